@@ -2,9 +2,14 @@
 //
 // This is the true 32-bit matrix product of the engine (no tensor-core mode of any
 // kind), and the fallback of the bfloat16 path for shapes the tensor-core kernel
-// refuses.  Any M, N, K >= 1.  Each output element is one accumulator that walks
-// k = 0..K-1 in ascending order, so the value at [m][n] does not depend on M or on
-// which other rows share the launch.
+// refuses.  Any M, N, K >= 1.  The order in which an output element's products are added depends
+// on the kernel alone, and which kernel runs on the types, K, ldx and the operands' alignment alone:
+// the value at [m][n] does not depend on M or on which other rows share the launch.
+//
+//   gemm_f32_kernel   fp32 throughout, rows that 16-byte copies can read (K, ldx multiples of 4):
+//                     eight partial sums an element (four quarters of every 64 k, even and odd k
+//                     apart), added in a fixed order.
+//   gemm_simt_kernel  everything else: one accumulator that walks k = 0..K-1.
 #include "common.cuh"
 
 using namespace fwb;
@@ -68,6 +73,148 @@ gemm_simt_kernel(const TX* __restrict__ X, const TW* __restrict__ W, TY* __restr
     }
 }
 
+// ---- fp32 operands in 16-byte pieces --------------------------------------------------------
+// Bound by the fp32 pipes from a few dozen rows on and by the weights' bytes below.  Both operands are
+// K-major, so they go to shared memory as they lie, by asynchronous 16-byte copies, three stages of
+// 64 k deep, and a thread reads four consecutive k of a row at once.  Rows are 68 floats apart, which
+// puts the eight rows that neighbouring lanes read on different banks.  Two k go through one packed
+// multiply-add (fma.rn.f32x2: two IEEE fp32 operations, half the issue slots), so an accumulator is a pair:
+// even k and odd k.  Four groups of 64 threads take 16 of the 64 k of every stage each: an output tile of
+// 64 x 32 keeps eight warps busy, and a 201 x 1024 product fills 128 SMs.
+// Measured on B200 (us; the kernel below this one, then this one): 201 x 9216 x 1024 289 -> 147,
+// 201 x 1024 x 4608 345 -> 147, 64 x 9216 x 1024 93 -> 38 (32 TFLOP/s), 8 x 1024 x 4608 314 -> 24,
+// 1 x 9216 x 1024 83 -> 23; relative error against 64 bits 5.7e-7 -> 2.1e-7 at K = 1024.
+constexpr int FK = 64, FSTRIDE = FK + 4, FSTAGES = 3;
+
+__device__ __forceinline__ void fma_pair(unsigned long long& acc, unsigned long long a, unsigned long long b) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ float pair_sum(unsigned long long v) {
+    return __uint_as_float((unsigned)v) + __uint_as_float((unsigned)(v >> 32));
+}
+
+template <int RM, int RN>
+constexpr int f32_smem_bytes() {
+    constexpr int ring = FSTAGES * 8 * (RM + RN) * FSTRIDE, partial = 3 * 64 * RM * RN;
+    return (ring > partial ? ring : partial) * 4;
+}
+
+// A tile of 8 RM rows x 8 RN columns; a thread of a group owns rows (lane & 7) + 8 i and columns (id / 8) + 8 j.
+template <int RM, int RN>
+__global__ void __launch_bounds__(256)
+gemm_f32_kernel(const float* __restrict__ X, const float* __restrict__ W, float* Y, const float* addend,
+                int M, int N, int K, int ldx, int ldy) {
+    constexpr int BM = 8 * RM, BN = 8 * RN, STAGE = (BM + BN) * FSTRIDE;
+    extern __shared__ __align__(16) float smem[];
+    fwb::pdl_entry();
+    const int tid = threadIdx.x, group = tid >> 6, id = tid & 63, tm = id & 7, tn = id >> 3;
+    const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
+    const int chunks = (K + FK - 1) / FK;
+
+    auto fetch = [&](int chunk) {
+        if (chunk < chunks) {
+            float* stage = smem + (chunk % FSTAGES) * STAGE;
+            const int k0 = chunk * FK;
+#pragma unroll
+            for (int i = 0; i < (BM + BN) * (FK / 4); i += 256) {
+                const int piece = i + tid, row = piece >> 4, k = k0 + (piece & 15) * 4;
+                const bool is_x = row < BM;
+                const int at = is_x ? m0 + row : n0 + row - BM;
+                const bool in = k < K && at < (is_x ? M : N);       // K is a multiple of 4: a piece is whole or absent
+                const float* src = is_x ? X + (in ? (size_t)at * ldx + k : 0) : W + (in ? (size_t)at * K + k : 0);
+                const uint32_t dst = (uint32_t)__cvta_generic_to_shared(stage + row * FSTRIDE + (piece & 15) * 4);
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(in ? 16 : 0)
+                             : "memory");
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    unsigned long long acc[RM][RN];
+#pragma unroll
+    for (int i = 0; i < RM; ++i)
+#pragma unroll
+        for (int j = 0; j < RN; ++j) acc[i][j] = 0ull;
+#pragma unroll
+    for (int s = 0; s < FSTAGES - 1; ++s) fetch(s);
+    for (int c = 0; c < chunks; ++c) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(FSTAGES - 2) : "memory");
+        __syncthreads();                       // chunk c has landed for everybody; chunk c - 1 is read by nobody
+        fetch(c + FSTAGES - 1);
+        const float* xs = smem + (c % FSTAGES) * STAGE + tm * FSTRIDE + group * 16;
+        const float* ws = smem + (c % FSTAGES) * STAGE + (BM + tn) * FSTRIDE + group * 16;
+#pragma unroll
+        for (int k = 0; k < 16; k += 4) {
+            ulonglong2 a[RM], b[RN];
+#pragma unroll
+            for (int i = 0; i < RM; ++i) a[i] = *reinterpret_cast<const ulonglong2*>(xs + i * 8 * FSTRIDE + k);
+#pragma unroll
+            for (int j = 0; j < RN; ++j) b[j] = *reinterpret_cast<const ulonglong2*>(ws + j * 8 * FSTRIDE + k);
+#pragma unroll
+            for (int i = 0; i < RM; ++i)
+#pragma unroll
+                for (int j = 0; j < RN; ++j) fma_pair(acc[i][j], a[i].x, b[j].x);
+#pragma unroll
+            for (int i = 0; i < RM; ++i)
+#pragma unroll
+                for (int j = 0; j < RN; ++j) fma_pair(acc[i][j], a[i].y, b[j].y);
+        }
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();                           // the ring is free: the groups' partial tiles go there
+    if (group > 0) {
+#pragma unroll
+        for (int i = 0; i < RM; ++i)
+#pragma unroll
+            for (int j = 0; j < RN; ++j) smem[(group - 1) * BM * BN + (tm + 8 * i) * BN + tn + 8 * j] = pair_sum(acc[i][j]);
+    }
+    __syncthreads();
+    if (group == 0) {
+#pragma unroll
+        for (int i = 0; i < RM; ++i)
+#pragma unroll
+            for (int j = 0; j < RN; ++j) {
+                const int at = (tm + 8 * i) * BN + tn + 8 * j;
+                smem[at] = ((pair_sum(acc[i][j]) + smem[at]) + smem[BM * BN + at]) + smem[2 * BM * BN + at];
+            }
+    }
+    __syncthreads();
+    for (int at = tid; at < BM * BN; at += 256) {
+        const int m = m0 + at / BN, n = n0 + at % BN;
+        if (m >= M || n >= N) continue;
+        float v = smem[at];
+        if (addend) v += addend[(size_t)m * ldy + n];
+        Y[(size_t)m * ldy + n] = v;
+    }
+}
+
+template <int RM, int RN>
+int launch_f32(const float* X, const float* W, float* Y, const float* addend, int M, int N, int K, int ldx, int ldy,
+               cudaStream_t stream) {
+    static bool configured = false;
+    if (!configured) {
+        cudaError_t e = cudaFuncSetAttribute(gemm_f32_kernel<RM, RN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             f32_smem_bytes<RM, RN>());
+        if (e != cudaSuccess) return (int)e;
+        configured = true;
+    }
+    const dim3 grid((M + 8 * RM - 1) / (8 * RM), (N + 8 * RN - 1) / (8 * RN));
+    if (grid.y > 65535) return FWB_TOO_LARGE;
+    fwb::pdl(gemm_f32_kernel<RM, RN>, grid, 256, f32_smem_bytes<RM, RN>(), stream)(X, W, Y, addend, M, N, K, ldx, ldy);
+    return fwb_launch_status();
+}
+
+// The tile: 16 or 32 rows for as few tokens; else the cheaper of 64 x 64 and 64 x 32 by rounds over the SMs
+// (a 64 x 32 tile takes about 0.6 of the other's time: fewer products an operand read).
+int dispatch_f32(const float* X, const float* W, float* Y, const float* addend, int M, int N, int K, int ldx, int ldy,
+                 cudaStream_t stream) {
+    if (M <= 16) return launch_f32<2, 2>(X, W, Y, addend, M, N, K, ldx, ldy, stream);
+    if (M <= 32) return launch_f32<4, 4>(X, W, Y, addend, M, N, K, ldx, ldy, stream);
+    const long rows = (M + 63) / 64;
+    const long square = (rows * ((N + 63) / 64) + 147) / 148, narrow = (rows * ((N + 31) / 32) + 147) / 148;
+    if (square * 10 <= narrow * 6) return launch_f32<8, 8>(X, W, Y, addend, M, N, K, ldx, ldy, stream);
+    return launch_f32<8, 4>(X, W, Y, addend, M, N, K, ldx, ldy, stream);
+}
+
 template <typename TX, typename TW, typename TY>
 int launch(const void* X, const void* W, void* Y, const float* addend, int M, int N, int K, int ldx,
            int ldy, cudaStream_t stream) {
@@ -91,7 +238,10 @@ FWB_API int fwb_gemm_simt(const void* X, int x_bf16, const void* W, int w_bf16, 
     using bf = __nv_bfloat16;
     const int key = (x_bf16 ? 4 : 0) | (w_bf16 ? 2 : 0) | (y_bf16 ? 1 : 0);
     switch (key) {
-        case 0: return launch<float, float, float>(X, W, Y, addend, M, N, K, ldx, ldy, stream);
+        case 0:
+            if (!(K & 3) && !(ldx & 3) && !((uintptr_t)X & 15) && !((uintptr_t)W & 15) && N <= 16 * 65535)
+                return dispatch_f32((const float*)X, (const float*)W, (float*)Y, addend, M, N, K, ldx, ldy, stream);
+            return launch<float, float, float>(X, W, Y, addend, M, N, K, ldx, ldy, stream);
         case 2: return launch<float, bf, float>(X, W, Y, addend, M, N, K, ldx, ldy, stream);
         case 4: return launch<bf, float, float>(X, W, Y, addend, M, N, K, ldx, ldy, stream);
         case 6: return launch<bf, bf, float>(X, W, Y, addend, M, N, K, ldx, ldy, stream);

@@ -109,6 +109,22 @@ def test_gemm_simt_fp32(M, N, K):
           x.double() @ w.double().T + add.double(), 1e-6, "gemm + addend")
 
 
+@pytest.mark.parametrize("M,N,K", [(1, 5, 4), (16, 17, 64), (17, 31, 68), (32, 33, 124), (33, 32, 128), (64, 64, 1028),
+                                   (65, 4800, 60), (201, 1024, 192), (130, 9473, 132)])
+def test_gemm_fp32_tiles(M, N, K):
+    """The 16-byte form: edges of its tiles and of its 64-wide steps; a row's value is the same in every tile.
+    The error of a sum of K products in eight parts is far below sqrt(K) roundings of their magnitude."""
+    from flyweight_b200.kernels import ops
+    g = torch.Generator().manual_seed(M * N + K)
+    x, w, add = torch.randn(M, K, generator=g), torch.randn(N, K, generator=g), torch.randn(M, N, generator=g)
+    exact = x.double() @ w.double().T
+    out = ops.gemm_simt(dev(x), dev(w), torch.float32)
+    assert ((out.cpu().double() - exact).abs() <= 2.0 ** -23 * (x.double().abs() @ w.double().abs().T)).all()
+    close(ops.gemm_simt(dev(x), dev(w), torch.float32, addend=dev(add)), exact + add.double(), 1e-6, "gemm + addend")
+    for rows in (1, min(M, 20), min(M, 40)):
+        assert torch.equal(ops.gemm_simt(dev(x[-rows:]), dev(w), torch.float32), out[-rows:])
+
+
 def test_gemm_row_does_not_depend_on_the_batch():
     from flyweight_b200.kernels import ops
     g = torch.Generator().manual_seed(5)
