@@ -263,6 +263,349 @@ delta_scan_kernel(const float* __restrict__ r, const float* __restrict__ p, floa
     }
 }
 
+// ---- runs of tokens: chunks of 32 ---------------------------------------------------------------------
+// The scan above walks a request token by token: 0.59 us a token whatever the heads, a chain of a copy, a barrier
+// and two reductions over lanes.  Over a chunk of C tokens behind the state S0 the same recurrence is
+//     u = T r,  r_i = beta_i (v_i - G_i S0^T k_i),  T = (I + A)^-1,  A_ij = beta_i D_ij k_i.k_j  (j < i)
+//     o_i = G_i S0^T q_i + sum_{j <= i} P_ij u_j,  P_ij = D_ij q_i.k_j
+//     S <- G_C S0 + sum_j D_Cj k_j u_j^T
+// with D_ij = g_{j+1} ... g_i and G_i = g_1 ... g_i, all products of decays (no logarithms: a difference of two
+// large sums would lose what a product of factors keeps).  T and P need no state: delta_chunk_kernel makes them for
+// every chunk and head at once; delta_runs_kernel then walks the chunks, one block per 16 columns of S and head, S
+// in shared memory, five small products a chunk in fp32 FMAs (packed in pairs, as in the fp32 matrix product).
+// T is a product of contractions (|k| = 1, beta < 1), so its entries stay below 1 and the sums lose nothing.
+constexpr int CHUNK = 32, CT = 36;                    // rows of T and P: 32 entries, then what a token has besides
+constexpr int CHUNK_FLOATS = 2 * CHUNK * CT;          // T | P of one chunk and head
+constexpr int AT_BETA = 32, AT_G = 32, AT_REST = 33;  // T[i][32] = beta_i; P[i][32] = G_i, P[i][33] = D_Ci
+
+__device__ __forceinline__ void fma_pair(unsigned long long& acc, unsigned long long a, unsigned long long b) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ float pair_sum(unsigned long long v) {
+    return __uint_as_float((unsigned)v) + __uint_as_float((unsigned)(v >> 32));
+}
+__device__ __forceinline__ unsigned long long pair_of(float v) {
+    const unsigned long long u = __float_as_uint(v);
+    return u | (u << 32);
+}
+
+// Chunk c of segment s and head h: scratch + (((seg_start[s] / 32 + s) + c) * H + h) * CHUNK_FLOATS: chunks of
+// different segments never meet, and T / 32 + S of them are enough.
+template <int D>
+__global__ void __launch_bounds__(256)
+delta_chunk_kernel(const float* __restrict__ r, const int* __restrict__ seg_start, float* __restrict__ scratch, DeltaShape sh) {
+    fwb::pdl_entry();
+    constexpr int STRIDE = D + 4;
+    __shared__ __align__(16) float kq[2 * CHUNK][STRIDE];             // k rows, then q rows
+    __shared__ float dots[2 * CHUNK][CHUNK + 1];                      // k_i.k_j, q_i.k_j
+    __shared__ __align__(16) float a_rows[CHUNK][CHUNK + 4];
+    __shared__ float beta[CHUNK], g[CHUNK];
+    const int seg = blockIdx.z, h = blockIdx.y;
+    const int begin = seg_start[seg], t0 = begin + blockIdx.x * CHUNK;
+    const int left = seg_start[seg + 1] - t0;
+    if (left <= 0) return;
+    const int n = left < CHUNK ? left : CHUNK, R = sh.r_width(), head = h / (sh.H / sh.G);
+    for (int i = threadIdx.x; i < 2 * CHUNK * (D / 4); i += blockDim.x) {
+        const int row = i / (D / 4), c = (i % (D / 4)) * 4, token = row % CHUNK;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (token < n)
+            v = *reinterpret_cast<const float4*>(r + (size_t)(t0 + token) * R + (row < CHUNK ? sh.cq() : 0) + head * D + c);
+        *reinterpret_cast<float4*>(&kq[row][c]) = v;
+    }
+    if (threadIdx.x < CHUNK) {
+        const bool in = (int)threadIdx.x < n;
+        const float* row = r + (size_t)(t0 + (in ? threadIdx.x : 0)) * R + sh.channels();
+        beta[threadIdx.x] = in ? row[h] : 0.0f;
+        g[threadIdx.x] = in ? row[sh.H + h] : 1.0f;
+    }
+    __syncthreads();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    {
+        const int row = warp * 8 + (lane & 7), col = lane >> 3;       // this thread's row, columns col + 4 j
+        unsigned long long acc[8], acc2[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[j] = acc2[j] = 0ull;
+#pragma unroll 4
+        for (int k = 0; k < D; k += 4) {
+            const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(&kq[row][k]);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(&kq[col + 4 * j][k]);
+                fma_pair(acc[j], a.x, b.x);
+                fma_pair(acc2[j], a.y, b.y);
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) dots[row][col + 4 * j] = pair_sum(acc[j]) + pair_sum(acc2[j]);
+    }
+    __syncthreads();
+    float* out = scratch + ((size_t)(begin / CHUNK + seg + blockIdx.x) * sh.H + h) * CHUNK_FLOATS;
+    float* p_out = out + CHUNK * CT;
+    // (the products of decays in 64 bits: a chunk's worth of roundings in one factor would go into whole rows)
+    if (warp == 0) {                                                  // A: lane j walks its column down
+        double d = 1.0;
+#pragma unroll 4
+        for (int i = 0; i < CHUNK; ++i) {
+            d = i > lane ? d * (double)g[i] : 1.0;
+            a_rows[i][lane] = i > lane ? beta[i] * ((float)d * dots[i][lane]) : 0.0f;
+        }
+        out[lane * CT + AT_BETA] = beta[lane];
+    } else if (warp == 1) {                                           // P
+        double d = 1.0;
+#pragma unroll 4
+        for (int i = 0; i < CHUNK; ++i) {
+            d = i > lane ? d * (double)g[i] : 1.0;
+            p_out[i * CT + lane] = i >= lane ? (float)d * dots[CHUNK + i][lane] : 0.0f;
+        }
+        p_out[lane * CT + AT_REST] = (float)d;                        // D_Cj: the last row's factor
+    } else if (warp == 2) {                                           // G_i
+        double d = 1.0;
+        for (int i = 0; i <= lane; ++i) d *= (double)g[i];
+        p_out[lane * CT + AT_G] = (float)d;
+    }
+    __syncwarp();
+    if (warp == 0) {                                                  // column `lane` of (I + A)^-1, forwards
+        float t[CHUNK];
+#pragma unroll
+        for (int i = 0; i < CHUNK; ++i) {
+            float s0 = 0.0f, s1 = 0.0f;
+#pragma unroll
+            for (int m = 0; m + 1 < i; m += 2) {
+                s0 = fmaf(a_rows[i][m], t[m], s0);
+                s1 = fmaf(a_rows[i][m + 1], t[m + 1], s1);
+            }
+            if (i & 1) s0 = fmaf(a_rows[i][i - 1], t[i - 1], s0);
+            t[i] = i == lane ? 1.0f : (i > lane ? -(s0 + s1) : 0.0f);
+            out[i * CT + lane] = t[i];
+        }
+    }
+}
+
+constexpr int RUN_COLS = 16;
+template <int D>
+struct RunLayout {                                     // floats
+    static constexpr int ROW = D + 4;
+    static constexpr int Q = CHUNK * ROW, V = 2 * CHUNK * ROW, TP = V + CHUNK * RUN_COLS, STAGE = TP + CHUNK_FLOATS;
+    static constexpr int S = 2 * STAGE, RED = S + RUN_COLS * ROW;     // S column by column
+    static constexpr int RED_FLOATS = 4 * 2 * CHUNK * 20;             // >= (256 / D - 1) * 16 * D, the state's partial sums
+    static constexpr int UT = RED + RED_FLOATS, UN = UT + 2 * RUN_COLS * CT, FLOATS = UN + CHUNK * RUN_COLS;
+};
+
+template <int D>
+__global__ void __launch_bounds__(256)
+delta_runs_kernel(const float* __restrict__ r, const float* __restrict__ p, const float* __restrict__ scratch,
+                  float* __restrict__ state, long long slot_stride, const int* __restrict__ seg_start,
+                  const int* __restrict__ seg_slot, float* __restrict__ o, DeltaShape sh) {
+    using Y = RunLayout<D>;
+    extern __shared__ __align__(16) float sm[];
+    fwb::pdl_wait();
+    const int seg = blockIdx.z, h = blockIdx.y, col0 = blockIdx.x * RUN_COLS;
+    const int t0 = seg_start[seg], t1 = seg_start[seg + 1];
+    if (t1 <= t0) return;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, e = sh.e, R = sh.r_width();
+    const int head = h / (sh.H / sh.G), chunks = (t1 - t0 + CHUNK - 1) / CHUNK;
+    float* slot = state + (size_t)seg_slot[seg] * slot_stride;
+    if (blockIdx.x == 0 && h == 0 && sh.L > 1) delta_conv_advance(p, slot, t0, t1 - t0, sh);
+    float* S = sm + Y::S;
+    float* red = sm + Y::RED;
+    float* rt = sm + Y::UT;                            // r, column by column [16][36]
+    float* ut = rt + RUN_COLS * CT;                    // u, column by column
+    float* un = sm + Y::UN;                            // D_Cj u_j, token by token [32][16]
+    for (int i = tid; i < RUN_COLS * (D / 4); i += 256) {
+        const int c = i / (D / 4), k = (i % (D / 4)) * 4;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (col0 + c < e) v = *reinterpret_cast<const float4*>(slot + ((size_t)h * e + col0 + c) * D + k);
+        *reinterpret_cast<float4*>(S + c * Y::ROW + k) = v;
+    }
+    const float* tp0 = scratch + ((size_t)(t0 / CHUNK + seg) * sh.H + h) * CHUNK_FLOATS;
+    auto copy = [&](float* dst, const float* src, bool in) {          // 16 bytes, or as many zeros
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
+                     "l"(src), "r"(in ? 16 : 0) : "memory");
+    };
+    auto fetch = [&](int c) {
+        if (c < chunks) {
+            float* stage = sm + (c & 1) * Y::STAGE;
+            const int first = t0 + c * CHUNK, n = t1 - first;
+            for (int i = tid; i < 2 * CHUNK * (D / 4); i += 256) {
+                const int row = i / (D / 4), k = (i % (D / 4)) * 4, token = row % CHUNK;
+                const bool in = token < n;
+                copy(stage + row * Y::ROW + k,
+                     r + (size_t)(in ? first + token : t0) * R + (row < CHUNK ? sh.cq() : 0) + head * D + k, in);
+            }
+            if (tid < CHUNK * RUN_COLS / 4) {
+                const int token = tid / 4, k = (tid % 4) * 4;
+                const bool in = token < n && col0 + k < e;
+                copy(stage + Y::V + token * RUN_COLS + k,
+                     r + (in ? (size_t)(first + token) * R + 2 * sh.cq() + h * e + col0 + k : (size_t)t0 * R), in);
+            }
+            const float* tp = tp0 + (size_t)c * sh.H * CHUNK_FLOATS;
+            for (int i = tid * 4; i < CHUNK_FLOATS; i += 1024) copy(stage + Y::TP + i, tp + i, true);
+        }
+        copy_async_commit();
+    };
+    fetch(0);
+    for (int c = 0; c < chunks; ++c) {
+        fetch(c + 1);                                  // (the stage was last read before the barrier that ends a chunk)
+        copy_async_wait<1>();
+        __syncthreads();
+        const float* stage = sm + (c & 1) * Y::STAGE;
+        const float* T = stage + Y::TP;
+        const float* P = T + CHUNK * CT;
+        const int n = t1 - t0 - c * CHUNK < CHUNK ? t1 - t0 - c * CHUNK : CHUNK;
+        {   // S0^T k and S0^T q: warps 0-3 the k rows, 4-7 the q rows, a quarter of the channels each
+            const int quarter = warp & 3, tm = lane & 7, tn = lane >> 3;
+            const float* rows = stage + (warp >> 2) * Y::Q + tm * Y::ROW + quarter * (D / 4);
+            const float* cols = S + tn * Y::ROW + quarter * (D / 4);
+            unsigned long long acc[4][4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) acc[i][j] = 0ull;
+#pragma unroll
+            for (int k = 0; k < D / 4; k += 4) {
+                ulonglong2 a[4], b[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) a[i] = *reinterpret_cast<const ulonglong2*>(rows + 8 * i * Y::ROW + k);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) b[j] = *reinterpret_cast<const ulonglong2*>(cols + 4 * j * Y::ROW + k);
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        fma_pair(acc[i][j], a[i].x, b[j].x);
+                        fma_pair(acc[i][j], a[i].y, b[j].y);
+                    }
+            }
+            float* to = red + quarter * (2 * CHUNK * 20) + ((warp >> 2) * CHUNK + tm) * 20 + tn;
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) to[i * 160 + 4 * j] = pair_sum(acc[i][j]);
+        }
+        __syncthreads();
+        const int row = tid >> 3, cc = tid & 7;        // token and columns cc, cc + 8 of the middle products
+        float from_state[2];
+        {
+            const float beta = T[row * CT + AT_BETA], G = P[row * CT + AT_G];
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                const float* at = red + row * 20 + cc + 8 * j;
+                const float ks = (at[0] + at[2 * CHUNK * 20]) + (at[4 * CHUNK * 20] + at[6 * CHUNK * 20]);
+                at += CHUNK * 20;
+                const float qs = (at[0] + at[2 * CHUNK * 20]) + (at[4 * CHUNK * 20] + at[6 * CHUNK * 20]);
+                rt[(cc + 8 * j) * CT + row] = beta * (stage[Y::V + row * RUN_COLS + cc + 8 * j] - G * ks);
+                from_state[j] = G * qs;
+            }
+        }
+        __syncthreads();
+        auto row_times = [&](const float* m_row, const float* columns, float (&v)[2]) {
+            unsigned long long s[2][2] = {{0ull, 0ull}, {0ull, 0ull}};
+#pragma unroll 4
+            for (int k = 0; k <= warp * 4; k += 4) {   // the warp's rows end there
+                const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(m_row + k);
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(columns + (cc + 8 * j) * CT + k);
+                    fma_pair(s[j][0], a.x, b.x);
+                    fma_pair(s[j][1], a.y, b.y);
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < 2; ++j) v[j] = pair_sum(s[j][0]) + pair_sum(s[j][1]);
+        };
+        {
+            float u[2];
+            row_times(T + row * CT, rt, u);
+            const float rest = P[row * CT + AT_REST];
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                ut[(cc + 8 * j) * CT + row] = u[j];
+                un[row * RUN_COLS + cc + 8 * j] = rest * u[j];
+            }
+        }
+        __syncthreads();
+        {
+            float v[2];
+            row_times(P + row * CT, ut, v);
+            if (row < n) {
+                float* at = o + ((size_t)(t0 + c * CHUNK + row) * sh.H + h) * e + col0;
+#pragma unroll
+                for (int j = 0; j < 2; ++j)
+                    if (col0 + cc + 8 * j < e) at[cc + 8 * j] = from_state[j] + v[j];
+            }
+        }
+        {   // S <- G_C S0 + sum_j k_j (D_Cj u_j): four channels x four columns a thread, the tokens in 256 / D parts
+            constexpr int QUADS = D / 4, PARTS = 256 / (4 * QUADS), TOKENS = CHUNK / PARTS;
+            const int quad = tid % QUADS, cg = (tid / QUADS) & 3, part = tid / (4 * QUADS);
+            unsigned long long acc[4][2];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) acc[j][0] = acc[j][1] = 0ull;
+#pragma unroll 4
+            for (int i = 0; i < TOKENS; ++i) {
+                const int token = part * TOKENS + i;
+                const ulonglong2 k = *reinterpret_cast<const ulonglong2*>(stage + token * Y::ROW + quad * 4);
+                const float4 u = *reinterpret_cast<const float4*>(un + token * RUN_COLS + cg * 4);
+                const unsigned long long uu[4] = {pair_of(u.x), pair_of(u.y), pair_of(u.z), pair_of(u.w)};
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    fma_pair(acc[j][0], k.x, uu[j]);
+                    fma_pair(acc[j][1], k.y, uu[j]);
+                }
+            }
+            ulonglong2* others = reinterpret_cast<ulonglong2*>(red);
+            if (part > 0)
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    others[((part - 1) * 4 + j) * (4 * QUADS) + cg * QUADS + quad] = make_ulonglong2(acc[j][0], acc[j][1]);
+            __syncthreads();
+            if (part == 0) {
+                const float last = P[(CHUNK - 1) * CT + AT_G];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    float4* at = reinterpret_cast<float4*>(S + (cg * 4 + j) * Y::ROW + quad * 4);
+                    float4 v = *at;
+                    float add[4] = {__uint_as_float((unsigned)acc[j][0]), __uint_as_float((unsigned)(acc[j][0] >> 32)),
+                                    __uint_as_float((unsigned)acc[j][1]), __uint_as_float((unsigned)(acc[j][1] >> 32))};
+#pragma unroll
+                    for (int other = 1; other < PARTS; ++other) {
+                        const float4 w = *reinterpret_cast<const float4*>(
+                            &others[((other - 1) * 4 + j) * (4 * QUADS) + cg * QUADS + quad]);
+                        add[0] += w.x, add[1] += w.y, add[2] += w.z, add[3] += w.w;
+                    }
+                    v.x = fmaf(last, v.x, add[0]), v.y = fmaf(last, v.y, add[1]);
+                    v.z = fmaf(last, v.z, add[2]), v.w = fmaf(last, v.w, add[3]);
+                    *at = v;
+                }
+            }
+        }
+        __syncthreads();
+    }
+    copy_async_wait<0>();
+    fwb::pdl_launch_dependents();
+    for (int i = tid; i < RUN_COLS * (D / 4); i += 256) {
+        const int c = i / (D / 4), k = (i % (D / 4)) * 4;
+        if (col0 + c < e)
+            *reinterpret_cast<float4*>(slot + ((size_t)h * e + col0 + c) * D + k) = *reinterpret_cast<float4*>(S + c * Y::ROW + k);
+    }
+}
+
+template <int D>
+int launch_runs(const float* r, const float* p, float* scratch, float* state, long long slot_stride, const int* seg_start,
+                const int* seg_slot, float* o, int longest, int n_segments, const DeltaShape& sh, cudaStream_t stream) {
+    constexpr int SMEM = RunLayout<D>::FLOATS * 4;
+    static bool configured = false;
+    if (!configured) {
+        cudaError_t err = cudaFuncSetAttribute(delta_runs_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+        if (err != cudaSuccess) return (int)err;
+        configured = true;
+    }
+    const dim3 chunks((longest + CHUNK - 1) / CHUNK, sh.H, n_segments);
+    fwb::pdl(delta_chunk_kernel<D>, chunks, 256, 0, stream)(r, seg_start, scratch, sh);
+    const dim3 grid((sh.e + RUN_COLS - 1) / RUN_COLS, sh.H, n_segments);
+    fwb::pdl(delta_runs_kernel<D>, grid, 256, SMEM, stream)(r, p, scratch, state, slot_stride, seg_start, seg_slot, o, sh);
+    return fwb_launch_status();
+}
+
 template <typename TO>
 __global__ void __launch_bounds__(128)
 gated_head_norm_kernel(const float* __restrict__ o, const float* __restrict__ gate, long long gate_stride,
@@ -287,10 +630,12 @@ gated_head_norm_kernel(const float* __restrict__ o, const float* __restrict__ ga
 // p: [T][2Gd + 2He + 2H] fp32 (q | k | v | gate | b | a).  taps: [2Gd + He][L] fp32.  a_log, dt_bias: [H].
 // state: [slots][slot_stride] fp32 with S at 0 and the convolution's inputs behind it.
 // r: [T][2Gd + He + 2H + G rounded up to a multiple of 4] fp32 scratch.  o: [T][H][e] fp32.
+// scratch: null (every token through the scan), or [T / 32 + n_segments][H][2][32][36] fp32 on a 16-byte border for
+// the chunked form, with `longest` the longest segment's tokens; sizes it does not take go through the scan.
 FWB_API int fwb_delta_rule(const float* p, const float* taps, const float* a_log, const float* dt_bias,
                            float* state, long long slot_stride, const int* seg_start, const int* seg_slot,
-                           const int* tok_seg, float* r, float* o, int T, int n_segments, int H, int G, int d,
-                           int e, int L, cudaStream_t stream) {
+                           const int* tok_seg, float* r, float* o, float* scratch, int longest, int T, int n_segments,
+                           int H, int G, int d, int e, int L, cudaStream_t stream) {
     if (T <= 0 || n_segments <= 0) return FWB_OK;
     if (!p || !taps || !a_log || !dt_bias || !state || !seg_start || !seg_slot || !tok_seg || !r || !o)
         return FWB_BAD_ARGUMENT;
@@ -307,6 +652,11 @@ FWB_API int fwb_delta_rule(const float* p, const float* taps, const float* a_log
                                                                      seg_start, seg_slot, tok_seg, r, sh);
     const bool vec = d % 4 == 0 && e % 4 == 0 && slot_stride % 4 == 0 && ((uintptr_t)state & 15) == 0 &&
                      ((uintptr_t)r & 15) == 0;
+    if (scratch && vec && (d == 64 || d == 128) && ((uintptr_t)scratch & 15) == 0) {
+        if (d == 64)
+            return launch_runs<64>(r, p, scratch, state, slot_stride, seg_start, seg_slot, o, longest, n_segments, sh, stream);
+        return launch_runs<128>(r, p, scratch, state, slot_stride, seg_start, seg_slot, o, longest, n_segments, sh, stream);
+    }
 #define FWB_SCAN(DPL, LPC)                                                                                 \
     do {                                                                                                   \
         const dim3 grid((e + 128 / LPC - 1) / (128 / LPC), H, n_segments);                                 \

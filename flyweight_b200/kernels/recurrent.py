@@ -16,6 +16,12 @@ def delta_state_size(heads: int, kv_heads: int, dim: int, vdim: int, taps: int) 
     return -(-size // 4) * 4            # slots start on 16-byte borders
 
 
+# From this many tokens of a step's longest segment on the recurrence runs in chunks of 32 tokens (head sizes 64 and
+# 128); shorter segments, decode steps above all, walk token by token.
+CHUNKS_FROM = 16
+_CHUNK_TOKENS, _CHUNK_FLOATS = 32, 2 * 32 * 36
+
+
 def delta_rule(p: torch.Tensor, taps: torch.Tensor, a_log: torch.Tensor, dt_bias: torch.Tensor,
                state: torch.Tensor, batch, heads: int, kv_heads: int, dim: int, vdim: int) -> torch.Tensor:
     """The gated delta rule over the step's tokens.  ``p``: fp32 [T][q | k | v | gate | b | a], the fused
@@ -44,9 +50,12 @@ def delta_rule(p: torch.Tensor, taps: torch.Tensor, a_log: torch.Tensor, dt_bias
     _i32("tok_seg", batch.tok_seg, T)
     r = torch.empty((T, -(-(channels + 2 * heads + kv_heads) // 4) * 4), dtype=torch.float32, device=p.device)
     o = torch.empty((T, heads, vdim), dtype=torch.float32, device=p.device)
+    chunked = batch.max_segment >= CHUNKS_FROM and dim in (64, 128) and vdim % 4 == 0 and stride % 4 == 0
+    scratch = torch.empty((T // _CHUNK_TOKENS + S) * heads * _CHUNK_FLOATS, dtype=torch.float32,
+                          device=p.device) if chunked else None
     lib.call("fwb_delta_rule", ptr(p), ptr(taps), ptr(a_log), ptr(dt_bias), ptr(state), c_longlong(stride),
-             ptr(batch.seg_start), ptr(batch.seg_slot), ptr(batch.tok_seg), ptr(r), ptr(o), T, S, heads, kv_heads,
-             dim, vdim, L, stream(), launches=2)
+             ptr(batch.seg_start), ptr(batch.seg_slot), ptr(batch.tok_seg), ptr(r), ptr(o), ptr(scratch),
+             batch.max_segment if chunked else 0, T, S, heads, kv_heads, dim, vdim, L, stream(), launches=3 if chunked else 2)
     return o
 
 

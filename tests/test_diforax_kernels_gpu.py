@@ -402,6 +402,60 @@ def test_delta_rule_whole_cut_and_one_by_one(shape, dtype):
         assert torch.isnan(cache.state[0]).all() and float(cache.state[3].abs().max()) == 0.0
 
 
+@pytest.mark.parametrize("H,G,d,e", [(2, 1, 128, 40), (3, 3, 64, 16), (2, 2, 128, 4), (4, 2, 64, 36)])
+@pytest.mark.parametrize("strong", [False, True])
+def test_delta_chunks_against_the_scan_and_64_bits(H, G, d, e, strong):
+    """The chunked form at the edges of its chunks of 32 and of its 16 columns, on a state that is not zero, with
+    keys that repeat and with decays down to e^-60 a token: as close to 64 bits as the token-by-token scan, up to
+    the handful of roundings more that a sum over a chunk has (both stay within 64 roundings of the largest value)."""
+    from flyweight_b200.kernels import recurrent
+    g = torch.Generator().manual_seed(H * d + e)
+    lengths, L, C = [31, 1, 32, 33, 97, 64], 1, 2 * G * d + H * e
+    T = sum(lengths)
+    p = torch.randn(T, C + H * e + 2 * H, generator=g, dtype=F64).float()
+    p[::3, G * d:2 * G * d] = p[0, G * d:2 * G * d]                   # the same key again and again
+    if strong:
+        p[:, C + H * e + H:] = 60.0 * torch.rand(T, H, generator=g).float()
+    taps, zeros = torch.ones(C, 1), torch.zeros(H)
+    start = torch.randn(7, recurrent.delta_state_size(H, G, d, e, L), generator=g, dtype=F64).float()
+    x = p.double()
+    act = x[:, :C] * torch.sigmoid(x[:, :C])
+    q, k = act[:, :G * d].view(T, G, d), act[:, G * d:2 * G * d].view(T, G, d)
+    q, k = (t * torch.rsqrt((t * t).sum(-1, keepdim=True) + 1e-6) for t in (q, k))
+    q, k = ((t * s).repeat_interleave(H // G, dim=1) for t, s in ((q, d ** -0.5), (k, 1.0)))
+    v, beta = act[:, 2 * G * d:].view(T, H, e), torch.sigmoid(x[:, C + H * e:C + H * e + H])
+    decay = torch.exp(-torch.nn.functional.softplus(x[:, C + H * e + H:]))
+    want, after, at = torch.empty(T, H, e, dtype=F64), start.double().clone(), 0
+    for s, n in enumerate(lengths):
+        S = after[s + 1, :H * d * e].view(H, e, d)
+        for t in range(at, at + n):
+            S *= decay[t][:, None, None]
+            u = beta[t][:, None] * (v[t] - torch.einsum("hed,hd->he", S, k[t]))
+            S += u[:, :, None] * k[t][:, None, :]
+            want[t] = torch.einsum("hed,hd->he", S, q[t])
+        at += n
+    starts = [sum(lengths[:i]) for i in range(len(lengths) + 1)]
+    batch = type("Batch", (), {})()
+    batch.n_segments, batch.max_segment = len(lengths), max(lengths)
+    i32 = lambda values: torch.tensor(values, dtype=torch.int32, device=DEV)
+    batch.seg_start, batch.seg_slot = i32(starts), i32(list(range(1, len(lengths) + 1)))
+    batch.tok_seg = i32([s for s, n in enumerate(lengths) for _ in range(n)])
+    errors = []
+    for chunked in (True, False):
+        recurrent.CHUNKS_FROM, before = (16 if chunked else 10 ** 9), recurrent.CHUNKS_FROM
+        try:
+            state = dev(start, torch.float32)
+            o = recurrent.delta_rule(dev(p, torch.float32), dev(taps), dev(zeros), dev(zeros), state, batch, H, G, d, e)
+        finally:
+            recurrent.CHUNKS_FROM = before
+        errors.append((float((o.cpu().double() - want).norm() / want.norm()),
+                       float((state.cpu().double() - after).norm() / after.norm())))
+        close(o.cpu().view(T, H, e), want, 64 * 2.0 ** -24, f"chunked {chunked}: read out")
+        close(state.cpu(), after, 64 * 2.0 ** -24, f"chunked {chunked}: state")
+    assert errors[0][0] <= 2 * errors[1][0] + 2.0 ** -24 and errors[0][1] <= 2 * errors[1][1] + 2.0 ** -24, errors
+    print("errors", errors)
+
+
 def test_the_delta_state_remembers_a_write_from_hundreds_of_tokens_ago():
     """One early token writes a value under a key that no later token touches (later keys are orthogonal
     to it and decay is switched off): a query for that key, 400 tokens and several steps later, reads the
