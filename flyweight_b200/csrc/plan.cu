@@ -34,6 +34,9 @@ int fwb_gemm_tcgen05(const void*, const void*, void*, const float*, int, int, in
                      int, int, int, float, cudaStream_t);
 int fwb_gemm_tcgen05_normed(const float*, const float*, const int*, float, const void*, void*, int, int, int,
                             int, int, int, int, int, int, int, float, cudaStream_t);
+int fwb_linear_rows(const void*, const void*, void*, const float*, int, int, int, int, int, int, int, float, cudaStream_t);
+int fwb_linear_rows_normed(const float*, const float*, const int*, float, const void*, void*, int, int, int, int, int,
+                           int, int, float, cudaStream_t);
 int fwb_gemm_tcgen05_pair(const void*, const void*, void*, int, int, int, int, int, int, int, int,
                           cudaStream_t);
 int fwb_shortconv(const void*, int, const float*, const float*, float*, const int*, const int*, const int*,
@@ -96,9 +99,10 @@ enum Option {
     OPT_ATTENTION_TCGEN05 = 9, // prompt portions through the tcgen05 attention kernel
     OPT_MIXED_SPLIT = 10,      // decoding requests at the head of a mixed step through the decode kernel
     OPT_LATENT_TENSORCORE = 11, // latent attention and its per-head products on tensor cores
-    OPT_COUNT = 12,
+    OPT_ROWS = 12,             // products of a few tokens on the weight reader
+    OPT_COUNT = 13,
 };
-int g_option[OPT_COUNT] = {1, 0, 1, 1, 1, 1, 0, 1, 0, 1, 1, 1};
+int g_option[OPT_COUNT] = {1, 0, 1, 1, 1, 1, 0, 1, 0, 1, 1, 1, 1};
 constexpr int FUSE_FROM_TOKENS = 16;
 constexpr int CLUSTER_MERGE_CTAS = 1024;
 
@@ -202,16 +206,27 @@ bool tc_accepts(const void* x, const void* w, int M, int K) {
     return g_option[OPT_TENSORCORE] && K % 8 == 0 && K >= 8 && aligned16(x) && aligned16(w) && M <= 65535 * 16;
 }
 
+// a few tokens: the weight reader (kernels/tensorcore.py: _rows_takes, _rows_takes_normed); N: rows of the matrix
+bool rows_takes(int M, int N, int K) {
+    if (!g_option[OPT_TENSORCORE] || !g_option[OPT_ROWS] || g_option[OPT_FORCED_SPLITS] > 0) return false;
+    static const long long limits[3][3] = {{8, 1 << 20, 1 << 26}, {16, 2048, 1 << 26}, {32, 1024, 1 << 24}};
+    for (const auto& limit : limits)
+        if (M <= limit[0] && K <= limit[1] && (long long)N * K <= limit[2]) return true;
+    return false;
+}
+bool rows_takes_normed(int M, int N, int K) { return M <= 8 && K <= 1024 && rows_takes(M, N, K); }
+
 bool normed_accepts(int M, int K, const void* w, int accumulators, int N) {
     if (!(g_option[OPT_TENSORCORE] && g_option[OPT_FUSE_NORM]) || M > 64 || K % 8 || !aligned16(w)) return false;
+    if (rows_takes(M, accumulators * N, K)) return rows_takes_normed(M, accumulators * N, K);
     if (M < FUSE_FROM_TOKENS && !g_option[OPT_FUSE_ALWAYS]) return false;
     const int splits = g_option[OPT_FORCED_SPLITS] > 0 ? g_option[OPT_FORCED_SPLITS]
                                                         : splits_for(M, N, K, accumulators);
     return ceil_div(K, 64) <= 8 * splits;
 }
 
-bool adds_in_place(const void* x, const void* w, int M, int K) {
-    return g_option[OPT_ADD_IN_PLACE] && (M >= FUSE_FROM_TOKENS || g_option[OPT_FUSE_ALWAYS]) &&
+bool adds_in_place(const void* x, const void* w, int M, int N, int K) {
+    return g_option[OPT_ADD_IN_PLACE] && (M >= FUSE_FROM_TOKENS || g_option[OPT_FUSE_ALWAYS] || rows_takes(M, N, K)) &&
            tc_accepts(x, w, M, K) && M <= 128;
 }
 
@@ -234,6 +249,10 @@ void tc_gemm(Launches& L, const void* x, const void* w, void* out, int out_bf16,
              int N, int K, cudaStream_t stream) {
     const bool in_place = addend && (const void*)addend == out;
     const int epilogue = addend ? EPI_ADD_F32 : (out_bf16 ? EPI_BF16 : EPI_F32);
+    if (rows_takes(M, N, K)) {
+        L.add(fwb_linear_rows(x, w, out, addend, M, N, K, N, N, epilogue, 0, 0.0f, stream));
+        return;
+    }
     const bool pair_ok = g_option[OPT_PAIRS] && M > 128 && !addend && !in_place && N >= 256;
     int splits = 0, stages = 0, tile_tokens = 0;
     bool pair = false, wide = false;
@@ -267,6 +286,10 @@ void tc_gemm(Launches& L, const void* x, const void* w, void* out, int out_bf16,
 // silu(x @ gate^T) * (x @ up^T) for w = [gate rows | up rows] ([2F][K]) -> out [M][F] bf16.
 void tc_swiglu(Launches& L, const void* x, const void* w, void* out, int M, int F, int K, cudaStream_t stream) {
     int splits = 1, stages = 0, tile_tokens = 0;
+    if (rows_takes(M, 2 * F, K)) {
+        L.add(fwb_linear_rows(x, w, out, nullptr, M, F, K, 2 * F, F, EPI_SWIGLU_BF16, F, 0.0f, stream));
+        return;
+    }
     if (M <= 64) {
         splits = g_option[OPT_FORCED_SPLITS] > 0 ? g_option[OPT_FORCED_SPLITS] : splits_for(M, F, K, 2);
         stages = ring_depth(M, F, splits, 2);
@@ -423,6 +446,11 @@ void run_norm_linear(Launches& L, const Op& op, const FwbStep& step, bool& pendi
     const int accumulators = swiglu ? 2 : 1;
     if (!pending && op.w_bf16 && act_bf16 && normed_accepts(M, op.K, op.w, accumulators, op.N)) {
         // the norm, the product (both products and silu(g)*u) in one kernel
+        if (rows_takes_normed(M, accumulators * op.N, op.K)) {
+            L.add(fwb_linear_rows_normed(op.x, op.v0, rows, op.eps, op.w, out, M, op.N, op.K, swiglu ? 2 * op.N : op.N,
+                                         op.N, op.epilogue, swiglu ? op.N : 0, 0.0f, stream));
+            return;
+        }
         int splits, stages, tile_tokens;
         if (swiglu) {
             splits = g_option[OPT_FORCED_SPLITS] > 0 ? g_option[OPT_FORCED_SPLITS] : splits_for(M, op.N, op.K, 2);
@@ -455,7 +483,7 @@ void run_norm_linear(Launches& L, const Op& op, const FwbStep& step, bool& pendi
 void run_linear_residual(Launches& L, const Op& op, const FwbStep& step, bool& pending, int act_bf16,
                          cudaStream_t stream) {
     const int M = step.T;
-    if (op.w_bf16 && act_bf16 && adds_in_place(op.in, op.w, M, op.K)) {
+    if (op.w_bf16 && act_bf16 && adds_in_place(op.in, op.w, M, op.N, op.K)) {
         tc_gemm(L, op.in, op.w, op.x, 0, op.x, M, op.N, op.K, stream);      // x += in @ w^T in the epilogue
         pending = false;
         return;

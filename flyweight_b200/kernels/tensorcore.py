@@ -64,6 +64,36 @@ def set_pairs_enabled(flag: bool) -> None:
     _use_pairs = bool(flag)
     lib.set_option("pairs", _use_pairs)
 
+# ---- decode steps of a few requests: csrc/linear_rows.cu -----------------------------------
+# A few tokens' products run on a kernel that streams weights straight to mma.sync instead of through tiles of tensor
+# memory: a decode step is a chain of small launches, and what counts is the time from the activations to the result.
+# (tokens, longest K, most weights): behind these lines the activations that every CTA reads cost more than that saves
+# (csrc/linear_rows.cu has the figures).
+ROWS_LIMITS = ((8, 1 << 20, 1 << 26), (16, 2048, 1 << 26), (32, 1024, 1 << 24))
+# The norm in front is folded in where K is one step of the kernel's walk: 1024 x 1024 at 8 tokens 3.3 us against 3.5 for
+# the norm's kernel and the product, 9216 x 1024 5.2 against 6.2; with K = 2048 it loses (6144 x 2048: 7.6 against 6.9).
+ROWS_NORMED_TO, ROWS_NORMED_K = 8, 1024
+_use_rows = True
+
+
+def set_rows_enabled(flag: bool) -> None:
+    """Products of a few tokens on the weight reader (on by default); off: the tcgen05 kernel."""
+    global _use_rows
+    _use_rows = bool(flag)
+    lib.set_option("rows", _use_rows)
+
+
+def _rows_takes(M: int, N: int, K: int) -> bool:
+    """``N``: rows of the matrix (gate and up together)."""
+    if not (_enabled and _use_rows) or _forced_splits is not None:
+        return False
+    return any(M <= tokens and K <= longest and N * K <= most for tokens, longest, most in ROWS_LIMITS)
+
+
+def _rows_takes_normed(M: int, N: int, K: int) -> bool:
+    return M <= ROWS_NORMED_TO and K <= ROWS_NORMED_K and _rows_takes(M, N, K)
+
+
 # Per-shape overrides found by measurement: (features, K, accumulators) -> (splits, stages);
 # 0 keeps the rule's choice.  Only decode-sized token counts (<= 64) consult it.
 TUNED = {}
@@ -191,7 +221,7 @@ def adds_in_place(x, w, residual) -> bool:
     """Whether ``gemm(x, w, fp32, addend=residual, out=residual)`` is available: the single-CTA
     kernel has the epilogue (every element is read and written by the same thread), the
     CTA-pair kernel of prompt-sized steps has not."""
-    return (_add_in_place and (x.shape[0] >= FUSE_FROM_TOKENS or _fuse_always)
+    return (_add_in_place and (x.shape[0] >= FUSE_FROM_TOKENS or _fuse_always or _rows_takes(x.shape[0], *w.shape))
             and accepts(x, w, torch.float32, residual) and x.shape[0] <= 128
             and residual.dtype == torch.float32 and residual.is_contiguous()
             and tuple(residual.shape) == (x.shape[0], w.shape[0]))
@@ -230,6 +260,10 @@ def gemm(x, w, out_dtype, addend=None, splits=None, stages=0, tile_tokens=0, wid
         epilogue = EPI_ADD_F32
     else:
         epilogue = EPI_F32 if out_dtype == torch.float32 else _output_epilogue(activation)
+    if free_choice and _rows_takes(M, N, K):
+        lib.call("fwb_linear_rows", ptr(x), ptr(w), ptr(out), ptr(addend), M, N, K, N, N, epilogue, 0,
+                 lib.c_float(0.0), stream(), tag=f"{N}x{K} rows")
+        return out
     if M <= 64 and (N, K, 1) in TUNED and _forced_splits is None:
         tuned = TUNED[(N, K, 1)]
         splits = splits or tuned[0] or None
@@ -263,6 +297,10 @@ def swiglu_gate_up(x, w_gate_up, splits=None, stages=0, tile_tokens=0, activatio
         raise KernelError("swiglu: weight must be [2F][K]")
     gated = _gated_epilogue(activation)
     out = torch.empty((M, F), dtype=torch.bfloat16, device=x.device)
+    if splits is None and not stages and not tile_tokens and _rows_takes(M, F2, K):
+        lib.call("fwb_linear_rows", ptr(x), ptr(w_gate_up), ptr(out), ptr(None), M, F, K, F2, F, gated, F,
+                 lib.c_float(limit), stream(), tag=f"swiglu {F}x{K} rows")
+        return out
     if M <= 64 and (F, K, 2) in TUNED and _forced_splits is None:
         tuned = TUNED[(F, K, 2)]
         splits = splits or tuned[0] or None
@@ -353,6 +391,8 @@ def normed_accepts(M: int, K: int, w, accumulators: int, N: int) -> bool:
     activation tiles inside the kernel stays off the critical path."""
     if not (_enabled and _fuse_norm) or w.dtype != torch.bfloat16 or M > 64 or K % 8 or not _aligned(w):
         return False
+    if _rows_takes(M, accumulators * N, K):
+        return _rows_takes_normed(M, accumulators * N, K)
     if M < FUSE_FROM_TOKENS and not _fuse_always:
         return False
     splits = _forced_splits if _forced_splits is not None else _splits_for(M, N, K, accumulators)
@@ -371,6 +411,11 @@ def gemm_normed(x_res, norm_weight, eps, w, out_dtype, rows=None, n_rows=None, s
     if w.shape[1] != K or norm_weight.numel() != K:
         raise KernelError(f"gemm: residual has {K} columns, weight has {w.shape[1]}, norm {norm_weight.numel()}")
     out = torch.empty((M, N), dtype=out_dtype, device=x_res.device)
+    if splits is None and not stages and not tile_tokens and _rows_takes_normed(M, N, K):
+        lib.call("fwb_linear_rows_normed", ptr(x_res), ptr(norm_weight), ptr(rows), lib.c_float(eps), ptr(w), ptr(out),
+                 M, N, K, N, N, EPI_F32 if out_dtype == torch.float32 else EPI_BF16, 0, lib.c_float(0.0), stream(),
+                 tag=f"normed {N}x{K} rows")
+        return out
     if splits is None:
         splits = pick_splits(M, N, K)
     stages = stages or _ring_depth(M, N, splits, 1)
@@ -395,6 +440,10 @@ def swiglu_gate_up_normed(x_res, norm_weight, eps, w_gate_up, splits=None, stage
         raise KernelError("swiglu: weight must be [2F][K] and the norm weight [K]")
     gated = _gated_epilogue(activation)
     out = torch.empty((M, F), dtype=torch.bfloat16, device=x_res.device)
+    if splits is None and not stages and not tile_tokens and _rows_takes_normed(M, F2, K):
+        lib.call("fwb_linear_rows_normed", ptr(x_res), ptr(norm_weight), ptr(None), lib.c_float(eps), ptr(w_gate_up),
+                 ptr(out), M, F, K, F2, F, gated, F, lib.c_float(limit), stream(), tag=f"normed swiglu {F}x{K} rows")
+        return out
     if splits is None:
         splits = _forced_splits if _forced_splits is not None else _splits_for(M, F, K, 2)
     stages = stages or _ring_depth(M, F, splits, 2)

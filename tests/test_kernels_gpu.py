@@ -125,6 +125,44 @@ def test_gemm_fp32_tiles(M, N, K):
         assert torch.equal(ops.gemm_simt(dev(x[-rows:]), dev(w), torch.float32), out[-rows:])
 
 
+@pytest.mark.parametrize("M", [1, 8, 9, 16, 17, 32])
+@pytest.mark.parametrize("N,K", [(8, 8), (17, 40), (1000, 264), (2048, 1024), (2488, 1032), (9216, 1024)])
+def test_products_of_a_few_tokens(M, N, K):
+    """The weight reader at the edges of its row groups, its feature groups and its chunks of K, with every epilogue,
+    against the same product in 64 bits: fp32 sums of K products of bfloat16 numbers, then one rounding."""
+    from flyweight_b200.kernels import ops, tensorcore
+    if not tensorcore._rows_takes(M, N, K):
+        pytest.skip("the tcgen05 kernel's size")
+    g = torch.Generator().manual_seed(M * N + K)
+    x, w = torch.randn(M, K, generator=g).bfloat16(), torch.randn(N, K, generator=g).bfloat16()
+    add = torch.randn(M, N, generator=g)
+    exact, size = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+    out = tensorcore.gemm(dev(x), dev(w), torch.float32)
+    assert ((out.cpu().double() - exact).abs() <= 2.0 ** -20 * size).all()
+    total = dev(add)
+    tensorcore.gemm(dev(x), dev(w), torch.float32, addend=total, out=total)
+    assert ((total.cpu().double() - exact - add.double()).abs() <= 2.0 ** -20 * size + 2.0 ** -23 * add.abs()).all()
+    half = tensorcore.gemm(dev(x), dev(w), torch.bfloat16)
+    assert torch.equal(half, out.bfloat16())
+    relu = tensorcore.gemm(dev(x), dev(w), torch.bfloat16, activation="relu_squared")
+    assert torch.equal(relu, (torch.relu(out) ** 2).bfloat16())
+    if M > 1 and M not in (17, 32):
+        # a row's value does not depend on its company (up to 16 rows; beyond, K is dealt to the warps otherwise)
+        assert torch.equal(tensorcore.gemm(dev(x[-1:]), dev(w), torch.float32), out[-1:])
+    if N % 2 == 0:
+        gate, up = exact[:, :N // 2], exact[:, N // 2:]
+        want = torch.nn.functional.silu(gate) * up
+        got = tensorcore.swiglu_gate_up(dev(x), dev(w)).cpu().double()
+        assert ((got - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -18 * (size[:, :N // 2] + 1) * (up.abs() + size[:, N // 2:] * 2.0 ** -18 + 1)).all()
+    if tensorcore._rows_takes_normed(M, N, K):
+        res, norm = torch.randn(40, K, generator=g), 1.0 + 0.1 * torch.randn(K, generator=g)
+        rows = torch.randperm(40, generator=g)[:M].to(torch.int32)
+        h = (res * norm).bfloat16().double()[rows.long()]
+        want = (h @ w.double().T) * torch.rsqrt((res.double()[rows.long()] ** 2).mean(1, keepdim=True) + 1e-5)
+        got = tensorcore.gemm_normed(dev(res), dev(norm), 1e-5, dev(w), torch.float32, rows=dev(rows))
+        assert ((got.cpu().double() - want).abs() <= 2.0 ** -19 * (h.abs() @ w.double().abs().T) * 2).all()
+
+
 def test_gemm_row_does_not_depend_on_the_batch():
     from flyweight_b200.kernels import ops
     g = torch.Generator().manual_seed(5)
