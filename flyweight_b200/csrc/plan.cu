@@ -37,7 +37,7 @@ int fwb_gemm_tcgen05_normed(const float*, const float*, const int*, float, const
 int fwb_linear_rows(const void*, const void*, void*, const float*, int, int, int, int, int, int, int, float, cudaStream_t);
 int fwb_linear_rows_normed(const float*, const float*, const int*, float, const void*, void*, int, int, int, int, int,
                            int, int, float, cudaStream_t);
-int fwb_gemm_tcgen05_pair(const void*, const void*, void*, int, int, int, int, int, int, int, int,
+int fwb_gemm_tcgen05_pair(const void*, const void*, void*, int, int, int, int, int, int, int, float,
                           cudaStream_t);
 int fwb_shortconv(const void*, int, const float*, const float*, float*, const int*, const int*, const int*,
                   void*, int, int, int, int, int, long long, cudaStream_t);
@@ -182,26 +182,6 @@ bool mid_size_choice(int M, int N, int K, int accumulators, bool pair_ok, int& t
     return pair;
 }
 
-int wave_cut(int M, int F) {
-    const int token_tiles = ceil_div(M, 256), feature_tiles = ceil_div(F, 128);
-    const int ctas = token_tiles * feature_tiles;
-    const int whole = ctas / SM_COUNT, left = ctas - whole * SM_COUNT;
-    if (whole == 0 || left == 0 || left > 0.75 * SM_COUNT) return 0;
-    const int cut = (whole * SM_COUNT) / token_tiles, rest = feature_tiles - cut;
-    if (cut <= 0 || rest <= 0 || rest * ceil_div(M, 128) > SM_COUNT) return 0;
-    return cut;
-}
-
-int pair_wave_cut(int M, int N) {
-    const int slots = SM_COUNT / 2, token_tiles = ceil_div(M, 256);
-    const int pairs = ceil_div(N, 512) * token_tiles;
-    const int whole = pairs / slots, left = pairs - whole * slots;
-    if (whole == 0 || left == 0 || left > 0.75 * slots) return 0;
-    const int cut = (whole * slots) / token_tiles, rest = N - cut * 512;
-    if (cut <= 0 || rest <= 0 || ceil_div(rest, 256) * token_tiles > slots) return 0;
-    return cut;
-}
-
 bool tc_accepts(const void* x, const void* w, int M, int K) {
     return g_option[OPT_TENSORCORE] && K % 8 == 0 && K >= 8 && aligned16(x) && aligned16(w) && M <= 65535 * 16;
 }
@@ -255,24 +235,11 @@ void tc_gemm(Launches& L, const void* x, const void* w, void* out, int out_bf16,
     }
     const bool pair_ok = g_option[OPT_PAIRS] && M > 128 && !addend && !in_place && N >= 256;
     int splits = 0, stages = 0, tile_tokens = 0;
-    bool pair = false, wide = false;
-    if (g_option[OPT_MID_SIZE_SPLIT] && M >= MID_FROM && M <= MID_TO) {
+    bool pair = pair_ok;
+    if (g_option[OPT_MID_SIZE_SPLIT] && M >= MID_FROM && M <= MID_TO)
         pair = mid_size_choice(M, N, K, 1, pair_ok, tile_tokens, splits);
-    } else if (pair_ok) {
-        pair = true;
-        wide = ceil_div(N, 256) * ceil_div(M, 256) > SM_COUNT / 2;
-    }
     if (pair) {
-        const int cut = wide ? pair_wave_cut(M, N) : 0;
-        const int out_bytes = out_bf16 ? 2 : 4;
-        if (cut) {
-            const int first = cut * 512;
-            L.add(fwb_gemm_tcgen05_pair(x, w, out, M, first, K, N, N, epilogue, 0, 1, stream));
-            L.add(fwb_gemm_tcgen05_pair(x, offset(w, (long long)first * K, 2), (void*)offset(out, first, out_bytes),
-                                        M, N - first, K, N - first, N, epilogue, 0, 0, stream));
-            return;
-        }
-        L.add(fwb_gemm_tcgen05_pair(x, w, out, M, N, K, N, N, epilogue, 0, wide ? 1 : 0, stream));
+        L.add(fwb_gemm_tcgen05_pair(x, w, out, M, N, K, N, N, epilogue, 0, 0.0f, stream));
         return;
     }
     if (!splits) splits = pick_splits(M, N, K);
@@ -297,12 +264,8 @@ void tc_swiglu(Launches& L, const void* x, const void* w, void* out, int M, int 
     }
     const bool mid = g_option[OPT_MID_SIZE_SPLIT] && M >= MID_FROM && M <= MID_TO;
     if (mid) mid_size_choice(M, F, K, 2, false, tile_tokens, splits);
-    const int cut = (M > 128 && splits == 1 && !stages && !tile_tokens && !mid) ? wave_cut(M, F) : 0;
-    if (cut) {
-        const int first = cut * 128;
-        L.add(fwb_gemm_tcgen05(x, w, out, nullptr, M, first, K, 2 * F, F, EPI_SWIGLU_BF16, F, 1, 0, 256, -1, 0.0f, stream));
-        L.add(fwb_gemm_tcgen05(x, offset(w, (long long)first * K, 2), (void*)offset(out, first, 2), nullptr, M,
-                               F - first, K, 2 * F - first, F, EPI_SWIGLU_BF16, F, 1, 0, 128, -1, 0.0f, stream));
+    else if (g_option[OPT_PAIRS] && M > 128 && splits == 1) {
+        L.add(fwb_gemm_tcgen05_pair(x, w, out, M, F, K, 2 * F, F, EPI_SWIGLU_BF16, F, 0.0f, stream));
         return;
     }
     L.add(fwb_gemm_tcgen05(x, w, out, nullptr, M, F, K, 2 * F, F, EPI_SWIGLU_BF16, F, splits, stages, tile_tokens,

@@ -245,12 +245,9 @@ def gemm(x, w, out_dtype, addend=None, splits=None, stages=0, tile_tokens=0, wid
     if free_choice and _mid_size_split and MID_FROM <= M <= MID_TO:
         kind, tile_tokens, splits = mid_size_choice(M, N, K, 1, pair_ok)
         if kind == "pair":
-            return gemm_pair(x, w, out_dtype, wide=False, activation=activation)
+            return gemm_pair(x, w, out_dtype, activation=activation)
     elif pair_ok and free_choice:
-        # prompt-sized: CTA pairs (cta_group::2); two feature blocks per pair when single blocks
-        # would make more CTAs than the GPU holds at once (measured at 2,048 tokens on B200)
-        pairs = -(-N // 256) * -(-M // 256)
-        return gemm_pair(x, w, out_dtype, wide=pairs > SM_COUNT // 2, activation=activation)
+        return gemm_pair(x, w, out_dtype, activation=activation)       # prompt-sized: CTA pairs (cta_group::2)
     if out is None:
         out = torch.empty((M, N), dtype=out_dtype, device=x.device)
     else:
@@ -316,17 +313,9 @@ def swiglu_gate_up(x, w_gate_up, splits=None, stages=0, tile_tokens=0, activatio
     mid = free_choice and _mid_size_split and MID_FROM <= M <= MID_TO
     if mid:
         _, tile_tokens, splits = mid_size_choice(M, F, K, 2, False)
-    cut = _wave_cut(M, F) if (M > 128 and splits == 1 and not stages and not tile_tokens and not mid) else 0
-    if cut:
-        # Prompt-sized: 256-token tiles make a number of CTAs that ends in a part-filled wave.  The
-        # feature tiles of the whole waves run as they are; the rest runs with 128-token tiles, twice
-        # as many CTAs of half the length, which fit one wave and start as the first launch drains.
-        first = cut * 128
-        lib.call("fwb_gemm_tcgen05", ptr(x), ptr(w_gate_up), ptr(out), ptr(None), M, first, K, F2, F,
-                 gated, F, 1, 0, 256, -1, lib.c_float(limit), stream(), tag=f"swiglu {F}x{K} first")
-        lib.call("fwb_gemm_tcgen05", ptr(x), _offset(w_gate_up, first * K), _offset(out, first), ptr(None), M,
-                 F - first, K, F2 - first, F, gated, F, 1, 0, 128, -1, lib.c_float(limit), stream(),
-                 tag=f"swiglu {F}x{K} rest")
+    if free_choice and not mid and _use_pairs and M > 128 and splits == 1:
+        lib.call("fwb_gemm_tcgen05_pair", ptr(x), ptr(w_gate_up), ptr(out), M, F, K, F2, F, gated, F,
+                 lib.c_float(limit), stream(), tag=f"swiglu {F}x{K}")
         return out
     lib.call("fwb_gemm_tcgen05", ptr(x), ptr(w_gate_up), ptr(out), ptr(None), M, F, K, F2, F,
              gated, F, splits, stages, tile_tokens, -1, lib.c_float(limit), stream(),
@@ -334,16 +323,9 @@ def swiglu_gate_up(x, w_gate_up, splits=None, stages=0, tile_tokens=0, activatio
     return out
 
 
-def _offset(tensor, elements: int):
-    """The address ``elements`` into a contiguous tensor (a slice without making a view)."""
-    return tensor.data_ptr() + elements * tensor.element_size()
-
-
 def _wave_cut(M: int, F: int) -> int:
-    """How many 128-feature tiles the first of two launches takes (0: one launch).  With one CTA
-    per SM, ``tiles`` CTAs take ceil(tiles / 148) rounds; when the last round would be less than
-    three quarters full and what is left fits one round of half-length CTAs, cutting there saves
-    most of a round (measured at 2,048 tokens, 8,192 features: 115.6 -> 110.6 us)."""
+    """How many 128-feature tiles the whole rounds of one-CTA gated tiles hold (0: no part-filled last round worth
+    cutting off).  The persistent CTA pairs run such products now; tests take ragged sizes from it."""
     token_tiles = -(-M // 256)
     feature_tiles = -(-F // 128)
     ctas = token_tiles * feature_tiles
@@ -461,8 +443,9 @@ def status() -> int:
 
 
 def gemm_pair(x, w, out_dtype, wide=False, activation=None) -> torch.Tensor:
-    """``x @ w.T`` on CTA pairs (tcgen05 cta_group::2): 256 features x 256 tokens per pair and
-    accumulator.  For prompt-sized steps; bf16 in, fp32 or bf16 out."""
+    """``x @ w.T`` on CTA pairs (tcgen05 cta_group::2), tiles of 256 features x 256 tokens, as many pairs as the GPU
+    holds.  For prompt-sized steps; bf16 in, fp32 or bf16 out.  (``wide`` asked for tiles of two feature blocks, which
+    the persistent pairs do not need: it changes nothing.)"""
     check_tensor("gemm input", x, torch.bfloat16)
     check_tensor("gemm weight", w, torch.bfloat16)
     M, K = x.shape
@@ -471,24 +454,13 @@ def gemm_pair(x, w, out_dtype, wide=False, activation=None) -> torch.Tensor:
         raise KernelError(f"gemm: input has {K} columns, weight has {w.shape[1]}")
     out = torch.empty((M, N), dtype=out_dtype, device=x.device)
     epilogue = EPI_F32 if out_dtype == torch.float32 else _output_epilogue(activation)
-    cut = _pair_wave_cut(M, N) if wide else 0
-    if cut:
-        # the wide blocks of the whole rounds, then the rest as narrow pairs that fit one round
-        first = cut * 512
-        lib.call("fwb_gemm_tcgen05_pair", ptr(x), ptr(w), ptr(out), M, first, K, N, N, epilogue, 0, 1, stream())
-        lib.call("fwb_gemm_tcgen05_pair", ptr(x), _offset(w, first * K), _offset(out, first), M, N - first, K,
-                 N - first, N, epilogue, 0, 0, stream())
-        return out
-    lib.call("fwb_gemm_tcgen05_pair", ptr(x), ptr(w), ptr(out), M, N, K, N, N, epilogue, 0,
-             1 if wide else 0, stream(), tag=f"{N}x{K}")
+    lib.call("fwb_gemm_tcgen05_pair", ptr(x), ptr(w), ptr(out), M, N, K, N, N, epilogue, 0, lib.c_float(0.0),
+             stream(), tag=f"{N}x{K}")
     return out
 
 
 def _pair_wave_cut(M: int, N: int) -> int:
-    """For the wide CTA-pair form (512 features a pair): how many 512-feature blocks the first of
-    two launches takes (0: one launch).  74 pairs run at a time; when the last round would be less
-    than three quarters full and what is left fits one round of one-block pairs (half the length),
-    cutting there saves most of half a round (in_proj at 2,048 tokens: 96 pairs = 1.3 rounds)."""
+    """The same for 512-feature blocks on CTA pairs."""
     slots = SM_COUNT // 2
     token_tiles = -(-M // 256)
     pairs = -(-N // 512) * token_tiles
@@ -511,5 +483,5 @@ def swiglu_gate_up_pair(x, w_gate_up) -> torch.Tensor:
     F = w_gate_up.shape[0] // 2
     out = torch.empty((M, F), dtype=torch.bfloat16, device=x.device)
     lib.call("fwb_gemm_tcgen05_pair", ptr(x), ptr(w_gate_up), ptr(out), M, F, K, 2 * F, F,
-             EPI_SWIGLU_BF16, F, 0, stream())
+             EPI_SWIGLU_BF16, F, lib.c_float(0.0), stream())
     return out
