@@ -93,6 +93,92 @@ delta_prepare_kernel(const float* __restrict__ p, const float* __restrict__ taps
     }
 }
 
+// The same for four taps and channel counts in fours, PREP tokens a block: their rows of p are read once, 16 bytes a
+// load, as a window that slides along (the kernel above reads every row once per tap), and only the channels of q and
+// k stop in shared memory on their way.
+constexpr int PREP = 4;
+__global__ void __launch_bounds__(512)
+delta_prepare_window_kernel(const float* __restrict__ p, const float* __restrict__ taps, const float* __restrict__ a_log,
+                            const float* __restrict__ dt_bias, const float* __restrict__ state, long long slot_stride,
+                            const int* __restrict__ seg_start, const int* __restrict__ seg_slot,
+                            const int* __restrict__ tok_seg, float* __restrict__ r, int T, DeltaShape sh) {
+    fwb::pdl_entry();
+    extern __shared__ __align__(16) float c[];    // [PREP][2 G d]: q and k behind convolution and silu
+    constexpr int L = 4;
+    const int t0 = blockIdx.x * PREP, tokens = T - t0 < PREP ? T - t0 : PREP;
+    const int C = sh.channels(), P = sh.p_width(), R = sh.r_width(), QK = 2 * sh.cq();
+    int local[PREP];                              // tokens of its request in front of a token in this step
+    const float* hist[PREP];
+#pragma unroll
+    for (int i = 0; i < PREP; ++i) {
+        const int t = i < tokens ? t0 + i : t0, seg = tok_seg[t];
+        local[i] = t - seg_start[seg];
+        hist[i] = state + (size_t)seg_slot[seg] * slot_stride + (size_t)sh.H * sh.d * sh.e;
+    }
+    for (int ch = threadIdx.x * 4; ch < C; ch += blockDim.x * 4) {
+        float4 window[PREP + L - 1];
+#pragma unroll
+        for (int i = 0; i < PREP + L - 1; ++i) {
+            const int t = t0 + i - (L - 1);
+            window[i] = t >= 0 && t < T ? *reinterpret_cast<const float4*>(p + (size_t)t * P + ch) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        float4 w[4];                              // the taps of four channels
+#pragma unroll
+        for (int j = 0; j < 4; ++j) w[j] = *reinterpret_cast<const float4*>(taps + (size_t)(ch + j) * L);
+#pragma unroll
+        for (int i = 0; i < PREP; ++i) {
+            if (i >= tokens) break;
+            float4 x[L];
+#pragma unroll
+            for (int j = 0; j < L; ++j) {
+                const int back = L - 1 - j;       // tap j multiplies the input `back` tokens ago
+                x[j] = window[i + j];
+                if (back > local[i]) {
+                    const float* from = hist[i] + (size_t)ch * (L - 1) + (L - 1) - (back - local[i]);
+                    x[j] = make_float4(from[0], from[L - 1], from[2 * (L - 1)], from[3 * (L - 1)]);
+                }
+            }
+            float4 v;
+            v.x = silu_f32(fmaf(w[0].w, x[3].x, fmaf(w[0].z, x[2].x, fmaf(w[0].y, x[1].x, w[0].x * x[0].x))));
+            v.y = silu_f32(fmaf(w[1].w, x[3].y, fmaf(w[1].z, x[2].y, fmaf(w[1].y, x[1].y, w[1].x * x[0].y))));
+            v.z = silu_f32(fmaf(w[2].w, x[3].z, fmaf(w[2].z, x[2].z, fmaf(w[2].y, x[1].z, w[2].x * x[0].z))));
+            v.w = silu_f32(fmaf(w[3].w, x[3].w, fmaf(w[3].z, x[2].w, fmaf(w[3].y, x[1].w, w[3].x * x[0].w))));
+            if (ch < QK) *reinterpret_cast<float4*>(c + i * QK + ch) = v;
+            else *reinterpret_cast<float4*>(r + (size_t)(t0 + i) * R + ch) = v;
+        }
+    }
+    __syncthreads();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+    const float q_scale = rsqrtf((float)sh.d);
+    for (int job = warp; job < tokens * sh.G; job += warps) {         // query head and key head `head` together
+        const int i = job / sh.G, head = job - i * sh.G;
+        const float* q = c + (size_t)i * QK + (size_t)head * sh.d;
+        const float* k = q + sh.cq();
+        float* out = r + (size_t)(t0 + i) * R;
+        float qq = 0.0f, kk = 0.0f, qk = 0.0f;
+        for (int n = lane; n < sh.d; n += 32) {
+            qq = fmaf(q[n], q[n], qq);
+            kk = fmaf(k[n], k[n], kk);
+            qk = fmaf(q[n], k[n], qk);
+        }
+        qq = warp_sum(qq), kk = warp_sum(kk), qk = warp_sum(qk);
+        const float inv_q = (1.0f / sqrtf(qq + 1e-6f)) * q_scale, inv_k = 1.0f / sqrtf(kk + 1e-6f);
+        for (int n = lane; n < sh.d; n += 32) {
+            out[(size_t)head * sh.d + n] = q[n] * inv_q;
+            out[(size_t)(sh.G + head) * sh.d + n] = k[n] * inv_k;
+        }
+        if (lane == 0) out[C + 2 * sh.H + head] = (qk * inv_q) * inv_k;      // q^ . k^, for the read-out
+    }
+    for (int job = threadIdx.x; job < tokens * sh.H; job += blockDim.x) {
+        const int i = job / sh.H, h = job - i * sh.H;
+        const float* row = p + (size_t)(t0 + i) * P + C + sh.cv();
+        const float a = row[sh.H + h] + dt_bias[h];
+        const float softplus = a > 20.0f ? a : log1pf(expf(a));
+        r[(size_t)(t0 + i) * R + C + h] = 1.0f / (1.0f + expf(-row[h]));
+        r[(size_t)(t0 + i) * R + C + sh.H + h] = expf(-expf(a_log[h]) * softplus);
+    }
+}
+
 // The request's last L-1 inputs of every channel, for the next step.  Runs in the kernel behind
 // delta_prepare (which reads the old ones): the first block of every segment's scan does it.
 __device__ __forceinline__ void delta_conv_advance(const float* __restrict__ p, float* __restrict__ slot, int t0,
@@ -645,11 +731,21 @@ FWB_API int fwb_delta_rule(const float* p, const float* taps, const float* a_log
     if (slot_stride < (long long)H * d * e + (long long)sh.channels() * (L - 1)) return FWB_BAD_ARGUMENT;
     const size_t smem = (size_t)sh.channels() * sizeof(float);
     if (smem > 160 * 1024 || n_segments > 65535 || H > 65535) return FWB_TOO_LARGE;
-    if (smem > 48 * 1024)
-        cudaFuncSetAttribute(delta_prepare_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    const int prepare_threads = sh.channels() >= 2048 ? 512 : (sh.channels() >= 512 ? 256 : 128);
-    fwb::pdl(delta_prepare_kernel, T, prepare_threads, smem, stream)(p, taps, a_log, dt_bias, state, slot_stride,
-                                                                     seg_start, seg_slot, tok_seg, r, sh);
+    // tokens in fours once there are enough of them, where 16-byte loads can read everything
+    const size_t window_smem = (size_t)PREP * 2 * sh.cq() * sizeof(float);
+    if (T >= 128 && L == 4 && sh.cq() % 2 == 0 && sh.cv() % 4 == 0 && sh.p_width() % 4 == 0 && window_smem <= 100 * 1024 &&
+        ((uintptr_t)p & 15) == 0 && ((uintptr_t)taps & 15) == 0 && ((uintptr_t)r & 15) == 0) {
+        if (window_smem > 48 * 1024)
+            cudaFuncSetAttribute(delta_prepare_window_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
+        fwb::pdl(delta_prepare_window_kernel, (T + PREP - 1) / PREP, 512, window_smem, stream)(
+            p, taps, a_log, dt_bias, state, slot_stride, seg_start, seg_slot, tok_seg, r, T, sh);
+    } else {
+        if (smem > 48 * 1024)
+            cudaFuncSetAttribute(delta_prepare_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        const int prepare_threads = sh.channels() >= 2048 ? 512 : (sh.channels() >= 512 ? 256 : 128);
+        fwb::pdl(delta_prepare_kernel, T, prepare_threads, smem, stream)(p, taps, a_log, dt_bias, state, slot_stride,
+                                                                         seg_start, seg_slot, tok_seg, r, sh);
+    }
     const bool vec = d % 4 == 0 && e % 4 == 0 && slot_stride % 4 == 0 && ((uintptr_t)state & 15) == 0 &&
                      ((uintptr_t)r & 15) == 0;
     if (scratch && vec && (d == 64 || d == 128) && ((uintptr_t)scratch & 15) == 0) {

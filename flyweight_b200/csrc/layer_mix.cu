@@ -46,6 +46,139 @@ rmsnorm_ranges_kernel(T* __restrict__ buf, long long row_stride, NormRange r0, N
         row[i] = from_f32<T>((to_f32<T>(row[i]) * inv) * r.weight[i]);
 }
 
+// ---- rows in registers --------------------------------------------------------------------------
+// The three norms of this file for rows that 256 threads hold in four-element pieces, VEC a thread: every row is read
+// once, its pieces asked for together, and the weights (nobody's output) before the wait.  In a decode step such a
+// launch is the chain of its loads and one reduction; the loops above wait for memory twice, and again for the weights.
+constexpr int VEC_FROM = 512, VEC_TO = 4096;       // row widths: below, most threads would have nothing to do
+
+template <typename T> __device__ __forceinline__ float4 load4(const T* p);
+template <> __device__ __forceinline__ float4 load4<float>(const float* p) { return *reinterpret_cast<const float4*>(p); }
+template <> __device__ __forceinline__ float4 load4<__nv_bfloat16>(const __nv_bfloat16* p) {
+    const uint2 v = *reinterpret_cast<const uint2*>(p);
+    const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v.x));
+    const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v.y));
+    return make_float4(a.x, a.y, b.x, b.y);
+}
+__device__ __forceinline__ void store4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
+__device__ __forceinline__ void store4(__nv_bfloat16* p, float4 v) {
+    __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
+    *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
+}
+__device__ __forceinline__ float squares(float4 v) { return fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, v.w * v.w))); }
+template <typename T>
+bool pieces_of_four(const T* p, long long stride) {
+    return stride % 4 == 0 && (uintptr_t)p % (4 * sizeof(T)) == 0;
+}
+
+template <typename T, int VEC>
+__global__ void __launch_bounds__(256)
+rmsnorm_ranges_vec_kernel(T* __restrict__ buf, long long row_stride, NormRange r0, NormRange r1, float eps) {
+    fwb::pdl_launch_dependents();
+    __shared__ float scratch[33];
+    const NormRange r = blockIdx.y == 0 ? r0 : r1;
+    T* row = buf + (size_t)blockIdx.x * row_stride + r.col0;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 v[VEC], w[VEC];
+#pragma unroll
+    for (int i = 0; i < VEC; ++i) {
+        const int c = (threadIdx.x + i * 256) * 4;
+        w[i] = c < r.width ? load4<float>(r.weight + c) : zero;
+    }
+    fwb::pdl_wait();
+    float ss = 0.0f;
+#pragma unroll
+    for (int i = 0; i < VEC; ++i) {
+        const int c = (threadIdx.x + i * 256) * 4;
+        v[i] = c < r.width ? load4<T>(row + c) : zero;
+    }
+#pragma unroll
+    for (int i = 0; i < VEC; ++i) ss += squares(v[i]);
+    const float inv = rsqrtf(block_sum(ss, scratch) / (float)r.count + eps);
+#pragma unroll
+    for (int i = 0; i < VEC; ++i) {
+        const int c = (threadIdx.x + i * 256) * 4;
+        if (c < r.width)
+            store4(row + c, make_float4((v[i].x * inv) * w[i].x, (v[i].y * inv) * w[i].y, (v[i].z * inv) * w[i].z,
+                                        (v[i].w * inv) * w[i].w));
+    }
+}
+
+template <int VEC>
+__global__ void __launch_bounds__(256)
+pair_norm_mean_vec_kernel(const float* __restrict__ a, const float* __restrict__ wa, const float* __restrict__ b,
+                          const float* __restrict__ wb, float eps, float* __restrict__ y, int H) {
+    fwb::pdl_launch_dependents();
+    __shared__ float scratch[33];
+    const size_t base = (size_t)blockIdx.x * H;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 u[VEC], v[VEC], wu[VEC], wv[VEC];
+#pragma unroll
+    for (int i = 0; i < VEC; ++i) {
+        const int c = (threadIdx.x + i * 256) * 4;
+        wu[i] = c < H ? load4<float>(wa + c) : zero;
+        wv[i] = c < H ? load4<float>(wb + c) : zero;
+    }
+    fwb::pdl_wait();
+#pragma unroll
+    for (int i = 0; i < VEC; ++i) {
+        const int c = (threadIdx.x + i * 256) * 4;
+        u[i] = c < H ? load4<float>(a + base + c) : zero;
+        v[i] = c < H ? load4<float>(b + base + c) : zero;
+    }
+    float sa = 0.0f, sb = 0.0f;
+#pragma unroll
+    for (int i = 0; i < VEC; ++i) sa += squares(u[i]), sb += squares(v[i]);
+    const float ia = rsqrtf(block_sum(sa, scratch) / (float)H + eps);
+    const float ib = rsqrtf(block_sum(sb, scratch) / (float)H + eps);
+#pragma unroll
+    for (int i = 0; i < VEC; ++i) {
+        const int c = (threadIdx.x + i * 256) * 4;
+        if (c < H)
+            store4(y + base + c, make_float4(0.5f * ((u[i].x * ia) * wu[i].x + (v[i].x * ib) * wv[i].x),
+                                             0.5f * ((u[i].y * ia) * wu[i].y + (v[i].y * ib) * wv[i].y),
+                                             0.5f * ((u[i].z * ia) * wu[i].z + (v[i].z * ib) * wv[i].z),
+                                             0.5f * ((u[i].w * ia) * wu[i].w + (v[i].w * ib) * wv[i].w)));
+    }
+}
+
+template <typename TG, typename TO, int VEC>
+__global__ void __launch_bounds__(256)
+gated_rmsnorm_vec_kernel(const float* __restrict__ o, const TG* __restrict__ gate, long long gate_stride,
+                         const float* __restrict__ w, float eps, TO* __restrict__ out, int H) {
+    fwb::pdl_launch_dependents();
+    __shared__ float scratch[33];
+    const size_t base = (size_t)blockIdx.x * H;
+    const TG* gr = gate + (size_t)blockIdx.x * gate_stride;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 v[VEC], g[VEC], wv[VEC];
+#pragma unroll
+    for (int i = 0; i < VEC; ++i) {
+        const int c = (threadIdx.x + i * 256) * 4;
+        wv[i] = c < H ? load4<float>(w + c) : zero;
+    }
+    fwb::pdl_wait();
+#pragma unroll
+    for (int i = 0; i < VEC; ++i) {
+        const int c = (threadIdx.x + i * 256) * 4;
+        v[i] = c < H ? load4<float>(o + base + c) : zero;
+        g[i] = c < H ? load4<TG>(gr + c) : zero;
+    }
+    float ss = 0.0f;
+#pragma unroll
+    for (int i = 0; i < VEC; ++i) ss += squares(v[i]);
+    const float inv = rsqrtf(block_sum(ss, scratch) / (float)H + eps);
+#pragma unroll
+    for (int i = 0; i < VEC; ++i) {
+        const int c = (threadIdx.x + i * 256) * 4;
+        if (c < H)
+            store4(out + base + c, make_float4(((v[i].x * inv) * wv[i].x) * sigmoid_f32(g[i].x),
+                                               ((v[i].y * inv) * wv[i].y) * sigmoid_f32(g[i].y),
+                                               ((v[i].z * inv) * wv[i].z) * sigmoid_f32(g[i].z),
+                                               ((v[i].w * inv) * wv[i].w) * sigmoid_f32(g[i].w)));
+    }
+}
+
 template <typename T>
 __global__ void value_mix_kernel(T* __restrict__ rows, long long row_stride, int col0, int width,
                                  T* __restrict__ first, const float* __restrict__ lam, int n_rows, int mix) {
@@ -175,6 +308,17 @@ gated_rmsnorm_kernel(const float* __restrict__ o, const TG* __restrict__ gate, l
         out[base + i] = from_f32<TO>(((o[base + i] * inv) * w[i]) * sigmoid_f32(to_f32<TG>(g[i])));
 }
 
+template <typename TG, typename TO>
+bool launch_gated_vec(const float* o, const TG* gate, long long gate_stride, const float* w, float eps, TO* out, int T, int H,
+                      cudaStream_t stream) {
+    if (H < VEC_FROM || H > VEC_TO || (H & 3) || !pieces_of_four(o, 0) || !pieces_of_four(gate, gate_stride) ||
+        !pieces_of_four(w, 0) || !pieces_of_four(out, 0))
+        return false;
+    if (H <= 2048) fwb::pdl(gated_rmsnorm_vec_kernel<TG, TO, 2>, T, 256, 0, stream)(o, gate, gate_stride, w, eps, out, H);
+    else fwb::pdl(gated_rmsnorm_vec_kernel<TG, TO, 4>, T, 256, 0, stream)(o, gate, gate_stride, w, eps, out, H);
+    return true;
+}
+
 inline int blocks_for(size_t n) { return (int)((n + 255) / 256 > 8192 ? 8192 : (n + 255) / 256); }
 
 }  // namespace
@@ -191,6 +335,20 @@ FWB_API int fwb_rmsnorm_ranges(void* buf, int is_bf16, long long row_stride, int
     if (width1 > 0 && (!w1 || count1 <= 0 || col1 < 0 || col1 + width1 > row_stride)) return FWB_BAD_ARGUMENT;
     const NormRange r0{col0, width0, count0, w0}, r1{col1, width1, count1 > 0 ? count1 : 1, w1};
     const dim3 grid(T, width1 > 0 ? 2 : 1);
+    const int widest = width1 > width0 ? width1 : width0;
+    const bool fours = is_bf16 ? pieces_of_four((bf*)buf, row_stride) : pieces_of_four((float*)buf, row_stride);
+    if (fours && widest >= VEC_FROM && widest <= VEC_TO && ((width0 | col0) & 3) == 0 && pieces_of_four(w0, 0) &&
+        (width1 <= 0 || (((width1 | col1) & 3) == 0 && pieces_of_four(w1, 0)))) {
+        // (a second range may be short: its idle threads cost nothing beside the first one's)
+        if (is_bf16) {
+            if (widest <= 2048) fwb::pdl(rmsnorm_ranges_vec_kernel<bf, 2>, grid, 256, 0, stream)((bf*)buf, row_stride, r0, r1, eps);
+            else fwb::pdl(rmsnorm_ranges_vec_kernel<bf, 4>, grid, 256, 0, stream)((bf*)buf, row_stride, r0, r1, eps);
+        } else {
+            if (widest <= 2048) fwb::pdl(rmsnorm_ranges_vec_kernel<float, 2>, grid, 256, 0, stream)((float*)buf, row_stride, r0, r1, eps);
+            else fwb::pdl(rmsnorm_ranges_vec_kernel<float, 4>, grid, 256, 0, stream)((float*)buf, row_stride, r0, r1, eps);
+        }
+        return fwb_launch_status();
+    }
     if (is_bf16) fwb::pdl(rmsnorm_ranges_kernel<bf>, grid, 256, 0, stream)((bf*)buf, row_stride, r0, r1, eps);
     else fwb::pdl(rmsnorm_ranges_kernel<float>, grid, 256, 0, stream)((float*)buf, row_stride, r0, r1, eps);
     return fwb_launch_status();
@@ -320,6 +478,12 @@ FWB_API int fwb_pair_norm_mean(const float* a, const float* wa, const float* b, 
                                int T, int H, cudaStream_t stream) {
     if (T <= 0) return FWB_OK;
     if (!a || !wa || !b || !wb || !y || H <= 0) return FWB_BAD_ARGUMENT;
+    if (H >= VEC_FROM && H <= VEC_TO && (((uintptr_t)a | (uintptr_t)wa | (uintptr_t)b | (uintptr_t)wb | (uintptr_t)y) & 15) == 0 &&
+        (H & 3) == 0) {
+        if (H <= 2048) fwb::pdl(pair_norm_mean_vec_kernel<2>, T, 256, 0, stream)(a, wa, b, wb, eps, y, H);
+        else fwb::pdl(pair_norm_mean_vec_kernel<4>, T, 256, 0, stream)(a, wa, b, wb, eps, y, H);
+        return fwb_launch_status();
+    }
     fwb::pdl(pair_norm_mean_kernel, T, 256, 0, stream)(a, wa, b, wb, eps, y, H);
     return fwb_launch_status();
 }
@@ -329,6 +493,10 @@ FWB_API int fwb_gated_rmsnorm(const float* o, const void* gate, int gate_bf16, l
                               float eps, void* out, int out_bf16, int T, int H, cudaStream_t stream) {
     if (T <= 0) return FWB_OK;
     if (!o || !gate || !w || !out || H <= 0 || gate_stride < H) return FWB_BAD_ARGUMENT;
+    const bool done = gate_bf16 ? out_bf16 && launch_gated_vec(o, (const bf*)gate, gate_stride, w, eps, (bf*)out, T, H, stream)
+                      : out_bf16 ? launch_gated_vec(o, (const float*)gate, gate_stride, w, eps, (bf*)out, T, H, stream)
+                                 : launch_gated_vec(o, (const float*)gate, gate_stride, w, eps, (float*)out, T, H, stream);
+    if (done) return fwb_launch_status();
     if (gate_bf16 && out_bf16)
         fwb::pdl(gated_rmsnorm_kernel<bf, bf>, T, 256, 0, stream)(o, (const bf*)gate, gate_stride, w, eps, (bf*)out, H);
     else if (!gate_bf16 && !out_bf16)

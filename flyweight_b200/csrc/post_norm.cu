@@ -41,6 +41,76 @@ rmsnorm_add_kernel(float* __restrict__ x, const float* __restrict__ y, const flo
     for (int i = threadIdx.x; i < H; i += blockDim.x) h[base + i] = from_f32<TO>((row[i] * inv2) * w2[i]);
 }
 
+// The same with a row in registers, VEC float4 a thread: y and x are asked for together and read once, the weights
+// before the wait (they are nobody's output).  Bound by memory at prompt sizes and by the chain of its two
+// reductions in a decode step; the kernel above reads y twice, 4 bytes a load.
+template <typename TO, int VEC, bool NEXT>
+__global__ void __launch_bounds__(256)
+rmsnorm_add_vec_kernel(float* __restrict__ x, const float* __restrict__ y, const float* __restrict__ w, float eps,
+                       const float* __restrict__ w2, float eps2, TO* __restrict__ h, int H) {
+    fwb::pdl_launch_dependents();
+    __shared__ float scratch[33];
+    const int n4 = H >> 2;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 wv[VEC], wn[NEXT ? VEC : 1];
+#pragma unroll
+    for (int i = 0; i < VEC; ++i) {
+        const int c = threadIdx.x + i * 256;
+        wv[i] = c < n4 ? reinterpret_cast<const float4*>(w)[c] : zero;
+        if (NEXT) wn[i] = c < n4 ? reinterpret_cast<const float4*>(w2)[c] : zero;
+    }
+    fwb::pdl_wait();
+    float4* xr = reinterpret_cast<float4*>(x + (size_t)blockIdx.x * H);
+    const float4* yr = reinterpret_cast<const float4*>(y + (size_t)blockIdx.x * H);
+    float4 v[VEC], r[VEC];
+#pragma unroll
+    for (int i = 0; i < VEC; ++i) {
+        const int c = threadIdx.x + i * 256;
+        v[i] = c < n4 ? yr[c] : zero;
+        r[i] = c < n4 ? xr[c] : zero;
+    }
+    float ss = 0.0f;
+#pragma unroll
+    for (int i = 0; i < VEC; ++i) ss += v[i].x * v[i].x + v[i].y * v[i].y + v[i].z * v[i].z + v[i].w * v[i].w;
+    const float inv = rsqrtf(block_sum(ss, scratch) / (float)H + eps);
+    float sx = 0.0f;
+#pragma unroll
+    for (int i = 0; i < VEC; ++i) {
+        const int c = threadIdx.x + i * 256;
+        r[i].x += (v[i].x * inv) * wv[i].x, r[i].y += (v[i].y * inv) * wv[i].y;
+        r[i].z += (v[i].z * inv) * wv[i].z, r[i].w += (v[i].w * inv) * wv[i].w;
+        if (c < n4) xr[c] = r[i];
+        sx += r[i].x * r[i].x + r[i].y * r[i].y + r[i].z * r[i].z + r[i].w * r[i].w;
+    }
+    if constexpr (NEXT) {
+        const float inv2 = rsqrtf(block_sum(sx, scratch) / (float)H + eps2);
+        TO* out = h + (size_t)blockIdx.x * H;
+#pragma unroll
+        for (int i = 0; i < VEC; ++i) {
+            const int c = threadIdx.x + i * 256;
+            if (c >= n4) continue;
+            const float a = (r[i].x * inv2) * wn[i].x, b = (r[i].y * inv2) * wn[i].y;
+            const float cc = (r[i].z * inv2) * wn[i].z, d = (r[i].w * inv2) * wn[i].w;
+            if (sizeof(TO) == 4) {
+                reinterpret_cast<float4*>(out)[c] = make_float4(a, b, cc, d);
+            } else {
+                __nv_bfloat162 lo = __floats2bfloat162_rn(a, b), hi = __floats2bfloat162_rn(cc, d);
+                reinterpret_cast<uint2*>(out)[c] = make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
+            }
+        }
+    }
+}
+
+template <typename TO, bool NEXT>
+void launch_vec(float* x, const float* y, const float* w, float eps, const float* w2, float eps2, TO* h, int T, int H,
+                cudaStream_t stream) {
+    const int vec = (H / 4 + 255) / 256;
+    if (vec == 1) fwb::pdl(rmsnorm_add_vec_kernel<TO, 1, NEXT>, T, 256, 0, stream)(x, y, w, eps, w2, eps2, h, H);
+    else if (vec == 2) fwb::pdl(rmsnorm_add_vec_kernel<TO, 2, NEXT>, T, 256, 0, stream)(x, y, w, eps, w2, eps2, h, H);
+    else if (vec == 3) fwb::pdl(rmsnorm_add_vec_kernel<TO, 3, NEXT>, T, 256, 0, stream)(x, y, w, eps, w2, eps2, h, H);
+    else fwb::pdl(rmsnorm_add_vec_kernel<TO, 4, NEXT>, T, 256, 0, stream)(x, y, w, eps, w2, eps2, h, H);
+}
+
 template <typename TI, typename TO>
 __global__ void gate_act_mul_kernel(const TI* __restrict__ gu, TO* __restrict__ out, int T, int F, int act,
                                     float limit) {
@@ -63,6 +133,14 @@ FWB_API int fwb_rmsnorm_add(float* x, const float* y, const float* w, float eps,
     if (!x || !y || !w || H <= 0 || (w2 && !h)) return FWB_BAD_ARGUMENT;
     const size_t smem = w2 ? (size_t)H * sizeof(float) : 0;
     if (smem > 160 * 1024) return FWB_TOO_LARGE;
+    // rows of 16-byte pieces that 256 threads hold in registers (shorter ones leave most of them idle)
+    const bool aligned = (((uintptr_t)x | (uintptr_t)y | (uintptr_t)w | (uintptr_t)w2 | (uintptr_t)h) & 15) == 0;
+    if ((H & 3) == 0 && H >= 512 && H <= 4096 && aligned) {
+        if (!w2) launch_vec<float, false>(x, y, w, eps, nullptr, 0.0f, nullptr, T, H, stream);
+        else if (h_bf16) launch_vec<__nv_bfloat16, true>(x, y, w, eps, w2, eps2, (__nv_bfloat16*)h, T, H, stream);
+        else launch_vec<float, true>(x, y, w, eps, w2, eps2, (float*)h, T, H, stream);
+        return fwb_launch_status();
+    }
     if (h_bf16) {
         if (smem > 48 * 1024)
             cudaFuncSetAttribute(rmsnorm_add_kernel<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

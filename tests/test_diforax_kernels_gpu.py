@@ -456,6 +456,37 @@ def test_delta_chunks_against_the_scan_and_64_bits(H, G, d, e, strong):
     print("errors", errors)
 
 
+def test_delta_inputs_of_many_short_segments():
+    """The convolution in front of the recurrence reads a window of rows that crosses requests: 60 requests of one to
+    five tokens in one step leave the bits and the states that each leaves in a step of its own."""
+    from flyweight_b200.kernels import recurrent
+    H, G, d, e, L = 4, 2, 16, 24, 4
+    C = 2 * G * d + H * e
+    g = torch.Generator().manual_seed(3)
+    lengths = [1 + (7 * i) % 5 for i in range(60)]
+    T = sum(lengths)
+    p = dev(torch.randn(T, C + H * e + 2 * H, generator=g))
+    taps, a_log, bias = dev(torch.randn(C, L, generator=g)), dev(torch.randn(H, generator=g)), dev(torch.randn(H, generator=g))
+    start = dev(torch.randn(61, recurrent.delta_state_size(H, G, d, e, L), generator=g))
+    i32 = lambda values: torch.tensor(values, dtype=torch.int32, device=DEV)
+
+    def run(p, lengths, slots, state):
+        batch = type("Batch", (), {})()
+        batch.n_segments, batch.max_segment = len(lengths), max(lengths)
+        batch.seg_start, batch.seg_slot = i32([sum(lengths[:i]) for i in range(len(lengths) + 1)]), i32(slots)
+        batch.tok_seg = i32([s for s, n in enumerate(lengths) for _ in range(n)])
+        return recurrent.delta_rule(p, taps, a_log, bias, state, batch, H, G, d, e)
+
+    assert T >= 128
+    together, apart = start.clone(), start.clone()
+    out = run(p, lengths, list(range(1, 61)), together)
+    at = 0
+    for s, n in enumerate(lengths):
+        assert torch.equal(run(p[at:at + n].contiguous(), [n], [s + 1], apart), out[at:at + n]), s
+        at += n
+    assert torch.equal(together, apart)
+
+
 def test_the_delta_state_remembers_a_write_from_hundreds_of_tokens_ago():
     """One early token writes a value under a key that no later token touches (later keys are orthogonal
     to it and decay is switched off): a query for that key, 400 tokens and several steps later, reads the

@@ -376,3 +376,39 @@ def test_dense_feed_forward_and_token_side_input(dtype):
         side.forward(ctx, x)
         want = h + P.token_side_input(h, torch.tensor(tokens), w, f"l{index}.side.", index, 8, EPS, rnd=rnd)
         close(x, want, TOL[dtype], f"side input of layer {index}")
+
+
+@pytest.mark.parametrize("H", [508, 512, 1020, 1024, 2048, 2052, 4096, 4100])
+def test_norms_whose_rows_stay_in_registers(H):
+    """Row widths around the edges of the forms that hold a row in 16-byte pieces, and rows and columns that such
+    pieces cannot take: all against 64 bits (a mean of H squares, a handful of roundings behind it)."""
+    from flyweight_b200.kernels import mixing, ops
+    g = torch.Generator().manual_seed(H)
+    rand = lambda *shape: torch.randn(*shape, generator=g)
+    unit = lambda t, count=None: t.double() * torch.rsqrt((t.double() ** 2).sum(-1, keepdim=True) / (count or t.shape[-1]) + EPS)
+    T, rel = 5, 2e-6
+    a, b, wa, wb = rand(T, H), rand(T, H), 1.0 + 0.1 * rand(H), 1.0 + 0.1 * rand(H)
+    close(mixing.pair_norm_mean(dev(a), dev(wa), dev(b), dev(wb), EPS),
+          0.5 * (unit(a) * wa.double() + unit(b) * wb.double()), rel, "pair")
+    for dtype in (torch.float32, torch.bfloat16):
+        for width, col in ((H + 8, 4), (H + 3, 2)):
+            wide = rand(T, width).to(dtype)
+            gate = wide[:, col:col + H]
+            want = unit(a) * wa.double() * torch.sigmoid(gate.double())
+            close(mixing.gated_rmsnorm(dev(a), dev(wide)[:, col:col + H], dev(wa), EPS, torch.bfloat16), want, 2.0 ** -8, "gated")
+            if dtype == torch.float32:
+                close(mixing.gated_rmsnorm(dev(a), dev(wide)[:, col:col + H], dev(wa), EPS, torch.float32), want, rel, "gated fp32")
+            rows = rand(T, width + 40).to(dtype)
+            out = dev(rows)
+            mixing.rmsnorm_ranges_(out, [(col, dev(wa), H - 4, EPS), (col + H, dev(wb[:32]), 32, EPS)])
+            want = rows.double().clone()
+            want[:, col:col + H] = unit(rows[:, col:col + H], H - 4) * wa.double()
+            want[:, col + H:col + H + 32] = unit(rows[:, col + H:col + H + 32]) * wb[:32].double()
+            close(out, want, rel if dtype == torch.float32 else 2.0 ** -8, "ranges")
+    for next_dtype in (None, torch.float32, torch.bfloat16):
+        x = dev(a)
+        h = ops.rmsnorm_add_(x, dev(b), dev(wa), EPS, None if next_dtype is None else dev(wb), EPS, next_dtype)
+        want = a.double() + unit(b) * wa.double()
+        close(x, want, rel, "sum")
+        if next_dtype is not None:
+            close(h, unit(want) * wb.double(), rel if next_dtype == torch.float32 else 2.0 ** -8, "next norm")
