@@ -41,7 +41,10 @@ constexpr int WARPS = 8, THREADS = 32 * (WARPS + 1);
 constexpr int SMEM_TARGET = 112 * 1024;        // two CTAs an SM
 constexpr int MAX_SLOTS = 8;
 constexpr long TWO_CTAS_FROM = 2 << 20;
-enum Epilogue : int { EPI_F32 = 0, EPI_BF16 = 1, EPI_ADD_F32 = 2, EPI_SWIGLU_BF16 = 3 };
+// EPI_CONV: the rows are B | C | x of a gated short convolution, a token per request: three accumulators, and the
+// epilogue is the convolution's step (csrc/shortconv.cu) on the bfloat16-rounded projections, state and all.
+enum Epilogue : int { EPI_F32 = 0, EPI_BF16 = 1, EPI_ADD_F32 = 2, EPI_SWIGLU_BF16 = 3, EPI_CONV = 4 };
+constexpr int accumulators_of(int epi) { return epi == EPI_CONV ? 3 : (epi == EPI_SWIGLU_BF16 ? 2 : 1); }
 
 struct RowsParams {
     const __nv_bfloat16* x;      // [M][K], or
@@ -58,6 +61,13 @@ struct RowsParams {
     int units;                   // groups of eight features of one accumulator per CTA
     int slots;                   // depth of the ring
     int* status;
+    // EPI_CONV: [N][conv_taps], [N] or null, a request's last conv_taps - 1 products at conv_slot[token] * conv_stride
+    const float* conv_w;
+    const float* conv_bias;
+    float* conv_state;
+    const int* conv_slot;
+    long long conv_stride;
+    int conv_taps;
 };
 
 __device__ __forceinline__ uint4 load_rows(const void* p) {     // written by the kernel before: not .nc
@@ -78,7 +88,7 @@ __host__ __device__ constexpr int row_stride(int K) { return ((2 * K + 127) & ~1
 // R8: groups of eight token rows.
 template <int R8, int KBLK, int EPI, bool NORMED>
 __global__ void __launch_bounds__(THREADS, 2) linear_rows_kernel(const RowsParams prm) {
-    constexpr int NACC = EPI == EPI_SWIGLU_BF16 ? 2 : 1;
+    constexpr int NACC = accumulators_of(EPI);
     constexpr int MT = (R8 + 1) / 2;                   // 16-row tiles of the product
     constexpr int CHUNK = WARPS * KBLK * 32, W_STRIDE = row_stride(CHUNK), SLOT = 8 * W_STRIDE;
     extern __shared__ __align__(128) uint8_t smem[];
@@ -117,8 +127,8 @@ __global__ void __launch_bounds__(THREADS, 2) linear_rows_kernel(const RowsParam
             if (lane == 0) mbar_expect_tx(&full_bar[slot], 8 * bytes);
             __syncwarp();
             if (lane < 8) {
-                const int feature = (unit0 + (NACC == 2 ? group >> 1 : group)) * 8 + lane;
-                const size_t row = (feature < prm.N ? feature : prm.N - 1) + (NACC == 2 && (group & 1) ? prm.up_row_offset : 0);
+                const int feature = (unit0 + group / NACC) * 8 + lane;
+                const size_t row = (feature < prm.N ? feature : prm.N - 1) + (size_t)(group % NACC) * prm.up_row_offset;
                 asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                              ::"r"(smem_u32(ring + slot * SLOT + lane * W_STRIDE)), "l"(prm.w + row * K + k), "r"(bytes),
                                "r"(smem_u32(&full_bar[slot])) : "memory");
@@ -277,7 +287,22 @@ __global__ void __launch_bounds__(THREADS, 2) linear_rows_kernel(const RowsParam
             for (int wp = 0; wp < WARPS; ++wp) v += p[(size_t)wp * prm.units * NACC * R8 * 64];
             sum[a] = v * inv_rms;
         }
-        if (EPI == EPI_F32) reinterpret_cast<float*>(prm.y)[at] = sum[0];
+        if constexpr (EPI == EPI_CONV) {
+            const int keep = prm.conv_taps - 1;
+            const float b = __bfloat162float(__float2bfloat16_rn(sum[0])), c = __bfloat162float(__float2bfloat16_rn(sum[1]));
+            const float u = b * __bfloat162float(__float2bfloat16_rn(sum[2]));
+            const float* taps = prm.conv_w + (size_t)f * prm.conv_taps;
+            float* kept = prm.conv_state + (size_t)prm.conv_slot[row] * prm.conv_stride + (size_t)f * keep;
+            float v = prm.conv_bias ? prm.conv_bias[f] : 0.0f;
+            for (int k = 0; k < keep; ++k) {
+                const float old = kept[k];
+                v = fmaf(taps[k], old, v);
+                if (k > 0) kept[k - 1] = old;
+            }
+            kept[keep - 1] = u;
+            v = fmaf(taps[keep], u, v);
+            reinterpret_cast<__nv_bfloat16*>(prm.y)[at] = __float2bfloat16_rn(c * v);
+        } else if (EPI == EPI_F32) reinterpret_cast<float*>(prm.y)[at] = sum[0];
         else if (EPI == EPI_ADD_F32) reinterpret_cast<float*>(prm.y)[at] = sum[0] + add;
         else if (EPI == EPI_BF16) reinterpret_cast<__nv_bfloat16*>(prm.y)[at] = __float2bfloat16_rn(output_act_f32(prm.act, sum[0]));
         else reinterpret_cast<__nv_bfloat16*>(prm.y)[at] = __float2bfloat16_rn(gated_fast(prm.act, prm.limit, sum[0], sum[NACC - 1]));
@@ -286,7 +311,7 @@ __global__ void __launch_bounds__(THREADS, 2) linear_rows_kernel(const RowsParam
 
 template <int R8, int KBLK, int EPI, bool NORMED>
 int launch(RowsParams prm, cudaStream_t stream) {
-    constexpr int NACC = EPI == EPI_SWIGLU_BF16 ? 2 : 1, SLOT = 8 * row_stride(WARPS * KBLK * 32);
+    constexpr int NACC = accumulators_of(EPI), SLOT = 8 * row_stride(WARPS * KBLK * 32);
     constexpr int MOST = 16 / (NACC * R8);             // units a CTA keeps partial sums of: 32 KiB
     const int all_units = (prm.N + 7) / 8;
     // two CTAs an SM, or as few more as the partial sums allow, evenly filled; one for a matrix that a single
@@ -341,7 +366,8 @@ FWB_API int fwb_linear_rows(const void* X, const void* W, void* Y, const float* 
     if (epilogue == EPI_SWIGLU_BF16 && (up_row_offset < N || w_rows < up_row_offset + N)) return FWB_BAD_ARGUMENT;
     if (epilogue != EPI_SWIGLU_BF16 && w_rows < N) return FWB_BAD_ARGUMENT;
     const RowsParams prm{(const __nv_bfloat16*)X, nullptr, nullptr, nullptr, 0.0f, (const __nv_bfloat16*)W, Y, addend,
-                         M, N, K, ldy, up_row_offset, act, gate_limit, 0, 0, status_word()};
+                         M, N, K, ldy, up_row_offset, act, gate_limit, 0, 0, status_word(),
+                         nullptr, nullptr, nullptr, nullptr, 0, 0};
     switch (epilogue) {
         case EPI_F32: return launch_rows<EPI_F32, false>(prm, stream);
         case EPI_BF16: return launch_rows<EPI_BF16, false>(prm, stream);
@@ -364,11 +390,30 @@ FWB_API int fwb_linear_rows_normed(const float* x_res, const float* norm_w, cons
     if (epilogue == EPI_SWIGLU_BF16 && (up_row_offset < N || w_rows < up_row_offset + N)) return FWB_BAD_ARGUMENT;
     if (epilogue != EPI_SWIGLU_BF16 && w_rows < N) return FWB_BAD_ARGUMENT;
     const RowsParams prm{nullptr, x_res, norm_w, rows, eps, (const __nv_bfloat16*)W, Y, nullptr,
-                         M, N, K, ldy, up_row_offset, act, gate_limit, 0, 0, status_word()};
+                         M, N, K, ldy, up_row_offset, act, gate_limit, 0, 0, status_word(),
+                         nullptr, nullptr, nullptr, nullptr, 0, 0};
     switch (epilogue) {
         case EPI_F32: return launch_rows<EPI_F32, true>(prm, stream);
         case EPI_BF16: return launch_rows<EPI_BF16, true>(prm, stream);
         case EPI_SWIGLU_BF16: return launch_rows<EPI_SWIGLU_BF16, true>(prm, stream);
         default: return FWB_UNSUPPORTED;
     }
+}
+
+// One step of a gated short convolution for requests of one token each: in_proj rows B | C | x ([3H][K], H below one
+// another) on X [M][K] bf16, or (norm_w given) on RMS-normed rows of the fp32 residual X, then
+// z[t][c] = C (bias + sum_k taps[c][k] u) with u = B x behind the `conv_taps` - 1 products in slots[t], which move on.
+// The projections are rounded to bfloat16 in between: the bits of fwb_linear_rows and fwb_shortconv.
+FWB_API int fwb_linear_rows_conv(const void* X, const float* norm_w, float eps, const void* W, const float* conv_w,
+                                 const float* conv_bias, float* state, long long state_stride, const int* slots, void* z,
+                                 int M, int H, int K, int conv_taps, cudaStream_t stream) {
+    if (M <= 0 || H <= 0) return FWB_OK;
+    if (!X || !W || !conv_w || !state || !slots || !z || K <= 0 || conv_taps < 2) return FWB_BAD_ARGUMENT;
+    if (!shape_ok(W, M, K, norm_w ? MAX_NORMED_ROWS : 16) || ((uintptr_t)X & 15)) return FWB_UNSUPPORTED;
+    if (norm_w && (((uintptr_t)norm_w & 15) || K > MAX_NORMED_K)) return FWB_UNSUPPORTED;
+    const RowsParams prm{(const __nv_bfloat16*)X, (const float*)X, norm_w, nullptr, eps, (const __nv_bfloat16*)W, z, nullptr,
+                         M, H, K, H, H, 0, 0.0f, 0, 0, status_word(),
+                         conv_w, conv_bias, state, slots, state_stride, conv_taps};
+    if (norm_w) return launch<1, 4, EPI_CONV, true>(prm, stream);
+    return M > 8 ? launch<2, 4, EPI_CONV, false>(prm, stream) : launch<1, 4, EPI_CONV, false>(prm, stream);
 }

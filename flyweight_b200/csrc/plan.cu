@@ -37,6 +37,8 @@ int fwb_gemm_tcgen05_normed(const float*, const float*, const int*, float, const
 int fwb_linear_rows(const void*, const void*, void*, const float*, int, int, int, int, int, int, int, float, cudaStream_t);
 int fwb_linear_rows_normed(const float*, const float*, const int*, float, const void*, void*, int, int, int, int, int,
                            int, int, float, cudaStream_t);
+int fwb_linear_rows_conv(const void*, const float*, float, const void*, const float*, const float*, float*, long long,
+                         const int*, void*, int, int, int, int, cudaStream_t);
 int fwb_gemm_tcgen05_pair(const void*, const void*, void*, int, int, int, int, int, int, int, float,
                           cudaStream_t);
 int fwb_shortconv(const void*, int, const float*, const float*, float*, const int*, const int*, const int*,
@@ -441,6 +443,28 @@ void run_norm_linear(Launches& L, const Op& op, const FwbStep& step, bool& pendi
         return;
     }
     linear(L, op.scratch, h_bf16, op.w, op.w_bf16, out, op.out_bf16, nullptr, M, op.N, op.K, stream);
+}
+
+// A step of one token per request: norm, in_proj and the short convolution behind it in one kernel, or the norm's and
+// one for the rest (kernels/tensorcore.py: conv_step).  False: the two operations run one after the other.
+bool run_conv_step(Launches& L, const Op& op, const Op& conv, const FwbStep& step, bool& pending, int act_bf16,
+                   cudaStream_t stream) {
+    const int M = step.T;
+    if (conv.kind != OP_SHORTCONV || conv.in != op.out || op.epilogue != EPI_BF16 || op.on_logit_rows || op.N != 3 * conv.K)
+        return false;
+    if (!act_bf16 || !op.w_bf16 || step.max_segment != 1 || step.S != M || M > 16 || op.K % 8 || !aligned16(op.w) ||
+        !rows_takes(M, op.N, op.K) || conv.out == op.scratch)
+        return false;
+    const int* slots = meta(step, META_SEG_SLOT);
+    const bool normed = !pending && g_option[OPT_FUSE_NORM] && rows_takes_normed(M, op.N, op.K) && aligned16(op.x);
+    if (!normed) {
+        L.add(fwb_rmsnorm(op.x, pending ? op.delta : nullptr, op.v0, op.scratch, 1, nullptr, M, op.K, op.eps, stream));
+        pending = false;
+    }
+    L.add(fwb_linear_rows_conv(normed ? (const void*)op.x : op.scratch, normed ? op.v0 : nullptr, op.eps, op.w, conv.v0,
+                               conv.v1, (float*)conv.pool_k, conv.stride, slots, conv.out, M, conv.K, op.K, conv.taps,
+                               stream));
+    return true;
 }
 
 void run_linear_residual(Launches& L, const Op& op, const FwbStep& step, bool& pending, int act_bf16,
@@ -988,6 +1012,10 @@ FWB_API int fwb_plan_run(void* handle, const void* step_ptr, int* launches, cuda
                                 op.flag, op.scale, stream));
                 break;
             case OP_NORM_LINEAR:
+                if (i + 1 < plan.ops.size() && run_conv_step(L, op, plan.ops[i + 1], step, pending, act_bf16, stream)) {
+                    ++i;
+                    break;
+                }
                 run_norm_linear(L, op, step, pending, act_bf16, stream);
                 break;
             case OP_LINEAR_RESIDUAL:

@@ -277,6 +277,46 @@ def gemm(x, w, out_dtype, addend=None, splits=None, stages=0, tile_tokens=0, wid
     return out
 
 
+def conv_step_accepts(h, w_in, batch, act_dtype) -> bool:
+    """A step of one token per request whose in_proj the weight reader takes does the short convolution in that
+    product's epilogue (measured in the decode step: a launch of 4 to 5 us less per convolution layer)."""
+    H = w_in.shape[0] // 3
+    return (act_dtype == torch.bfloat16 and w_in.dtype == torch.bfloat16 and batch.max_segment == 1
+            and batch.n_tokens == batch.n_segments <= 16 and w_in.shape[1] % 8 == 0 and _aligned(w_in)
+            and _rows_takes(batch.n_tokens, 3 * H, w_in.shape[1]))
+
+
+def conv_step(h, w_in, taps, bias, state, batch) -> torch.Tensor:
+    """``shortconv(linear(h, w_in))`` of a step of one token per request, in one kernel: ``h`` bf16 rows, or a norm not
+    yet applied to rows of the residual."""
+    K, H, L = w_in.shape[1], w_in.shape[0] // 3, taps.shape[1]
+    M = batch.n_tokens
+    norm_w, eps = None, 0.0
+    if isinstance(h, torch.Tensor):
+        x = h
+    elif h.kind == "rmsnorm" and h.rows is None and _fuse_norm and _rows_takes_normed(M, 3 * H, K) and _aligned(h.x):
+        x, norm_w, eps = h.x, h.weight, h.eps
+        check_tensor("norm weight", norm_w, torch.float32, (K,))
+    else:
+        x = h.materialize(torch.bfloat16)
+    check_tensor("conv step input", x, torch.bfloat16 if norm_w is None else torch.float32)
+    check_tensor("conv step weight", w_in, torch.bfloat16)
+    check_tensor("conv taps", taps, torch.float32, (H, L))
+    if bias is not None:
+        check_tensor("conv bias", bias, torch.float32, (H,))
+    if x.numel() != M * K:
+        raise KernelError(f"conv step: {x.numel()} inputs for {M} tokens of {K}")
+    if (not state.is_cuda or state.dtype != torch.float32 or tuple(state.shape[1:]) != (H, L - 1)
+            or state.stride(2) != 1 or state.stride(1) != L - 1 or (state.shape[0] > 1 and state.stride(0) < H * (L - 1))):
+        raise KernelError(f"conv state must be CUDA fp32 [slots][{H}][{L - 1}] with contiguous slots")
+    stride = state.stride(0) if state.shape[0] > 1 else H * (L - 1)
+    check_tensor("seg_slot", batch.seg_slot, torch.int32, (M,))
+    out = torch.empty((M, H), dtype=torch.bfloat16, device=x.device)
+    lib.call("fwb_linear_rows_conv", ptr(x), ptr(norm_w), lib.c_float(eps), ptr(w_in), ptr(taps), ptr(bias), ptr(state),
+             lib.c_longlong(stride), ptr(batch.seg_slot), ptr(out), M, H, K, L, stream(), tag=f"{H}x{K} conv step")
+    return out
+
+
 def swiglu_accepts(x, w_gate_up) -> bool:
     return accepts(x, w_gate_up, torch.bfloat16)
 

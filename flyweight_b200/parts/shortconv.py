@@ -59,7 +59,11 @@ class GatedShortConv(Mixer):
         return FixedState((self.hidden, self.taps_len - 1))
 
     def forward(self, ctx, h, cache, residual=None):
+        from ..kernels import tensorcore
         batch = ctx.batch
+        if tensorcore.conv_step_accepts(h, self.w_in, batch, ctx.precision.act_dtype):
+            z = tensorcore.conv_step(h, self.w_in, self.taps, self.bias, cache.state, batch)
+            return ops.linear_into_residual(z, self.w_out, residual)
         # B|C|x in the activation dtype: the conv kernel widens them and multiplies in fp32
         p = ops.linear(h, self.w_in, ctx.precision.act_dtype)
         z = ops.shortconv(p, self.taps, self.bias, cache.state, batch.seg_start, batch.seg_slot,
@@ -70,9 +74,9 @@ class GatedShortConv(Mixer):
         """The same three operations for the native step plan (``engine/plan.py``)."""
         from ..engine.plan import EPI_ACT
         act = builder.act_dtype
+        z = builder.tokens(self.hidden, act)        # (before the norm's rows: the one-token form reads those and writes z)
         p = builder.tokens(3 * self.hidden, act)
         builder.norm_linear(norm, self.w_in, EPI_ACT, p, "conv in_proj")
-        z = builder.tokens(self.hidden, act)
         builder.shortconv(p, self.taps, self.bias, cache.state, z)
         builder.free(p)
         builder.linear_residual(z, self.w_out, "conv out_proj")

@@ -163,6 +163,33 @@ def test_products_of_a_few_tokens(M, N, K):
         assert ((got.cpu().double() - want).abs() <= 2.0 ** -19 * (h.abs() @ w.double().abs().T) * 2).all()
 
 
+@pytest.mark.parametrize("M,H,K,L", [(1, 64, 64, 3), (8, 200, 264, 3), (9, 24, 1032, 2), (16, 512, 512, 4), (8, 1000, 1000, 3)])
+@pytest.mark.parametrize("biased", [False, True])
+def test_a_convolution_step_in_the_projection(M, H, K, L, biased):
+    """One token per request: the projection with the convolution in its epilogue leaves the bits and the state of the
+    two kernels, with the norm folded in (few tokens, short rows) and without."""
+    from flyweight_b200.kernels import ops, tensorcore
+    from flyweight_b200.parts.base import DeferredNorm
+    g = torch.Generator().manual_seed(M * H + K)
+    x, w = dev(torch.randn(M, K, generator=g)), dev((torch.randn(3 * H, K, generator=g) / K ** 0.5).bfloat16())
+    taps, norm = dev(torch.randn(H, L, generator=g)), dev(1.0 + 0.1 * torch.randn(K, generator=g))
+    bias = dev(torch.randn(H, generator=g)) if biased else None
+    state = torch.randn(M + 3, H, L - 1, generator=g)
+    batch = type("Batch", (), {})()
+    i32 = lambda values: torch.tensor(values, dtype=torch.int32, device=DEV)
+    batch.n_tokens = batch.n_segments = M
+    batch.max_segment, batch.seg_start, batch.tok_seg = 1, i32(list(range(M + 1))), i32(list(range(M)))
+    batch.seg_slot = i32(torch.randperm(M + 3, generator=g)[:M].tolist())
+    for h in (DeferredNorm(x, norm, 1e-5), x.bfloat16()):
+        one, two = dev(state), dev(state)
+        assert tensorcore.conv_step_accepts(h, w, batch, torch.bfloat16)
+        got = tensorcore.conv_step(h, w, taps, bias, one, batch)
+        p = ops.linear(h, w, torch.bfloat16)
+        want = ops.shortconv(p, taps, bias, two, batch.seg_start, batch.seg_slot, batch.tok_seg, M, torch.bfloat16)
+        assert torch.equal(got, want) and torch.equal(one, two)
+    assert tensorcore.status() == 0
+
+
 def test_gemm_row_does_not_depend_on_the_batch():
     from flyweight_b200.kernels import ops
     g = torch.Generator().manual_seed(5)
