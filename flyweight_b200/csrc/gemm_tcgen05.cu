@@ -738,11 +738,10 @@ FWB_API int fwb_gemm_tcgen05_grouped(const void* X, const void* W, void* Y, cons
     if (epilogue != EPI_SWIGLU_BF16 && group_w_rows < N) return FWB_BAD_ARGUMENT;
     if (tile_rows != 16 && tile_rows != 32 && tile_rows != 64 && tile_rows != 128) return FWB_BAD_ARGUMENT;
     if ((N + BM - 1) / BM > 65535) return FWB_TOO_LARGE;
-    // full token tiles and enough features: two 128-feature tiles a CTA, the rows read once for both
-    if (tile_rows == 128 && N >= 2 * BM) {
-        if (epilogue == EPI_F32) epilogue = EPI_F32_WIDE;
-        else if (epilogue == EPI_BF16) epilogue = EPI_BF16_WIDE;
-    }
+    // full token tiles: persistent CTA pairs
+    if (tile_rows == 128)
+        return gemm_pair_grouped(X, W, Y, offsets, tiles, max_tiles, A, N, K, n_groups, group_w_rows, ldy, epilogue, gate_act,
+                                 up_row_offset, gate_limit, stream);
     Params prm;
     prm.y = Y;
     prm.addend = nullptr;
@@ -769,7 +768,6 @@ FWB_API int fwb_gemm_tcgen05_grouped(const void* X, const void* W, void* Y, cons
     switch (tile_rows) {
         case 16: return launch_epi<16>(epilogue, map_w, map_x, prm, 1, stream);
         case 32: return launch_epi<32>(epilogue, map_w, map_x, prm, 1, stream);
-        case 64: return launch_epi<64>(epilogue, map_w, map_x, prm, 1, stream);
-        default: return launch_epi<128>(epilogue, map_w, map_x, prm, 1, stream);
+        default: return launch_epi<64>(epilogue, map_w, map_x, prm, 1, stream);
     }
 }

@@ -37,17 +37,19 @@ namespace {
 
 constexpr int EPI_WARPS = 16;          // four per quarter of the TMEM lanes
 constexpr int THREADS = 64 + 32 * EPI_WARPS;   // warp 0 producer, warp 1 MMA, then the epilogue warps
-constexpr int BN = 256;                // tokens per tile (128 per CTA in shared memory)
-constexpr int HALF_N = BN / 2;
 constexpr int SM_PAIRS = 148 / 2;
-constexpr int STAGES = 6;
 constexpr int A_BYTES = BM * BK * 2;                    // 16 KiB: this CTA's 128 rows of A
-constexpr int STAGE_BYTES = A_BYTES + HALF_N * BK * 2;  // + its 128 tokens
 constexpr int TRADE_FLOATS = 8 * 32;                    // what a warp hands over of 16 columns
 enum PairEpilogue : int { PAIR_F32 = 0, PAIR_BF16 = 1, PAIR_SWIGLU_BF16 = 3 };
-constexpr int smem_bytes(int epi) {
-    return STAGES * STAGE_BYTES + (epi == PAIR_SWIGLU_BF16 ? 2 * EPI_WARPS * TRADE_FLOATS * 4 : 0) + 1024 + 512;
-}
+// BN: tokens per tile, half of them in each CTA's shared memory
+template <int BN>
+struct PairTile {
+    static constexpr int HALF_N = BN / 2;
+    static constexpr int STAGE_BYTES = A_BYTES + HALF_N * BK * 2;
+    static constexpr int STAGES = 192 * 1024 / STAGE_BYTES;
+    static constexpr int TRADE_BYTES = 2 * EPI_WARPS * TRADE_FLOATS * 4;
+    static constexpr int smem_bytes(bool gated) { return STAGES * STAGE_BYTES + (gated ? TRADE_BYTES : 0) + 1024 + 512; }
+};
 
 struct PairParams {
     void* y;
@@ -55,8 +57,14 @@ struct PairParams {
     int up_row_offset;
     int gate_act;          // SwiGLU: the gate's activation (GATE_*); bf16 outputs: OUTPUT_*
     float gate_limit;
-    int token_tiles, tiles;
+    int token_tiles, feature_tiles;
     int* status;
+    // Grouped form: the rows of X are sorted by group (see fwb_gemm_tcgen05_grouped); group_tiles[0] token tiles,
+    // then their (group, first row) pairs; a group's rows end at group_offsets[group + 1], its matrix begins
+    // group * group_w_rows rows down W.
+    const int* group_tiles;
+    const int* group_offsets;
+    int group_w_rows;
 };
 
 __device__ __forceinline__ void umma_bf16_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
@@ -107,16 +115,18 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar_cluster_addr) {
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar_cluster_addr) : "memory");
 }
 
-template <int EPI>
+template <int EPI, int BN, bool GROUPED>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                  const PairParams prm) {
     constexpr bool GATED = EPI == PAIR_SWIGLU_BF16;
     constexpr int CTA_FEATURES = GATED ? BM / 2 : BM;    // features a CTA has of a tile
+    using T = PairTile<BN>;
+    constexpr int STAGES = T::STAGES, STAGE_BYTES = T::STAGE_BYTES, HALF_N = T::HALF_N;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     float* trade = reinterpret_cast<float*>(tiles + STAGES * STAGE_BYTES);
-    uint64_t* full_bar = reinterpret_cast<uint64_t*>(tiles + STAGES * STAGE_BYTES + (GATED ? 2 * EPI_WARPS * TRADE_FLOATS * 4 : 0));
+    uint64_t* full_bar = reinterpret_cast<uint64_t*>(tiles + STAGES * STAGE_BYTES + (GATED ? T::TRADE_BYTES : 0));
     uint64_t* empty_bar = full_bar + STAGES;
     uint64_t* acc_full = empty_bar + STAGES;             // [2]: in both CTAs
     uint64_t* acc_empty = acc_full + 2;                  // [2]: the leader's, arrived on by both CTAs' epilogue warps
@@ -148,44 +158,69 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     tc_fence_after();
     const uint32_t tmem_base = *tmem_holder;
 
+    // the list of token tiles is the work of an earlier kernel of this step: nothing is read before it is done
+    if (GROUPED) pdl_wait();
+    const int token_tiles = GROUPED ? prm.group_tiles[0] : prm.token_tiles;
+    const int tiles_all = token_tiles * prm.feature_tiles;
     // token tiles are the fast index: pairs that run together share weight tiles in L2
-    auto tokens_of = [&](int tile) { return (tile % prm.token_tiles) * BN; };
-    auto features_of = [&](int tile) { return (tile / prm.token_tiles) * 2 * CTA_FEATURES + (int)rank * CTA_FEATURES; };
+    struct Place {
+        int tok0, m_end, f, w_row;                       // first token, the rows' end, this CTA's first feature and row of W
+    };
+    auto place_of = [&](int tile) {
+        Place at;
+        const int token_tile = tile % token_tiles;
+        at.f = (tile / token_tiles) * 2 * CTA_FEATURES + (int)rank * CTA_FEATURES;
+        if (GROUPED) {
+            const int group = prm.group_tiles[1 + 2 * token_tile];
+            at.tok0 = prm.group_tiles[2 + 2 * token_tile];
+            at.m_end = prm.group_offsets[group + 1];
+            at.w_row = at.f + group * prm.group_w_rows;
+        } else {
+            at.tok0 = token_tile * BN;
+            at.m_end = prm.M;
+            at.w_row = at.f;
+        }
+        return at;
+    };
 
     if (warp == 0) {
         if (lane == 0) {
             // every load of the pair reports to the leader's barrier of its stage; the leader arms it
             // with the bytes of both CTAs
-            auto load_w = [&](int s, int tile, int kb) {
+            auto load_w = [&](int s, const Place& at, int kb) {
                 uint8_t* stage = tiles + (size_t)s * STAGE_BYTES;
                 const uint32_t bar = cluster_addr(&full_bar[s], 0);
-                const int f = features_of(tile);
                 if (rank == 0) mbar_expect_tx(&full_bar[s], 2 * STAGE_BYTES);
-                tma_load_2d_pair(stage, &map_w, bar, kb * BK, f);
-                if (GATED) tma_load_2d_pair(stage + A_BYTES / 2, &map_w, bar, kb * BK, prm.up_row_offset + f);
+                tma_load_2d_pair(stage, &map_w, bar, kb * BK, at.w_row);
+                if (GATED) tma_load_2d_pair(stage + A_BYTES / 2, &map_w, bar, kb * BK, prm.up_row_offset + at.w_row);
             };
-            auto load_x = [&](int s, int tile, int kb) {
+            auto load_x = [&](int s, const Place& at, int kb) {
                 tma_load_2d_pair(tiles + (size_t)s * STAGE_BYTES + A_BYTES, &map_x, cluster_addr(&full_bar[s], 0), kb * BK,
-                                 tokens_of(tile) + (int)rank * HALF_N);
+                                 at.tok0 + (int)rank * HALF_N);
             };
-            const int ahead = n_kb < STAGES ? n_kb : STAGES;
-            for (int i = 0; i < ahead; ++i) load_w(i, first_tile, i);   // weights first: nothing in the stream writes them
-            pdl_wait();
-            for (int i = 0; i < ahead; ++i) load_x(i, first_tile, i);
+            const int ahead = first_tile >= tiles_all ? 0 : n_kb < STAGES ? n_kb : STAGES;
+            if (ahead) {
+                const Place at = place_of(first_tile);
+                for (int i = 0; i < ahead; ++i) load_w(i, at, i);      // weights first: nothing in the stream writes them
+                if (!GROUPED) pdl_wait();
+                for (int i = 0; i < ahead; ++i) load_x(i, at, i);
+            }
             int s = ahead % STAGES;
             uint32_t parity = ahead == STAGES ? 0 : 1;   // of the empty barrier; the ring's first round waits for nothing
             bool ok = true;
-            for (int tile = first_tile; tile < prm.tiles && ok; tile += tile_step)
+            for (int tile = first_tile; tile < tiles_all && ok; tile += tile_step) {
+                const Place at = place_of(tile);
                 for (int kb = tile == first_tile ? ahead : 0; kb < n_kb; ++kb) {
                     ok = mbar_wait(&empty_bar[s], parity, abort_flag, 11, prm.status);
                     if (!ok) break;
-                    load_w(s, tile, kb);
-                    load_x(s, tile, kb);
+                    load_w(s, at, kb);
+                    load_x(s, at, kb);
                     if (++s == STAGES) {
                         s = 0;
                         parity ^= 1;
                     }
                 }
+            }
         }
     } else if (warp == 1) {
         if (lane == 0 && rank == 0) {
@@ -193,7 +228,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
             bool ok = true;
             int s = 0, turn = 0;
             uint32_t parity = 0;
-            for (int tile = first_tile; tile < prm.tiles && ok; tile += tile_step, ++turn) {
+            for (int tile = first_tile; tile < tiles_all && ok; tile += tile_step, ++turn) {
                 const int b = turn & 1;
                 // both CTAs' epilogues have read what this accumulator held two tiles ago
                 if (turn >= 2) ok = mbar_wait_cluster(&acc_empty[b], ((turn >> 1) - 1) & 1, abort_flag, 17, prm.status);
@@ -222,22 +257,23 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
 
     // ---------------------------------------------------------------- epilogue (both CTAs)
     if (warp >= 2) {
-        pdl_wait();
+        if (!GROUPED) pdl_wait();
         const int quarter = warp & 3, group = (warp - 2) >> 2;
         const uint32_t lane_base = tmem_base + ((uint32_t)(quarter * 32) << 16);
         constexpr int PER_GROUP = BN / (EPI_WARPS / 4);  // the warps of a quarter of the TMEM lanes share the token columns
         int turn = 0;
-        for (int tile = first_tile; tile < prm.tiles; tile += tile_step, ++turn) {
+        for (int tile = first_tile; tile < tiles_all; tile += tile_step, ++turn) {
             const int b = turn & 1;
             bool ready = mbar_wait(&acc_full[b], (turn >> 1) & 1, abort_flag, 15, prm.status);
             // (after a wait that gave up nobody reads or stores, but everybody keeps meeting his partner's barriers)
             ready = __all_sync(0xffffffffu, ready && !*abort_flag);
             tc_fence_after();
-            const int tok0 = tokens_of(tile) + group * PER_GROUP;
+            const Place at_tile = place_of(tile);
+            const int tok0 = at_tile.tok0 + group * PER_GROUP, m_end = at_tile.m_end;
             const uint32_t from = lane_base + b * BN + group * PER_GROUP;
             if constexpr (GATED) {
                 const bool up = quarter >= 2;
-                const int f = features_of(tile) + (quarter & 1) * 32 + lane;
+                const int f = at_tile.f + (quarter & 1) * 32 + lane;
                 float* mine = trade + (size_t)(warp - 2) * TRADE_FLOATS + lane;
                 const float* theirs = trade + (size_t)((warp - 2) ^ 2) * TRADE_FLOATS + lane;
                 const int barrier = 1 + group * 2 + (quarter & 1);
@@ -254,13 +290,13 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
                         const float other = theirs[buffer + j * 32];
                         const float g = up ? other : v[j], u = up ? v[8 + j] : other;
                         const int t = tok0 + c0 + (up ? 8 : 0) + j;
-                        if (ready && t < prm.M && f < prm.N)
+                        if (ready && t < m_end && f < prm.N)
                             reinterpret_cast<__nv_bfloat16*>(prm.y)[(size_t)t * prm.ldy + f] =
                                 __float2bfloat16_rn(gated_fast(prm.gate_act, prm.gate_limit, g, u));
                     }
                 }
             } else {
-                const int f = features_of(tile) + quarter * 32 + lane;
+                const int f = at_tile.f + quarter * 32 + lane;
 #pragma unroll 1
                 for (int c0 = 0; c0 < PER_GROUP && ready; c0 += 16) {
                     float v[16];
@@ -268,7 +304,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
 #pragma unroll
                     for (int j = 0; j < 16; ++j) {
                         const int t = tok0 + c0 + j;
-                        if (t >= prm.M || f >= prm.N) continue;
+                        if (t >= m_end || f >= prm.N) continue;
                         const size_t at = (size_t)t * prm.ldy + f;
                         if (EPI == PAIR_F32) reinterpret_cast<float*>(prm.y)[at] = v[j];
                         else reinterpret_cast<__nv_bfloat16*>(prm.y)[at] = __float2bfloat16_rn(output_act_f32(prm.gate_act, v[j]));
@@ -286,19 +322,20 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     if (warp == 1) tmem_dealloc_pair(tmem_base, 512);
 }
 
-template <int EPI>
-int launch(const CUtensorMap& map_w, const CUtensorMap& map_x, const PairParams& prm, cudaStream_t stream) {
-    auto kernel = gemm_pair_kernel<EPI>;
+template <int EPI, int BN, bool GROUPED>
+int launch(const CUtensorMap& map_w, const CUtensorMap& map_x, const PairParams& prm, long most_tiles, cudaStream_t stream) {
+    auto kernel = gemm_pair_kernel<EPI, BN, GROUPED>;
+    constexpr int SMEM = PairTile<BN>::smem_bytes(EPI == PAIR_SWIGLU_BF16);
     static bool configured = false;
     if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes(EPI));
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
         if (e != cudaSuccess) return (int)e;
         configured = true;
     }
     cudaLaunchConfig_t config = {};
-    config.gridDim = dim3(2 * (prm.tiles < SM_PAIRS ? prm.tiles : SM_PAIRS), 1, 1);
+    config.gridDim = dim3(2 * (unsigned)(most_tiles < SM_PAIRS ? most_tiles : SM_PAIRS), 1, 1);
     config.blockDim = dim3(THREADS);
-    config.dynamicSmemBytes = smem_bytes(EPI);
+    config.dynamicSmemBytes = SMEM;
     config.stream = stream;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -338,19 +375,63 @@ FWB_API int fwb_gemm_tcgen05_pair(const void* X, const void* W, void* Y, int M, 
     prm.up_row_offset = up_row_offset;
     prm.gate_act = gate_act;
     prm.gate_limit = gate_limit;
-    prm.token_tiles = (M + BN - 1) / BN;
     prm.status = status_word();
+    prm.group_tiles = prm.group_offsets = nullptr;
+    prm.group_w_rows = 0;
     const int features = gated ? BM : 2 * BM;            // of a tile
-    const long tiles = (long)prm.token_tiles * ((N + features - 1) / features);
+    prm.feature_tiles = (N + features - 1) / features;
+    // 128-token tiles where 256 would leave half of the pairs without one (1,024 features at 2,048 tokens)
+    const bool narrow = (long)prm.feature_tiles * ((M + 255) / 256) * 2 <= SM_PAIRS;
+    const int bn = narrow ? 128 : 256;
+    prm.token_tiles = (M + bn - 1) / bn;
+    const long tiles = (long)prm.token_tiles * prm.feature_tiles;
     if (tiles > 1073741823L) return FWB_TOO_LARGE;
-    prm.tiles = (int)tiles;
     CUtensorMap map_w, map_x;
     if (!make_map(&map_w, W, w_rows, K, gated ? BM / 2 : BM)) return FWB_UNSUPPORTED;
-    if (!make_map(&map_x, X, M, K, HALF_N)) return FWB_UNSUPPORTED;
+    if (!make_map(&map_x, X, M, K, bn / 2)) return FWB_UNSUPPORTED;
     switch (epilogue) {
-        case PAIR_F32: return launch<PAIR_F32>(map_w, map_x, prm, stream);
-        case PAIR_BF16: return launch<PAIR_BF16>(map_w, map_x, prm, stream);
-        case PAIR_SWIGLU_BF16: return launch<PAIR_SWIGLU_BF16>(map_w, map_x, prm, stream);
+        case PAIR_F32:
+            return narrow ? launch<PAIR_F32, 128, false>(map_w, map_x, prm, tiles, stream)
+                          : launch<PAIR_F32, 256, false>(map_w, map_x, prm, tiles, stream);
+        case PAIR_BF16:
+            return narrow ? launch<PAIR_BF16, 128, false>(map_w, map_x, prm, tiles, stream)
+                          : launch<PAIR_BF16, 256, false>(map_w, map_x, prm, tiles, stream);
+        case PAIR_SWIGLU_BF16:
+            return narrow ? launch<PAIR_SWIGLU_BF16, 128, false>(map_w, map_x, prm, tiles, stream)
+                          : launch<PAIR_SWIGLU_BF16, 256, false>(map_w, map_x, prm, tiles, stream);
         default: return FWB_UNSUPPORTED;
+    }
+}
+
+// The grouped form of fwb_gemm_tcgen05_grouped (its arguments, checked there) for token tiles of 128 rows.
+int fwb::tc5::gemm_pair_grouped(const void* X, const void* W, void* Y, const int* offsets, const int* tiles, int max_tiles,
+                                int A, int N, int K, int n_groups, int group_w_rows, int ldy, int epilogue, int gate_act,
+                                int up_row_offset, float gate_limit, cudaStream_t stream) {
+    const bool gated = epilogue == PAIR_SWIGLU_BF16;
+    PairParams prm;
+    prm.y = Y;
+    prm.M = A;
+    prm.N = N;
+    prm.K = K;
+    prm.ldy = ldy;
+    prm.up_row_offset = up_row_offset;
+    prm.gate_act = gate_act;
+    prm.gate_limit = gate_limit;
+    prm.status = status_word();
+    prm.group_tiles = tiles;
+    prm.group_offsets = offsets;
+    prm.group_w_rows = group_w_rows;
+    const int features = gated ? BM : 2 * BM;
+    prm.feature_tiles = (N + features - 1) / features;
+    prm.token_tiles = max_tiles;
+    const long most = (long)max_tiles * prm.feature_tiles;
+    if (most > 1073741823L) return FWB_TOO_LARGE;
+    CUtensorMap map_w, map_x;
+    if (!make_map(&map_w, W, (long)n_groups * group_w_rows, K, gated ? BM / 2 : BM)) return FWB_UNSUPPORTED;
+    if (!make_map(&map_x, X, A, K, 64)) return FWB_UNSUPPORTED;
+    switch (epilogue) {
+        case PAIR_F32: return launch<PAIR_F32, 128, true>(map_w, map_x, prm, most, stream);
+        case PAIR_BF16: return launch<PAIR_BF16, 128, true>(map_w, map_x, prm, most, stream);
+        default: return launch<PAIR_SWIGLU_BF16, 128, true>(map_w, map_x, prm, most, stream);
     }
 }

@@ -19,6 +19,11 @@ constexpr unsigned WAIT_LIMIT = 1u << 22;
 // gave up.  (Host function; kernels get the pointer as a parameter.)  Null if it cannot be found.
 int* status_word();
 
+// The CTA-pair product over groups of rows with a matrix each, 128-row tiles (host function, gemm_tcgen05_pair.cu).
+int gemm_pair_grouped(const void* X, const void* W, void* Y, const int* offsets, const int* tiles, int max_tiles, int A,
+                      int N, int K, int n_groups, int group_w_rows, int ldy, int epilogue, int gate_act, int up_row_offset,
+                      float gate_limit, cudaStream_t stream);
+
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }

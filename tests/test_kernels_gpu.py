@@ -1148,6 +1148,38 @@ def test_tcgen05_cta_pair_swiglu(M, F, K):
     assert tc.status() == 0
 
 
+@pytest.mark.parametrize("epilogue", ["float32", "bfloat16", "gated"])
+@pytest.mark.parametrize("N,K", [(64, 40), (136, 264), (512, 128), (600, 1032)])
+def test_grouped_products_on_cta_pairs(N, K, epilogue):
+    """Rows sorted by group, 128-row tiles on persistent CTA pairs: empty groups, groups of one row, of a tile, of a
+    tile and a row, more tiles than pairs, and a list that is shorter than the grid was sized for."""
+    from flyweight_b200.kernels import lib, tensorcore as tc
+    from flyweight_b200.kernels.lib import ptr, stream
+    sizes = [1, 0, 128, 129, 127, 300, 0, 64, 2000, 5]
+    g = torch.Generator().manual_seed(N + K)
+    A, E, rows = sum(sizes), len(sizes), 2 * N if epilogue == "gated" else N
+    x = torch.randn(A, K, generator=g).bfloat16()
+    w = (torch.randn(E, rows, K, generator=g) / math.sqrt(K)).bfloat16()
+    starts = [sum(sizes[:i]) for i in range(E + 1)]
+    tiles = [(e, starts[e] + r) for e in range(E) for r in range(0, sizes[e], 128)]
+    most = A // 128 + E + 1
+    flat = torch.zeros(1 + 2 * most, dtype=torch.int32)
+    flat[0] = len(tiles)
+    flat[1:1 + 2 * len(tiles)] = torch.tensor(tiles, dtype=torch.int32).flatten()
+    want = torch.cat([x[starts[e]:starts[e + 1]].double() @ w[e].double().T for e in range(E)])
+    if epilogue == "gated":
+        want = torch.nn.functional.silu(want[:, :N]) * want[:, N:]
+    out_dtype = torch.float32 if epilogue == "float32" else torch.bfloat16
+    guard = torch.full((A + 2, N), 7.0, dtype=out_dtype, device=DEV)
+    code = {"float32": tc.EPI_F32, "bfloat16": tc.EPI_BF16, "gated": tc.EPI_SWIGLU_BF16}[epilogue]
+    x_d, w_d, o_d, t_d = dev(x), dev(w), torch.tensor(starts, dtype=torch.int32, device=DEV), flat.to(DEV)
+    lib.call("fwb_gemm_tcgen05_grouped", ptr(x_d), ptr(w_d), guard[1:].data_ptr(), ptr(o_d), ptr(t_d), most, 128, A, N, K, E,
+             rows, N, code, N if epilogue == "gated" else 0, lib.c_float(0.0), stream())
+    assert tc.status() == 0
+    close(guard[1:1 + A], want, 1e-5 if epilogue == "float32" else 2.0 ** -8, "grouped product")
+    assert (guard[0] == 7.0).all() and (guard[1 + A] == 7.0).all()
+
+
 @pytest.mark.parametrize("M,N,K", [(65, 2048, 8192), (128, 384, 4168), (300, 2048, 4096), (256, 2048, 8192),
                                    (700, 260, 4104), (200, 1000, 5000)])
 @pytest.mark.parametrize("out_dtype", [torch.float32, torch.bfloat16])
