@@ -40,7 +40,7 @@ constexpr int THREADS = 64 + 32 * EPI_WARPS;   // warp 0 producer, warp 1 MMA, t
 constexpr int SM_PAIRS = 148 / 2;
 constexpr int A_BYTES = BM * BK * 2;                    // 16 KiB: this CTA's 128 rows of A
 constexpr int TRADE_FLOATS = 8 * 32;                    // what a warp hands over of 16 columns
-enum PairEpilogue : int { PAIR_F32 = 0, PAIR_BF16 = 1, PAIR_SWIGLU_BF16 = 3 };
+enum PairEpilogue : int { PAIR_F32 = 0, PAIR_BF16 = 1, PAIR_ADD_F32 = 2, PAIR_SWIGLU_BF16 = 3 };
 // BN: tokens per tile, half of them in each CTA's shared memory
 template <int BN>
 struct PairTile {
@@ -300,13 +300,22 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
 #pragma unroll 1
                 for (int c0 = 0; c0 < PER_GROUP && ready; c0 += 16) {
                     float v[16];
+                    float sum[EPI == PAIR_ADD_F32 ? 16 : 1];
+                    if constexpr (EPI == PAIR_ADD_F32) {          // Y += the product: asked for in front of the accumulator
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) {
+                            const int t = tok0 + c0 + j;
+                            sum[j] = t < m_end && f < prm.N ? reinterpret_cast<const float*>(prm.y)[(size_t)t * prm.ldy + f] : 0.0f;
+                        }
+                    }
                     tmem_ld16(from + c0, v);
 #pragma unroll
                     for (int j = 0; j < 16; ++j) {
                         const int t = tok0 + c0 + j;
                         if (t >= m_end || f >= prm.N) continue;
                         const size_t at = (size_t)t * prm.ldy + f;
-                        if (EPI == PAIR_F32) reinterpret_cast<float*>(prm.y)[at] = v[j];
+                        if (EPI == PAIR_ADD_F32) reinterpret_cast<float*>(prm.y)[at] = v[j] + sum[EPI == PAIR_ADD_F32 ? j : 0];
+                        else if (EPI == PAIR_F32) reinterpret_cast<float*>(prm.y)[at] = v[j];
                         else reinterpret_cast<__nv_bfloat16*>(prm.y)[at] = __float2bfloat16_rn(output_act_f32(prm.gate_act, v[j]));
                     }
                 }
@@ -352,8 +361,8 @@ int launch(const CUtensorMap& map_w, const CUtensorMap& map_x, const PairParams&
 
 }  // namespace
 
-// X: [M][K] bf16, W: [w_rows][K] bf16, Y: [M][ldy] fp32 (epilogue 0) or bf16 (1, 3).
-// epilogue: 0 = fp32, 1 = bf16 (an output activation in the bits above), 3 = SwiGLU (N = F, up rows at
+// X: [M][K] bf16, W: [w_rows][K] bf16, Y: [M][ldy] fp32 (epilogues 0, 2) or bf16 (1, 3).
+// epilogue: 0 = fp32, 1 = bf16 (an output activation in the bits above), 2 = fp32, Y += the product, 3 = SwiGLU (N = F, up rows at
 // up_row_offset; the gate's activation in the bits above, its parameter in gate_limit).
 // K % 8 == 0, bases 16-byte aligned.
 FWB_API int fwb_gemm_tcgen05_pair(const void* X, const void* W, void* Y, int M, int N, int K, int w_rows,
@@ -396,6 +405,9 @@ FWB_API int fwb_gemm_tcgen05_pair(const void* X, const void* W, void* Y, int M, 
         case PAIR_BF16:
             return narrow ? launch<PAIR_BF16, 128, false>(map_w, map_x, prm, tiles, stream)
                           : launch<PAIR_BF16, 256, false>(map_w, map_x, prm, tiles, stream);
+        case PAIR_ADD_F32:
+            return narrow ? launch<PAIR_ADD_F32, 128, false>(map_w, map_x, prm, tiles, stream)
+                          : launch<PAIR_ADD_F32, 256, false>(map_w, map_x, prm, tiles, stream);
         case PAIR_SWIGLU_BF16:
             return narrow ? launch<PAIR_SWIGLU_BF16, 128, false>(map_w, map_x, prm, tiles, stream)
                           : launch<PAIR_SWIGLU_BF16, 256, false>(map_w, map_x, prm, tiles, stream);

@@ -207,9 +207,14 @@ bool normed_accepts(int M, int K, const void* w, int accumulators, int N) {
     return ceil_div(K, 64) <= 8 * splits;
 }
 
+// (kernels/tensorcore.py: _pairs_add)
+bool pairs_add(int M, int N) {
+    return g_option[OPT_PAIRS] && M > (g_option[OPT_MID_SIZE_SPLIT] ? MID_TO : 128) && N >= 256;
+}
+
 bool adds_in_place(const void* x, const void* w, int M, int N, int K) {
-    return g_option[OPT_ADD_IN_PLACE] && (M >= FUSE_FROM_TOKENS || g_option[OPT_FUSE_ALWAYS] || rows_takes(M, N, K)) &&
-           tc_accepts(x, w, M, K) && M <= 128;
+    const bool small = M <= 128 && (M >= FUSE_FROM_TOKENS || g_option[OPT_FUSE_ALWAYS] || rows_takes(M, N, K));
+    return g_option[OPT_ADD_IN_PLACE] && (small || pairs_add(M, N)) && tc_accepts(x, w, M, K);
 }
 
 struct Launches {
@@ -233,6 +238,10 @@ void tc_gemm(Launches& L, const void* x, const void* w, void* out, int out_bf16,
     const int epilogue = addend ? EPI_ADD_F32 : (out_bf16 ? EPI_BF16 : EPI_F32);
     if (rows_takes(M, N, K)) {
         L.add(fwb_linear_rows(x, w, out, addend, M, N, K, N, N, epilogue, 0, 0.0f, stream));
+        return;
+    }
+    if (in_place && pairs_add(M, N)) {
+        L.add(fwb_gemm_tcgen05_pair(x, w, out, M, N, K, N, N, EPI_ADD_F32, 0, 0.0f, stream));
         return;
     }
     const bool pair_ok = g_option[OPT_PAIRS] && M > 128 && !addend && !in_place && N >= 256;
