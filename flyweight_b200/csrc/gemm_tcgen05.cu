@@ -90,7 +90,7 @@ struct Tile {
     static constexpr int DEFAULT_STAGES = MAX_STAGES > 6 ? 6 : MAX_STAGES;
     static constexpr int COLS = BN * NACC;                      // TMEM columns in use
     static constexpr int TMEM_COLS = COLS <= 32 ? 32 : (COLS <= 64 ? 64 : (COLS <= 128 ? 128 : (COLS <= 256 ? 256 : 512)));
-    static constexpr int PARTIAL_BYTES = (BN <= 64 || NACC == 1) ? COLS * BM * 4 : 0;   // fp32 partial tile for split-K
+    static constexpr int PARTIAL_BYTES = (BN <= 96 || NACC == 1) ? COLS * BM * 4 : 0;   // fp32 partial tile for split-K
     static constexpr int data_bytes(int stages) {
         return stages * STAGE_BYTES > PARTIAL_BYTES ? stages * STAGE_BYTES : PARTIAL_BYTES;
     }
@@ -560,7 +560,8 @@ FWB_API int fwb_gemm_tcgen05(const void* X, const void* W, void* Y, const float*
     if (epilogue != EPI_SWIGLU_BF16 && w_rows < N) return FWB_BAD_ARGUMENT;
     if (splits < 1 || splits > 8) return FWB_BAD_ARGUMENT;
     int bn = M <= 16 ? 16 : (M <= 32 ? 32 : (M <= 64 ? 64 : (M <= 128 ? 128 : 256)));
-    if (tile_tokens == 16 || tile_tokens == 32 || tile_tokens == 64 || tile_tokens == 128 || tile_tokens == 256) {
+    if (tile_tokens == 16 || tile_tokens == 32 || tile_tokens == 64 || tile_tokens == 96 || tile_tokens == 128 ||
+        tile_tokens == 256) {
         if (tile_tokens < bn) bn = tile_tokens;                            // a smaller tile: more CTAs
     } else if (tile_tokens != 0) {
         return FWB_BAD_ARGUMENT;
@@ -609,6 +610,7 @@ FWB_API int fwb_gemm_tcgen05(const void* X, const void* W, void* Y, const float*
         case 16: return launch_epi<16>(epilogue, map_w, map_x, prm, splits, stream);
         case 32: return launch_epi<32>(epilogue, map_w, map_x, prm, splits, stream);
         case 64: return launch_epi<64>(epilogue, map_w, map_x, prm, splits, stream);
+        case 96: return launch_epi<96>(epilogue, map_w, map_x, prm, splits, stream);
         case 128: return launch_epi<128>(epilogue, map_w, map_x, prm, splits, stream);
         default: return launch_epi<256>(epilogue, map_w, map_x, prm, splits, stream);
     }

@@ -95,7 +95,7 @@ enum Option {
     OPT_MID_SIZE_SPLIT = 3,    // 128-token tiles with a split K for narrow products with a long K
     OPT_FUSE_NORM = 4,         // norms folded into the product that follows
     OPT_ADD_IN_PLACE = 5,      // residual sums in the product's epilogue
-    OPT_FUSE_ALWAYS = 6,       // ... at every decode-sized token count (default: from 16 tokens)
+    OPT_FUSE_ALWAYS = 6,       // norms in tcgen05 products too, and both at every decode-sized token count
     OPT_ATTENTION_MMA = 7,     // tensor-core attention kernels at all
     OPT_FORCE_TILED = 8,       // single decode tokens through the tiled attention kernel
     OPT_ATTENTION_TCGEN05 = 9, // prompt portions through the tcgen05 attention kernel
@@ -146,6 +146,28 @@ int pick_splits(int M, int N, int K) {
     if (g_option[OPT_FORCED_SPLITS] > 0) return M <= 64 ? g_option[OPT_FORCED_SPLITS] : 1;
     if (M > 64) return 1;
     return splits_for(M, N, K, 1);
+}
+
+// 33 to 128 tokens, two rings of weights an SM (kernels/tensorcore.py: two_rings).
+bool two_rings(int M, int N, int K, int accumulators, int& tile, int& splits, int& stages) {
+    if (g_option[OPT_FORCED_SPLITS] > 0 || M <= 32 || M > 128) return false;
+    const int tiles = ceil_div(N, 128), k_blocks = ceil_div(K, 64);
+    if (accumulators == 2) {
+        const int t = M <= 64 ? (k_blocks >= 32 ? 64 : 32) : 96;
+        if ((M > 64 && k_blocks < 32) || M > 96 || k_blocks < 16 || tiles * ceil_div(M, t) * 4 > 2 * SM_COUNT) return false;
+        tile = t, splits = 4, stages = 2;
+        return true;
+    }
+    if (M <= 64 || !g_option[OPT_MID_SIZE_SPLIT]) return false;
+    if (k_blocks >= 64 && tiles * 2 * 8 <= 2 * SM_COUNT) {
+        tile = 64, splits = 8, stages = 4;
+        return true;
+    }
+    if (k_blocks >= 16 && tiles >= 40 && tiles <= SM_COUNT / 2) {
+        tile = M <= 96 ? 96 : 64, splits = 4, stages = 3;
+        return true;
+    }
+    return false;
 }
 
 // 65 to 512 tokens: the cost model of kernels/tensorcore.py (mid_size_choice), in hundredths of a
@@ -201,7 +223,7 @@ bool rows_takes_normed(int M, int N, int K) { return M <= 8 && K <= 1024 && rows
 bool normed_accepts(int M, int K, const void* w, int accumulators, int N) {
     if (!(g_option[OPT_TENSORCORE] && g_option[OPT_FUSE_NORM]) || M > 64 || K % 8 || !aligned16(w)) return false;
     if (rows_takes(M, accumulators * N, K)) return rows_takes_normed(M, accumulators * N, K);
-    if (M < FUSE_FROM_TOKENS && !g_option[OPT_FUSE_ALWAYS]) return false;
+    if (!g_option[OPT_FUSE_ALWAYS]) return false;
     const int splits = g_option[OPT_FORCED_SPLITS] > 0 ? g_option[OPT_FORCED_SPLITS]
                                                         : splits_for(M, N, K, accumulators);
     return ceil_div(K, 64) <= 8 * splits;
@@ -247,7 +269,8 @@ void tc_gemm(Launches& L, const void* x, const void* w, void* out, int out_bf16,
     const bool pair_ok = g_option[OPT_PAIRS] && M > 128 && !addend && !in_place && N >= 256;
     int splits = 0, stages = 0, tile_tokens = 0;
     bool pair = pair_ok;
-    if (g_option[OPT_MID_SIZE_SPLIT] && M >= MID_FROM && M <= MID_TO)
+    if (two_rings(M, N, K, 1, tile_tokens, splits, stages)) pair = false;
+    else if (g_option[OPT_MID_SIZE_SPLIT] && M >= MID_FROM && M <= MID_TO)
         pair = mid_size_choice(M, N, K, 1, pair_ok, tile_tokens, splits);
     if (pair) {
         L.add(fwb_gemm_tcgen05_pair(x, w, out, M, N, K, N, N, epilogue, 0, 0.0f, stream));
@@ -268,14 +291,15 @@ void tc_swiglu(Launches& L, const void* x, const void* w, void* out, int M, int 
         L.add(fwb_linear_rows(x, w, out, nullptr, M, F, K, 2 * F, F, EPI_SWIGLU_BF16, F, 0.0f, stream));
         return;
     }
-    if (M <= 64) {
+    const bool rings = two_rings(M, F, K, 2, tile_tokens, splits, stages);
+    if (!rings && M <= 64) {
         splits = g_option[OPT_FORCED_SPLITS] > 0 ? g_option[OPT_FORCED_SPLITS] : splits_for(M, F, K, 2);
         stages = ring_depth(M, F, splits, 2);
         tile_tokens = decode_tile(M, F);
     }
-    const bool mid = g_option[OPT_MID_SIZE_SPLIT] && M >= MID_FROM && M <= MID_TO;
+    const bool mid = !rings && g_option[OPT_MID_SIZE_SPLIT] && M >= MID_FROM && M <= MID_TO;
     if (mid) mid_size_choice(M, F, K, 2, false, tile_tokens, splits);
-    else if (g_option[OPT_PAIRS] && M > 128 && splits == 1) {
+    else if (!rings && g_option[OPT_PAIRS] && M > 128 && splits == 1) {
         L.add(fwb_gemm_tcgen05_pair(x, w, out, M, F, K, 2 * F, F, EPI_SWIGLU_BF16, F, 0.0f, stream));
         return;
     }

@@ -161,6 +161,29 @@ def _splits_for(M: int, N: int, K: int, accumulators: int) -> int:
     return splits
 
 
+def two_rings(M: int, N: int, K: int, accumulators: int):
+    """33 to 128 tokens, matrices that are still read like a decode step's: (token tile, slices of K, stages) with two
+    CTAs, so two rings of weights, on an SM -- one leaves HBM waiting for its latency -- or None for the general rules.
+    Measured on B200 (us, the general rule's choice and this one): gated 8192 x 2048 at 64 tokens 23.9 and 20.1, at 77
+    23.9 and 22.1; gated 4608 x 1024 at 64 14.8 and 11.3; 2048 x 8192 at 77 17.7 and 13.8, at 128 18.2 and 14.0;
+    6144 x 2048 at 77 13.6 and 11.9, at 128 14.2 and 12.7.  csrc/plan.cu has the same rule."""
+    if _forced_splits is not None or M <= 32 or M > 128:
+        return None
+    tiles, k_blocks = -(-N // 128), -(-K // 64)
+    if accumulators == 2:
+        tile = (64 if k_blocks >= 32 else 32) if M <= 64 else 96
+        if (M > 64 and k_blocks < 32) or M > 96 or k_blocks < 16 or tiles * -(-M // tile) * 4 > 2 * SM_COUNT:
+            return None
+        return tile, 4, 2
+    if M <= 64 or not _mid_size_split:
+        return None
+    if k_blocks >= 64 and tiles * 2 * 8 <= 2 * SM_COUNT:
+        return 64, 8, 4
+    if k_blocks >= 16 and 40 <= tiles <= SM_COUNT // 2:
+        return (96 if M <= 96 else 64), 4, 3
+    return None
+
+
 # ---- 65 to 512 tokens: which tile, how many slices of K, or CTA pairs ----------------------
 # Between decode-sized steps (a weight streamer on every SM) and prompt-sized ones (256-token
 # tiles that fill the GPU) a product has few output tiles, and a CTA's walk over K is bound by
@@ -254,7 +277,10 @@ def gemm(x, w, out_dtype, addend=None, splits=None, stages=0, tile_tokens=0, wid
         lib.call("fwb_gemm_tcgen05_pair", ptr(x), ptr(w), ptr(out), M, N, K, N, N, EPI_ADD_F32, 0, lib.c_float(0.0),
                  stream(), tag=f"{N}x{K} added")
         return out
-    if free_choice and _mid_size_split and MID_FROM <= M <= MID_TO:
+    rings = two_rings(M, N, K, 1) if free_choice else None
+    if rings:
+        tile_tokens, splits, stages = rings
+    elif free_choice and _mid_size_split and MID_FROM <= M <= MID_TO:
         kind, tile_tokens, splits = mid_size_choice(M, N, K, 1, pair_ok)
         if kind == "pair":
             return gemm_pair(x, w, out_dtype, activation=activation)
@@ -357,6 +383,10 @@ def swiglu_gate_up(x, w_gate_up, splits=None, stages=0, tile_tokens=0, activatio
         if len(tuned) > 2:
             tile_tokens = tile_tokens or tuned[2]
     free_choice = splits is None and not stages and not tile_tokens
+    rings = two_rings(M, F, K, 2) if free_choice else None
+    if rings:
+        tile_tokens, splits, stages = rings
+        free_choice = False
     if splits is None:
         splits = (_forced_splits if _forced_splits is not None else _splits_for(M, F, K, 2)) if M <= 64 else 1
     if M <= 64:
@@ -395,10 +425,11 @@ def _wave_cut(M: int, F: int) -> int:
 _fuse_norm = True
 _add_in_place = True
 _fuse_always = False
-# Measured inside the decode step of LFM2-1.2B on B200: folding the norms into the products
-# (and the residual sums into the epilogues) takes 2-3 % off the step from 16 tokens on; below
-# that the separate norm kernel is faster, because the next product's first weight tiles are
-# fetched while it runs.
+# Residual sums go into the products' epilogues from 16 tokens on (2-3 % of the decode step of LFM2-1.2B); below that
+# only where the weight reader runs the product.  Norms are not folded into the tcgen05 products any more unless
+# ``fuse_always`` asks for it: with the activations of a whole row to build, the product waits longer than the norm's
+# own kernel takes (us, folded and apart: 6144 x 2048 at 64 tokens 20.3 and 11.3, at 16 13.2 and 8.6; 2048 x 2048 at 64
+# 8.8 and 7.7; gated 8192 x 2048 at 24 17.1 and 16.8).
 FUSE_FROM_TOKENS = 16
 
 
@@ -427,7 +458,7 @@ def normed_accepts(M: int, K: int, w, accumulators: int, N: int) -> bool:
         return False
     if _rows_takes(M, accumulators * N, K):
         return _rows_takes_normed(M, accumulators * N, K)
-    if M < FUSE_FROM_TOKENS and not _fuse_always:
+    if not _fuse_always:
         return False
     splits = _forced_splits if _forced_splits is not None else _splits_for(M, N, K, accumulators)
     return -(-K // 64) <= 8 * splits

@@ -1180,6 +1180,33 @@ def test_grouped_products_on_cta_pairs(N, K, epilogue):
     assert (guard[0] == 7.0).all() and (guard[1 + A] == 7.0).all()
 
 
+@pytest.mark.parametrize("M,N,K", [(65, 256, 1032), (96, 384, 264), (97, 1000, 512), (200, 130, 2048)])
+@pytest.mark.parametrize("splits", [1, 2, 4])
+def test_token_tiles_of_96(M, N, K, splits):
+    """One and two accumulators over 96 tokens, slices of K merged in a cluster, two stages and three."""
+    from flyweight_b200.kernels import tensorcore as tc
+    g = torch.Generator().manual_seed(M + N)
+    x = torch.randn(M, K, generator=g).bfloat16()
+    w = (torch.randn(2 * N, K, generator=g) / math.sqrt(K)).bfloat16()
+    want = x.double() @ w.double().T
+    close(tc.gemm(dev(x), dev(w), torch.float32, splits=splits, stages=3, tile_tokens=96), want, 1e-5, "96 tokens")
+    close(tc.swiglu_gate_up(dev(x), dev(w), splits=splits, stages=2, tile_tokens=96),
+          torch.nn.functional.silu(want[:, :N]) * want[:, N:], 2.0 ** -8, "96 tokens, gated")
+    assert tc.status() == 0
+
+
+@pytest.mark.parametrize("M,N,K", [(513, 256, 64), (600, 1000, 264), (2048, 2048, 128)])
+def test_cta_pairs_add_into_their_output(M, N, K):
+    from flyweight_b200.kernels import tensorcore as tc
+    g = torch.Generator().manual_seed(M + N)
+    x, w = dev(torch.randn(M, K, generator=g).bfloat16()), dev((torch.randn(N, K, generator=g) / math.sqrt(K)).bfloat16())
+    total = dev(torch.randn(M, N, generator=g))
+    want = total + tc.gemm(x, w, torch.float32)
+    assert tc.adds_in_place(x, w, total)
+    tc.gemm(x, w, torch.float32, addend=total, out=total)
+    assert torch.equal(total, want) and tc.status() == 0
+
+
 @pytest.mark.parametrize("M,N,K", [(65, 2048, 8192), (128, 384, 4168), (300, 2048, 4096), (256, 2048, 8192),
                                    (700, 260, 4104), (200, 1000, 5000)])
 @pytest.mark.parametrize("out_dtype", [torch.float32, torch.bfloat16])
