@@ -148,22 +148,26 @@ int pick_splits(int M, int N, int K) {
     return splits_for(M, N, K, 1);
 }
 
-// 33 to 128 tokens, two rings of weights an SM (kernels/tensorcore.py: two_rings).
+constexpr int MID_FROM = 65, MID_TO = 512;       // between decode steps and prompts
+
+// 33 to 512 tokens, two rings of weights an SM (kernels/tensorcore.py: two_rings).
 bool two_rings(int M, int N, int K, int accumulators, int& tile, int& splits, int& stages) {
-    if (g_option[OPT_FORCED_SPLITS] > 0 || M <= 32 || M > 128) return false;
-    const int tiles = ceil_div(N, 128), k_blocks = ceil_div(K, 64);
+    if (g_option[OPT_FORCED_SPLITS] > 0 || M <= 32 || M > MID_TO) return false;
+    const int tiles = ceil_div(N, 128), k_blocks = ceil_div(K, 64), most = 2 * SM_COUNT;
     if (accumulators == 2) {
         const int t = M <= 64 ? (k_blocks >= 32 ? 64 : 32) : 96;
-        if ((M > 64 && k_blocks < 32) || M > 96 || k_blocks < 16 || tiles * ceil_div(M, t) * 4 > 2 * SM_COUNT) return false;
+        if ((M > 64 && k_blocks < 32) || M > 96 || k_blocks < 16 || tiles * ceil_div(M, t) * 4 > most) return false;
         tile = t, splits = 4, stages = 2;
         return true;
     }
     if (M <= 64 || !g_option[OPT_MID_SIZE_SPLIT]) return false;
-    if (k_blocks >= 64 && tiles * 2 * 8 <= 2 * SM_COUNT) {
-        tile = 64, splits = 8, stages = 4;
-        return true;
-    }
-    if (k_blocks >= 16 && tiles >= 40 && tiles <= SM_COUNT / 2) {
+    if (k_blocks >= 64)
+        for (int t = 64; t <= 96; t += 32)
+            if (tiles * ceil_div(M, t) * 8 <= most) {
+                tile = t, splits = 8, stages = t == 64 ? 4 : 3;
+                return true;
+            }
+    if (M <= 128 && k_blocks >= 16 && tiles >= 40 && tiles <= SM_COUNT / 2) {
         tile = M <= 96 ? 96 : 64, splits = 4, stages = 3;
         return true;
     }
@@ -172,7 +176,6 @@ bool two_rings(int M, int N, int K, int accumulators, int& tile, int& splits, in
 
 // 65 to 512 tokens: the cost model of kernels/tensorcore.py (mid_size_choice), in hundredths of a
 // microsecond.  Returns true for CTA pairs, else sets the token tile and the slices of K.
-constexpr int MID_FROM = 65, MID_TO = 512;
 bool mid_size_choice(int M, int N, int K, int accumulators, bool pair_ok, int& tile_out, int& splits_out) {
     static const int tiles[3] = {64, 128, 256};
     static const int block_cost[2][3] = {{38, 38, 42}, {63, 58, 84}};
@@ -297,9 +300,10 @@ void tc_swiglu(Launches& L, const void* x, const void* w, void* out, int M, int 
         stages = ring_depth(M, F, splits, 2);
         tile_tokens = decode_tile(M, F);
     }
-    const bool mid = !rings && g_option[OPT_MID_SIZE_SPLIT] && M >= MID_FROM && M <= MID_TO;
-    if (mid) mid_size_choice(M, F, K, 2, false, tile_tokens, splits);
-    else if (!rings && g_option[OPT_PAIRS] && M > 128 && splits == 1) {
+    const bool pairs = !rings && g_option[OPT_PAIRS] && M > 128 && splits == 1;
+    if (!rings && !pairs && g_option[OPT_MID_SIZE_SPLIT] && M >= MID_FROM && M <= MID_TO)
+        mid_size_choice(M, F, K, 2, false, tile_tokens, splits);
+    else if (pairs) {
         L.add(fwb_gemm_tcgen05_pair(x, w, out, M, F, K, 2 * F, F, EPI_SWIGLU_BF16, F, 0.0f, stream));
         return;
     }

@@ -162,24 +162,27 @@ def _splits_for(M: int, N: int, K: int, accumulators: int) -> int:
 
 
 def two_rings(M: int, N: int, K: int, accumulators: int):
-    """33 to 128 tokens, matrices that are still read like a decode step's: (token tile, slices of K, stages) with two
+    """33 to 512 tokens, matrices that are still read like a decode step's: (token tile, slices of K, stages) with two
     CTAs, so two rings of weights, on an SM -- one leaves HBM waiting for its latency -- or None for the general rules.
     Measured on B200 (us, the general rule's choice and this one): gated 8192 x 2048 at 64 tokens 23.9 and 20.1, at 77
-    23.9 and 22.1; gated 4608 x 1024 at 64 14.8 and 11.3; 2048 x 8192 at 77 17.7 and 13.8, at 128 18.2 and 14.0;
-    6144 x 2048 at 77 13.6 and 11.9, at 128 14.2 and 12.7.  csrc/plan.cu has the same rule."""
-    if _forced_splits is not None or M <= 32 or M > 128:
+    23.9 and 22.1; gated 4608 x 1024 at 64 14.8 and 11.3; 2048 x 8192 at 77 17.7 and 13.8, at 160 19.5 and 15.9;
+    1024 x 4608 at 256 13.2 and 10.9; 6144 x 2048 at 77 13.6 and 11.9, at 128 14.2 and 12.7.  csrc/plan.cu has the
+    same rule."""
+    if _forced_splits is not None or M <= 32 or M > MID_TO:
         return None
-    tiles, k_blocks = -(-N // 128), -(-K // 64)
+    tiles, k_blocks, most = -(-N // 128), -(-K // 64), 2 * SM_COUNT
     if accumulators == 2:
         tile = (64 if k_blocks >= 32 else 32) if M <= 64 else 96
-        if (M > 64 and k_blocks < 32) or M > 96 or k_blocks < 16 or tiles * -(-M // tile) * 4 > 2 * SM_COUNT:
+        if (M > 64 and k_blocks < 32) or M > 96 or k_blocks < 16 or tiles * -(-M // tile) * 4 > most:
             return None
         return tile, 4, 2
     if M <= 64 or not _mid_size_split:
         return None
-    if k_blocks >= 64 and tiles * 2 * 8 <= 2 * SM_COUNT:
-        return 64, 8, 4
-    if k_blocks >= 16 and 40 <= tiles <= SM_COUNT // 2:
+    if k_blocks >= 64:
+        for tile, stages in ((64, 4), (96, 3)):
+            if tiles * -(-M // tile) * 8 <= most:
+                return tile, 8, stages
+    if M <= 128 and k_blocks >= 16 and 40 <= tiles <= SM_COUNT // 2:
         return (96 if M <= 96 else 64), 4, 3
     return None
 
@@ -392,10 +395,10 @@ def swiglu_gate_up(x, w_gate_up, splits=None, stages=0, tile_tokens=0, activatio
     if M <= 64:
         stages = stages or _ring_depth(M, F, splits, 2)
         tile_tokens = tile_tokens or _decode_tile(M, F)
-    mid = free_choice and _mid_size_split and MID_FROM <= M <= MID_TO
-    if mid:
+    pairs = free_choice and _use_pairs and M > 128 and splits == 1
+    if free_choice and not pairs and _mid_size_split and MID_FROM <= M <= MID_TO:
         _, tile_tokens, splits = mid_size_choice(M, F, K, 2, False)
-    if free_choice and not mid and _use_pairs and M > 128 and splits == 1:
+    if pairs:
         lib.call("fwb_gemm_tcgen05_pair", ptr(x), ptr(w_gate_up), ptr(out), M, F, K, F2, F, gated, F,
                  lib.c_float(limit), stream(), tag=f"swiglu {F}x{K}")
         return out
