@@ -9,8 +9,8 @@
 // itself) and silu; q and k are then made unit vectors per head (x / sqrt(sum x^2 + 1e-6)); query
 // head h uses q/k head h / (H / G).  beta = sigmoid(b), g = exp(-exp(A_log) softplus(a + dt_bias)).
 //
-// Three kernels (everything fp32):
-//   delta_prepare   one block per token: convolution + silu, unit vectors, beta and g
+// Kernels (everything fp32; segments of many tokens also take delta_chunk and delta_runs, further down):
+//   delta_prepare   one block per token (or per four): convolution + silu, unit vectors, beta and g
 //                   -> r[t] = [ q^: G d | k^: G d | v: H e | beta: H | g: H | q^.k^: G ]
 //   delta_scan      one block per (16 or 32 columns of S, head, segment): the recurrence over the
 //                   segment's tokens in order.  A column of S evolves independently of the others;
@@ -20,8 +20,9 @@
 //                   step (behind delta_prepare, which reads the old ones).
 //   gated_head_norm out[t][h] = weight * o / sqrt(mean(o^2) + eps) * silu(gate)
 // A request's slot is [ S: H d e | conv inputs: C (L-1) ] fp32, zero when the request starts.  A
-// token's result depends on its request's earlier tokens only through that slot, and every sum runs
-// in an order fixed by the sizes, so it does not depend on how the sequence was cut into steps.
+// token's result depends on its request's earlier tokens only through that slot.  In the scan every sum runs in an
+// order fixed by the sizes, so it does not depend on how the sequence was cut into steps; the chunks of a long
+// segment start where the segment does, so another cut is another order of the same fp32 sums.
 #include "common.cuh"
 
 using namespace fwb;

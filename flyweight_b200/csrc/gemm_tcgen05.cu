@@ -6,7 +6,7 @@
 // a CTA owns 128 features x BN tokens, the accumulator D[128 x BN] lives in tensor memory
 // with one feature per TMEM lane and one token per column.  With BN = 16..64 the kernel is a
 // weight streamer for decode (every weight byte is read once, the few tokens ride along);
-// with BN = 256 it is the ordinary 128x256 tile for prefill.  One kernel, five BN.
+// with BN = 256 it is the ordinary 128x256 tile for prefill.  One kernel, six BN.
 //
 // Roles inside a CTA (192 or 576 threads): warp 0 = TMA producer (one elected lane issues
 // cp.async.bulk.tensor loads of 128B-swizzled [rows x 64] boxes into a ring of stages),
@@ -542,7 +542,7 @@ int launch_epi(int epi, const CUtensorMap& map_w, const CUtensorMap& map_x, cons
 
 // X: [M][K] bf16; W: [rows][K] bf16 (rows = N, or >= up_row_offset + N for SwiGLU);
 // Y: [M][ldy] (fp32 for epilogues 0 and 2, bf16 for 1 and 3).  `splits` (1..8) CTAs share the
-// K range of a tile as a cluster; with splits > 1 the token tile must be <= 128 wide (64 for SwiGLU).
+// K range of a tile as a cluster; with splits > 1 the token tile must be <= 128 wide (96 for SwiGLU).
 // `stages` sets the depth of the shared-memory ring (0: the default).  `tile_tokens` (0: by M)
 // may ask for a smaller token tile than M would pick (more CTAs); `wide` gives a CTA two feature tiles.
 // K must be a multiple of 8 (TMA strides are multiples of 16 bytes) and both base
