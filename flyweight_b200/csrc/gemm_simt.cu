@@ -77,34 +77,35 @@ gemm_simt_kernel(const TX* __restrict__ X, const TW* __restrict__ W, TY* __restr
 // Bound by the fp32 pipes from a few dozen rows on and by the weights' bytes below.  Both operands are
 // K-major, so they go to shared memory as they lie, by asynchronous 16-byte copies, three stages of
 // 64 k deep, and a thread reads four consecutive k of a row at once.  Rows are 68 floats apart, which
-// puts the eight rows that neighbouring lanes read on different banks.  Two k go through one packed
-// multiply-add (fma.rn.f32x2: two IEEE fp32 operations, half the issue slots), so an accumulator is a pair:
-// even k and odd k.  Four groups of 64 threads take 16 of the 64 k of every stage each: an output tile of
+// puts the eight rows that neighbouring lanes read on different banks.  An accumulator is a pair: even k and
+// odd k, plain multiply-adds (packed ones, fma.rn.f32x2, gave the same bits and took 147 us instead of 89 for
+// 201 x 1024 x 4608).  Four groups of 64 threads take 16 of the 64 k of every stage each: an output tile of
 // 64 x 32 keeps eight warps busy, and a 201 x 1024 product fills 128 SMs.
-// Measured on B200 (us; the kernel below this one, then this one): 201 x 9216 x 1024 289 -> 147,
-// 201 x 1024 x 4608 345 -> 147, 64 x 9216 x 1024 93 -> 38 (32 TFLOP/s), 8 x 1024 x 4608 314 -> 24,
+// Measured on B200 (us; the kernel below this one, then this one): 201 x 9216 x 1024 289 -> 121,
+// 201 x 1024 x 4608 345 -> 92, 64 x 9216 x 1024 93 -> 38 (32 TFLOP/s), 8 x 1024 x 4608 314 -> 24,
 // 1 x 9216 x 1024 83 -> 23; relative error against 64 bits 5.7e-7 -> 2.1e-7 at K = 1024.
 constexpr int FK = 64, FSTRIDE = FK + 4, FSTAGES = 3;
 
-__device__ __forceinline__ void fma_pair(unsigned long long& acc, unsigned long long a, unsigned long long b) {
-    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
-}
-__device__ __forceinline__ float pair_sum(unsigned long long v) {
-    return __uint_as_float((unsigned)v) + __uint_as_float((unsigned)(v >> 32));
+__device__ __forceinline__ void fma_four(float2& acc, const float4& a, const float4& b) {
+    acc.x = fmaf(a.x, b.x, acc.x);
+    acc.y = fmaf(a.y, b.y, acc.y);
+    acc.x = fmaf(a.z, b.z, acc.x);
+    acc.y = fmaf(a.w, b.w, acc.y);
 }
 
 template <int RM, int RN>
 constexpr int f32_smem_bytes() {
-    constexpr int ring = FSTAGES * 8 * (RM + RN) * FSTRIDE, partial = 3 * 64 * RM * RN;
+    constexpr int ring = FSTAGES * 8 * (RM + RN) * FSTRIDE, partial = 3 * 8 * RM * (8 * RN + 4);
     return (ring > partial ? ring : partial) * 4;
 }
 
 // A tile of 8 RM rows x 8 RN columns; a thread of a group owns rows (lane & 7) + 8 i and columns (id / 8) + 8 j.
-template <int RM, int RN>
-__global__ void __launch_bounds__(256)
+template <int RM, int RN, int PER_SM>
+__global__ void __launch_bounds__(256, PER_SM)
 gemm_f32_kernel(const float* __restrict__ X, const float* __restrict__ W, float* Y, const float* addend,
                 int M, int N, int K, int ldx, int ldy) {
     constexpr int BM = 8 * RM, BN = 8 * RN, STAGE = (BM + BN) * FSTRIDE;
+    constexpr int PROW = BN + 4;               // rows of a partial tile: a warp's 8 rows x 4 columns on 32 banks
     extern __shared__ __align__(16) float smem[];
     fwb::pdl_entry();
     const int tid = threadIdx.x, group = tid >> 6, id = tid & 63, tm = id & 7, tn = id >> 3;
@@ -118,6 +119,7 @@ gemm_f32_kernel(const float* __restrict__ X, const float* __restrict__ W, float*
 #pragma unroll
             for (int i = 0; i < (BM + BN) * (FK / 4); i += 256) {
                 const int piece = i + tid, row = piece >> 4, k = k0 + (piece & 15) * 4;
+                if ((BM + BN) * (FK / 4) % 256 != 0 && row >= BM + BN) break;
                 const bool is_x = row < BM;
                 const int at = is_x ? m0 + row : n0 + row - BM;
                 const bool in = k < K && at < (is_x ? M : N);       // K is a multiple of 4: a piece is whole or absent
@@ -129,11 +131,11 @@ gemm_f32_kernel(const float* __restrict__ X, const float* __restrict__ W, float*
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    unsigned long long acc[RM][RN];
+    float2 acc[RM][RN];
 #pragma unroll
     for (int i = 0; i < RM; ++i)
 #pragma unroll
-        for (int j = 0; j < RN; ++j) acc[i][j] = 0ull;
+        for (int j = 0; j < RN; ++j) acc[i][j] = make_float2(0.0f, 0.0f);
 #pragma unroll
     for (int s = 0; s < FSTAGES - 1; ++s) fetch(s);
     for (int c = 0; c < chunks; ++c) {
@@ -144,19 +146,15 @@ gemm_f32_kernel(const float* __restrict__ X, const float* __restrict__ W, float*
         const float* ws = smem + (c % FSTAGES) * STAGE + (BM + tn) * FSTRIDE + group * 16;
 #pragma unroll
         for (int k = 0; k < 16; k += 4) {
-            ulonglong2 a[RM], b[RN];
+            float4 a[RM], b[RN];
 #pragma unroll
-            for (int i = 0; i < RM; ++i) a[i] = *reinterpret_cast<const ulonglong2*>(xs + i * 8 * FSTRIDE + k);
+            for (int i = 0; i < RM; ++i) a[i] = *reinterpret_cast<const float4*>(xs + i * 8 * FSTRIDE + k);
 #pragma unroll
-            for (int j = 0; j < RN; ++j) b[j] = *reinterpret_cast<const ulonglong2*>(ws + j * 8 * FSTRIDE + k);
-#pragma unroll
-            for (int i = 0; i < RM; ++i)
-#pragma unroll
-                for (int j = 0; j < RN; ++j) fma_pair(acc[i][j], a[i].x, b[j].x);
+            for (int j = 0; j < RN; ++j) b[j] = *reinterpret_cast<const float4*>(ws + j * 8 * FSTRIDE + k);
 #pragma unroll
             for (int i = 0; i < RM; ++i)
 #pragma unroll
-                for (int j = 0; j < RN; ++j) fma_pair(acc[i][j], a[i].y, b[j].y);
+                for (int j = 0; j < RN; ++j) fma_four(acc[i][j], a[i], b[j]);
         }
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
@@ -165,7 +163,7 @@ gemm_f32_kernel(const float* __restrict__ X, const float* __restrict__ W, float*
 #pragma unroll
         for (int i = 0; i < RM; ++i)
 #pragma unroll
-            for (int j = 0; j < RN; ++j) smem[(group - 1) * BM * BN + (tm + 8 * i) * BN + tn + 8 * j] = pair_sum(acc[i][j]);
+            for (int j = 0; j < RN; ++j) smem[(group - 1) * BM * PROW + (tm + 8 * i) * PROW + tn + 8 * j] = acc[i][j].x + acc[i][j].y;
     }
     __syncthreads();
     if (group == 0) {
@@ -173,46 +171,63 @@ gemm_f32_kernel(const float* __restrict__ X, const float* __restrict__ W, float*
         for (int i = 0; i < RM; ++i)
 #pragma unroll
             for (int j = 0; j < RN; ++j) {
-                const int at = (tm + 8 * i) * BN + tn + 8 * j;
-                smem[at] = ((pair_sum(acc[i][j]) + smem[at]) + smem[BM * BN + at]) + smem[2 * BM * BN + at];
+                const int at = (tm + 8 * i) * PROW + tn + 8 * j;
+                smem[at] = (((acc[i][j].x + acc[i][j].y) + smem[at]) + smem[BM * PROW + at]) + smem[2 * BM * PROW + at];
             }
     }
     __syncthreads();
     for (int at = tid; at < BM * BN; at += 256) {
         const int m = m0 + at / BN, n = n0 + at % BN;
         if (m >= M || n >= N) continue;
-        float v = smem[at];
+        float v = smem[at / BN * PROW + at % BN];
         if (addend) v += addend[(size_t)m * ldy + n];
         Y[(size_t)m * ldy + n] = v;
     }
 }
 
-template <int RM, int RN>
+template <int RM, int RN, int PER_SM>
 int launch_f32(const float* X, const float* W, float* Y, const float* addend, int M, int N, int K, int ldx, int ldy,
                cudaStream_t stream) {
     static bool configured = false;
     if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_f32_kernel<RM, RN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        cudaError_t e = cudaFuncSetAttribute(gemm_f32_kernel<RM, RN, PER_SM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              f32_smem_bytes<RM, RN>());
         if (e != cudaSuccess) return (int)e;
         configured = true;
     }
     const dim3 grid((M + 8 * RM - 1) / (8 * RM), (N + 8 * RN - 1) / (8 * RN));
     if (grid.y > 65535) return FWB_TOO_LARGE;
-    fwb::pdl(gemm_f32_kernel<RM, RN>, grid, 256, f32_smem_bytes<RM, RN>(), stream)(X, W, Y, addend, M, N, K, ldx, ldy);
+    fwb::pdl(gemm_f32_kernel<RM, RN, PER_SM>, grid, 256, f32_smem_bytes<RM, RN>(), stream)(X, W, Y, addend, M, N, K, ldx, ldy);
     return fwb_launch_status();
 }
 
-// The tile: 16 or 32 rows for as few tokens; else the cheaper of 64 x 64 and 64 x 32 by rounds over the SMs
-// (a 64 x 32 tile takes about 0.6 of the other's time: fewer products an operand read).
+// The tile: 16 or 32 rows for as few tokens; else 40 to 64 rows by 64 or 32 columns, whichever takes the least time by
+// rounds over the SMs: 201 rows are four tiles of 56 or of 64.  A tile's time goes with its products and a constant
+// (64 x 64: 143 us for four rounds at K = 1,024; 64 x 32: 25 us for one, 60 us for three).
 int dispatch_f32(const float* X, const float* W, float* Y, const float* addend, int M, int N, int K, int ldx, int ldy,
                  cudaStream_t stream) {
-    if (M <= 16) return launch_f32<2, 2>(X, W, Y, addend, M, N, K, ldx, ldy, stream);
-    if (M <= 32) return launch_f32<4, 4>(X, W, Y, addend, M, N, K, ldx, ldy, stream);
-    const long rows = (M + 63) / 64;
-    const long square = (rows * ((N + 63) / 64) + 147) / 148, narrow = (rows * ((N + 31) / 32) + 147) / 148;
-    if (square * 10 <= narrow * 6) return launch_f32<8, 8>(X, W, Y, addend, M, N, K, ldx, ldy, stream);
-    return launch_f32<8, 4>(X, W, Y, addend, M, N, K, ldx, ldy, stream);
+    if (M <= 16) return launch_f32<2, 2, 2>(X, W, Y, addend, M, N, K, ldx, ldy, stream);
+    if (M <= 32) return launch_f32<4, 4, 2>(X, W, Y, addend, M, N, K, ldx, ldy, stream);
+    int rm = 8, rn = 8;
+    bool alone = true;                         // a tile has an SM to itself: all the registers a thread can use
+    long best = -1;
+    for (int r = 8; r >= 5; --r)
+        for (int c = 8; c >= 4; c -= 4) {
+            const long tiles = (long)((M + 8 * r - 1) / (8 * r)) * ((N + 8 * c - 1) / (8 * c));
+            const long cost = ((tiles + 147) / 148) * (r * c + 12);
+            if (best < 0 || cost < best) best = cost, rm = r, rn = c, alone = c == 8 || tiles <= 148;
+        }
+#define FWB_F32(RM)                                                                                        \
+    if (rm == RM)                                                                                          \
+        return rn == 8 ? launch_f32<RM, 8, 1>(X, W, Y, addend, M, N, K, ldx, ldy, stream)                  \
+               : alone ? launch_f32<RM, 4, 1>(X, W, Y, addend, M, N, K, ldx, ldy, stream)                  \
+                       : launch_f32<RM, 4, 2>(X, W, Y, addend, M, N, K, ldx, ldy, stream)
+    FWB_F32(8);
+    FWB_F32(7);
+    FWB_F32(6);
+    FWB_F32(5);
+#undef FWB_F32
+    return FWB_UNSUPPORTED;
 }
 
 template <typename TX, typename TW, typename TY>
