@@ -17,7 +17,8 @@ def delta_state_size(heads: int, kv_heads: int, dim: int, vdim: int, taps: int) 
 
 
 # From this many tokens of a step's longest segment on the recurrence runs in chunks of 32 tokens (head sizes 64 and
-# 128); shorter segments, decode steps above all, walk token by token.
+# 128); shorter segments, decode steps above all, walk token by token.  Measured on B200 (16 heads of 128, one segment, all
+# launches, us in chunks and by the scan): 8 tokens 30.9 and 31.5, 16 31.0 and 34.1, 32 31.3 and 40.8, 64 34.6 and 53.2.
 CHUNKS_FROM = 16
 _CHUNK_TOKENS, _CHUNK_FLOATS = 32, 2 * 32 * 36
 
