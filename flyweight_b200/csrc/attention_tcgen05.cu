@@ -417,7 +417,7 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k,
                 if (seen < KEYS) {
                     // only the last tile: clear the V rows beyond it (whole 128-byte rows of every box)
                     const int u = u0 + j + LEAD, s = u % L::STAGES;   // the step that brought this V tile
-                    ok = mbar_wait(&full[s], (u / L::STAGES) & 1, abort_flag, 17, prm.status);
+                    ok = __all_sync(0xffffffffu, mbar_wait(&full[s], (u / L::STAGES) & 1, abort_flag, 17, prm.status));
                     uint8_t* v_tile = v_s + (size_t)s * L::KV_BYTES;
                     const int chunks = (KEYS - seen) * 8;
                     for (int b = 0; b < L::BOXES; ++b)

@@ -186,7 +186,7 @@ __device__ __forceinline__ void produce_normed_tiles(const Params& prm, uint8_t*
             if (i >= STAGES) {
                 // the slot comes free only after tiles already written here have been announced
                 announce(i);
-                ok = mbar_wait(&empty_bar[s], ((i / STAGES) - 1) & 1, abort_flag, 4, prm.status);
+                ok = __all_sync(0xffffffffu, mbar_wait(&empty_bar[s], ((i / STAGES) - 1) & 1, abort_flag, 4, prm.status));
             }
             if (!ok) break;
             uint8_t* b_tile = tiles + (size_t)s * T::STAGE_BYTES + NACC * T::A_BYTES;

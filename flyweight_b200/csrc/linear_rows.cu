@@ -117,12 +117,15 @@ __global__ void __launch_bounds__(THREADS, 2) linear_rows_kernel(const RowsParam
     }
     __syncthreads();
 
+    int asked = 0;                                     // the weight warp's copies into the ring so far, eight rows each
     if (warp == WARPS) {
         // ---- weights
         int slot = 0, group = 0, k = 0;
         uint32_t parity = 1;                           // of the empty barrier: the ring's first round waits for nothing
-        for (int step = 0; step < steps; ++step) {
-            if (step >= slots && !mbar_wait(&empty_bar[slot], parity, abort_flag, 21, prm.status)) break;
+        for (; asked < steps; ++asked) {
+            // (the lanes poll each for itself and go on together: a vote, or one that gave up would leave the others behind)
+            if (asked >= slots && !__all_sync(0xffffffffu, mbar_wait(&empty_bar[slot], parity, abort_flag, 21, prm.status)))
+                break;
             const uint32_t bytes = (uint32_t)(K - k < CHUNK ? K - k : CHUNK) * 2;
             if (lane == 0) mbar_expect_tx(&full_bar[slot], 8 * bytes);
             __syncwarp();
@@ -136,7 +139,6 @@ __global__ void __launch_bounds__(THREADS, 2) linear_rows_kernel(const RowsParam
             if (++group == groups) group = 0, k += CHUNK;
             if (++slot == slots) slot = 0, parity ^= 1;
         }
-        if (*abort_flag) __nanosleep(1000000);         // gave up: the copies in flight end before the memory is freed
     }
     if (NORMED && warp < WARPS) {
         // the norm's weight, a warp's own k only, while the kernel before this one still runs
@@ -213,7 +215,7 @@ __global__ void __launch_bounds__(THREADS, 2) linear_rows_kernel(const RowsParam
             if (chunk + 1 < chunks) fetch_rows(x_k);
             const int live = K - w_k - warp * KBLK * 32 - t * 8;      // this lane's k below K, from its first one on
             for (int group = 0; group < groups; ++group) {
-                ok = mbar_wait(&full_bar[slot], parity, abort_flag, 22, prm.status);
+                ok = __all_sync(0xffffffffu, mbar_wait(&full_bar[slot], parity, abort_flag, 22, prm.status));
                 if (!ok) break;
                 const uint8_t* from = ring + slot * SLOT + g * W_STRIDE + (warp * KBLK * 32 + t * 8) * 2;
                 uint4 wv[KBLK];
@@ -262,7 +264,15 @@ __global__ void __launch_bounds__(THREADS, 2) linear_rows_kernel(const RowsParam
         }
     }
     __syncthreads();
-    if (*abort_flag) return;
+    if (*abort_flag) {
+        // somebody gave up: the copies still in flight land before the block's shared memory is another's.  The slot's
+        // last phase, for each slot, with a limit of its own (the abort flag would end mbar_wait at once)
+        if (warp == WARPS && lane < slots && asked > lane) {
+            const uint32_t last = (uint32_t)((asked - 1 - lane) / slots) & 1;
+            for (unsigned spin = 0; spin < WAIT_LIMIT && !mbar_test(&full_bar[lane], last); ++spin) __nanosleep(64);
+        }
+        return;
+    }
 
     // ---- the warps' sums together, and what the caller wants done with them
     const int width = units * 8;
