@@ -181,8 +181,7 @@ __global__ void __launch_bounds__(THREADS, 2) linear_rows_kernel(const RowsParam
         // ---- the walk: chunk by chunk of K, in every chunk group by group of features
         int slot = 0, w_k = 0;
         uint32_t parity = 0;
-        bool ok = true;
-        for (int chunk = 0; chunk < chunks && ok; ++chunk) {
+        for (int chunk = 0; chunk < chunks; ++chunk) {
             uint4 xv[KBLK][R8];
 #pragma unroll
             for (int b = 0; b < KBLK; ++b) {
@@ -215,8 +214,9 @@ __global__ void __launch_bounds__(THREADS, 2) linear_rows_kernel(const RowsParam
             if (chunk + 1 < chunks) fetch_rows(x_k);
             const int live = K - w_k - warp * KBLK * 32 - t * 8;      // this lane's k below K, from its first one on
             for (int group = 0; group < groups; ++group) {
-                ok = __all_sync(0xffffffffu, mbar_wait(&full_bar[slot], parity, abort_flag, 22, prm.status));
-                if (!ok) break;
+                // (nothing goes by the answer: after a wait that gave up every later one ends at its first poll, the sums
+                // are worth nothing and nobody stores them.  A vote here costs 4 % of a decode step)
+                mbar_wait(&full_bar[slot], parity, abort_flag, 22, prm.status);
                 const uint8_t* from = ring + slot * SLOT + g * W_STRIDE + (warp * KBLK * 32 + t * 8) * 2;
                 uint4 wv[KBLK];
 #pragma unroll
