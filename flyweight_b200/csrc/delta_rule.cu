@@ -590,9 +590,13 @@ delta_runs_kernel(const float* __restrict__ r, const float* __restrict__ p, cons
 #pragma unroll 4
             for (int k = 0; k <= warp * 4; k += 4) {   // the warp's rows end there
                 const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(m_row + k);
+                const int left = row - k;              // entries behind the row's own token are left out, not multiplied
+                                                       // by zero: what is not finite there stays there
 #pragma unroll
                 for (int j = 0; j < 2; ++j) {
-                    const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(columns + (cc + 8 * j) * CT + k);
+                    ulonglong2 b = *reinterpret_cast<const ulonglong2*>(columns + (cc + 8 * j) * CT + k);
+                    if (left < 1) b.x &= 0xffffffffull;
+                    if (left < 3) b.y &= left < 2 ? 0ull : 0xffffffffull;
                     fma_pair(s[j][0], a.x, b.x);
                     fma_pair(s[j][1], a.y, b.y);
                 }

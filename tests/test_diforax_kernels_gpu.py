@@ -456,6 +456,37 @@ def test_delta_chunks_against_the_scan_and_64_bits(H, G, d, e, strong):
     print("errors", errors)
 
 
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("part,bad", [("k", "nan"), ("v", "nan"), ("v", "inf"), ("q", "nan")])
+def test_a_value_that_is_not_finite_reaches_no_earlier_token(d, part, bad):
+    """Token 37 of 75 brings a NaN or an infinity in one head's query, key or value: the tokens before it keep the bits
+    that they have without it, and what is not finite behind it is what the token-by-token scan has there."""
+    from flyweight_b200.kernels import recurrent
+    H = G = 2
+    e, n, at = 36, 75, 37
+    C = 2 * G * d + H * e
+    g = torch.Generator().manual_seed(d)
+    p = torch.randn(n, C + H * e + 2 * H, generator=g)
+    broken = p.clone()
+    broken[at, {"q": 0, "k": G * d, "v": 2 * G * d}[part] + 5] = float(bad)
+    start = torch.randn(2, recurrent.delta_state_size(H, G, d, e, 1), generator=g)
+
+    def run(p, chunks_from):
+        batch = Feeder(1, slots={0: 1}).batch([(0, n)])
+        recurrent.CHUNKS_FROM, before = chunks_from, recurrent.CHUNKS_FROM
+        try:
+            state = dev(start)
+            return recurrent.delta_rule(dev(p), dev(torch.ones(C, 1)), dev(torch.zeros(H)), dev(torch.zeros(H)), state,
+                                        batch, H, G, d, e).cpu()
+        finally:
+            recurrent.CHUNKS_FROM = before
+
+    whole, scanned, chunked = run(p, 16), run(broken, 10 ** 9), run(broken, 16)
+    assert torch.equal(chunked[:at], whole[:at])
+    assert torch.equal(chunked.isfinite(), scanned.isfinite())
+    assert not bool(chunked[at].isfinite().all())
+
+
 def test_delta_inputs_of_many_short_segments():
     """The convolution in front of the recurrence reads a window of rows that crosses requests: 60 requests of one to
     five tokens in one step leave the bits and the states that each leaves in a step of its own."""
