@@ -20,9 +20,10 @@
 //                   step (behind delta_prepare, which reads the old ones).
 //   gated_head_norm out[t][h] = weight * o / sqrt(mean(o^2) + eps) * silu(gate)
 // A request's slot is [ S: H d e | conv inputs: C (L-1) ] fp32, zero when the request starts.  A
-// token's result depends on its request's earlier tokens only through that slot.  In the scan every sum runs in an
-// order fixed by the sizes, so it does not depend on how the sequence was cut into steps; the chunks of a long
-// segment start where the segment does, so another cut is another order of the same fp32 sums.
+// token's result depends on its request's earlier tokens only through that slot, and on nothing of the segments beside
+// its own in the step: a segment's own length decides between scan and chunks.  In the scan every sum runs in an order
+// fixed by the sizes, so it does not depend on how the sequence was cut into steps; the chunks of a long segment start
+// where the segment does, so another cut is another order of the same sums.
 #include "common.cuh"
 
 using namespace fwb;
@@ -221,7 +222,7 @@ template <int DPL, int LPC, bool VEC>
 __global__ void __launch_bounds__(128)
 delta_scan_kernel(const float* __restrict__ r, const float* __restrict__ p, float* __restrict__ state,
                   long long slot_stride, const int* __restrict__ seg_start, const int* __restrict__ seg_slot,
-                  float* __restrict__ o, DeltaShape sh) {
+                  float* __restrict__ o, int below, DeltaShape sh) {
     // The next kernel is released only behind the token loop: its blocks would otherwise sit on the SMs for
     // the whole scan, whose one warp a scheduler is slowed by every other resident warp.
     fwb::pdl_wait();
@@ -232,7 +233,7 @@ delta_scan_kernel(const float* __restrict__ r, const float* __restrict__ p, floa
     __shared__ float scalars[STAGES][4];                              // beta, g, q.k
     const int seg = blockIdx.z, h = blockIdx.y;
     const int t0 = seg_start[seg], t1 = seg_start[seg + 1];
-    if (t1 <= t0) return;
+    if (t1 <= t0 || t1 - t0 >= below) return;                         // (a segment of that many tokens goes by chunks)
     const int d = sh.d, e = sh.e, R = sh.r_width();
     const int kv_head = h / (sh.H / sh.G);
     const int col_local = threadIdx.x / LPC, sub = threadIdx.x % LPC;
@@ -377,10 +378,11 @@ __device__ __forceinline__ unsigned long long pair_of(float v) {
 }
 
 // Chunk c of segment s and head h: scratch + (((seg_start[s] / 32 + s) + c) * H + h) * CHUNK_FLOATS: chunks of
-// different segments never meet, and T / 32 + S of them are enough.
+// different segments never meet, and T / 32 + S of them are enough.  Segments shorter than `from` are the scan's.
 template <int D>
 __global__ void __launch_bounds__(256)
-delta_chunk_kernel(const float* __restrict__ r, const int* __restrict__ seg_start, float* __restrict__ scratch, DeltaShape sh) {
+delta_chunk_kernel(const float* __restrict__ r, const int* __restrict__ seg_start, float* __restrict__ scratch, int from,
+                   DeltaShape sh) {
     fwb::pdl_entry();
     constexpr int STRIDE = D + 4;
     __shared__ __align__(16) float kq[2 * CHUNK][STRIDE];             // k rows, then q rows
@@ -388,9 +390,9 @@ delta_chunk_kernel(const float* __restrict__ r, const int* __restrict__ seg_star
     __shared__ __align__(16) float a_rows[CHUNK][CHUNK + 4];
     __shared__ float beta[CHUNK], g[CHUNK];
     const int seg = blockIdx.z, h = blockIdx.y;
-    const int begin = seg_start[seg], t0 = begin + blockIdx.x * CHUNK;
-    const int left = seg_start[seg + 1] - t0;
-    if (left <= 0) return;
+    const int begin = seg_start[seg], end = seg_start[seg + 1], t0 = begin + blockIdx.x * CHUNK;
+    const int left = end - t0;
+    if (left <= 0 || end - begin < from) return;
     const int n = left < CHUNK ? left : CHUNK, R = sh.r_width(), head = h / (sh.H / sh.G);
     for (int i = threadIdx.x; i < 2 * CHUNK * (D / 4); i += blockDim.x) {
         const int row = i / (D / 4), c = (i % (D / 4)) * 4, token = row % CHUNK;
@@ -482,13 +484,13 @@ template <int D>
 __global__ void __launch_bounds__(256)
 delta_runs_kernel(const float* __restrict__ r, const float* __restrict__ p, const float* __restrict__ scratch,
                   float* __restrict__ state, long long slot_stride, const int* __restrict__ seg_start,
-                  const int* __restrict__ seg_slot, float* __restrict__ o, DeltaShape sh) {
+                  const int* __restrict__ seg_slot, float* __restrict__ o, int from, DeltaShape sh) {
     using Y = RunLayout<D>;
     extern __shared__ __align__(16) float sm[];
     fwb::pdl_wait();
     const int seg = blockIdx.z, h = blockIdx.y, col0 = blockIdx.x * RUN_COLS;
     const int t0 = seg_start[seg], t1 = seg_start[seg + 1];
-    if (t1 <= t0) return;
+    if (t1 <= t0 || t1 - t0 < from) return;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, e = sh.e, R = sh.r_width();
     const int head = h / (sh.H / sh.G), chunks = (t1 - t0 + CHUNK - 1) / CHUNK;
     float* slot = state + (size_t)seg_slot[seg] * slot_stride;
@@ -680,9 +682,11 @@ delta_runs_kernel(const float* __restrict__ r, const float* __restrict__ p, cons
     }
 }
 
+// Segments `first` .. of at least `from` tokens, the longest of `longest`.
 template <int D>
 int launch_runs(const float* r, const float* p, float* scratch, float* state, long long slot_stride, const int* seg_start,
-                const int* seg_slot, float* o, int longest, int n_segments, const DeltaShape& sh, cudaStream_t stream) {
+                const int* seg_slot, float* o, int first, int from, int longest, int n_segments, const DeltaShape& sh,
+                cudaStream_t stream) {
     constexpr int SMEM = RunLayout<D>::FLOATS * 4;
     static bool configured = false;
     if (!configured) {
@@ -690,10 +694,11 @@ int launch_runs(const float* r, const float* p, float* scratch, float* state, lo
         if (err != cudaSuccess) return (int)err;
         configured = true;
     }
-    const dim3 chunks((longest + CHUNK - 1) / CHUNK, sh.H, n_segments);
-    fwb::pdl(delta_chunk_kernel<D>, chunks, 256, 0, stream)(r, seg_start, scratch, sh);
-    const dim3 grid((sh.e + RUN_COLS - 1) / RUN_COLS, sh.H, n_segments);
-    fwb::pdl(delta_runs_kernel<D>, grid, 256, SMEM, stream)(r, p, scratch, state, slot_stride, seg_start, seg_slot, o, sh);
+    const dim3 chunks((longest + CHUNK - 1) / CHUNK, sh.H, n_segments - first);
+    fwb::pdl(delta_chunk_kernel<D>, chunks, 256, 0, stream)(r, seg_start + first, scratch, from, sh);
+    const dim3 grid((sh.e + RUN_COLS - 1) / RUN_COLS, sh.H, n_segments - first);
+    fwb::pdl(delta_runs_kernel<D>, grid, 256, SMEM, stream)(r, p, scratch, state, slot_stride, seg_start + first,
+                                                            seg_slot + first, o, from, sh);
     return fwb_launch_status();
 }
 
@@ -721,12 +726,14 @@ gated_head_norm_kernel(const float* __restrict__ o, const float* __restrict__ ga
 // p: [T][2Gd + 2He + 2H] fp32 (q | k | v | gate | b | a).  taps: [2Gd + He][L] fp32.  a_log, dt_bias: [H].
 // state: [slots][slot_stride] fp32 with S at 0 and the convolution's inputs behind it.
 // r: [T][2Gd + He + 2H + G rounded up to a multiple of 4] fp32 scratch.  o: [T][H][e] fp32.
-// scratch: null (every token through the scan), or [T / 32 + n_segments][H][2][32][36] fp32 on a 16-byte border for
-// the chunked form, with `longest` the longest segment's tokens; sizes it does not take go through the scan.
+// scratch: null (every token through the scan), or [T / 32 + n_segments][H][2][32][36] fp32 on a 16-byte border: segments
+// of `from` tokens and more go by chunks, the others through the scan; sizes that the chunks do not take all go through the
+// scan.  The caller says where to look: no segment of the first `first` has `from` tokens, none behind the first `scanned`
+// has fewer, and the longest has `longest`.
 FWB_API int fwb_delta_rule(const float* p, const float* taps, const float* a_log, const float* dt_bias,
                            float* state, long long slot_stride, const int* seg_start, const int* seg_slot,
-                           const int* tok_seg, float* r, float* o, float* scratch, int longest, int T, int n_segments,
-                           int H, int G, int d, int e, int L, cudaStream_t stream) {
+                           const int* tok_seg, float* r, float* o, float* scratch, int from, int longest, int first,
+                           int scanned, int T, int n_segments, int H, int G, int d, int e, int L, cudaStream_t stream) {
     if (T <= 0 || n_segments <= 0) return FWB_OK;
     if (!p || !taps || !a_log || !dt_bias || !state || !seg_start || !seg_slot || !tok_seg || !r || !o)
         return FWB_BAD_ARGUMENT;
@@ -734,6 +741,9 @@ FWB_API int fwb_delta_rule(const float* p, const float* taps, const float* a_log
     if (L > MAX_TAPS || d > 256) return FWB_TOO_LARGE;
     const DeltaShape sh{H, G, d, e, L};
     if (slot_stride < (long long)H * d * e + (long long)sh.channels() * (L - 1)) return FWB_BAD_ARGUMENT;
+    if (scratch && (from <= 0 || longest <= 0 || longest > T || first < 0 || first > n_segments || scanned < first ||
+                    scanned > n_segments))
+        return FWB_BAD_ARGUMENT;
     const size_t smem = (size_t)sh.channels() * sizeof(float);
     if (smem > 160 * 1024 || n_segments > 65535 || H > 65535) return FWB_TOO_LARGE;
     // tokens in fours once there are enough of them, where 16-byte loads can read everything
@@ -753,27 +763,33 @@ FWB_API int fwb_delta_rule(const float* p, const float* taps, const float* a_log
     }
     const bool vec = d % 4 == 0 && e % 4 == 0 && slot_stride % 4 == 0 && ((uintptr_t)state & 15) == 0 &&
                      ((uintptr_t)r & 15) == 0;
-    if (scratch && vec && (d == 64 || d == 128) && ((uintptr_t)scratch & 15) == 0) {
-        if (d == 64)
-            return launch_runs<64>(r, p, scratch, state, slot_stride, seg_start, seg_slot, o, longest, n_segments, sh, stream);
-        return launch_runs<128>(r, p, scratch, state, slot_stride, seg_start, seg_slot, o, longest, n_segments, sh, stream);
-    }
+    const bool runs = scratch && vec && (d == 64 || d == 128) && ((uintptr_t)scratch & 15) == 0;
+    const int below = runs ? from : 2147483647, scans = runs ? scanned : n_segments;
 #define FWB_SCAN(DPL, LPC)                                                                                 \
     do {                                                                                                   \
-        const dim3 grid((e + 128 / LPC - 1) / (128 / LPC), H, n_segments);                                 \
+        const dim3 grid((e + 128 / LPC - 1) / (128 / LPC), H, scans);                                      \
         if (vec)                                                                                           \
             fwb::pdl(delta_scan_kernel<DPL, LPC, true>, grid, 128, 0, stream)(r, p, state, slot_stride,    \
-                                                                              seg_start, seg_slot, o, sh); \
+                                                                              seg_start, seg_slot, o, below, sh); \
         else                                                                                               \
             fwb::pdl(delta_scan_kernel<DPL, LPC, false>, grid, 128, 0, stream)(r, p, state, slot_stride,   \
-                                                                               seg_start, seg_slot, o, sh); \
+                                                                               seg_start, seg_slot, o, below, sh); \
     } while (0)
-    if (d <= 16) FWB_SCAN(4, 4);
-    else if (d <= 32) FWB_SCAN(8, 4);
-    else if (d <= 64) FWB_SCAN(16, 4);
-    else if (d <= 128) FWB_SCAN(16, 8);
-    else FWB_SCAN(32, 8);
+    if (scans > 0) {
+        if (d <= 16) FWB_SCAN(4, 4);
+        else if (d <= 32) FWB_SCAN(8, 4);
+        else if (d <= 64) FWB_SCAN(16, 4);
+        else if (d <= 128) FWB_SCAN(16, 8);
+        else FWB_SCAN(32, 8);
+    }
 #undef FWB_SCAN
+    if (runs && first < n_segments) {
+        const int status = d == 64 ? launch_runs<64>(r, p, scratch, state, slot_stride, seg_start, seg_slot, o, first, from,
+                                                     longest, n_segments, sh, stream)
+                                   : launch_runs<128>(r, p, scratch, state, slot_stride, seg_start, seg_slot, o, first, from,
+                                                      longest, n_segments, sh, stream);
+        if (status != FWB_OK) return status;
+    }
     return fwb_launch_status();
 }
 

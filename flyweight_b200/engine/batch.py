@@ -168,6 +168,16 @@ class StepBatch:
             cached = self._tiles[(tokens_per_tile, first_segment)] = (dev[:n], dev[n:], n)
         return cached
 
+    def split_by_length(self, tokens: int):
+        """``(first, behind)``: no segment in front of ``first`` has ``tokens`` tokens or more, none from ``behind`` on
+        has fewer.  Found once per step and length."""
+        key = ("length", tokens)
+        if key not in self._tiles:
+            long = [index for index, seg in enumerate(self.segments) if len(seg.tokens) >= tokens]
+            short = [index for index, seg in enumerate(self.segments) if len(seg.tokens) < tokens]
+            self._tiles[key] = (long[0] if long else self.n_segments, short[-1] + 1 if short else 0)
+        return self._tiles[key]
+
     def visible_pages(self, page_size: int, first_segment: int = 0):
         """The pages that the segments from ``first_segment`` on may see, listed one after the other: (page_seg,
         page_no, table, n_pages), int32 on the device -- segment and logical page of every entry, and a block table

@@ -16,8 +16,8 @@ def delta_state_size(heads: int, kv_heads: int, dim: int, vdim: int, taps: int) 
     return -(-size // 4) * 4            # slots start on 16-byte borders
 
 
-# From this many tokens of a step's longest segment on the recurrence runs in chunks of 32 tokens (head sizes 64 and
-# 128); shorter segments, decode steps above all, walk token by token.  Measured on B200 (16 heads of 128, one segment, all
+# A segment of this many tokens and more runs in chunks of 32 tokens (head sizes 64 and 128); shorter ones, decoding
+# requests above all, walk token by token, whatever else the step holds.  Measured on B200 (16 heads of 128, one segment, all
 # launches, us in chunks and by the scan): 8 tokens 30.9 and 31.5, 16 31.0 and 34.1, 32 31.3 and 40.8, 64 34.6 and 53.2.
 CHUNKS_FROM = 16
 _CHUNK_TOKENS, _CHUNK_FLOATS = 32, 2 * 32 * 36
@@ -52,11 +52,16 @@ def delta_rule(p: torch.Tensor, taps: torch.Tensor, a_log: torch.Tensor, dt_bias
     r = torch.empty((T, -(-(channels + 2 * heads + kv_heads) // 4) * 4), dtype=torch.float32, device=p.device)
     o = torch.empty((T, heads, vdim), dtype=torch.float32, device=p.device)
     chunked = batch.max_segment >= CHUNKS_FROM and dim in (64, 128) and vdim % 4 == 0 and stride % 4 == 0
-    scratch = torch.empty((T // _CHUNK_TOKENS + S) * heads * _CHUNK_FLOATS, dtype=torch.float32,
-                          device=p.device) if chunked else None
+    scratch, first, scanned = None, 0, S
+    if chunked:
+        scratch = torch.empty((T // _CHUNK_TOKENS + S) * heads * _CHUNK_FLOATS, dtype=torch.float32, device=p.device)
+        split = getattr(batch, "split_by_length", None)          # (a batch that cannot say: both forms look at every segment)
+        if split is not None:
+            first, scanned = split(CHUNKS_FROM)
     lib.call("fwb_delta_rule", ptr(p), ptr(taps), ptr(a_log), ptr(dt_bias), ptr(state), c_longlong(stride),
              ptr(batch.seg_start), ptr(batch.seg_slot), ptr(batch.tok_seg), ptr(r), ptr(o), ptr(scratch),
-             batch.max_segment if chunked else 0, T, S, heads, kv_heads, dim, vdim, L, stream(), launches=3 if chunked else 2)
+             CHUNKS_FROM if chunked else 0, batch.max_segment if chunked else 0, first, scanned, T, S, heads, kv_heads, dim,
+             vdim, L, stream(), launches=1 + (scanned > 0) + (2 if chunked else 0))
     return o
 
 

@@ -487,6 +487,41 @@ def test_a_value_that_is_not_finite_reaches_no_earlier_token(d, part, bad):
     assert not bool(chunked[at].isfinite().all())
 
 
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("told", [True, False])
+def test_a_segment_of_the_delta_rule_does_not_see_its_company(d, told):
+    """Decoding requests, short portions and long ones in one step, on both sides of the line between scan and chunks
+    and in any order: outputs and states have the bits that each segment leaves in a step of its own, whether or not
+    the batch says where the long ones are."""
+    from flyweight_b200.kernels import recurrent
+    H, G, e, L = 4, 2, 20, 4
+    C, line = 2 * G * d + H * e, recurrent.CHUNKS_FROM
+    g = torch.Generator().manual_seed(d)
+    taps, a_log, bias = dev(torch.randn(C, L, generator=g)), dev(torch.randn(H, generator=g)), dev(torch.randn(H, generator=g))
+    for lengths in ([1] * 6 + [line + 33], [line, 1, line - 1, 2 * line + 1, 5, 1], [1, 1, line - 1], [line + 7, 2 * line]):
+        T = sum(lengths)
+        p = dev(torch.randn(T, C + H * e + 2 * H, generator=g))
+        start = dev(torch.randn(len(lengths), recurrent.delta_state_size(H, G, d, e, L), generator=g))
+
+        def run(p, members, state):
+            feeder = Feeder(len(lengths), n_pages=400, slots={s: s for s in range(len(lengths))})
+            batch = feeder.batch([(s, lengths[s]) for s in members])
+            if not told:
+                plain = type("Batch", (), {})()
+                for name in ("n_segments", "max_segment", "seg_start", "seg_slot", "tok_seg"):
+                    setattr(plain, name, getattr(batch, name))
+                batch = plain
+            return recurrent.delta_rule(p, taps, a_log, bias, state, batch, H, G, d, e)
+
+        together, apart = start.clone(), start.clone()
+        out = run(p, range(len(lengths)), together)
+        at = 0
+        for s, n in enumerate(lengths):
+            assert torch.equal(run(p[at:at + n].contiguous(), [s], apart), out[at:at + n]), (lengths, s)
+            at += n
+        assert torch.equal(together, apart), lengths
+
+
 def test_delta_inputs_of_many_short_segments():
     """The convolution in front of the recurrence reads a window of rows that crosses requests: 60 requests of one to
     five tokens in one step leave the bits and the states that each leaves in a step of its own."""
