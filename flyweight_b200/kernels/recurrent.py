@@ -24,10 +24,12 @@ _CHUNK_TOKENS, _CHUNK_FLOATS = 32, 2 * 32 * 36
 
 
 def delta_rule(p: torch.Tensor, taps: torch.Tensor, a_log: torch.Tensor, dt_bias: torch.Tensor,
-               state: torch.Tensor, batch, heads: int, kv_heads: int, dim: int, vdim: int) -> torch.Tensor:
+               state: torch.Tensor, batch, heads: int, kv_heads: int, dim: int, vdim: int,
+               chunks: bool = True) -> torch.Tensor:
     """The gated delta rule over the step's tokens.  ``p``: fp32 [T][q | k | v | gate | b | a], the fused
     projection; ``taps``: fp32 [2 kv_heads dim + heads vdim][L]; ``state``: fp32 [slots][delta_state_size],
-    read at the head of every segment and advanced.  Returns o, fp32 [T][heads][vdim]."""
+    read at the head of every segment and advanced.  Returns o, fp32 [T][heads][vdim].  ``chunks``: long segments may go
+    by chunks; False walks every one token by token, so that the bits do not depend on where a sequence was cut."""
     check_tensor("delta projection", p, torch.float32)
     T = p.shape[0]
     channels = 2 * kv_heads * dim + heads * vdim
@@ -51,7 +53,7 @@ def delta_rule(p: torch.Tensor, taps: torch.Tensor, a_log: torch.Tensor, dt_bias
     _i32("tok_seg", batch.tok_seg, T)
     r = torch.empty((T, -(-(channels + 2 * heads + kv_heads) // 4) * 4), dtype=torch.float32, device=p.device)
     o = torch.empty((T, heads, vdim), dtype=torch.float32, device=p.device)
-    chunked = batch.max_segment >= CHUNKS_FROM and dim in (64, 128) and vdim % 4 == 0 and stride % 4 == 0
+    chunked = chunks and batch.max_segment >= CHUNKS_FROM and dim in (64, 128) and vdim % 4 == 0 and stride % 4 == 0
     scratch, first, scanned = None, 0, S
     if chunked:
         scratch = torch.empty((T // _CHUNK_TOKENS + S) * heads * _CHUNK_FLOATS, dtype=torch.float32, device=p.device)

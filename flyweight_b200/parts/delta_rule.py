@@ -88,8 +88,9 @@ class GatedDeltaRule(Mixer):
 
     def forward(self, ctx, h, cache):
         p = ops.linear(h, self.w_in, torch.float32)
+        # 32-bit runs keep one order of sums however a sequence is cut: token by token
         o = recurrent.delta_rule(p, self.taps, self.a_log, self.dt_bias, cache.state, ctx.batch, self.n_heads,
-                                 self.n_kv, self.dim, self.vdim)
+                                 self.n_kv, self.dim, self.vdim, chunks=ctx.precision.act_dtype != torch.float32)
         gate_at = 2 * self._qk + self._v
         z = recurrent.gated_head_norm(o, p[:, gate_at:gate_at + self._v], self.norm, self.eps,
                                       ctx.precision.act_dtype)

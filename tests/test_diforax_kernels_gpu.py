@@ -522,6 +522,27 @@ def test_a_segment_of_the_delta_rule_does_not_see_its_company(d, told):
         assert torch.equal(together, apart), lengths
 
 
+def test_delta_rule_in_32_bits_has_the_same_bits_however_it_is_cut():
+    """A whole sequence, portions of many sizes and single tokens, in float32 at a head size that has a chunked form:
+    outputs and the state's slot agree bit for bit."""
+    from flyweight_b200.kernels.recurrent import delta_state_size
+    from flyweight_b200.parts import build_mixer
+    heads, kv, dim, vdim, taps, hidden = 4, 2, 64, 128, 4, 128
+    g = torch.Generator().manual_seed(1)
+    w = delta_weights(g, heads, kv, dim, vdim, taps, hidden, torch.float32)
+    h = [torch.randn(n, hidden, generator=g) for n in (333, 150)]
+    part = build_mixer(delta_spec(heads, kv, dim, vdim, taps, hidden))
+    part.bind(lambda n: w[n].to(torch.float32), precision_of(torch.float32), DEV)
+    results = []
+    for sizes in ([1000], [257, 40, 3], [64, 1, 129], [1]):
+        cache = type("Cache", (), {})()
+        cache.state = torch.zeros((3, delta_state_size(heads, kv, dim, vdim, taps)), device=DEV)
+        got = run_part(part, precision_of(torch.float32), h, cuts_of([333, 150], sizes), cache, Feeder(2, slots={0: 2, 1: 0}))
+        results.append((got, cache.state))
+    for got, state in results[1:]:
+        assert all(torch.equal(got[s], results[0][0][s]) for s in got) and torch.equal(state, results[0][1])
+
+
 def test_delta_inputs_of_many_short_segments():
     """The convolution in front of the recurrence reads a window of rows that crosses requests: 60 requests of one to
     five tokens in one step leave the bits and the states that each leaves in a step of its own."""
