@@ -9,7 +9,8 @@
 // itself) and silu; q and k are then made unit vectors per head (x / sqrt(sum x^2 + 1e-6)); query
 // head h uses q/k head h / (H / G).  beta = sigmoid(b), g = exp(-exp(A_log) softplus(a + dt_bias)).
 //
-// Kernels (everything fp32; segments of many tokens also take delta_chunk and delta_runs, further down):
+// Kernels (everything fp32; segments of many tokens also take delta_chunk and delta_runs, further down, which sum over
+// their chunks in 64 bits):
 //   delta_prepare   one block per token (or per four): convolution + silu, unit vectors, beta and g
 //                   -> r[t] = [ q^: G d | k^: G d | v: H e | beta: H | g: H | q^.k^: G ]
 //   delta_scan      one block per (16 or 32 columns of S, head, segment): the recurrence over the
@@ -360,10 +361,21 @@ delta_scan_kernel(const float* __restrict__ r, const float* __restrict__ p, floa
 // with D_ij = g_{j+1} ... g_i and G_i = g_1 ... g_i, all products of decays (no logarithms: a difference of two
 // large sums would lose what a product of factors keeps).  T and P need no state: delta_chunk_kernel makes them for
 // every chunk and head at once; delta_runs_kernel then walks the chunks, one block per 16 columns of S and head, S
-// in shared memory, five small products a chunk in fp32 FMAs (packed in pairs, as in the fp32 matrix product).
-// T is a product of contractions (|k| = 1, beta < 1), so its entries stay below 1 and the sums lose nothing.
-constexpr int CHUNK = 32, CT = 36;                    // rows of T and P: 32 entries, then what a token has besides
-constexpr int CHUNK_FLOATS = 2 * CHUNK * CT;          // T | P of one chunk and head
+// in shared memory, five small products a chunk.
+//
+// What the chunk adds to the scan's roundings would be those of T, P, u and of sums over 32 tokens (2.5 times the scan's
+// error under strong decays, 1.9 under moderate ones, all in 32 bits).  So the products with T and P, the dot products
+// behind those two and the state's update run in 64 bits; only the 128-channel sums S0^T k and S0^T q, S itself and the
+// results are 32 bits wide.  Error against 64 bits over the scan's, 600 tokens on B200, keys behind silu, keys that come
+// again, keys that nearly coincide and keys of both signs, decays from none to e^-60 a token: 0.76 to 0.92 in the
+// read-out, 0.72 to 1.00 in the state (what is left is the inputs' own rounding).  64-bit multiply-adds run at half the
+// rate of 32-bit ones here and do not bind; 16 heads of 128, 2,048 tokens, all launches: 302 us in 32 bits, 388 so, 900
+// by the scan.
+//
+// A token reads nothing of a later one: T and P are summed up to the token's own column, so a value that is not finite
+// stays where the scan leaves it.
+constexpr int CHUNK = 32, CT = 34;                    // rows of T and P: 32 entries, then what a token has besides
+constexpr int CHUNK_DOUBLES = 2 * CHUNK * CT;         // T | P of one chunk and head
 constexpr int AT_BETA = 32, AT_G = 32, AT_REST = 33;  // T[i][32] = beta_i; P[i][32] = G_i, P[i][33] = D_Ci
 
 __device__ __forceinline__ void fma_pair(unsigned long long& acc, unsigned long long a, unsigned long long b) {
@@ -372,99 +384,109 @@ __device__ __forceinline__ void fma_pair(unsigned long long& acc, unsigned long 
 __device__ __forceinline__ float pair_sum(unsigned long long v) {
     return __uint_as_float((unsigned)v) + __uint_as_float((unsigned)(v >> 32));
 }
-__device__ __forceinline__ unsigned long long pair_of(float v) {
-    const unsigned long long u = __float_as_uint(v);
-    return u | (u << 32);
-}
 
-// Chunk c of segment s and head h: scratch + (((seg_start[s] / 32 + s) + c) * H + h) * CHUNK_FLOATS: chunks of
+// Chunk c of segment s and head h: scratch + (((seg_start[s] / 32 + s) + c) * H + h) * CHUNK_DOUBLES: chunks of
 // different segments never meet, and T / 32 + S of them are enough.  Segments shorter than `from` are the scan's.
+// A block's dot products are 16 x 16 a warp, four rows and two columns a thread, 64 channels of k and q at a time as
+// doubles in shared memory; the products and the rows of A take that room afterwards.
 template <int D>
-__global__ void __launch_bounds__(256)
-delta_chunk_kernel(const float* __restrict__ r, const int* __restrict__ seg_start, float* __restrict__ scratch, int from,
+__global__ void __launch_bounds__(256, 2)
+delta_chunk_kernel(const float* __restrict__ r, const int* __restrict__ seg_start, double* __restrict__ scratch, int from,
                    DeltaShape sh) {
     fwb::pdl_entry();
-    constexpr int STRIDE = D + 4;
-    __shared__ __align__(16) float kq[2 * CHUNK][STRIDE];             // k rows, then q rows
-    __shared__ float dots[2 * CHUNK][CHUNK + 1];                      // k_i.k_j, q_i.k_j
-    __shared__ __align__(16) float a_rows[CHUNK][CHUNK + 4];
-    __shared__ float beta[CHUNK], g[CHUNK];
+    constexpr int PART = 64, STRIDE = PART + 2, DOTS = CHUNK + 1, A_ROW = CHUNK + 2;
+    __shared__ __align__(16) double pool[2 * CHUNK * STRIDE];         // k rows, then q rows
+    double* dots = pool;                                              // [64][33]: k_i.k_j, q_i.k_j
+    double* a_rows = pool + 2 * CHUNK * DOTS;                         // [32][34]
+    static_assert(2 * CHUNK * DOTS % 2 == 0 && 2 * CHUNK * DOTS + CHUNK * A_ROW <= 2 * CHUNK * STRIDE, "the pool holds both");
+    __shared__ double beta[CHUNK], g[CHUNK];
     const int seg = blockIdx.z, h = blockIdx.y;
     const int begin = seg_start[seg], end = seg_start[seg + 1], t0 = begin + blockIdx.x * CHUNK;
     const int left = end - t0;
     if (left <= 0 || end - begin < from) return;
     const int n = left < CHUNK ? left : CHUNK, R = sh.r_width(), head = h / (sh.H / sh.G);
-    for (int i = threadIdx.x; i < 2 * CHUNK * (D / 4); i += blockDim.x) {
-        const int row = i / (D / 4), c = (i % (D / 4)) * 4, token = row % CHUNK;
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (token < n)
-            v = *reinterpret_cast<const float4*>(r + (size_t)(t0 + token) * R + (row < CHUNK ? sh.cq() : 0) + head * D + c);
-        *reinterpret_cast<float4*>(&kq[row][c]) = v;
-    }
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x < CHUNK) {
         const bool in = (int)threadIdx.x < n;
         const float* row = r + (size_t)(t0 + (in ? threadIdx.x : 0)) * R + sh.channels();
-        beta[threadIdx.x] = in ? row[h] : 0.0f;
-        g[threadIdx.x] = in ? row[sh.H + h] : 1.0f;
+        beta[threadIdx.x] = in ? (double)row[h] : 0.0;
+        g[threadIdx.x] = in ? (double)row[sh.H + h] : 1.0;
     }
-    __syncthreads();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    {
-        const int row = warp * 8 + (lane & 7), col = lane >> 3;       // this thread's row, columns col + 4 j
-        unsigned long long acc[8], acc2[8];
+    // warps 0-3 the k rows 16 by 16, 4-7 the q rows; nobody needs columns 16-31 of rows 0-15
+    const int row0 = (warp >> 2) * CHUNK + (warp & 2) * 8 + (lane & 3), col0 = (warp & 1) * 16 + (lane >> 2);
+    const bool needed = (warp & 3) != 1;
+    double acc[4][2];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) acc[j] = acc2[j] = 0ull;
+    for (int i = 0; i < 4; ++i) acc[i][0] = acc[i][1] = 0.0;
+    for (int part = 0; part < D; part += PART) {
+        if (part > 0) __syncthreads();
+        for (int i = threadIdx.x; i < 2 * CHUNK * (PART / 4); i += 256) {
+            const int row = i / (PART / 4), c = (i % (PART / 4)) * 4, token = row % CHUNK;
+            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (token < n)
+                v = *reinterpret_cast<const float4*>(r + (size_t)(t0 + token) * R + (row < CHUNK ? sh.cq() : 0) + head * D +
+                                                     part + c);
+            *reinterpret_cast<double2*>(&pool[row * STRIDE + c]) = make_double2(v.x, v.y);
+            *reinterpret_cast<double2*>(&pool[row * STRIDE + c + 2]) = make_double2(v.z, v.w);
+        }
+        __syncthreads();
+        if (needed) {
 #pragma unroll 4
-        for (int k = 0; k < D; k += 4) {
-            const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(&kq[row][k]);
+            for (int k = 0; k < PART; k += 2) {
+                double2 a[4], b[2];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(&kq[col + 4 * j][k]);
-                fma_pair(acc[j], a.x, b.x);
-                fma_pair(acc2[j], a.y, b.y);
+                for (int i = 0; i < 4; ++i) a[i] = *reinterpret_cast<const double2*>(&pool[(row0 + 4 * i) * STRIDE + k]);
+#pragma unroll
+                for (int j = 0; j < 2; ++j) b[j] = *reinterpret_cast<const double2*>(&pool[(col0 + 8 * j) * STRIDE + k]);
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int j = 0; j < 2; ++j) acc[i][j] = fma(a[i].y, b[j].y, fma(a[i].x, b[j].x, acc[i][j]));
             }
         }
-#pragma unroll
-        for (int j = 0; j < 8; ++j) dots[row][col + 4 * j] = pair_sum(acc[j]) + pair_sum(acc2[j]);
     }
+    __syncthreads();                                                  // k and q have been read: the pool is free
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) dots[(row0 + 4 * i) * DOTS + col0 + 8 * j] = acc[i][j];
     __syncthreads();
-    float* out = scratch + ((size_t)(begin / CHUNK + seg + blockIdx.x) * sh.H + h) * CHUNK_FLOATS;
-    float* p_out = out + CHUNK * CT;
-    // (the products of decays in 64 bits: a chunk's worth of roundings in one factor would go into whole rows)
+    double* out = scratch + ((size_t)(begin / CHUNK + seg + blockIdx.x) * sh.H + h) * CHUNK_DOUBLES;
+    double* p_out = out + CHUNK * CT;
     if (warp == 0) {                                                  // A: lane j walks its column down
         double d = 1.0;
 #pragma unroll 4
         for (int i = 0; i < CHUNK; ++i) {
-            d = i > lane ? d * (double)g[i] : 1.0;
-            a_rows[i][lane] = i > lane ? beta[i] * ((float)d * dots[i][lane]) : 0.0f;
+            d = i > lane ? d * g[i] : 1.0;
+            a_rows[i * A_ROW + lane] = i > lane ? beta[i] * (d * dots[i * DOTS + lane]) : 0.0;
         }
         out[lane * CT + AT_BETA] = beta[lane];
     } else if (warp == 1) {                                           // P
         double d = 1.0;
 #pragma unroll 4
         for (int i = 0; i < CHUNK; ++i) {
-            d = i > lane ? d * (double)g[i] : 1.0;
-            p_out[i * CT + lane] = i >= lane ? (float)d * dots[CHUNK + i][lane] : 0.0f;
+            d = i > lane ? d * g[i] : 1.0;
+            p_out[i * CT + lane] = i >= lane ? d * dots[(CHUNK + i) * DOTS + lane] : 0.0;
         }
-        p_out[lane * CT + AT_REST] = (float)d;                        // D_Cj: the last row's factor
+        p_out[lane * CT + AT_REST] = d;                               // D_Cj: the last row's factor
     } else if (warp == 2) {                                           // G_i
         double d = 1.0;
-        for (int i = 0; i <= lane; ++i) d *= (double)g[i];
-        p_out[lane * CT + AT_G] = (float)d;
+        for (int i = 0; i <= lane; ++i) d *= g[i];
+        p_out[lane * CT + AT_G] = d;
     }
     __syncwarp();
     if (warp == 0) {                                                  // column `lane` of (I + A)^-1, forwards
-        float t[CHUNK];
+        double t[CHUNK];
 #pragma unroll
         for (int i = 0; i < CHUNK; ++i) {
-            float s0 = 0.0f, s1 = 0.0f;
+            double s0 = 0.0, s1 = 0.0;
 #pragma unroll
             for (int m = 0; m + 1 < i; m += 2) {
-                s0 = fmaf(a_rows[i][m], t[m], s0);
-                s1 = fmaf(a_rows[i][m + 1], t[m + 1], s1);
+                s0 = fma(a_rows[i * A_ROW + m], t[m], s0);
+                s1 = fma(a_rows[i * A_ROW + m + 1], t[m + 1], s1);
             }
-            if (i & 1) s0 = fmaf(a_rows[i][i - 1], t[i - 1], s0);
-            t[i] = i == lane ? 1.0f : (i > lane ? -(s0 + s1) : 0.0f);
+            if (i & 1) s0 = fma(a_rows[i * A_ROW + i - 1], t[i - 1], s0);
+            t[i] = i == lane ? 1.0 : (i > lane ? -(s0 + s1) : 0.0);
             out[i * CT + lane] = t[i];
         }
     }
@@ -472,17 +494,23 @@ delta_chunk_kernel(const float* __restrict__ r, const int* __restrict__ seg_star
 
 constexpr int RUN_COLS = 16;
 template <int D>
-struct RunLayout {                                     // floats
+struct RunLayout {                                     // floats (T, P, r and u: two a value, on 16-byte borders)
     static constexpr int ROW = D + 4;
-    static constexpr int Q = CHUNK * ROW, V = 2 * CHUNK * ROW, TP = V + CHUNK * RUN_COLS, STAGE = TP + CHUNK_FLOATS;
-    static constexpr int S = 2 * STAGE, RED = S + RUN_COLS * ROW;     // S column by column
-    static constexpr int RED_FLOATS = 4 * 2 * CHUNK * 20;             // >= (256 / D - 1) * 16 * D, the state's partial sums
-    static constexpr int UT = RED + RED_FLOATS, UN = UT + 2 * RUN_COLS * CT, FLOATS = UN + CHUNK * RUN_COLS;
+    static constexpr int K = 0, V = 2 * CHUNK * ROW, Q = V + 2 * CHUNK * RUN_COLS, TP = Q + CHUNK * ROW;     // k and v: two chunks
+    static constexpr int S = TP + 2 * CHUNK_DOUBLES, RT = S + RUN_COLS * ROW, RED = RT + 2 * RUN_COLS * CT;  // S column by column
+    static constexpr int RED_FLOATS = 4 * 2 * CHUNK * 20, FLOATS = RED + RED_FLOATS;
+    static constexpr int UT = RED, UN = UT + 2 * RUN_COLS * CT;       // where the quarters' sums lay: they have been read
+    static_assert(UN + 2 * CHUNK * RUN_COLS <= FLOATS && Q % 4 == 0 && TP % 4 == 0 && RT % 4 == 0 && RED % 4 == 0, "it fits");
+    static_assert(FLOATS * 4 <= 112 * 1024, "two blocks an SM");
 };
 
+// Bound by latency: five barriers a chunk with little between them, 4.9 us a chunk for a block that has an SM to itself
+// (one prompt of 16 heads is 128 blocks).  So what a chunk needs lies once in shared memory where its place comes free in
+// time (q behind the first products, T and P behind the last), k and v twice, and two blocks share an SM where several
+// segments bring them.
 template <int D>
-__global__ void __launch_bounds__(256)
-delta_runs_kernel(const float* __restrict__ r, const float* __restrict__ p, const float* __restrict__ scratch,
+__global__ void __launch_bounds__(256, 2)
+delta_runs_kernel(const float* __restrict__ r, const float* __restrict__ p, const double* __restrict__ scratch,
                   float* __restrict__ state, long long slot_stride, const int* __restrict__ seg_start,
                   const int* __restrict__ seg_slot, float* __restrict__ o, int from, DeltaShape sh) {
     using Y = RunLayout<D>;
@@ -497,53 +525,68 @@ delta_runs_kernel(const float* __restrict__ r, const float* __restrict__ p, cons
     if (blockIdx.x == 0 && h == 0 && sh.L > 1) delta_conv_advance(p, slot, t0, t1 - t0, sh);
     float* S = sm + Y::S;
     float* red = sm + Y::RED;
-    float* rt = sm + Y::UT;                            // r, column by column [16][36]
-    float* ut = rt + RUN_COLS * CT;                    // u, column by column
-    float* un = sm + Y::UN;                            // D_Cj u_j, token by token [32][16]
+    double* rt = reinterpret_cast<double*>(sm + Y::RT);               // r, column by column [16][34]
+    double* ut = reinterpret_cast<double*>(sm + Y::UT);               // u, column by column
+    double* un = reinterpret_cast<double*>(sm + Y::UN);               // D_Cj u_j, token by token [32][16]
     for (int i = tid; i < RUN_COLS * (D / 4); i += 256) {
         const int c = i / (D / 4), k = (i % (D / 4)) * 4;
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
         if (col0 + c < e) v = *reinterpret_cast<const float4*>(slot + ((size_t)h * e + col0 + c) * D + k);
         *reinterpret_cast<float4*>(S + c * Y::ROW + k) = v;
     }
-    const float* tp0 = scratch + ((size_t)(t0 / CHUNK + seg) * sh.H + h) * CHUNK_FLOATS;
-    auto copy = [&](float* dst, const float* src, bool in) {          // 16 bytes, or as many zeros
+    const double* tp0 = scratch + ((size_t)(t0 / CHUNK + seg) * sh.H + h) * CHUNK_DOUBLES;
+    auto copy = [&](float* dst, const void* src, bool in) {           // 16 bytes, or as many zeros
         asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
                      "l"(src), "r"(in ? 16 : 0) : "memory");
     };
-    auto fetch = [&](int c) {
+    // rows of k or q (from column `at` of r's rows) of chunk c
+    auto fetch_rows = [&](float* to, int c, int at) {
+        const int first = t0 + c * CHUNK, n = t1 - first;
+        for (int i = tid; i < CHUNK * (D / 4); i += 256) {
+            const int token = i / (D / 4), k = (i % (D / 4)) * 4;
+            const bool in = token < n;
+            copy(to + token * Y::ROW + k, r + (size_t)(in ? first + token : t0) * R + at + head * D + k, in);
+        }
+    };
+    auto fetch_kv = [&](int c) {
         if (c < chunks) {
-            float* stage = sm + (c & 1) * Y::STAGE;
+            fetch_rows(sm + Y::K + (c & 1) * CHUNK * Y::ROW, c, sh.cq());
             const int first = t0 + c * CHUNK, n = t1 - first;
-            for (int i = tid; i < 2 * CHUNK * (D / 4); i += 256) {
-                const int row = i / (D / 4), k = (i % (D / 4)) * 4, token = row % CHUNK;
-                const bool in = token < n;
-                copy(stage + row * Y::ROW + k,
-                     r + (size_t)(in ? first + token : t0) * R + (row < CHUNK ? sh.cq() : 0) + head * D + k, in);
-            }
             if (tid < CHUNK * RUN_COLS / 4) {
                 const int token = tid / 4, k = (tid % 4) * 4;
                 const bool in = token < n && col0 + k < e;
-                copy(stage + Y::V + token * RUN_COLS + k,
+                copy(sm + Y::V + (c & 1) * CHUNK * RUN_COLS + token * RUN_COLS + k,
                      r + (in ? (size_t)(first + token) * R + 2 * sh.cq() + h * e + col0 + k : (size_t)t0 * R), in);
             }
-            const float* tp = tp0 + (size_t)c * sh.H * CHUNK_FLOATS;
-            for (int i = tid * 4; i < CHUNK_FLOATS; i += 1024) copy(stage + Y::TP + i, tp + i, true);
         }
         copy_async_commit();
     };
-    fetch(0);
+    auto fetch_q = [&](int c) {
+        if (c < chunks) fetch_rows(sm + Y::Q, c, 0);
+        copy_async_commit();
+    };
+    auto fetch_tp = [&](int c) {
+        if (c < chunks) {
+            const double* tp = tp0 + (size_t)c * sh.H * CHUNK_DOUBLES;
+            for (int i = tid * 2; i < CHUNK_DOUBLES; i += 512) copy(sm + Y::TP + 2 * i, tp + i, true);
+        }
+        copy_async_commit();
+    };
+    fetch_kv(0);
+    fetch_q(0);
+    fetch_tp(0);
+    const double* T = reinterpret_cast<const double*>(sm + Y::TP);
+    const double* P = T + CHUNK * CT;
     for (int c = 0; c < chunks; ++c) {
-        fetch(c + 1);                                  // (the stage was last read before the barrier that ends a chunk)
-        copy_async_wait<1>();
+        copy_async_wait<1>();                          // k, v and q of this chunk; T and P may still be on their way
         __syncthreads();
-        const float* stage = sm + (c & 1) * Y::STAGE;
-        const float* T = stage + Y::TP;
-        const float* P = T + CHUNK * CT;
+        fetch_kv(c + 1);                               // (its places were last read in front of the barrier)
+        const float* ks_rows = sm + Y::K + (c & 1) * CHUNK * Y::ROW;
+        const float* vs = sm + Y::V + (c & 1) * CHUNK * RUN_COLS;
         const int n = t1 - t0 - c * CHUNK < CHUNK ? t1 - t0 - c * CHUNK : CHUNK;
         {   // S0^T k and S0^T q: warps 0-3 the k rows, 4-7 the q rows, a quarter of the channels each
             const int quarter = warp & 3, tm = lane & 7, tn = lane >> 3;
-            const float* rows = stage + (warp >> 2) * Y::Q + tm * Y::ROW + quarter * (D / 4);
+            const float* rows = (warp < 4 ? ks_rows : sm + Y::Q) + tm * Y::ROW + quarter * (D / 4);
             const float* cols = S + tn * Y::ROW + quarter * (D / 4);
             unsigned long long acc[4][4];
 #pragma unroll
@@ -571,45 +614,44 @@ delta_runs_kernel(const float* __restrict__ r, const float* __restrict__ p, cons
 #pragma unroll
                 for (int j = 0; j < 4; ++j) to[i * 160 + 4 * j] = pair_sum(acc[i][j]);
         }
+        copy_async_wait<1>();                          // T and P; the next chunk's k and v may still be on their way
         __syncthreads();
+        fetch_q(c + 1);
         const int row = tid >> 3, cc = tid & 7;        // token and columns cc, cc + 8 of the middle products
-        float from_state[2];
+        double from_state[2];
         {
-            const float beta = T[row * CT + AT_BETA], G = P[row * CT + AT_G];
+            const double beta = T[row * CT + AT_BETA], G = P[row * CT + AT_G];
 #pragma unroll
             for (int j = 0; j < 2; ++j) {
                 const float* at = red + row * 20 + cc + 8 * j;
                 const float ks = (at[0] + at[2 * CHUNK * 20]) + (at[4 * CHUNK * 20] + at[6 * CHUNK * 20]);
                 at += CHUNK * 20;
                 const float qs = (at[0] + at[2 * CHUNK * 20]) + (at[4 * CHUNK * 20] + at[6 * CHUNK * 20]);
-                rt[(cc + 8 * j) * CT + row] = beta * (stage[Y::V + row * RUN_COLS + cc + 8 * j] - G * ks);
-                from_state[j] = G * qs;
+                rt[(cc + 8 * j) * CT + row] = beta * ((double)vs[row * RUN_COLS + cc + 8 * j] - G * (double)ks);
+                from_state[j] = G * (double)qs;
             }
         }
         __syncthreads();
-        auto row_times = [&](const float* m_row, const float* columns, float (&v)[2]) {
-            unsigned long long s[2][2] = {{0ull, 0ull}, {0ull, 0ull}};
+        // one row of T or P times two columns, up to the row's own token
+        auto row_times = [&](const double* m_row, const double* columns, double (&v)[2]) {
+            double s[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
 #pragma unroll 4
-            for (int k = 0; k <= warp * 4; k += 4) {   // the warp's rows end there
-                const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(m_row + k);
-                const int left = row - k;              // entries behind the row's own token are left out, not multiplied
-                                                       // by zero: what is not finite there stays there
+            for (int k = 0; k <= row; k += 2) {
+                const double2 a = *reinterpret_cast<const double2*>(m_row + k);
 #pragma unroll
                 for (int j = 0; j < 2; ++j) {
-                    ulonglong2 b = *reinterpret_cast<const ulonglong2*>(columns + (cc + 8 * j) * CT + k);
-                    if (left < 1) b.x &= 0xffffffffull;
-                    if (left < 3) b.y &= left < 2 ? 0ull : 0xffffffffull;
-                    fma_pair(s[j][0], a.x, b.x);
-                    fma_pair(s[j][1], a.y, b.y);
+                    const double2 b = *reinterpret_cast<const double2*>(columns + (cc + 8 * j) * CT + k);
+                    s[j][0] = fma(a.x, b.x, s[j][0]);
+                    if (k < row) s[j][1] = fma(a.y, b.y, s[j][1]);
                 }
             }
 #pragma unroll
-            for (int j = 0; j < 2; ++j) v[j] = pair_sum(s[j][0]) + pair_sum(s[j][1]);
+            for (int j = 0; j < 2; ++j) v[j] = s[j][0] + s[j][1];
         };
         {
-            float u[2];
+            double u[2];
             row_times(T + row * CT, rt, u);
-            const float rest = P[row * CT + AT_REST];
+            const double rest = P[row * CT + AT_REST];
 #pragma unroll
             for (int j = 0; j < 2; ++j) {
                 ut[(cc + 8 * j) * CT + row] = u[j];
@@ -618,60 +660,42 @@ delta_runs_kernel(const float* __restrict__ r, const float* __restrict__ p, cons
         }
         __syncthreads();
         {
-            float v[2];
+            double v[2];
             row_times(P + row * CT, ut, v);
             if (row < n) {
                 float* at = o + ((size_t)(t0 + c * CHUNK + row) * sh.H + h) * e + col0;
 #pragma unroll
                 for (int j = 0; j < 2; ++j)
-                    if (col0 + cc + 8 * j < e) at[cc + 8 * j] = from_state[j] + v[j];
+                    if (col0 + cc + 8 * j < e) at[cc + 8 * j] = (float)(from_state[j] + v[j]);
             }
         }
-        {   // S <- G_C S0 + sum_j k_j (D_Cj u_j): four channels x four columns a thread, the tokens in 256 / D parts
-            constexpr int QUADS = D / 4, PARTS = 256 / (4 * QUADS), TOKENS = CHUNK / PARTS;
-            const int quad = tid % QUADS, cg = (tid / QUADS) & 3, part = tid / (4 * QUADS);
-            unsigned long long acc[4][2];
+        {   // S <- G_C S0 + sum_j k_j (D_Cj u_j): two channels and COLS columns a thread, all tokens
+            constexpr int PAIRS = D / 2, COLS = RUN_COLS * PAIRS / 256;
+            const int pair = tid % PAIRS, first = (tid / PAIRS) * COLS;
+            double acc[COLS][2];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) acc[j][0] = acc[j][1] = 0ull;
+            for (int j = 0; j < COLS; ++j) acc[j][0] = acc[j][1] = 0.0;
 #pragma unroll 4
-            for (int i = 0; i < TOKENS; ++i) {
-                const int token = part * TOKENS + i;
-                const ulonglong2 k = *reinterpret_cast<const ulonglong2*>(stage + token * Y::ROW + quad * 4);
-                const float4 u = *reinterpret_cast<const float4*>(un + token * RUN_COLS + cg * 4);
-                const unsigned long long uu[4] = {pair_of(u.x), pair_of(u.y), pair_of(u.z), pair_of(u.w)};
+            for (int token = 0; token < CHUNK; ++token) {
+                const float2 k = *reinterpret_cast<const float2*>(ks_rows + token * Y::ROW + pair * 2);
+                const double kx = k.x, ky = k.y;
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    fma_pair(acc[j][0], k.x, uu[j]);
-                    fma_pair(acc[j][1], k.y, uu[j]);
+                for (int j = 0; j < COLS; j += 2) {
+                    const double2 u = *reinterpret_cast<const double2*>(un + token * RUN_COLS + first + j);
+                    acc[j][0] = fma(kx, u.x, acc[j][0]), acc[j][1] = fma(ky, u.x, acc[j][1]);
+                    acc[j + 1][0] = fma(kx, u.y, acc[j + 1][0]), acc[j + 1][1] = fma(ky, u.y, acc[j + 1][1]);
                 }
             }
-            ulonglong2* others = reinterpret_cast<ulonglong2*>(red);
-            if (part > 0)
+            const double last = P[(CHUNK - 1) * CT + AT_G];
 #pragma unroll
-                for (int j = 0; j < 4; ++j)
-                    others[((part - 1) * 4 + j) * (4 * QUADS) + cg * QUADS + quad] = make_ulonglong2(acc[j][0], acc[j][1]);
-            __syncthreads();
-            if (part == 0) {
-                const float last = P[(CHUNK - 1) * CT + AT_G];
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    float4* at = reinterpret_cast<float4*>(S + (cg * 4 + j) * Y::ROW + quad * 4);
-                    float4 v = *at;
-                    float add[4] = {__uint_as_float((unsigned)acc[j][0]), __uint_as_float((unsigned)(acc[j][0] >> 32)),
-                                    __uint_as_float((unsigned)acc[j][1]), __uint_as_float((unsigned)(acc[j][1] >> 32))};
-#pragma unroll
-                    for (int other = 1; other < PARTS; ++other) {
-                        const float4 w = *reinterpret_cast<const float4*>(
-                            &others[((other - 1) * 4 + j) * (4 * QUADS) + cg * QUADS + quad]);
-                        add[0] += w.x, add[1] += w.y, add[2] += w.z, add[3] += w.w;
-                    }
-                    v.x = fmaf(last, v.x, add[0]), v.y = fmaf(last, v.y, add[1]);
-                    v.z = fmaf(last, v.z, add[2]), v.w = fmaf(last, v.w, add[3]);
-                    *at = v;
-                }
+            for (int j = 0; j < COLS; ++j) {
+                float2* at = reinterpret_cast<float2*>(S + (first + j) * Y::ROW + pair * 2);
+                const float2 v = *at;
+                *at = make_float2((float)fma(last, (double)v.x, acc[j][0]), (float)fma(last, (double)v.y, acc[j][1]));
             }
         }
-        __syncthreads();
+        __syncthreads();                               // S is whole, and T and P have been read
+        fetch_tp(c + 1);
     }
     copy_async_wait<0>();
     fwb::pdl_launch_dependents();
@@ -684,20 +708,23 @@ delta_runs_kernel(const float* __restrict__ r, const float* __restrict__ p, cons
 
 // Segments `first` .. of at least `from` tokens, the longest of `longest`.
 template <int D>
-int launch_runs(const float* r, const float* p, float* scratch, float* state, long long slot_stride, const int* seg_start,
+int launch_runs(const float* r, const float* p, double* scratch, float* state, long long slot_stride, const int* seg_start,
                 const int* seg_slot, float* o, int first, int from, int longest, int n_segments, const DeltaShape& sh,
                 cudaStream_t stream) {
-    constexpr int SMEM = RunLayout<D>::FLOATS * 4;
+    // blocks that fit the SMs one by one must not pair up on some of them (128 blocks, started in the shadow of the kernel
+    // in front: 552 us for 2,048 tokens in pairs, 400 apart): they ask for more than half of an SM's shared memory
+    constexpr int SMEM = RunLayout<D>::FLOATS * 4, ALONE = 120 * 1024;
     static bool configured = false;
     if (!configured) {
-        cudaError_t err = cudaFuncSetAttribute(delta_runs_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+        cudaError_t err = cudaFuncSetAttribute(delta_runs_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, ALONE);
         if (err != cudaSuccess) return (int)err;
         configured = true;
     }
     const dim3 chunks((longest + CHUNK - 1) / CHUNK, sh.H, n_segments - first);
     fwb::pdl(delta_chunk_kernel<D>, chunks, 256, 0, stream)(r, seg_start + first, scratch, from, sh);
     const dim3 grid((sh.e + RUN_COLS - 1) / RUN_COLS, sh.H, n_segments - first);
-    fwb::pdl(delta_runs_kernel<D>, grid, 256, SMEM, stream)(r, p, scratch, state, slot_stride, seg_start + first,
+    const bool alone = (long)grid.x * grid.y * grid.z <= 148;
+    fwb::pdl(delta_runs_kernel<D>, grid, 256, alone ? ALONE : SMEM, stream)(r, p, scratch, state, slot_stride, seg_start + first,
                                                             seg_slot + first, o, from, sh);
     return fwb_launch_status();
 }
@@ -726,13 +753,13 @@ gated_head_norm_kernel(const float* __restrict__ o, const float* __restrict__ ga
 // p: [T][2Gd + 2He + 2H] fp32 (q | k | v | gate | b | a).  taps: [2Gd + He][L] fp32.  a_log, dt_bias: [H].
 // state: [slots][slot_stride] fp32 with S at 0 and the convolution's inputs behind it.
 // r: [T][2Gd + He + 2H + G rounded up to a multiple of 4] fp32 scratch.  o: [T][H][e] fp32.
-// scratch: null (every token through the scan), or [T / 32 + n_segments][H][2][32][36] fp32 on a 16-byte border: segments
+// scratch: null (every token through the scan), or [T / 32 + n_segments][H][2][32][34] fp64 on a 16-byte border: segments
 // of `from` tokens and more go by chunks, the others through the scan; sizes that the chunks do not take all go through the
 // scan.  The caller says where to look: no segment of the first `first` has `from` tokens, none behind the first `scanned`
 // has fewer, and the longest has `longest`.
 FWB_API int fwb_delta_rule(const float* p, const float* taps, const float* a_log, const float* dt_bias,
                            float* state, long long slot_stride, const int* seg_start, const int* seg_slot,
-                           const int* tok_seg, float* r, float* o, float* scratch, int from, int longest, int first,
+                           const int* tok_seg, float* r, float* o, double* scratch, int from, int longest, int first,
                            int scanned, int T, int n_segments, int H, int G, int d, int e, int L, cudaStream_t stream) {
     if (T <= 0 || n_segments <= 0) return FWB_OK;
     if (!p || !taps || !a_log || !dt_bias || !state || !seg_start || !seg_slot || !tok_seg || !r || !o)

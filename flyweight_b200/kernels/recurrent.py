@@ -20,7 +20,7 @@ def delta_state_size(heads: int, kv_heads: int, dim: int, vdim: int, taps: int) 
 # requests above all, walk token by token, whatever else the step holds.  Measured on B200 (16 heads of 128, one segment, all
 # launches, us in chunks and by the scan): 8 tokens 30.9 and 31.5, 16 31.0 and 34.1, 32 31.3 and 40.8, 64 34.6 and 53.2.
 CHUNKS_FROM = 16
-_CHUNK_TOKENS, _CHUNK_FLOATS = 32, 2 * 32 * 36
+_CHUNK_TOKENS, _CHUNK_DOUBLES = 32, 2 * 32 * 34
 
 
 def delta_rule(p: torch.Tensor, taps: torch.Tensor, a_log: torch.Tensor, dt_bias: torch.Tensor,
@@ -56,7 +56,7 @@ def delta_rule(p: torch.Tensor, taps: torch.Tensor, a_log: torch.Tensor, dt_bias
     chunked = chunks and batch.max_segment >= CHUNKS_FROM and dim in (64, 128) and vdim % 4 == 0 and stride % 4 == 0
     scratch, first, scanned = None, 0, S
     if chunked:
-        scratch = torch.empty((T // _CHUNK_TOKENS + S) * heads * _CHUNK_FLOATS, dtype=torch.float32, device=p.device)
+        scratch = torch.empty((T // _CHUNK_TOKENS + S) * heads * _CHUNK_DOUBLES, dtype=torch.float64, device=p.device)
         split = getattr(batch, "split_by_length", None)          # (a batch that cannot say: both forms look at every segment)
         if split is not None:
             first, scanned = split(CHUNKS_FROM)

@@ -406,8 +406,8 @@ def test_delta_rule_whole_cut_and_one_by_one(shape, dtype):
 @pytest.mark.parametrize("strong", [False, True])
 def test_delta_chunks_against_the_scan_and_64_bits(H, G, d, e, strong):
     """The chunked form at the edges of its chunks of 32 and of its 16 columns, on a state that is not zero, with
-    keys that repeat and with decays down to e^-60 a token: as close to 64 bits as the token-by-token scan, up to
-    the handful of roundings more that a sum over a chunk has (both stay within 64 roundings of the largest value)."""
+    keys that repeat and with decays down to e^-60 a token: as close to 64 bits as the token-by-token scan (one rounding
+    more for what differs by chance in so few tokens; both stay within 64 roundings of the largest value)."""
     from flyweight_b200.kernels import recurrent
     g = torch.Generator().manual_seed(H * d + e)
     lengths, L, C = [31, 1, 32, 33, 97, 64], 1, 2 * G * d + H * e
@@ -452,7 +452,7 @@ def test_delta_chunks_against_the_scan_and_64_bits(H, G, d, e, strong):
                        float((state.cpu().double() - after).norm() / after.norm())))
         close(o.cpu().view(T, H, e), want, 64 * 2.0 ** -24, f"chunked {chunked}: read out")
         close(state.cpu(), after, 64 * 2.0 ** -24, f"chunked {chunked}: state")
-    assert errors[0][0] <= 2 * errors[1][0] + 2.0 ** -24 and errors[0][1] <= 2 * errors[1][1] + 2.0 ** -24, errors
+    assert errors[0][0] <= errors[1][0] + 2.0 ** -24 and errors[0][1] <= errors[1][1] + 2.0 ** -24, errors
     print("errors", errors)
 
 
@@ -541,6 +541,63 @@ def test_delta_rule_in_32_bits_has_the_same_bits_however_it_is_cut():
         results.append((got, cache.state))
     for got, state in results[1:]:
         assert all(torch.equal(got[s], results[0][0][s]) for s in got) and torch.equal(state, results[0][1])
+
+
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("keys,decay", [("silu", "weak"), ("silu", "strong"), ("repeated", "moderate"), ("aligned", "none"),
+                                        ("signed", "weak")])
+def test_delta_chunks_are_no_further_from_64_bits_than_the_scan(keys, decay, d):
+    """600 tokens of the inputs that the recurrence meets (keys behind silu, keys that come again, keys that nearly
+    coincide, keys of both signs; decays from none to e^-60 a token): the error of the chunked form in the read-out and
+    in the state is at most the token-by-token scan's (2 % for chance, where it is that of the rounded inputs)."""
+    from flyweight_b200.kernels import recurrent
+    H, G, e, n = 4, 4, 32, 600
+    C = 2 * G * d + H * e
+    g = torch.Generator().manual_seed(7)
+    p = torch.randn(n, C + H * e + 2 * H, generator=g)
+    key = slice(G * d, 2 * G * d)
+    if keys == "repeated":
+        p[::3, key] = p[0, key]
+    elif keys == "aligned":
+        p[:, key] = 2.0 + p[0, key].abs() + 0.01 * p[:, key]
+        p[:, C + H * e:C + H * e + H] = 4.0                            # beta = 0.98
+    elif keys == "signed":
+        p[:, :2 * G * d] = 8.0 + p[:, :2 * G * d]                      # silu is close to the identity; taps make it signed
+    a = p[:, C + H * e + H:]
+    a_log = torch.zeros(H)
+    if decay == "none":
+        a[:] = -60.0
+    elif decay == "weak":
+        a_log[:] = -3.0
+    elif decay == "strong":
+        a[:] = 60.0 * torch.rand(n, H, generator=g)
+    taps, zeros = torch.ones(C, 1), torch.zeros(H)
+    if keys == "signed":
+        taps = torch.where(torch.rand(C, 1, generator=g) < 0.5, -0.25, 1.0)
+    start = 0.1 * torch.randn(2, recurrent.delta_state_size(H, G, d, e, 1), generator=g)
+    x = p.double()
+    act = x[:, :C] * taps[:, 0].double()
+    act = act * torch.sigmoid(act)
+    unit = lambda t: t * torch.rsqrt((t * t).sum(-1, keepdim=True) + 1e-6)
+    q, k = unit(act[:, :G * d].view(n, G, d)) * d ** -0.5, unit(act[:, key].view(n, G, d))
+    v, beta = act[:, 2 * G * d:].view(n, H, e), torch.sigmoid(x[:, C + H * e:C + H * e + H])
+    fade = torch.exp(-torch.exp(a_log.double()) * torch.nn.functional.softplus(x[:, C + H * e + H:]))
+    S, want = start[1].double()[:H * d * e].view(H, e, d).clone(), torch.empty(n, H, e, dtype=F64)
+    for t in range(n):
+        S *= fade[t][:, None, None]
+        u = beta[t][:, None] * (v[t] - torch.einsum("hed,hd->he", S, k[t]))
+        S += u[:, :, None] * k[t][:, None, :]
+        want[t] = torch.einsum("hed,hd->he", S, q[t])
+    errors = []
+    for chunks in (True, False):
+        batch = Feeder(1, slots={0: 1}).batch([(0, n)])
+        state = dev(start)
+        o = recurrent.delta_rule(dev(p), dev(taps), dev(a_log), dev(zeros), state, batch, H, G, d, e, chunks=chunks)
+        after = state[1, :H * d * e].cpu().double().view(H, e, d)
+        errors.append((float((o.cpu().double() - want).norm() / want.norm()), float((after - S).norm() / S.norm())))
+    print("errors", errors)
+    assert n >= recurrent.CHUNKS_FROM
+    assert errors[0][0] <= 1.02 * errors[1][0] and errors[0][1] <= 1.02 * errors[1][1], errors
 
 
 def test_delta_inputs_of_many_short_segments():
