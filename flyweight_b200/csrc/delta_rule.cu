@@ -367,7 +367,7 @@ delta_scan_kernel(const float* __restrict__ r, const float* __restrict__ p, floa
 // error under strong decays, 1.9 under moderate ones, all in 32 bits).  So the products with T and P, the dot products
 // behind those two and the state's update run in 64 bits; only the 128-channel sums S0^T k and S0^T q, S itself and the
 // results are 32 bits wide.  Error against 64 bits over the scan's, 600 tokens on B200, keys behind silu, keys that come
-// again, keys that nearly coincide and keys of both signs, decays from none to e^-60 a token: 0.76 to 0.92 in the
+// again, keys that nearly coincide and keys of both signs, decays from none to e^-60 a token: 0.76 to 0.90 in the
 // read-out, 0.72 to 1.00 in the state (what is left is the inputs' own rounding).  64-bit multiply-adds run at half the
 // rate of 32-bit ones here and do not bind; 16 heads of 128, 2,048 tokens, all launches: 302 us in 32 bits, 388 so, 900
 // by the scan.
@@ -504,7 +504,7 @@ struct RunLayout {                                     // floats (T, P, r and u:
     static_assert(FLOATS * 4 <= 112 * 1024, "two blocks an SM");
 };
 
-// Bound by latency: five barriers a chunk with little between them, 4.9 us a chunk for a block that has an SM to itself
+// Bound by latency: five barriers a chunk with little between them, 4.7 us a chunk for a block that has an SM to itself
 // (one prompt of 16 heads is 128 blocks).  So what a chunk needs lies once in shared memory where its place comes free in
 // time (q behind the first products, T and P behind the last), k and v twice, and two blocks share an SM where several
 // segments bring them.

@@ -17,9 +17,14 @@ def delta_state_size(heads: int, kv_heads: int, dim: int, vdim: int, taps: int) 
 
 
 # A segment of this many tokens and more runs in chunks of 32 tokens (head sizes 64 and 128); shorter ones, decoding
-# requests above all, walk token by token, whatever else the step holds.  Measured on B200 (16 heads of 128, one segment, all
-# launches, us in chunks and by the scan): 8 tokens 30.9 and 31.5, 16 31.0 and 34.1, 32 31.3 and 40.8, 64 34.6 and 53.2.
-CHUNKS_FROM = 16
+# requests above all, walk token by token, whatever else the step holds.  Measured on B200 (16 heads of 128, all
+# launches, us a layer with that segment in chunks, and with every segment by the scan):
+#   one segment of 64 tokens 54 and 68, of 128 63 and 93, of 512 118 and 368, of 2,048 388 and 900;
+#   behind 8 decoding requests 64 tokens 84 and 69, 96 88 and 85, 128 96 and 112; behind 64, 96 tokens 117 and 112,
+#   128 121 and 122, 512 174 and 302;  4 segments of 128 101 and 138, 8 of 128 175 and 171, 8 of 256 321 and 323.
+# Steps that fill the SMs several times over are dearer in chunks (16 of 128 320 and 286, 16 of 512 1,144 and 1,043): the
+# line cannot follow the number of segments without a request's bits following its company.
+CHUNKS_FROM = 128
 _CHUNK_TOKENS, _CHUNK_DOUBLES = 32, 2 * 32 * 34
 
 
