@@ -348,6 +348,7 @@ int launch(RowsParams prm, cudaStream_t stream) {
 }
 
 constexpr int MAX_ROWS = 32, MAX_NORMED_ROWS = 8, MAX_NORMED_K = 1024;    // normed: K in one chunk
+constexpr int MAX_CONV_TAPS = 16;
 
 template <int EPI, bool NORMED>
 int launch_rows(const RowsParams& prm, cudaStream_t stream) {
@@ -418,7 +419,9 @@ FWB_API int fwb_linear_rows_conv(const void* X, const float* norm_w, float eps, 
                                  const float* conv_bias, float* state, long long state_stride, const int* slots, void* z,
                                  int M, int H, int K, int conv_taps, cudaStream_t stream) {
     if (M <= 0 || H <= 0) return FWB_OK;
-    if (!X || !W || !conv_w || !state || !slots || !z || K <= 0 || conv_taps < 2) return FWB_BAD_ARGUMENT;
+    if (!X || !W || !conv_w || !state || !slots || !z || K <= 0) return FWB_BAD_ARGUMENT;
+    if (conv_taps < 2 || conv_taps > MAX_CONV_TAPS) return FWB_UNSUPPORTED;       // as fwb_shortconv
+    if (state_stride < (long long)H * (conv_taps - 1)) return FWB_BAD_ARGUMENT;
     if (!shape_ok(W, M, K, norm_w ? MAX_NORMED_ROWS : 16) || ((uintptr_t)X & 15)) return FWB_UNSUPPORTED;
     if (norm_w && (((uintptr_t)norm_w & 15) || K > MAX_NORMED_K)) return FWB_UNSUPPORTED;
     const RowsParams prm{(const __nv_bfloat16*)X, (const float*)X, norm_w, nullptr, eps, (const __nv_bfloat16*)W, z, nullptr,

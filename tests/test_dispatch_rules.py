@@ -36,3 +36,16 @@ def test_the_measured_points_of_the_slicing_rule():
     assert chosen(128, 65)[0] == 2                  # one piece would be 1.4 rounds of the SMs
     assert chosen(8, 513) == (8, 65, True)          # 8 x 32,768 keys
     assert chosen(1, 1985)[0] >= 32 and not chosen(1, 1985)[2]      # one long request: a merge kernel
+
+
+def test_a_convolution_step_refuses_what_the_convolution_refuses():
+    """Fewer than two taps, more than sixteen, a slot shorter than its contents: the argument checks of the C entries
+    answer before anything is launched, the folded step as the convolution's own kernel."""
+    from flyweight_b200.kernels import lib
+    unsupported, bad = -2, -1
+    here = 4096                                     # a pointer that nobody reads
+    for taps, stride, want in ((1, 1024, unsupported), (17, 1 << 20, unsupported), (3, 127, bad)):
+        alone = lib.library().fwb_shortconv(here, 1, here, None, here, here, here, here, here, 1, 4, 4, 64, taps, stride, None)
+        folded = lib.library().fwb_linear_rows_conv(here, None, 0.0, here, here, None, here, stride, here, here, 4, 64, 256,
+                                                    taps, None)
+        assert alone == folded == want, (taps, stride)
