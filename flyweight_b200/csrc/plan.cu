@@ -223,8 +223,9 @@ bool rows_takes(int M, int N, int K) {
 }
 bool rows_takes_normed(int M, int N, int K) { return M <= 8 && K <= 1024 && rows_takes(M, N, K); }
 
-bool normed_accepts(int M, int K, const void* w, int accumulators, int N) {
+bool normed_accepts(int M, int K, const void* w, const void* x, const void* norm_w, int accumulators, int N) {
     if (!(g_option[OPT_TENSORCORE] && g_option[OPT_FUSE_NORM]) || M > 64 || K % 8 || !aligned16(w)) return false;
+    if (!aligned16(x) || !aligned16(norm_w)) return false;
     if (rows_takes(M, accumulators * N, K)) return rows_takes_normed(M, accumulators * N, K);
     if (!g_option[OPT_FUSE_ALWAYS]) return false;
     const int splits = g_option[OPT_FORCED_SPLITS] > 0 ? g_option[OPT_FORCED_SPLITS]
@@ -446,7 +447,7 @@ void run_norm_linear(Launches& L, const Op& op, const FwbStep& step, bool& pendi
     void* out = op.on_logit_rows && op.out == nullptr ? step.logits : op.out;
     const bool swiglu = op.epilogue == EPI_SWIGLU_BF16;
     const int accumulators = swiglu ? 2 : 1;
-    if (!pending && op.w_bf16 && act_bf16 && normed_accepts(M, op.K, op.w, accumulators, op.N)) {
+    if (!pending && op.w_bf16 && act_bf16 && normed_accepts(M, op.K, op.w, op.x, op.v0, accumulators, op.N)) {
         // the norm, the product (both products and silu(g)*u) in one kernel
         if (rows_takes_normed(M, accumulators * op.N, op.K)) {
             L.add(fwb_linear_rows_normed(op.x, op.v0, rows, op.eps, op.w, out, M, op.N, op.K, swiglu ? 2 * op.N : op.N,
@@ -493,7 +494,8 @@ bool run_conv_step(Launches& L, const Op& op, const Op& conv, const FwbStep& ste
         !rows_takes(M, op.N, op.K) || conv.out == op.scratch)
         return false;
     const int* slots = meta(step, META_SEG_SLOT);
-    const bool normed = !pending && g_option[OPT_FUSE_NORM] && rows_takes_normed(M, op.N, op.K) && aligned16(op.x);
+    const bool normed = !pending && g_option[OPT_FUSE_NORM] && rows_takes_normed(M, op.N, op.K) && aligned16(op.x) &&
+                        aligned16(op.v0);
     if (!normed) {
         L.add(fwb_rmsnorm(op.x, pending ? op.delta : nullptr, op.v0, op.scratch, 1, nullptr, M, op.K, op.eps, stream));
         pending = false;

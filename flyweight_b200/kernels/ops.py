@@ -154,7 +154,7 @@ def linear(x, w: torch.Tensor, out_dtype: torch.dtype,
     from . import tensorcore
     if not isinstance(x, torch.Tensor):                       # a DeferredNorm
         if (addend is None and x.kind == "rmsnorm"
-                and tensorcore.normed_accepts(x.n_rows, x.x.shape[-1], w, 1, w.shape[0])):
+                and tensorcore.normed_accepts(x.n_rows, x.x.shape[-1], w, 1, w.shape[0], x)):
             return tensorcore.gemm_normed(x.x, x.weight, x.eps, w, out_dtype, rows=x.rows, n_rows=x.n_rows)
         x = x.materialize(torch.float32 if w.dtype == torch.float32 else torch.bfloat16)
     if w.dtype == torch.float32:

@@ -322,6 +322,8 @@ def conv_step_accepts(h, w_in, batch, act_dtype) -> bool:
     """A step of one token per request whose in_proj the weight reader takes does the short convolution in that
     product's epilogue (measured in the decode step: a launch of 4 to 5 us less per convolution layer)."""
     H = w_in.shape[0] // 3
+    if isinstance(h, torch.Tensor) and (h.dtype != torch.bfloat16 or not _aligned(h)):
+        return False                                            # (the projection on its own takes those)
     return (act_dtype == torch.bfloat16 and w_in.dtype == torch.bfloat16 and batch.max_segment == 1
             and batch.n_tokens == batch.n_segments <= 16 and w_in.shape[1] % 8 == 0 and _aligned(w_in)
             and _rows_takes(batch.n_tokens, 3 * H, w_in.shape[1]))
@@ -335,7 +337,7 @@ def conv_step(h, w_in, taps, bias, state, batch) -> torch.Tensor:
     norm_w, eps = None, 0.0
     if isinstance(h, torch.Tensor):
         x = h
-    elif h.kind == "rmsnorm" and h.rows is None and _fuse_norm and _rows_takes_normed(M, 3 * H, K) and _aligned(h.x):
+    elif h.kind == "rmsnorm" and h.rows is None and _fuse_norm and _rows_takes_normed(M, 3 * H, K) and _norm_aligned(h):
         x, norm_w, eps = h.x, h.weight, h.eps
         check_tensor("norm weight", norm_w, torch.float32, (K,))
     else:
@@ -454,11 +456,17 @@ def set_norm_fusion(flag: bool) -> None:
     lib.set_option("add_in_place", _add_in_place)
 
 
-def normed_accepts(M: int, K: int, w, accumulators: int, N: int) -> bool:
+def _norm_aligned(norm) -> bool:
+    return _aligned(norm.x) and _aligned(norm.weight)
+
+
+def normed_accepts(M: int, K: int, w, accumulators: int, N: int, norm=None) -> bool:
     """Decode-sized token counts whose K slice per CTA is short enough that building the
     activation tiles inside the kernel stays off the critical path."""
     if not (_enabled and _fuse_norm) or w.dtype != torch.bfloat16 or M > 64 or K % 8 or not _aligned(w):
         return False
+    if norm is not None and not _norm_aligned(norm):
+        return False                                            # (rows or a weight off a 16-byte border: the norm's kernel)
     if _rows_takes(M, accumulators * N, K):
         return _rows_takes_normed(M, accumulators * N, K)
     if not _fuse_always:

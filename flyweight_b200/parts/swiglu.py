@@ -53,7 +53,7 @@ class SwiGLU(FeedForward):
         act = ctx.precision.act_dtype
         if not isinstance(h, torch.Tensor):                   # a norm not yet applied
             if h.kind == "rmsnorm" and tensorcore.normed_accepts(h.n_rows, self.hidden, self.w_gate_up, 2,
-                                                                  self.ffn_dim):
+                                                                  self.ffn_dim, h):
                 # the norm, both products and silu(g)*u in one kernel
                 a = tensorcore.swiglu_gate_up_normed(h.x, h.weight, h.eps, self.w_gate_up,
                                                      activation=self.activation)

@@ -190,6 +190,45 @@ def test_a_convolution_step_in_the_projection(M, H, K, L, biased):
     assert tensorcore.status() == 0
 
 
+@pytest.mark.parametrize("off", ["residual", "weight", "rows"])
+def test_few_tokens_off_a_16_byte_border(off):
+    """A residual, a norm's weight or bfloat16 rows that begin four or two bytes behind a 16-byte border, and float32
+    rows: the folded forms need the border, so the norm's kernel and the general products take such calls."""
+    from flyweight_b200.kernels import ops, tensorcore
+    from flyweight_b200.parts.base import DeferredNorm
+    M, K, H, L = 4, 256, 64, 3
+    g = torch.Generator().manual_seed(3)
+
+    def place(t, shifted):
+        flat = torch.empty(t.numel() + 1, dtype=t.dtype, device=DEV)
+        view = flat[1 if shifted else 0:][:t.numel()].view(t.shape)
+        return view.copy_(t)
+
+    x, norm = torch.randn(M, K, generator=g), 1.0 + 0.1 * torch.randn(K, generator=g)
+    w, taps = dev((torch.randn(3 * H, K, generator=g) / K ** 0.5).bfloat16()), dev(torch.randn(H, L, generator=g))
+    state, i32 = torch.randn(M, H, L - 1, generator=g), lambda values: torch.tensor(values, dtype=torch.int32, device=DEV)
+    batch = type("Batch", (), {})()
+    batch.n_tokens = batch.n_segments = M
+    batch.max_segment, batch.seg_start, batch.tok_seg, batch.seg_slot = 1, i32([0, 1, 2, 3, 4]), i32([0, 1, 2, 3]), i32([2, 0, 3, 1])
+    plain = ops.rmsnorm(dev(x), dev(norm), 1e-5, torch.bfloat16)
+    want = ops.linear(plain, w, torch.bfloat16)
+    if off != "rows":
+        h = DeferredNorm(place(x, off == "residual"), place(norm, off == "weight"), 1e-5)
+        close(ops.linear(h, w, torch.bfloat16), want, 2.0 ** -6, "norm and product")
+        want = ops.linear(h.materialize(torch.bfloat16), w, torch.bfloat16)
+        one = dev(state)
+        assert tensorcore.conv_step_accepts(h, w, batch, torch.bfloat16)
+        got = tensorcore.conv_step(h, w, taps, None, one, batch)
+        two = dev(state)
+        assert torch.equal(got, ops.shortconv(want, taps, None, two, batch.seg_start, batch.seg_slot, batch.tok_seg, M,
+                                              torch.bfloat16)) and torch.equal(one, two)
+    else:
+        for h in (place(plain.cpu(), True), plain.float()):
+            assert not tensorcore.conv_step_accepts(h, w, batch, torch.bfloat16)
+            close(ops.linear(h, w, torch.bfloat16), want, 2.0 ** -6, "product")
+    assert tensorcore.status() == 0
+
+
 def test_gemm_row_does_not_depend_on_the_batch():
     from flyweight_b200.kernels import ops
     g = torch.Generator().manual_seed(5)
