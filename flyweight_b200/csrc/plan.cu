@@ -669,6 +669,29 @@ FWB_API int fwb_get_option(int option) {
     return option < 0 || option >= OPT_COUNT ? -1 : g_option[option];
 }
 
+// What the rules above say of a product of M tokens (N features, K, one or two accumulators), for a comparison with
+// kernels/tensorcore.py, which states them again.  out[13]: the weight reader takes it, and with the norm folded in; two
+// rings: token tile (0: no), slices of K, stages; sums in place on the pairs; 65 to 512 tokens: pairs, token tile, slices
+// of K; decode-sized: token tile, slices of K as chosen for one accumulator, slices by the rule, ring depth for those.
+FWB_API int fwb_product_rules(int M, int N, int K, int accumulators, int* out) {
+    if (M <= 0 || N <= 0 || K <= 0 || accumulators < 1 || accumulators > 2 || !out) return FWB_BAD_ARGUMENT;
+    for (int i = 0; i < 13; ++i) out[i] = 0;
+    out[0] = rows_takes(M, accumulators * N, K);
+    out[1] = rows_takes_normed(M, accumulators * N, K);
+    int tile = 0, splits = 0, stages = 0;
+    if (two_rings(M, N, K, accumulators, tile, splits, stages)) out[2] = tile, out[3] = splits, out[4] = stages;
+    out[5] = pairs_add(M, N);
+    if (M >= MID_FROM && M <= MID_TO) {
+        out[6] = mid_size_choice(M, N, K, accumulators, accumulators == 1 && M > 128 && N >= 256, tile, splits);
+        if (!out[6]) out[7] = tile, out[8] = splits;
+    }
+    out[9] = decode_tile(M, N);
+    out[10] = pick_splits(M, N, K);
+    out[11] = splits_for(M, N, K, accumulators);
+    out[12] = ring_depth(M, N, out[11], accumulators);
+    return FWB_OK;
+}
+
 FWB_API void* fwb_plan_create(int act_bf16) {
     Plan* plan = new Plan();
     plan->act_bf16 = act_bf16 ? 1 : 0;

@@ -49,3 +49,33 @@ def test_a_convolution_step_refuses_what_the_convolution_refuses():
         folded = lib.library().fwb_linear_rows_conv(here, None, 0.0, here, here, None, here, stride, here, here, 4, 64, 256,
                                                     taps, None)
         assert alone == folded == want, (taps, stride)
+
+
+@pytest.mark.parametrize("switch", ["none", "rows", "mid_size_split", "pairs", "forced_splits"])
+def test_the_products_rules_are_the_same_in_both_languages(switch):
+    """The native step plan states the rules of ``kernels/tensorcore.py`` again: over token counts on both sides of every
+    line, ragged and even features and K, plain and gated, and with each switch turned, both choose the same."""
+    import ctypes
+    from flyweight_b200.kernels import lib, tensorcore as tc
+    turn = {"none": lambda on: None, "rows": tc.set_rows_enabled, "mid_size_split": tc.set_mid_size_split,
+            "pairs": tc.set_pairs_enabled, "forced_splits": lambda on: tc.force_splits(None if on else 2)}[switch]
+    out = (ctypes.c_int * 13)()
+    turn(False)
+    try:
+        for M in (1, 7, 8, 9, 16, 17, 32, 33, 48, 64, 65, 77, 96, 97, 100, 128, 129, 160, 192, 256, 300, 512, 513, 2048):
+            for N in (8, 130, 384, 1000, 1024, 2048, 3072, 3840, 4608, 5120, 6144, 8192, 9472, 9600, 16384, 65536):
+                for K in (8, 64, 504, 1024, 1032, 2048, 4096, 4608, 8192, 10752):
+                    for acc in (1, 2):
+                        assert lib.library().fwb_product_rules(M, N, K, acc, ctypes.addressof(out)) == 0
+                        rings = tc.two_rings(M, N, K, acc) or (0, 0, 0)
+                        mid = (False, 0, 0)
+                        if tc.MID_FROM <= M <= tc.MID_TO:
+                            kind, tile, splits = tc.mid_size_choice(M, N, K, acc, acc == 1 and M > 128 and N >= 256)
+                            mid = (True, 0, 0) if kind == "pair" else (False, tile, splits)
+                        splits = tc._splits_for(M, N, K, acc)
+                        want = (tc._rows_takes(M, acc * N, K), tc._rows_takes_normed(M, acc * N, K), *rings,
+                                tc._pairs_add(M, N), *mid, tc._decode_tile(M, N), tc.pick_splits(M, N, K), splits,
+                                tc._ring_depth(M, N, splits, acc))
+                        assert tuple(out) == tuple(int(v) for v in want), (M, N, K, acc)
+    finally:
+        turn(True)
