@@ -69,9 +69,9 @@ constexpr int epi_warps(int bn) { return bn >= 128 ? 16 : 4; }
 constexpr int threads_for(int bn) { return 64 + 32 * epi_warps(bn); }   // + producer and MMA warps
 constexpr int SMEM_BUDGET = 200 * 1024;
 
-// The WIDE forms give a CTA two adjacent 128-feature tiles (two accumulators over the same
-// token tile): per MMA the activations are read from L2 once for 256 features, which is what
-// keeps the tensor pipe fed at prefill sizes.
+// The WIDE forms (token tiles of 128 and 256) give a CTA two adjacent 128-feature tiles (two accumulators
+// over the same token tile): per MMA the activations are read from L2 once for 256 features.  Prompts take
+// the CTA pairs instead; these run where a caller asks for them or has switched the pairs off.
 enum Epilogue : int { EPI_F32 = 0, EPI_BF16 = 1, EPI_ADD_F32 = 2, EPI_SWIGLU_BF16 = 3,
                       EPI_F32_WIDE = 4, EPI_BF16_WIDE = 5 };
 constexpr bool epi_wide(int epi) { return epi == EPI_F32_WIDE || epi == EPI_BF16_WIDE; }
@@ -532,10 +532,13 @@ int launch_epi(int epi, const CUtensorMap& map_w, const CUtensorMap& map_x, cons
         case EPI_BF16: return launch<BN, EPI_BF16>(map_w, map_x, prm, splits, stream);
         case EPI_ADD_F32: return launch<BN, EPI_ADD_F32>(map_w, map_x, prm, splits, stream);
         case EPI_SWIGLU_BF16: return launch<BN, EPI_SWIGLU_BF16>(map_w, map_x, prm, splits, stream);
-        case EPI_F32_WIDE: return launch<BN, EPI_F32_WIDE>(map_w, map_x, prm, splits, stream);
-        case EPI_BF16_WIDE: return launch<BN, EPI_BF16_WIDE>(map_w, map_x, prm, splits, stream);
-        default: return FWB_UNSUPPORTED;
+        default: break;
     }
+    if constexpr (BN >= 128) {
+        if (epi == EPI_F32_WIDE) return launch<BN, EPI_F32_WIDE>(map_w, map_x, prm, splits, stream);
+        if (epi == EPI_BF16_WIDE) return launch<BN, EPI_BF16_WIDE>(map_w, map_x, prm, splits, stream);
+    }
+    return FWB_UNSUPPORTED;
 }
 
 }  // namespace

@@ -93,7 +93,6 @@ __device__ __forceinline__ void tmem_alloc_pair(uint32_t* holder, uint32_t cols)
 __device__ __forceinline__ void tmem_dealloc_pair(uint32_t addr, uint32_t cols) {
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(addr), "r"(cols) : "memory");
 }
-// One arrival on the barrier at the same offset in CTA `rank` of the cluster.
 // Cluster-window address of `ptr`'s offset in CTA `rank`.
 __device__ __forceinline__ uint32_t cluster_addr(const void* ptr, uint32_t rank) {
     uint32_t remote;

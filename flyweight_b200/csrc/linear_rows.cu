@@ -20,8 +20,9 @@
 //   * Activations are read as A fragments from global memory, one chunk ahead; the NORMED form reads rows
 //     of the fp32 residual, makes bf16(x * w) of them and keeps the rows' sums of squares for
 //     the epilogue: (W (x w)) r = W (x w r).
-//   * The warps' partial sums meet in shared memory and are added in warp order: the result depends
-//     neither on the number of tokens nor on how the features are cut over CTAs.
+//   * The warps' partial sums meet in shared memory and are added in warp order: the result does not depend on
+//     how the features are cut over CTAs, nor on the number of tokens up to 16 (17 to 32 deal K to the warps in
+//     shorter steps, which is another order of the same sums).
 // Every wait on an mbarrier is bounded as in the tcgen05 products.
 //
 // Measured on B200 in a chain of launches over 300 MB of weights (us; tcgen05 kernel, this one; HBM time):
@@ -364,7 +365,7 @@ bool shape_ok(const void* w, int M, int K, int most) { return M <= most && (K & 
 
 }  // namespace
 
-// X: [M][K] bf16, M <= 16; W: [rows][K] bf16; Y: [M][ldy].  Epilogues 0 fp32, 1 bf16 (with an output activation in
+// X: [M][K] bf16, M <= 32; W: [rows][K] bf16; Y: [M][ldy].  Epilogues 0 fp32, 1 bf16 (with an output activation in
 // the bits above the code), 2 fp32 + addend (which may be Y), 3 gated, as fwb_gemm_tcgen05.
 FWB_API int fwb_linear_rows(const void* X, const void* W, void* Y, const float* addend, int M, int N, int K, int w_rows,
                             int ldy, int epilogue, int up_row_offset, float gate_limit, cudaStream_t stream) {
@@ -411,7 +412,7 @@ FWB_API int fwb_linear_rows_normed(const float* x_res, const float* norm_w, cons
     }
 }
 
-// One step of a gated short convolution for requests of one token each: in_proj rows B | C | x ([3H][K], H below one
+// One step of a gated short convolution for requests of one token each (M <= 16, or 8 with the norm): in_proj rows B | C | x ([3H][K], H below one
 // another) on X [M][K] bf16, or (norm_w given) on RMS-normed rows of the fp32 residual X, then
 // z[t][c] = C (bias + sum_k taps[c][k] u) with u = B x behind the `conv_taps` - 1 products in slots[t], which move on.
 // The projections are rounded to bfloat16 in between: the bits of fwb_linear_rows and fwb_shortconv.

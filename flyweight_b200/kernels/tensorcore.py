@@ -410,23 +410,6 @@ def swiglu_gate_up(x, w_gate_up, splits=None, stages=0, tile_tokens=0, activatio
     return out
 
 
-def _wave_cut(M: int, F: int) -> int:
-    """How many 128-feature tiles the whole rounds of one-CTA gated tiles hold (0: no part-filled last round worth
-    cutting off).  The persistent CTA pairs run such products now; tests take ragged sizes from it."""
-    token_tiles = -(-M // 256)
-    feature_tiles = -(-F // 128)
-    ctas = token_tiles * feature_tiles
-    whole = ctas // SM_COUNT
-    left = ctas - whole * SM_COUNT
-    if whole == 0 or left == 0 or left > 0.75 * SM_COUNT:
-        return 0
-    cut = (whole * SM_COUNT) // token_tiles
-    rest = feature_tiles - cut
-    if cut <= 0 or rest <= 0 or rest * -(-M // 128) > SM_COUNT:
-        return 0
-    return cut
-
-
 _fuse_norm = True
 _add_in_place = True
 _fuse_always = False
@@ -536,10 +519,9 @@ def status() -> int:
     return int(lib.library().fwb_gemm_tcgen05_status())
 
 
-def gemm_pair(x, w, out_dtype, wide=False, activation=None) -> torch.Tensor:
+def gemm_pair(x, w, out_dtype, activation=None) -> torch.Tensor:
     """``x @ w.T`` on CTA pairs (tcgen05 cta_group::2), tiles of 256 features x 256 tokens, as many pairs as the GPU
-    holds.  For prompt-sized steps; bf16 in, fp32 or bf16 out.  (``wide`` asked for tiles of two feature blocks, which
-    the persistent pairs do not need: it changes nothing.)"""
+    holds.  For prompt-sized steps; bf16 in, fp32 or bf16 out."""
     check_tensor("gemm input", x, torch.bfloat16)
     check_tensor("gemm weight", w, torch.bfloat16)
     M, K = x.shape
@@ -551,22 +533,6 @@ def gemm_pair(x, w, out_dtype, wide=False, activation=None) -> torch.Tensor:
     lib.call("fwb_gemm_tcgen05_pair", ptr(x), ptr(w), ptr(out), M, N, K, N, N, epilogue, 0, lib.c_float(0.0),
              stream(), tag=f"{N}x{K}")
     return out
-
-
-def _pair_wave_cut(M: int, N: int) -> int:
-    """The same for 512-feature blocks on CTA pairs."""
-    slots = SM_COUNT // 2
-    token_tiles = -(-M // 256)
-    pairs = -(-N // 512) * token_tiles
-    whole = pairs // slots
-    left = pairs - whole * slots
-    if whole == 0 or left == 0 or left > 0.75 * slots:
-        return 0
-    cut = (whole * slots) // token_tiles
-    rest = N - cut * 512
-    if cut <= 0 or rest <= 0 or -(-rest // 256) * token_tiles > slots:
-        return 0
-    return cut
 
 
 def swiglu_gate_up_pair(x, w_gate_up) -> torch.Tensor:

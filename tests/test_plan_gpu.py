@@ -106,7 +106,7 @@ def test_decoding_requests_at_the_head_of_a_step_beside_portions():
     same_steps(runners, steps, "singles then a portion")
 
 
-@pytest.mark.parametrize("switch", ["fuse_always", "pinned", "no_tensor_cores", "no_mixed_split"])
+@pytest.mark.parametrize("switch", ["fuse_always", "pinned", "no_tensor_cores", "no_mixed_split", "no_rows"])
 def test_the_switches_reach_both_paths(switch):
     from flyweight_b200.kernels import attention, tensorcore
     name = "A"
@@ -126,6 +126,9 @@ def test_the_switches_reach_both_paths(switch):
             tensorcore.set_enabled(False)
             attention.set_mma_enabled(False)
             undo += [lambda: tensorcore.set_enabled(True), lambda: attention.set_mma_enabled(True)]
+        elif switch == "no_rows":
+            tensorcore.set_rows_enabled(False)
+            undo.append(lambda: tensorcore.set_rows_enabled(True))
         else:
             attention.set_mixed_split(False)
             undo.append(lambda: attention.set_mixed_split(True))
