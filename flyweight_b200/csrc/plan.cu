@@ -153,21 +153,22 @@ constexpr int MID_FROM = 65, MID_TO = 512;       // between decode steps and pro
 // 33 to 512 tokens, two rings of weights an SM (kernels/tensorcore.py: two_rings).
 bool two_rings(int M, int N, int K, int accumulators, int& tile, int& splits, int& stages) {
     if (g_option[OPT_FORCED_SPLITS] > 0 || M <= 32 || M > MID_TO) return false;
-    const int tiles = ceil_div(N, 128), k_blocks = ceil_div(K, 64), most = 2 * SM_COUNT;
+    const int tiles = ceil_div(N, 128), k_blocks = ceil_div(K, 64);
     if (accumulators == 2) {
         const int t = M <= 64 ? (k_blocks >= 32 ? 64 : 32) : 96;
-        if ((M > 64 && k_blocks < 32) || M > 96 || k_blocks < 16 || tiles * ceil_div(M, t) * 4 > most) return false;
+        if ((M > 64 && k_blocks < 32) || M > 96 || k_blocks < 16 || tiles * ceil_div(M, t) > (t == 32 ? 74 : 70))
+            return false;
         tile = t, splits = 4, stages = 2;
         return true;
     }
     if (M <= 64 || !g_option[OPT_MID_SIZE_SPLIT]) return false;
     if (k_blocks >= 64)
         for (int t = 64; t <= 96; t += 32)
-            if (tiles * ceil_div(M, t) * 8 <= most) {
+            if (tiles * ceil_div(M, t) <= (t == 96 && (M <= 96 || (M > 128 && M <= 192)) ? 37 : 33)) {
                 tile = t, splits = 8, stages = t == 64 ? 4 : 3;
                 return true;
             }
-    if (M <= 128 && k_blocks >= 16 && tiles >= 40 && tiles <= SM_COUNT / 2) {
+    if (M <= 128 && k_blocks >= 16 && tiles >= 40 && tiles <= (M <= 96 ? 70 : 52)) {
         tile = M <= 96 ? 96 : 64, splits = 4, stages = 3;
         return true;
     }

@@ -166,23 +166,30 @@ def two_rings(M: int, N: int, K: int, accumulators: int):
     CTAs, so two rings of weights, on an SM -- one leaves HBM waiting for its latency -- or None for the general rules.
     Measured on B200 (us, the general rule's choice and this one): gated 8192 x 2048 at 64 tokens 23.9 and 20.1, at 77
     23.9 and 22.1; gated 4608 x 1024 at 64 14.8 and 11.3; 2048 x 8192 at 77 17.7 and 13.8, at 160 19.5 and 15.9;
-    1024 x 4608 at 256 13.2 and 10.9; 6144 x 2048 at 77 13.6 and 11.9, at 128 14.2 and 12.7.  csrc/plan.cu has the
-    same rule."""
+    1024 x 4608 at 256 13.2 and 10.9; 6144 x 2048 at 77 13.6 and 11.9, at 128 14.2 and 12.7.
+
+    The lines: all clusters have to be resident at once (a cluster's CTAs lie in one GPC).  Of clusters of four 70 are with
+    two CTAs an SM, 104 with three (8960 x 2048 at 77 tokens 15.2 and 13.8, 9216 x 2048 15.2 and 21.9; 6656 x 2048 at 128
+    14.5 and 12.9, 6912 x 2048 14.7 and 18.7; gated 8960 x 2048 at 64 24.9 and 21.2, 9216 x 2048 24.9 and 32.3), of
+    clusters of eight 33 (2048 x 4096 at 77 11.7 and 10.3, 2176 x 4096 12.2 and 15.4).  34 to 37 of eight are taken where
+    the general choice needs two rounds as well (4352 x 4096 at 77 24.3 and 20.3; 2176 x 4096 at 160 22.6 and 17.7).  Below
+    5,120 features with a short K the general choice is level or better (3840 x 1024 at 77 7.9 and 8.3).  csrc/plan.cu has
+    the same rule."""
     if _forced_splits is not None or M <= 32 or M > MID_TO:
         return None
-    tiles, k_blocks, most = -(-N // 128), -(-K // 64), 2 * SM_COUNT
+    tiles, k_blocks = -(-N // 128), -(-K // 64)
     if accumulators == 2:
         tile = (64 if k_blocks >= 32 else 32) if M <= 64 else 96
-        if (M > 64 and k_blocks < 32) or M > 96 or k_blocks < 16 or tiles * -(-M // tile) * 4 > most:
+        if (M > 64 and k_blocks < 32) or M > 96 or k_blocks < 16 or tiles * -(-M // tile) > (74 if tile == 32 else 70):
             return None
         return tile, 4, 2
     if M <= 64 or not _mid_size_split:
         return None
     if k_blocks >= 64:
         for tile, stages in ((64, 4), (96, 3)):
-            if tiles * -(-M // tile) * 8 <= most:
+            if tiles * -(-M // tile) <= (37 if tile == 96 and (M <= 96 or 128 < M <= 192) else 33):
                 return tile, 8, stages
-    if M <= 128 and k_blocks >= 16 and 40 <= tiles <= SM_COUNT // 2:
+    if M <= 128 and k_blocks >= 16 and 40 <= tiles <= (70 if M <= 96 else 52):
         return (96 if M <= 96 else 64), 4, 3
     return None
 

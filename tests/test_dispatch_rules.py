@@ -79,3 +79,22 @@ def test_the_products_rules_are_the_same_in_both_languages(switch):
                         assert tuple(out) == tuple(int(v) for v in want), (M, N, K, acc)
     finally:
         turn(True)
+
+
+def test_two_rings_of_weights_keep_their_clusters_resident():
+    """A cluster of CTAs lies in one GPC: on this chip 70 clusters of four fit at two CTAs an SM, 104 at three, 33 of eight.
+    A choice beyond that takes a second round, longer than the choice it replaced (9216 x 2048 at 77 tokens 15.2 -> 21.9
+    us), but for the sizes where that one has a second round too."""
+    from flyweight_b200.kernels import tensorcore as tc
+    for M in (33, 64, 65, 96, 97, 128, 129, 160, 192, 193, 256, 300, 384, 512):
+        for tiles in range(1, 160):
+            for k_blocks in (16, 31, 32, 64, 128):
+                for acc in (1, 2):
+                    choice = tc.two_rings(M, tiles * 128, k_blocks * 64, acc)
+                    if choice is None:
+                        continue
+                    tile, splits, stages = choice
+                    an_sm = min(3, 227 * 1024 // (stages * (acc * 16384 + tile * 128) + 2560))
+                    clusters, fit = tiles * -(-M // tile), {(4, 2): 70, (4, 3): 104, (8, 2): 33}[splits, an_sm]
+                    two_rounds_anyway = splits == 8 and tile == 96 and (tiles >= 34 or 128 < M <= 192 and tiles >= 17)
+                    assert clusters <= fit or (two_rounds_anyway and clusters <= 37), (M, tiles, k_blocks, acc, choice)
