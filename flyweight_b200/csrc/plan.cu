@@ -214,13 +214,34 @@ bool tc_accepts(const void* x, const void* w, int M, int K) {
     return g_option[OPT_TENSORCORE] && K % 8 == 0 && K >= 8 && aligned16(x) && aligned16(w) && M <= 65535 * 16;
 }
 
-// a few tokens: the weight reader (kernels/tensorcore.py: _rows_takes, _rows_takes_normed); N: rows of the matrix
+// a few tokens: the weight reader (kernels/tensorcore.py: _rows_takes and what it calls); N: rows of the matrix
+bool rows_on() { return g_option[OPT_TENSORCORE] && g_option[OPT_ROWS] && g_option[OPT_FORCED_SPLITS] <= 0; }
+double rows_share(int N) {
+    const int units = ceil_div(N, 8), per_cta = ceil_div(units, 2 * SM_COUNT), ctas = ceil_div(units, per_cta);
+    return units <= 2 * SM_COUNT ? 1.0 : (double)units / ((double)SM_COUNT * per_cta * ceil_div(ctas, SM_COUNT));
+}
+bool all_resident(int M, int N, int K) {
+    const int splits = splits_for(M, N, K, 1), clusters = ceil_div(N, 128) * ceil_div(M, decode_tile(M, N));
+    const int an_sm = ceil_div(clusters * splits, SM_COUNT);
+    return clusters <= (splits == 1 ? SM_COUNT : splits == 2 ? SM_COUNT / 2 : splits == 4 ? 35 : 16) * an_sm;
+}
 bool rows_takes(int M, int N, int K) {
-    if (!g_option[OPT_TENSORCORE] || !g_option[OPT_ROWS] || g_option[OPT_FORCED_SPLITS] > 0) return false;
-    static const long long limits[3][3] = {{8, 1 << 20, 1 << 26}, {16, 2048, 1 << 26}, {32, 1024, 1 << 24}};
-    for (const auto& limit : limits)
-        if (M <= limit[0] && K <= limit[1] && (long long)N * K <= limit[2]) return true;
-    return false;
+    const long long weights = (long long)N * K;
+    if (!rows_on() || M > 32 || weights > 1 << 26) return false;
+    if (M <= 8) {
+        if (K <= 1024) return N <= (K < 512 ? 24 : 32) * K;
+        if (K < 2048) return N <= 7 * K;
+        return K <= 4096 || rows_share(N) >= 0.85;
+    }
+    if (M <= 16) {
+        if (K <= 1024) return N <= (K < 512 ? 12 : 24) * K && (K < 512 || N <= 18432);
+        return K <= 2048 && N <= (M <= 12 && K >= 1920 ? 8192 : 4096);
+    }
+    if (K > 1024 || weights > 1 << 24) return false;
+    return (N <= (K < 512 ? 12 : 18) * K && N <= (1 << 22) / K) || (N <= 9472 && !all_resident(M, N, K));
+}
+bool rows_takes_conv(int M, int N, int K) {
+    return rows_on() && (long long)N * K <= 1 << 26 && (M <= 8 || (M <= 16 && K <= 2048));
 }
 bool rows_takes_normed(int M, int N, int K) { return M <= 8 && K <= 1024 && rows_takes(M, N, K); }
 
@@ -492,10 +513,10 @@ bool run_conv_step(Launches& L, const Op& op, const Op& conv, const FwbStep& ste
     if (conv.kind != OP_SHORTCONV || conv.in != op.out || op.epilogue != EPI_BF16 || op.on_logit_rows || op.N != 3 * conv.K)
         return false;
     if (!act_bf16 || !op.w_bf16 || step.max_segment != 1 || step.S != M || M > 16 || op.K % 8 || !aligned16(op.w) ||
-        !rows_takes(M, op.N, op.K) || conv.out == op.scratch)
+        !rows_takes_conv(M, op.N, op.K) || conv.out == op.scratch)
         return false;
     const int* slots = meta(step, META_SEG_SLOT);
-    const bool normed = !pending && g_option[OPT_FUSE_NORM] && rows_takes_normed(M, op.N, op.K) && aligned16(op.x) &&
+    const bool normed = !pending && g_option[OPT_FUSE_NORM] && M <= 8 && op.K <= 1024 && aligned16(op.x) &&
                         aligned16(op.v0);
     if (!normed) {
         L.add(fwb_rmsnorm(op.x, pending ? op.delta : nullptr, op.v0, op.scratch, 1, nullptr, M, op.K, op.eps, stream));
@@ -671,12 +692,13 @@ FWB_API int fwb_get_option(int option) {
 }
 
 // What the rules above say of a product of M tokens (N features, K, one or two accumulators), for a comparison with
-// kernels/tensorcore.py, which states them again.  out[13]: the weight reader takes it, and with the norm folded in; two
+// kernels/tensorcore.py, which states them again.  out[14]: the weight reader takes it, and with the norm folded in; two
 // rings: token tile (0: no), slices of K, stages; sums in place on the pairs; 65 to 512 tokens: pairs, token tile, slices
-// of K; decode-sized: token tile, slices of K as chosen for one accumulator, slices by the rule, ring depth for those.
+// of K; decode-sized: token tile, slices of K as chosen for one accumulator, slices by the rule, ring depth for those; the
+// weight reader with a convolution's step.
 FWB_API int fwb_product_rules(int M, int N, int K, int accumulators, int* out) {
     if (M <= 0 || N <= 0 || K <= 0 || accumulators < 1 || accumulators > 2 || !out) return FWB_BAD_ARGUMENT;
-    for (int i = 0; i < 13; ++i) out[i] = 0;
+    for (int i = 0; i < 14; ++i) out[i] = 0;
     out[0] = rows_takes(M, accumulators * N, K);
     out[1] = rows_takes_normed(M, accumulators * N, K);
     int tile = 0, splits = 0, stages = 0;
@@ -690,6 +712,7 @@ FWB_API int fwb_product_rules(int M, int N, int K, int accumulators, int* out) {
     out[10] = pick_splits(M, N, K);
     out[11] = splits_for(M, N, K, accumulators);
     out[12] = ring_depth(M, N, out[11], accumulators);
+    out[13] = rows_takes_conv(M, N, K);
     return FWB_OK;
 }
 

@@ -67,9 +67,17 @@ def set_pairs_enabled(flag: bool) -> None:
 # ---- decode steps of a few requests: csrc/linear_rows.cu -----------------------------------
 # A few tokens' products run on a kernel that streams weights straight to mma.sync instead of through tiles of tensor
 # memory: a decode step is a chain of small launches, and what counts is the time from the activations to the result.
-# (tokens, longest K, most weights): behind these lines the activations that every CTA reads cost more than that saves
-# (csrc/linear_rows.cu has the figures).
-ROWS_LIMITS = ((8, 1 << 20, 1 << 26), (16, 2048, 1 << 26), (32, 1024, 1 << 24))
+# The lines (us on B200, tcgen05 kernel and this one; more sizes in csrc/linear_rows.cu), N being the matrix's rows:
+#  * The walk over K goes 1,024 at a time, so a shorter K leaves warps idle and one a little longer than a step or two
+#    pays for steps half empty: 8 tokens, 16384 x 512 8.2 and 6.9, 32768 x 512 8.4 and 11.0, 65536 x 1024 22.7 and 25.2,
+#    8192 x 1536 8.9 and 7.4, 28672 x 1536 16.6 and 18.5.
+#  * Every CTA reads all activations and keeps partial sums of its features: with 9 and more tokens wide matrices take
+#    another round of CTAs (16 tokens, 18432 x 1024 +-0, 19456 x 1024 1.2 times, 65536 x 1024 23.6 and 35.3).
+#  * With a long K the tcgen05 kernel cuts K finely, and a share of features that leaves SMs idle decides: 8 tokens,
+#    4864 x 5120 1.13 times its time (share 0.69), 6144 x 5120 1.02 (0.87), 4096 x 5120 0.8 (0.87).
+#  * 17 to 32 tokens besides where the tcgen05 kernel's clusters would not all be resident (see ``two_rings``):
+#    9216 x 1024 at 24 11.4 and 8.1, against 9728 x 1024 7.4 and 10.8.
+ROWS_LONG_K, ROWS_LEAST_SHARE = 4096, 0.85
 # The norm in front is folded in where K is one step of the kernel's walk: 1024 x 1024 at 8 tokens 3.3 us against 3.5 for
 # the norm's kernel and the product, 9216 x 1024 5.2 against 6.2; with K = 2048 it loses (6144 x 2048: 7.6 against 6.9).
 ROWS_NORMED_TO, ROWS_NORMED_K = 8, 1024
@@ -85,13 +93,51 @@ def set_rows_enabled(flag: bool) -> None:
 
 def _rows_takes(M: int, N: int, K: int) -> bool:
     """``N``: rows of the matrix (gate and up together)."""
-    if not (_enabled and _use_rows) or _forced_splits is not None:
+    if not (_enabled and _use_rows) or _forced_splits is not None or M > 32 or N * K > 1 << 26:
         return False
-    return any(M <= tokens and K <= longest and N * K <= most for tokens, longest, most in ROWS_LIMITS)
+    if M <= 8:
+        if K <= 1024:
+            return N <= (24 if K < 512 else 32) * K
+        if K < 2048:
+            return N <= 7 * K
+        return K <= ROWS_LONG_K or _rows_share(N) >= ROWS_LEAST_SHARE
+    if M <= 16:
+        if K <= 1024:
+            return N <= (12 * K if K < 512 else min(24 * K, 18432))
+        return K <= 2048 and N <= (8192 if M <= 12 and K >= 1920 else 4096)
+    if K > 1024 or N * K > 1 << 24:
+        return False
+    return N <= min((12 if K < 512 else 18) * K, (1 << 22) // K) or (N <= 9472 and not _all_resident(M, N, K))
+
+
+def _rows_share(N: int) -> float:
+    """How even the weight reader's CTAs (up to 8 tokens: two an SM, groups of eight features) lie on the SMs: the mean
+    over the fullest."""
+    units = -(-N // 8)
+    if units <= 2 * SM_COUNT:
+        return 1.0                  # one group a CTA
+    per_cta = -(-units // (2 * SM_COUNT))
+    ctas = -(-units // per_cta)
+    return units / (SM_COUNT * per_cta * -(-ctas // SM_COUNT))
+
+
+def _all_resident(M: int, N: int, K: int) -> bool:
+    """Whether the clusters of the tcgen05 kernel's choice for a decode-sized product all run at once."""
+    splits = _splits_for(M, N, K, 1)
+    clusters = -(-N // 128) * -(-M // _decode_tile(M, N))
+    an_sm = -(-clusters * splits // SM_COUNT)
+    return clusters <= {1: SM_COUNT, 2: SM_COUNT // 2, 4: 35, 8: 16}[splits] * an_sm
 
 
 def _rows_takes_normed(M: int, N: int, K: int) -> bool:
     return M <= ROWS_NORMED_TO and K <= ROWS_NORMED_K and _rows_takes(M, N, K)
+
+
+def _rows_takes_conv(M: int, N: int, K: int) -> bool:
+    """A convolution step saves the convolution's launch, 4 to 5 us, which outweighs what the product itself may lose."""
+    if not (_enabled and _use_rows) or _forced_splits is not None:
+        return False
+    return N * K <= 1 << 26 and (M <= 8 or (M <= 16 and K <= 2048))
 
 
 # Per-shape overrides found by measurement: (features, K, accumulators) -> (splits, stages);
@@ -333,7 +379,7 @@ def conv_step_accepts(h, w_in, batch, act_dtype) -> bool:
         return False                                            # (the projection on its own takes those)
     return (act_dtype == torch.bfloat16 and w_in.dtype == torch.bfloat16 and batch.max_segment == 1
             and batch.n_tokens == batch.n_segments <= 16 and w_in.shape[1] % 8 == 0 and _aligned(w_in)
-            and _rows_takes(batch.n_tokens, 3 * H, w_in.shape[1]))
+            and _rows_takes_conv(batch.n_tokens, 3 * H, w_in.shape[1]))
 
 
 def conv_step(h, w_in, taps, bias, state, batch) -> torch.Tensor:
@@ -344,7 +390,7 @@ def conv_step(h, w_in, taps, bias, state, batch) -> torch.Tensor:
     norm_w, eps = None, 0.0
     if isinstance(h, torch.Tensor):
         x = h
-    elif h.kind == "rmsnorm" and h.rows is None and _fuse_norm and _rows_takes_normed(M, 3 * H, K) and _norm_aligned(h):
+    elif h.kind == "rmsnorm" and h.rows is None and _fuse_norm and M <= ROWS_NORMED_TO and K <= ROWS_NORMED_K and _norm_aligned(h):
         x, norm_w, eps = h.x, h.weight, h.eps
         check_tensor("norm weight", norm_w, torch.float32, (K,))
     else:

@@ -59,12 +59,12 @@ def test_the_products_rules_are_the_same_in_both_languages(switch):
     from flyweight_b200.kernels import lib, tensorcore as tc
     turn = {"none": lambda on: None, "rows": tc.set_rows_enabled, "mid_size_split": tc.set_mid_size_split,
             "pairs": tc.set_pairs_enabled, "forced_splits": lambda on: tc.force_splits(None if on else 2)}[switch]
-    out = (ctypes.c_int * 13)()
+    out = (ctypes.c_int * 14)()
     turn(False)
     try:
-        for M in (1, 7, 8, 9, 16, 17, 32, 33, 48, 64, 65, 77, 96, 97, 100, 128, 129, 160, 192, 256, 300, 512, 513, 2048):
-            for N in (8, 130, 384, 1000, 1024, 2048, 3072, 3840, 4608, 5120, 6144, 8192, 9472, 9600, 16384, 65536):
-                for K in (8, 64, 504, 1024, 1032, 2048, 4096, 4608, 8192, 10752):
+        for M in (1, 7, 8, 9, 12, 13, 16, 17, 32, 33, 48, 64, 65, 77, 96, 97, 100, 128, 129, 160, 192, 256, 300, 512, 513, 2048):
+            for N in (8, 130, 384, 1000, 1024, 2048, 3072, 3840, 4608, 4864, 5120, 6144, 8192, 9216, 9600, 16384, 65536):
+                for K in (8, 64, 256, 504, 512, 1024, 1032, 1912, 2048, 4096, 4608, 8192, 10752):
                     for acc in (1, 2):
                         assert lib.library().fwb_product_rules(M, N, K, acc, ctypes.addressof(out)) == 0
                         rings = tc.two_rings(M, N, K, acc) or (0, 0, 0)
@@ -75,7 +75,7 @@ def test_the_products_rules_are_the_same_in_both_languages(switch):
                         splits = tc._splits_for(M, N, K, acc)
                         want = (tc._rows_takes(M, acc * N, K), tc._rows_takes_normed(M, acc * N, K), *rings,
                                 tc._pairs_add(M, N), *mid, tc._decode_tile(M, N), tc.pick_splits(M, N, K), splits,
-                                tc._ring_depth(M, N, splits, acc))
+                                tc._ring_depth(M, N, splits, acc), tc._rows_takes_conv(M, N, K))
                         assert tuple(out) == tuple(int(v) for v in want), (M, N, K, acc)
     finally:
         turn(True)
@@ -98,3 +98,15 @@ def test_two_rings_of_weights_keep_their_clusters_resident():
                     clusters, fit = tiles * -(-M // tile), {(4, 2): 70, (4, 3): 104, (8, 2): 33}[splits, an_sm]
                     two_rounds_anyway = splits == 8 and tile == 96 and (tiles >= 34 or 128 < M <= 192 and tiles >= 17)
                     assert clusters <= fit or (two_rounds_anyway and clusters <= 37), (M, tiles, k_blocks, acc, choice)
+
+
+def test_the_weight_reader_leaves_what_it_is_slower_at():
+    """Sizes on both sides of its lines (measured beside the rule): a head of 65,536 features over 1,024 channels, short
+    K under many features, wide matrices from nine tokens on, shares that leave SMs idle under a long K."""
+    from flyweight_b200.kernels import tensorcore as tc
+    for M, N, K in ((1, 65536, 1024), (8, 65536, 1024), (16, 65536, 1024), (8, 32768, 512), (8, 28672, 1536), (8, 4864, 5120),
+                    (16, 19456, 1024), (16, 9216, 1536), (16, 6144, 2048), (24, 9728, 1024), (32, 8192, 1024), (32, 16384, 512)):
+        assert not tc._rows_takes(M, N, K), (M, N, K)
+    for M, N, K in ((1, 1024, 1024), (8, 9216, 1024), (8, 32768, 1024), (8, 2048, 8192), (8, 16384, 2048), (8, 6144, 5120),
+                    (16, 18432, 1024), (16, 2048, 2048), (12, 6144, 2048), (24, 3072, 1024), (24, 9216, 1024), (32, 8192, 512)):
+        assert tc._rows_takes(M, N, K), (M, N, K)
