@@ -543,15 +543,16 @@ void run_linear_residual(Launches& L, const Op& op, const FwbStep& step, bool& p
 void decode_splits(int n_tokens, int n_kv, int max_tiles, int head_dim, int& splits, int& tiles_per_split,
                    bool& in_cluster) {
     // the same rule as kernels/attention.py: decode_splits (the measurements are quoted there): as many
-    // slices as keep every CTA resident at once, of 8 (2 below one CTA an SM) to 128 tiles; else the fewest that fill the SMs'
-    // last round to 85 %
+    // slices as keep every CTA resident at once, of 8 (2 below one CTA an SM, where that pays) to 128 tiles; else the
+    // fewest that fill the SMs' last round to 85 %
     const long pairs = (long)n_tokens * n_kv > 1 ? (long)n_tokens * n_kv : 1;
     const long resident = (long)SM_COUNT * (head_dim <= 64 ? 5 : 3);
     int least = 1;
     while (least * 128 < max_tiles && least < 64) least *= 2;
+    const int pays_from = pairs * 4 <= SM_COUNT ? (head_dim <= 64 ? 6 : 8) : (head_dim <= 64 ? 10 : 12);
     int choice = 0;
     for (int s = least; s <= 64 && pairs * s <= resident &&
-                        (s == least || s * 8 <= max_tiles || (s <= 8 && s * 2 <= max_tiles && pairs * s <= SM_COUNT));
+                        (s == least || s * 8 <= max_tiles || (s <= 8 && s * 2 <= max_tiles && pays_from <= max_tiles && pairs * s <= SM_COUNT));
          s *= 2)
         choice = s;
     if (!choice)
@@ -713,6 +714,15 @@ FWB_API int fwb_product_rules(int M, int N, int K, int accumulators, int* out) {
     out[11] = splits_for(M, N, K, accumulators);
     out[12] = ring_depth(M, N, out[11], accumulators);
     out[13] = rows_takes_conv(M, N, K);
+    return FWB_OK;
+}
+
+// The slices of a decode step's contexts: out[3] = slices, tiles a slice, merged in a cluster.
+FWB_API int fwb_decode_attention_rule(int n_tokens, int n_kv, int max_tiles, int head_dim, int* out) {
+    if (n_tokens <= 0 || n_kv <= 0 || max_tiles <= 0 || !out) return FWB_BAD_ARGUMENT;
+    bool in_cluster = false;
+    decode_splits(n_tokens, n_kv, max_tiles, head_dim, out[0], out[1], in_cluster);
+    out[2] = in_cluster;
     return FWB_OK;
 }
 

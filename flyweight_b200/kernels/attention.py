@@ -91,7 +91,10 @@ def decode_splits(n_tokens: int, n_kv: int, max_tiles: int, head_dim: int = 64):
     # them as that allows: 8 x 4,096 keys in 8 slices (512 CTAs) 15.5 us, 16 x 4,096 in 4 slices 25.4 us
     # (in 8: 32.7), 32 x 4,096 in 2 slices 45.9 us (in 8: 52.9), 64 x 4,096 in one piece 83.7 us (in 8:
     # 91.8).  A slice has at least 8 tiles -- 2 while the CTAs do not fill the SMs and merge as a cluster (1 x 1,000
-    # keys: 8.4 us in 2 slices, 5.9 in 4, 4.8 in 8) -- and at most 128: the grid is laid out for the longest request
+    # keys: 8.4 us in 2 slices, 5.9 in 4, 4.8 in 8), from as many tiles on as pay for the merge (head size 64: 8 pairs of
+    # token and KV head, 6 tiles 5.6 us in one piece and 5.0 in two, 64 pairs 8 tiles 7.0 and 7.3, 10 tiles 8.6 and 7.4;
+    # head size 128: 8 pairs 5 tiles 6.4 and 7.0, 8 tiles 8.2 and, in four, 5.3; 64 pairs 8 tiles 9.2 and 10.2, 12 tiles
+    # 12.7 and 12.0) -- and at most 128: the grid is laid out for the longest request
     # of the step, and one long request among short ones must not walk its context alone.  Where the
     # CTAs cannot all be resident, the fewest slices that fill the last round of the SMs to 85 % (128 x
     # 4,096 in one piece is 1.4 rounds: 182 us; in two slices 163 us).  Up to 8 slices merge inside the
@@ -101,11 +104,15 @@ def decode_splits(n_tokens: int, n_kv: int, max_tiles: int, head_dim: int = 64):
     least = 1
     while least * 128 < max_tiles and least < 64:
         least *= 2
+    if pairs * 4 <= SM_COUNT:
+        pays_from = 6 if head_dim <= 64 else 8
+    else:
+        pays_from = 10 if head_dim <= 64 else 12
     choice = 0
     splits = least
     while splits <= 64 and pairs * splits <= resident and (
             splits == least or splits * 8 <= max_tiles
-            or (splits <= 8 and splits * 2 <= max_tiles and pairs * splits <= SM_COUNT)):
+            or (splits <= 8 and max(splits * 2, pays_from) <= max_tiles and pairs * splits <= SM_COUNT)):
         choice = splits
         splits *= 2
     if not choice:

@@ -110,3 +110,19 @@ def test_the_weight_reader_leaves_what_it_is_slower_at():
     for M, N, K in ((1, 1024, 1024), (8, 9216, 1024), (8, 32768, 1024), (8, 2048, 8192), (8, 16384, 2048), (8, 6144, 5120),
                     (16, 18432, 1024), (16, 2048, 2048), (12, 6144, 2048), (24, 3072, 1024), (24, 9216, 1024), (32, 8192, 512)):
         assert tc._rows_takes(M, N, K), (M, N, K)
+
+
+def test_the_slicing_rule_is_the_same_in_both_languages_and_merges_only_what_pays():
+    import ctypes
+    from flyweight_b200.kernels import lib
+    out = (ctypes.c_int * 3)()
+    for head_dim in (64, 128):
+        for n_kv in (1, 2, 4, 8):
+            for n_tokens in (1, 2, 4, 8, 9, 16, 18, 32, 37, 64, 74, 75, 128, 300):
+                for max_tiles in (*range(1, 33), 64, 65, 129, 513, 1985, 9000):
+                    chosen = attention.decode_splits(n_tokens, n_kv, max_tiles, head_dim)
+                    assert lib.library().fwb_decode_attention_rule(n_tokens, n_kv, max_tiles, head_dim, ctypes.addressof(out)) == 0
+                    assert tuple(out) == tuple(int(v) for v in chosen), (n_tokens, n_kv, max_tiles, head_dim)
+    slices = lambda pairs, tiles, head_dim: attention.decode_splits(pairs, 1, tiles, head_dim)[0]
+    assert slices(8, 5, 64) == 1 and slices(8, 6, 64) == 2 and slices(64, 8, 64) == 1 and slices(64, 10, 64) == 2
+    assert slices(8, 7, 128) == 1 and slices(8, 8, 128) == 4 and slices(64, 8, 128) == 1 and slices(64, 12, 128) == 2
