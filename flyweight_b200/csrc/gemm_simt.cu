@@ -78,12 +78,12 @@ gemm_simt_kernel(const TX* __restrict__ X, const TW* __restrict__ W, TY* __restr
 // K-major, so they go to shared memory as they lie, by asynchronous 16-byte copies, three stages of
 // 64 k deep, and a thread reads four consecutive k of a row at once.  Rows are 68 floats apart, which
 // puts the eight rows that neighbouring lanes read on different banks.  An accumulator is a pair: even k and
-// odd k, plain multiply-adds (packed ones, fma.rn.f32x2, gave the same bits and took 147 us instead of 89 for
+// odd k, plain multiply-adds (packed ones, fma.rn.f32x2, gave the same bits and took 1.6 times as long for
 // 201 x 1024 x 4608).  Four groups of 64 threads take 16 of the 64 k of every stage each: an output tile of
 // 64 x 32 keeps eight warps busy, and a 201 x 1024 product fills 128 SMs.
-// Measured on B200 (us; the kernel below this one, then this one): 201 x 9216 x 1024 289 -> 121,
-// 201 x 1024 x 4608 345 -> 92, 64 x 9216 x 1024 93 -> 38 (32 TFLOP/s), 8 x 1024 x 4608 314 -> 24,
-// 1 x 9216 x 1024 83 -> 23; relative error against 64 bits 5.7e-7 -> 2.1e-7 at K = 1024.
+// Measured on B200 in a chain of launches over 300 MB of weights (us; gemm_simt_kernel, then this one):
+// 201 x 9216 x 1024 288 -> 121, 201 x 1024 x 4608 378 -> 76, 64 x 9216 x 1024 100 -> 39 (31 TFLOP/s),
+// 8 x 1024 x 4608 403 -> 35, 1 x 9216 x 1024 94 -> 21; relative error against 64 bits 5.7e-7 -> 2.1e-7 at K = 1024.
 constexpr int FK = 64, FSTRIDE = FK + 4, FSTAGES = 3;
 
 __device__ __forceinline__ void fma_four(float2& acc, const float4& a, const float4& b) {
