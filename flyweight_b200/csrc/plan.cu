@@ -235,7 +235,7 @@ bool rows_takes(int M, int N, int K) {
     }
     if (M <= 16) {
         if (K <= 1024) return N <= (K < 512 ? 12 : 24) * K && (K < 512 || N <= 18432);
-        return K <= 2048 && N <= (M <= 12 && K >= 1920 ? 8192 : 4096);
+        return K < 1920 ? N <= 4096 : K <= 2048 && (N <= 8192 || (N >= 13312 && N <= 18432));
     }
     if (K > 1024 || weights > 1 << 24) return false;
     return (N <= (K < 512 ? 12 : 18) * K && N <= (1 << 22) / K) || (N <= 9472 && !all_resident(M, N, K));

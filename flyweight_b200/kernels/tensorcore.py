@@ -73,6 +73,8 @@ def set_pairs_enabled(flag: bool) -> None:
 #    8192 x 1536 8.9 and 7.4, 28672 x 1536 16.6 and 18.5.
 #  * Every CTA reads all activations and keeps partial sums of its features: with 9 and more tokens wide matrices take
 #    another round of CTAs (16 tokens, 18432 x 1024 +-0, 19456 x 1024 1.2 times, 65536 x 1024 23.6 and 35.3).
+#    Up to 18,432 features over 2,048 channels they win but for the middle (12 tokens: 8192 9.6 and 8.8, 9728 x 2048 behind
+#    a norm 11.5 and 11.7, 12288 12.9 and 13.5, 16384 16.4 and 14.6, where the tcgen05 kernel's CTAs make a round and a half).
 #  * With a long K the tcgen05 kernel cuts K finely, and a share of features that leaves SMs idle decides: 8 tokens,
 #    4864 x 5120 1.13 times its time (share 0.69), 6144 x 5120 1.02 (0.87), 4096 x 5120 0.8 (0.87).
 #  * 17 to 32 tokens besides where the tcgen05 kernel's clusters would not all be resident (see ``two_rings``):
@@ -104,7 +106,9 @@ def _rows_takes(M: int, N: int, K: int) -> bool:
     if M <= 16:
         if K <= 1024:
             return N <= (12 * K if K < 512 else min(24 * K, 18432))
-        return K <= 2048 and N <= (8192 if M <= 12 and K >= 1920 else 4096)
+        if K < 1920:
+            return N <= 4096
+        return K <= 2048 and (N <= 8192 or 13312 <= N <= 18432)
     if K > 1024 or N * K > 1 << 24:
         return False
     return N <= min((12 if K < 512 else 18) * K, (1 << 22) // K) or (N <= 9472 and not _all_resident(M, N, K))

@@ -63,7 +63,7 @@ def test_the_products_rules_are_the_same_in_both_languages(switch):
     turn(False)
     try:
         for M in (1, 7, 8, 9, 12, 13, 16, 17, 32, 33, 48, 64, 65, 77, 96, 97, 100, 128, 129, 160, 192, 256, 300, 512, 513, 2048):
-            for N in (8, 130, 384, 1000, 1024, 2048, 3072, 3840, 4608, 4864, 5120, 6144, 8192, 9216, 9600, 16384, 65536):
+            for N in (8, 130, 384, 1000, 1024, 2048, 3072, 3840, 4608, 4864, 5120, 6144, 8192, 9216, 9600, 13312, 16384, 65536):
                 for K in (8, 64, 256, 504, 512, 1024, 1032, 1912, 2048, 4096, 4608, 8192, 10752):
                     for acc in (1, 2):
                         assert lib.library().fwb_product_rules(M, N, K, acc, ctypes.addressof(out)) == 0
@@ -105,10 +105,10 @@ def test_the_weight_reader_leaves_what_it_is_slower_at():
     K under many features, wide matrices from nine tokens on, shares that leave SMs idle under a long K."""
     from flyweight_b200.kernels import tensorcore as tc
     for M, N, K in ((1, 65536, 1024), (8, 65536, 1024), (16, 65536, 1024), (8, 32768, 512), (8, 28672, 1536), (8, 4864, 5120),
-                    (16, 19456, 1024), (16, 9216, 1536), (16, 6144, 2048), (24, 9728, 1024), (32, 8192, 1024), (32, 16384, 512)):
+                    (16, 19456, 1024), (16, 9216, 1536), (16, 12288, 2048), (24, 9728, 1024), (32, 8192, 1024), (32, 16384, 512)):
         assert not tc._rows_takes(M, N, K), (M, N, K)
     for M, N, K in ((1, 1024, 1024), (8, 9216, 1024), (8, 32768, 1024), (8, 2048, 8192), (8, 16384, 2048), (8, 6144, 5120),
-                    (16, 18432, 1024), (16, 2048, 2048), (12, 6144, 2048), (24, 3072, 1024), (24, 9216, 1024), (32, 8192, 512)):
+                    (16, 18432, 1024), (16, 2048, 2048), (12, 6144, 2048), (16, 16384, 2048), (24, 3072, 1024), (24, 9216, 1024), (32, 8192, 512)):
         assert tc._rows_takes(M, N, K), (M, N, K)
 
 
