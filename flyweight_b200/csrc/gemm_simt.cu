@@ -1,16 +1,18 @@
 // Y[M][N] = X[M][K] * W[N][K]^T (+ addend), plain SIMT with fp32 FMA accumulation.
 //
-// This is the true 32-bit matrix product of the engine (no tensor-core mode of any
-// kind), and the fallback of the bfloat16 path for shapes the tensor-core kernel
-// refuses.  Any M, N, K >= 1.  The order in which an output element's products are added depends
+// This is the true 32-bit matrix product of the engine, and the fallback of the bfloat16
+// path for shapes the tensor-core kernel refuses.  Any M, N, K >= 1.  The order in which an output element's products are added depends
 // on the kernel alone, and which kernel runs on the types, K, ldx and the operands' alignment alone:
 // the value at [m][n] does not depend on M or on which other rows share the launch.
 //
+//   gemm_f32_tcgen05.cu   fp32 throughout, 16-byte copies, N and K from 128 on: exact thirds of
+//                     the values on the tensor cores, closer to the exact sum than the others.
 //   gemm_f32_kernel   fp32 throughout, rows that 16-byte copies can read (K, ldx multiples of 4):
 //                     eight partial sums an element (four quarters of every 64 k, even and odd k
 //                     apart), added in a fixed order.
 //   gemm_simt_kernel  everything else: one accumulator that walks k = 0..K-1.
 #include "common.cuh"
+#include "gemm_f32.cuh"
 
 using namespace fwb;
 
@@ -254,6 +256,8 @@ FWB_API int fwb_gemm_simt(const void* X, int x_bf16, const void* W, int w_bf16, 
     const int key = (x_bf16 ? 4 : 0) | (w_bf16 ? 2 : 0) | (y_bf16 ? 1 : 0);
     switch (key) {
         case 0:
+            if (!(K & 3) && !(ldx & 3) && !((uintptr_t)X & 15) && !((uintptr_t)W & 15) && gemm_f32_split_takes(N, K))
+                return gemm_f32_split((const float*)X, (const float*)W, (float*)Y, addend, M, N, K, ldx, ldy, stream);
             if (!(K & 3) && !(ldx & 3) && !((uintptr_t)X & 15) && !((uintptr_t)W & 15) && N <= 16 * 65535)
                 return dispatch_f32((const float*)X, (const float*)W, (float*)Y, addend, M, N, K, ldx, ldy, stream);
             return launch<float, float, float>(X, W, Y, addend, M, N, K, ldx, ldy, stream);

@@ -123,10 +123,6 @@ struct Params {
     int group_w_rows;
 };
 
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-
 // NORMED forms, run by the 128 threads of the four epilogue warps: for every 64-wide block of
 // this CTA's K slice, write bf16(x[t][k] * w[k]) for the tile's tokens into the ring slot's B
 // tile (128-byte rows, 16-byte chunks XOR-swizzled by row: what TMA would have left) and arrive
