@@ -493,14 +493,22 @@ delta_chunk_kernel(const float* __restrict__ r, const int* __restrict__ seg_star
 }
 
 constexpr int RUN_COLS = 16;
+constexpr int COL = 36, UN_ROW = 20;                   // columns of r and u, rows of D_Cj u_j: a fragment's 16 values on 16 banks
+
+// d[8][8] += a[8][4] b[4][8]: a lane has a[lane / 4][lane % 4], b[lane % 4][lane / 4], d[lane / 4][2 (lane % 4) + 0, 1].
+__device__ __forceinline__ void mma_f64(double (&d)[2], double a, double b) {
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+                 : "+d"(d[0]), "+d"(d[1]) : "d"(a), "d"(b));
+}
+
 template <int D>
 struct RunLayout {                                     // floats (T, P, r and u: two a value, on 16-byte borders)
     static constexpr int ROW = D + 4;
     static constexpr int K = 0, V = 2 * CHUNK * ROW, Q = V + 2 * CHUNK * RUN_COLS, TP = Q + CHUNK * ROW;     // k and v: two chunks
-    static constexpr int S = TP + 2 * CHUNK_DOUBLES, RT = S + RUN_COLS * ROW, RED = RT + 2 * RUN_COLS * CT;  // S column by column
+    static constexpr int S = TP + 2 * CHUNK_DOUBLES, RT = S + RUN_COLS * ROW, RED = RT + 2 * RUN_COLS * COL;  // S column by column
     static constexpr int RED_FLOATS = 4 * 2 * CHUNK * 20, FLOATS = RED + RED_FLOATS;
-    static constexpr int UT = RED, UN = UT + 2 * RUN_COLS * CT;       // where the quarters' sums lay: they have been read
-    static_assert(UN + 2 * CHUNK * RUN_COLS <= FLOATS && Q % 4 == 0 && TP % 4 == 0 && RT % 4 == 0 && RED % 4 == 0, "it fits");
+    static constexpr int UT = RED, UN = UT + 2 * RUN_COLS * COL;      // where the quarters' sums lay: they have been read
+    static_assert(UN + 2 * CHUNK * UN_ROW <= FLOATS && Q % 4 == 0 && TP % 4 == 0 && RT % 4 == 0 && RED % 4 == 0, "it fits");
     static_assert(FLOATS * 4 <= 112 * 1024, "two blocks an SM");
 };
 
@@ -525,9 +533,9 @@ delta_runs_kernel(const float* __restrict__ r, const float* __restrict__ p, cons
     if (blockIdx.x == 0 && h == 0 && sh.L > 1) delta_conv_advance(p, slot, t0, t1 - t0, sh);
     float* S = sm + Y::S;
     float* red = sm + Y::RED;
-    double* rt = reinterpret_cast<double*>(sm + Y::RT);               // r, column by column [16][34]
+    double* rt = reinterpret_cast<double*>(sm + Y::RT);               // r, column by column [16][COL]
     double* ut = reinterpret_cast<double*>(sm + Y::UT);               // u, column by column
-    double* un = reinterpret_cast<double*>(sm + Y::UN);               // D_Cj u_j, token by token [32][16]
+    double* un = reinterpret_cast<double*>(sm + Y::UN);               // D_Cj u_j, token by token [32][UN_ROW]
     for (int i = tid; i < RUN_COLS * (D / 4); i += 256) {
         const int c = i / (D / 4), k = (i % (D / 4)) * 4;
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -617,82 +625,97 @@ delta_runs_kernel(const float* __restrict__ r, const float* __restrict__ p, cons
         copy_async_wait<1>();                          // T and P; the next chunk's k and v may still be on their way
         __syncthreads();
         fetch_q(c + 1);
-        const int row = tid >> 3, cc = tid & 7;        // token and columns cc, cc + 8 of the middle products
+        // the middle products: a warp has 8 tokens and 8 columns, a lane a token and two neighbouring columns
+        const int g = lane >> 2, t = lane & 3, tokens0 = (warp >> 1) * 8, row = tokens0 + g, cc = (warp & 1) * 8 + 2 * t;
         double from_state[2];
+        bool plain = false;
         {
             const double beta = T[row * CT + AT_BETA], G = P[row * CT + AT_G];
 #pragma unroll
             for (int j = 0; j < 2; ++j) {
-                const float* at = red + row * 20 + cc + 8 * j;
+                const float* at = red + row * 20 + cc + j;
                 const float ks = (at[0] + at[2 * CHUNK * 20]) + (at[4 * CHUNK * 20] + at[6 * CHUNK * 20]);
                 at += CHUNK * 20;
                 const float qs = (at[0] + at[2 * CHUNK * 20]) + (at[4 * CHUNK * 20] + at[6 * CHUNK * 20]);
-                rt[(cc + 8 * j) * CT + row] = beta * ((double)vs[row * RUN_COLS + cc + 8 * j] - G * (double)ks);
+                const double one = beta * ((double)vs[row * RUN_COLS + cc + j] - G * (double)ks);
+                rt[(cc + j) * COL + row] = one;
+                plain |= !isfinite(one);
                 from_state[j] = G * (double)qs;
             }
         }
-        __syncthreads();
-        // one row of T or P times two columns, up to the row's own token
-        auto row_times = [&](const double* m_row, const double* columns, double (&v)[2]) {
-            double s[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
-#pragma unroll 4
-            for (int k = 0; k <= row; k += 2) {
-                const double2 a = *reinterpret_cast<const double2*>(m_row + k);
-#pragma unroll
-                for (int j = 0; j < 2; ++j) {
-                    const double2 b = *reinterpret_cast<const double2*>(columns + (cc + 8 * j) * CT + k);
-                    s[j][0] = fma(a.x, b.x, s[j][0]);
-                    if (k < row) s[j][1] = fma(a.y, b.y, s[j][1]);
+        // A token's row of T or P times the columns, up to the row's own token: rows end in zeros, which the tensor cores
+        // multiply with later tokens' values all the same.  Where one of those is not finite, the row is added up to
+        // its end instead.
+        auto rows_times = [&](const double* m, const double* columns, bool plain_sums, double (&v)[2]) {
+            v[0] = v[1] = 0.0;
+            if (!plain_sums) {
+                double odd[2] = {0.0, 0.0};
+                for (int k = 0; k < tokens0 + 8; k += 8) {
+                    const double* a = m + row * CT + k + t;
+                    const double* b = columns + ((warp & 1) * 8 + g) * COL + k + t;
+                    mma_f64(v, a[0], b[0]);
+                    mma_f64(odd, a[4], b[4]);
                 }
+                v[0] += odd[0], v[1] += odd[1];
+            } else {
+                for (int k = 0; k <= row; ++k)
+                    for (int j = 0; j < 2; ++j) v[j] = fma(m[row * CT + k], columns[(cc + j) * COL + k], v[j]);
             }
-#pragma unroll
-            for (int j = 0; j < 2; ++j) v[j] = s[j][0] + s[j][1];
         };
+        plain = __syncthreads_or(plain);
         {
             double u[2];
-            row_times(T + row * CT, rt, u);
+            rows_times(T, rt, plain, u);
             const double rest = P[row * CT + AT_REST];
+            plain = false;
 #pragma unroll
             for (int j = 0; j < 2; ++j) {
-                ut[(cc + 8 * j) * CT + row] = u[j];
-                un[row * RUN_COLS + cc + 8 * j] = rest * u[j];
+                ut[(cc + j) * COL + row] = u[j];
+                un[row * UN_ROW + cc + j] = rest * u[j];
+                plain |= !isfinite(u[j]);
             }
         }
-        __syncthreads();
+        plain = __syncthreads_or(plain);
         {
             double v[2];
-            row_times(P + row * CT, ut, v);
+            rows_times(P, ut, plain, v);
             if (row < n) {
                 float* at = o + ((size_t)(t0 + c * CHUNK + row) * sh.H + h) * e + col0;
 #pragma unroll
                 for (int j = 0; j < 2; ++j)
-                    if (col0 + cc + 8 * j < e) at[cc + 8 * j] = (float)(from_state[j] + v[j]);
+                    if (col0 + cc + j < e) at[cc + j] = (float)(from_state[j] + v[j]);
             }
         }
-        {   // S <- G_C S0 + sum_j k_j (D_Cj u_j): two channels and COLS columns a thread, all tokens
-            constexpr int PAIRS = D / 2, COLS = RUN_COLS * PAIRS / 256;
-            const int pair = tid % PAIRS, first = (tid / PAIRS) * COLS;
-            double acc[COLS][2];
+        {   // S <- G_C S0 + sum_j k_j (D_Cj u_j), all tokens
+            constexpr int M_TILES = D / 8, PER_WARP = M_TILES * 2 / 8;      // tiles of 8 channels by 8 columns
+            const double last = P[(CHUNK - 1) * CT + AT_G];
+            const int n0 = PER_WARP == 2 ? (warp & 1) * 8 : 0, m0 = PER_WARP == 2 ? (warp >> 1) * 16 : warp * 16;
+            // D = 128: two tiles of channels, both of columns; D = 64: two of channels, one of columns
+            double acc[2][PER_WARP / 2][2];
 #pragma unroll
-            for (int j = 0; j < COLS; ++j) acc[j][0] = acc[j][1] = 0.0;
-#pragma unroll 4
-            for (int token = 0; token < CHUNK; ++token) {
-                const float2 k = *reinterpret_cast<const float2*>(ks_rows + token * Y::ROW + pair * 2);
-                const double kx = k.x, ky = k.y;
+            for (int i = 0; i < 2; ++i)
 #pragma unroll
-                for (int j = 0; j < COLS; j += 2) {
-                    const double2 u = *reinterpret_cast<const double2*>(un + token * RUN_COLS + first + j);
-                    acc[j][0] = fma(kx, u.x, acc[j][0]), acc[j][1] = fma(ky, u.x, acc[j][1]);
-                    acc[j + 1][0] = fma(kx, u.y, acc[j + 1][0]), acc[j + 1][1] = fma(ky, u.y, acc[j + 1][1]);
+                for (int j = 0; j < PER_WARP / 2; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+#pragma unroll
+            for (int k = 0; k < CHUNK; k += 4) {
+                const float* a = ks_rows + (k + t) * Y::ROW + m0 + g;
+                const double a0 = a[0], a1 = a[8];
+#pragma unroll
+                for (int j = 0; j < PER_WARP / 2; ++j) {
+                    const double b = un[(k + t) * UN_ROW + n0 + 8 * j + g];
+                    mma_f64(acc[0][j], a0, b);
+                    mma_f64(acc[1][j], a1, b);
                 }
             }
-            const double last = P[(CHUNK - 1) * CT + AT_G];
 #pragma unroll
-            for (int j = 0; j < COLS; ++j) {
-                float2* at = reinterpret_cast<float2*>(S + (first + j) * Y::ROW + pair * 2);
-                const float2 v = *at;
-                *at = make_float2((float)fma(last, (double)v.x, acc[j][0]), (float)fma(last, (double)v.y, acc[j][1]));
-            }
+            for (int i = 0; i < 2; ++i)
+#pragma unroll
+                for (int j = 0; j < PER_WARP / 2; ++j)
+#pragma unroll
+                    for (int x = 0; x < 2; ++x) {
+                        float* at = S + (n0 + 8 * j + 2 * t + x) * Y::ROW + m0 + 8 * i + g;
+                        *at = (float)fma(last, (double)*at, acc[i][j][x]);
+                    }
         }
         __syncthreads();                               // S is whole, and T and P have been read
         fetch_tp(c + 1);

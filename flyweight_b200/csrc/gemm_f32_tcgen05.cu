@@ -415,7 +415,15 @@ int launch(const CUtensorMap& map_w, const CUtensorMap& map_x, const SplitParams
 
 }  // namespace
 
-bool fwb::gemm_f32_split_takes(int N, int K) { return N >= 128 && K >= 128 && N <= 128 * 65535; }
+// By the matrix alone, so that a row's bits do not depend on the batch.  Smaller matrices leave most SMs without a tile, and
+// what a CTA needs to start (tensor memory, rings) shows: us, multiply-adds then this, 1 | 64 | 201 tokens: 128 x 128 8.3 8.5 |
+// 8.9 8.3 | 8.5 12.5; 256 x 512 8.6 8.3 | 8.8 8.4 | 8.6 14.1; 1024 x 1024 10.5 11.0 | 15.2 8.4 | 19.0 16.4; 3072 x 1024
+// 11.9 11.1 | 22.5 11.6 | 47.7 22.0; 9216 x 1024 21.0 12.6 | 38.8 16.4 | 121 34.5; 1024 x 4608 40.5 12.5 | 60.3 17.0 |
+// 76.3 39.0; 65536 x 1024 130 68 | 260 92 | 832 230.  Relative error at K = 1,024 2.1e-7, then 0.9e-7 (one slice of 1,024:
+// 1.2e-7), at 4,608 4.3e-7 and 1.1e-7, at 128 0.9e-7 and 0.7e-7.
+bool fwb::gemm_f32_split_takes(int N, int K) {
+    return N >= 128 && K >= 128 && (long)N * K >= 1L << 20 && N <= 128 * 65535;
+}
 
 int fwb::gemm_f32_split(const float* X, const float* W, float* Y, const float* addend, int M, int N, int K, int ldx, int ldy,
                         cudaStream_t stream) {

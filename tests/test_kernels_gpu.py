@@ -125,6 +125,47 @@ def test_gemm_fp32_tiles(M, N, K):
         assert torch.equal(ops.gemm_simt(dev(x[-rows:]), dev(w), torch.float32), out[-rows:])
 
 
+@pytest.mark.parametrize("M", [1, 16, 17, 65, 112, 113, 209])
+@pytest.mark.parametrize("N,K", [(8192, 128), (8193, 132), (1025, 1028), (259, 8200), (19000, 160)])
+def test_gemm_fp32_thirds(M, N, K):
+    """The tensor-core form: edges of its tiles of tokens, features and k, one slice of K and several.  Six of nine
+    partial products (the rest below 2^-26 of a product), sums of 32 cut off at 2^-23, then rounded sums: within
+    2^-22 of the products' magnitudes; rows do not depend on the batch."""
+    from flyweight_b200.kernels import ops
+    g = torch.Generator().manual_seed(M * N + K)
+    x, w, add = torch.randn(M, K, generator=g), torch.randn(N, K, generator=g), torch.randn(M, N, generator=g)
+    exact = x.double() @ w.double().T
+    out = ops.gemm_simt(dev(x), dev(w), torch.float32)
+    assert ((out.cpu().double() - exact).abs() <= 2.0 ** -22 * (x.double().abs() @ w.double().abs().T)).all()
+    close(ops.gemm_simt(dev(x), dev(w), torch.float32, addend=dev(add)), exact + add.double(), 1e-6, "gemm + addend")
+    for rows in (1, min(M, 20), min(M, 70)):
+        assert torch.equal(ops.gemm_simt(dev(x[-rows:]), dev(w), torch.float32), out[-rows:])
+
+
+def test_gemm_fp32_thirds_odd_values():
+    """Values that have no three bfloat16 parts: the multiply-adds' answer, and nobody else's changes."""
+    from flyweight_b200.kernels import ops
+    g = torch.Generator().manual_seed(3)
+    x, w = torch.randn(20, 1024, generator=g), torch.randn(1030, 1024, generator=g)
+    plain = ops.gemm_simt(dev(x), dev(w), torch.float32).cpu()
+    x[1, 5], x[2, 7], x[3, 1023], w[9, 3] = float("inf"), float("nan"), 3.4e38, float("-inf")
+    w[:, 1023] = w[:, 1023].clamp(-0.9, 0.9)
+    x[4] *= 1e-36                                        # parts below the smallest normal value
+    x[5] = 0.0
+    exact = x.double() @ w.double().T
+    out = ops.gemm_simt(dev(x), dev(w), torch.float32).cpu()
+    finite = exact.abs() <= 3.4028235e38
+    assert torch.equal(torch.isnan(out), torch.isnan(exact)) and torch.equal(out[exact.isinf()], exact[exact.isinf()].float())
+    scale = x.double().abs() @ w.double().abs().T
+    assert ((out.double() - exact).abs()[finite] <= (2.0 ** -19 * scale)[finite]).all()
+    same = [i for i in range(20) if i not in (1, 2, 3, 4, 5)]
+    clean = torch.ones(1030, dtype=torch.bool)
+    clean[9] = False
+    untouched = torch.randn(20, 1024, generator=torch.Generator().manual_seed(3))
+    again = ops.gemm_simt(dev(untouched), dev(w), torch.float32).cpu()
+    assert torch.equal(out[same][:, clean], again[same][:, clean]) and torch.isfinite(plain).all()
+
+
 @pytest.mark.parametrize("M", [1, 8, 9, 16, 17, 32])
 @pytest.mark.parametrize("N,K", [(8, 8), (17, 40), (1000, 264), (2048, 1024), (2488, 1032), (9216, 1024)])
 def test_products_of_a_few_tokens(M, N, K):
