@@ -385,20 +385,31 @@ __device__ __forceinline__ float pair_sum(unsigned long long v) {
     return __uint_as_float((unsigned)v) + __uint_as_float((unsigned)(v >> 32));
 }
 
+// d[8][8] += a[8][4] b[4][8]: a lane has a[lane / 4][lane % 4], b[lane % 4][lane / 4], d[lane / 4][2 (lane % 4) + 0, 1].
+__device__ __forceinline__ void mma_f64(double (&d)[2], double a, double b) {
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+                 : "+d"(d[0]), "+d"(d[1]) : "d"(a), "d"(b));
+}
+
 // Chunk c of segment s and head h: scratch + (((seg_start[s] / 32 + s) + c) * H + h) * CHUNK_DOUBLES: chunks of
 // different segments never meet, and T / 32 + S of them are enough.  Segments shorter than `from` are the scan's.
-// A block's dot products are 16 x 16 a warp, four rows and two columns a thread, 64 channels of k and q at a time as
-// doubles in shared memory; the products and the rows of A take that room afterwards.
+// The dot products are 8 x 8 tiles of the 64-bit tensor cores, a warp eight rows of k or q and the tiles up to its own
+// tokens; (I + A)^-1 is two inverses of 16 tokens side by side in a warp and T21 = -T22 A21 T11 over the block.  With
+// multiply-adds from doubles in shared memory and one substitution of 32 steps, two blocks an SM, it took 57 us a layer
+// of 2,048 tokens and 16 heads.
 template <int D>
-__global__ void __launch_bounds__(256, 2)
+__global__ void __launch_bounds__(256, 4)
 delta_chunk_kernel(const float* __restrict__ r, const int* __restrict__ seg_start, double* __restrict__ scratch, int from,
                    DeltaShape sh) {
     fwb::pdl_entry();
-    constexpr int PART = 64, STRIDE = PART + 2, DOTS = CHUNK + 1, A_ROW = CHUNK + 2;
-    __shared__ __align__(16) double pool[2 * CHUNK * STRIDE];         // k rows, then q rows
+    constexpr int ROW = D + 4, DOTS = CHUNK + 1, A_ROW = CHUNK + 2, HALF = CHUNK / 2;
+    constexpr int DOUBLES = 2 * CHUNK * DOTS + 2 * CHUNK * A_ROW, LOADED = CHUNK * ROW;      // (floats, two to a double)
+    __shared__ __align__(16) double pool[DOUBLES > LOADED ? DOUBLES : LOADED];
+    float* rows = reinterpret_cast<float*>(pool);                     // [64][D + 4]: k, then q
     double* dots = pool;                                              // [64][33]: k_i.k_j, q_i.k_j
     double* a_rows = pool + 2 * CHUNK * DOTS;                         // [32][34]
-    static_assert(2 * CHUNK * DOTS % 2 == 0 && 2 * CHUNK * DOTS + CHUNK * A_ROW <= 2 * CHUNK * STRIDE, "the pool holds both");
+    double* t_rows = a_rows + CHUNK * A_ROW;                          // [32][34]
+    double* u = pool;                                                 // [16][16], where k's dot products were
     __shared__ double beta[CHUNK], g[CHUNK];
     const int seg = blockIdx.z, h = blockIdx.y;
     const int begin = seg_start[seg], end = seg_start[seg + 1], t0 = begin + blockIdx.x * CHUNK;
@@ -412,44 +423,35 @@ delta_chunk_kernel(const float* __restrict__ r, const int* __restrict__ seg_star
         beta[threadIdx.x] = in ? (double)row[h] : 0.0;
         g[threadIdx.x] = in ? (double)row[sh.H + h] : 1.0;
     }
-    // warps 0-3 the k rows 16 by 16, 4-7 the q rows; nobody needs columns 16-31 of rows 0-15
-    const int row0 = (warp >> 2) * CHUNK + (warp & 2) * 8 + (lane & 3), col0 = (warp & 1) * 16 + (lane >> 2);
-    const bool needed = (warp & 3) != 1;
+#pragma unroll
+    for (int i = threadIdx.x; i < 2 * CHUNK * (D / 4); i += 256) {
+        const int row = i / (D / 4), c = (i % (D / 4)) * 4, token = row % CHUNK;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (token < n)
+            v = *reinterpret_cast<const float4*>(r + (size_t)(t0 + token) * R + (row < CHUNK ? sh.cq() : 0) + head * D + c);
+        *reinterpret_cast<float4*>(rows + row * ROW + c) = v;
+    }
+    __syncthreads();
+    // warps 0-3 eight k rows each, 4-7 eight q rows; nobody needs the columns of later tokens
+    const int own = warp & 3, row0 = (warp >> 2) * CHUNK + own * 8, at = (lane >> 2) * ROW + (lane & 3);
     double acc[4][2];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) acc[i][0] = acc[i][1] = 0.0;
-    for (int part = 0; part < D; part += PART) {
-        if (part > 0) __syncthreads();
-        for (int i = threadIdx.x; i < 2 * CHUNK * (PART / 4); i += 256) {
-            const int row = i / (PART / 4), c = (i % (PART / 4)) * 4, token = row % CHUNK;
-            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (token < n)
-                v = *reinterpret_cast<const float4*>(r + (size_t)(t0 + token) * R + (row < CHUNK ? sh.cq() : 0) + head * D +
-                                                     part + c);
-            *reinterpret_cast<double2*>(&pool[row * STRIDE + c]) = make_double2(v.x, v.y);
-            *reinterpret_cast<double2*>(&pool[row * STRIDE + c + 2]) = make_double2(v.z, v.w);
-        }
-        __syncthreads();
-        if (needed) {
+    for (int j = 0; j < 4; ++j) acc[j][0] = acc[j][1] = 0.0;
 #pragma unroll 4
-            for (int k = 0; k < PART; k += 2) {
-                double2 a[4], b[2];
+    for (int k = 0; k < D; k += 4) {
+        const double a = rows[row0 * ROW + at + k];
 #pragma unroll
-                for (int i = 0; i < 4; ++i) a[i] = *reinterpret_cast<const double2*>(&pool[(row0 + 4 * i) * STRIDE + k]);
-#pragma unroll
-                for (int j = 0; j < 2; ++j) b[j] = *reinterpret_cast<const double2*>(&pool[(col0 + 8 * j) * STRIDE + k]);
-#pragma unroll
-                for (int i = 0; i < 4; ++i)
-#pragma unroll
-                    for (int j = 0; j < 2; ++j) acc[i][j] = fma(a[i].y, b[j].y, fma(a[i].x, b[j].x, acc[i][j]));
-            }
-        }
+        for (int j = 0; j < 4; ++j)
+            if (j <= own) mma_f64(acc[j], a, (double)rows[j * 8 * ROW + at + k]);
     }
     __syncthreads();                                                  // k and q have been read: the pool is free
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 2; ++j) dots[(row0 + 4 * i) * DOTS + col0 + 8 * j] = acc[i][j];
+    for (int j = 0; j < 4; ++j)
+        if (j <= own) {
+            double* to = dots + (row0 + (lane >> 2)) * DOTS + j * 8 + 2 * (lane & 3);
+            to[0] = acc[j][0];
+            to[1] = acc[j][1];
+        }
     __syncthreads();
     double* out = scratch + ((size_t)(begin / CHUNK + seg + blockIdx.x) * sh.H + h) * CHUNK_DOUBLES;
     double* p_out = out + CHUNK * CT;
@@ -460,7 +462,25 @@ delta_chunk_kernel(const float* __restrict__ r, const int* __restrict__ seg_star
             d = i > lane ? d * g[i] : 1.0;
             a_rows[i * A_ROW + lane] = i > lane ? beta[i] * (d * dots[i * DOTS + lane]) : 0.0;
         }
-        out[lane * CT + AT_BETA] = beta[lane];
+        __syncwarp();
+        // column `lane` of the inverse inside its half, forwards
+        const int base = lane & HALF, column = lane & (HALF - 1);
+        double t[HALF];
+#pragma unroll
+        for (int i = 0; i < HALF; ++i) {
+            const double* row = a_rows + (base + i) * A_ROW + base;
+            double s0 = 0.0, s1 = 0.0;
+#pragma unroll
+            for (int m = 0; m + 1 < i; m += 2) {
+                s0 = fma(row[m], t[m], s0);
+                s1 = fma(row[m + 1], t[m + 1], s1);
+            }
+            if (i & 1) s0 = fma(row[i - 1], t[i - 1], s0);
+            t[i] = i == column ? 1.0 : (i > column ? -(s0 + s1) : 0.0);
+            t_rows[(base + i) * A_ROW + lane] = t[i];
+        }
+        if (lane >= HALF)
+            for (int i = 0; i < HALF; ++i) t_rows[i * A_ROW + lane] = 0.0;
     } else if (warp == 1) {                                           // P
         double d = 1.0;
 #pragma unroll 4
@@ -473,33 +493,24 @@ delta_chunk_kernel(const float* __restrict__ r, const int* __restrict__ seg_star
         double d = 1.0;
         for (int i = 0; i <= lane; ++i) d *= g[i];
         p_out[lane * CT + AT_G] = d;
+        out[lane * CT + AT_BETA] = beta[lane];
     }
-    __syncwarp();
-    if (warp == 0) {                                                  // column `lane` of (I + A)^-1, forwards
-        double t[CHUNK];
+    __syncthreads();
+    const int i = threadIdx.x >> 4, j = threadIdx.x & (HALF - 1);     // an element of the lower left quarter
+    double sum = 0.0;
+    for (int l = j; l < HALF; ++l) sum = fma(a_rows[(HALF + i) * A_ROW + l], t_rows[l * A_ROW + j], sum);
+    u[i * HALF + j] = sum;
+    __syncthreads();
+    sum = 0.0;
+    for (int m = 0; m <= i; ++m) sum = fma(t_rows[(HALF + i) * A_ROW + HALF + m], u[m * HALF + j], sum);
+    t_rows[(HALF + i) * A_ROW + j] = -sum;
+    __syncthreads();
 #pragma unroll
-        for (int i = 0; i < CHUNK; ++i) {
-            double s0 = 0.0, s1 = 0.0;
-#pragma unroll
-            for (int m = 0; m + 1 < i; m += 2) {
-                s0 = fma(a_rows[i * A_ROW + m], t[m], s0);
-                s1 = fma(a_rows[i * A_ROW + m + 1], t[m + 1], s1);
-            }
-            if (i & 1) s0 = fma(a_rows[i * A_ROW + i - 1], t[i - 1], s0);
-            t[i] = i == lane ? 1.0 : (i > lane ? -(s0 + s1) : 0.0);
-            out[i * CT + lane] = t[i];
-        }
-    }
+    for (int x = threadIdx.x; x < CHUNK * CHUNK; x += 256) out[(x / CHUNK) * CT + x % CHUNK] = t_rows[(x / CHUNK) * A_ROW + x % CHUNK];
 }
 
 constexpr int RUN_COLS = 16;
 constexpr int COL = 36, UN_ROW = 20;                   // columns of r and u, rows of D_Cj u_j: a fragment's 16 values on 16 banks
-
-// d[8][8] += a[8][4] b[4][8]: a lane has a[lane / 4][lane % 4], b[lane % 4][lane / 4], d[lane / 4][2 (lane % 4) + 0, 1].
-__device__ __forceinline__ void mma_f64(double (&d)[2], double a, double b) {
-    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-                 : "+d"(d[0]), "+d"(d[1]) : "d"(a), "d"(b));
-}
 
 template <int D>
 struct RunLayout {                                     // floats (T, P, r and u: two a value, on 16-byte borders)
