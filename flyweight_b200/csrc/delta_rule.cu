@@ -98,9 +98,10 @@ delta_prepare_kernel(const float* __restrict__ p, const float* __restrict__ taps
 
 // The same for four taps and channel counts in fours, PREP tokens a block: their rows of p are read once, 16 bytes a
 // load, as a window that slides along (the kernel above reads every row once per tap), and only the channels of q and
-// k stop in shared memory on their way.
+// k stop in shared memory on their way.  Blocks (.., 0) have q and k, blocks (.., 1) the values: three small blocks an SM
+// wait for their loads, norms and scalars in turn.
 constexpr int PREP = 4;
-__global__ void __launch_bounds__(512)
+__global__ void __launch_bounds__(256, 3)
 delta_prepare_window_kernel(const float* __restrict__ p, const float* __restrict__ taps, const float* __restrict__ a_log,
                             const float* __restrict__ dt_bias, const float* __restrict__ state, long long slot_stride,
                             const int* __restrict__ seg_start, const int* __restrict__ seg_slot,
@@ -118,7 +119,8 @@ delta_prepare_window_kernel(const float* __restrict__ p, const float* __restrict
         local[i] = t - seg_start[seg];
         hist[i] = state + (size_t)seg_slot[seg] * slot_stride + (size_t)sh.H * sh.d * sh.e;
     }
-    for (int ch = threadIdx.x * 4; ch < C; ch += blockDim.x * 4) {
+    const int stop = blockIdx.y ? C : QK;
+    for (int ch = (blockIdx.y ? QK : 0) + threadIdx.x * 4; ch < stop; ch += blockDim.x * 4) {
         float4 window[PREP + L - 1];
 #pragma unroll
         for (int i = 0; i < PREP + L - 1; ++i) {
@@ -150,6 +152,7 @@ delta_prepare_window_kernel(const float* __restrict__ p, const float* __restrict
             else *reinterpret_cast<float4*>(r + (size_t)(t0 + i) * R + ch) = v;
         }
     }
+    if (blockIdx.y) return;
     __syncthreads();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
     const float q_scale = rsqrtf((float)sh.d);
@@ -814,7 +817,7 @@ FWB_API int fwb_delta_rule(const float* p, const float* taps, const float* a_log
         ((uintptr_t)p & 15) == 0 && ((uintptr_t)taps & 15) == 0 && ((uintptr_t)r & 15) == 0) {
         if (window_smem > 48 * 1024)
             cudaFuncSetAttribute(delta_prepare_window_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
-        fwb::pdl(delta_prepare_window_kernel, (T + PREP - 1) / PREP, 512, window_smem, stream)(
+        fwb::pdl(delta_prepare_window_kernel, dim3((T + PREP - 1) / PREP, 2), 256, window_smem, stream)(
             p, taps, a_log, dt_bias, state, slot_stride, seg_start, seg_slot, tok_seg, r, T, sh);
     } else {
         if (smem > 48 * 1024)
