@@ -119,18 +119,19 @@ def sigmoid_gate_mul_(y: torch.Tensor, gate: torch.Tensor, heads: int, head_dim:
     return y
 
 
-def sigmoid_gate_cols_mul_(y: torch.Tensor, rows: torch.Tensor, col0: int, heads: int, head_dim: int) -> torch.Tensor:
-    """``y[t][h][c] *= sigmoid(rows[t][col0 + h])``: a gate per head that lies in columns of another buffer (a
-    fused projection's last columns), of its own dtype; in place."""
+def sigmoid_gate_cols_mul_(y: torch.Tensor, rows: torch.Tensor, col0: int, heads: int, head_dim: int,
+                           per_channel: bool = False) -> torch.Tensor:
+    """``y[t][h][c] *= sigmoid(rows[t][col0 + h])``, or ``sigmoid(rows[t][col0 + h * head_dim + c])``: a gate per head or
+    per channel that lies in columns of another buffer (a fused projection's last columns), of its own dtype; in place."""
     check_tensor("attention output", y)
     check_tensor("projection rows", rows)
-    T = y.shape[0]
-    if y.numel() != T * heads * head_dim or rows.shape[0] != T or col0 + heads > rows.shape[1]:
+    T, width = y.shape[0], head_dim if per_channel else 1
+    if y.numel() != T * heads * head_dim or rows.shape[0] != T or col0 + heads * width > rows.shape[1]:
         raise KernelError("the gated rows and the gate's columns do not fit")
     if rows.dtype == torch.bfloat16 and y.dtype != torch.bfloat16:
         raise KernelError("a 16-bit gate on 32-bit rows has no kernel")
     lib.call("fwb_sigmoid_gate_mul_strided", ptr(y), is_bf16(y), rows.data_ptr() + col0 * rows.element_size(),
-             is_bf16(rows), c_longlong(rows.shape[1]), T, heads, head_dim, 1, stream())
+             is_bf16(rows), c_longlong(rows.shape[1]), T, heads, head_dim, width, stream())
     return y
 
 
