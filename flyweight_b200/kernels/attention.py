@@ -141,27 +141,18 @@ def set_rope_fusion(flag: bool) -> None:
     _fuse_rope = bool(flag)
 
 
-FUSE_ROPE_CLUSTER_CTAS = 256
-
-
-def decode_fusable(ctx, qkv, cache, block_table, n_heads: int, rotary_dim: int, window: int = 0) -> bool:
-    """Whether ``fused_decode_attention`` takes this step: single tokens only, everything bfloat16, a
-    shape the tensor-core decode kernel has, a rotary width the 16-byte lanes can pair up -- and a
-    launch that gains by it.  Measured in the decode step of LFM2-1.2B: batch 1 (64 CTAs in clusters)
-    0.783 -> 0.775 ms, batch 64 (512 CTAs, no clusters) 1.56 -> 1.53 ms, but batch 8 (512 CTAs in clusters
-    of 8) 0.867 -> 0.881 ms: the kernel of its own was the window in which that many clusters found
-    their SMs and fetched their first tiles, so such launches keep it."""
+def decode_fusable(ctx, qkv, cache, n_heads: int, rotary_dim: int, window: int = 0) -> bool:
+    """Whether ``fused_decode_attention`` takes this step: single tokens only, everything bfloat16, a shape the
+    tensor-core decode kernel has, a rotary width the 16-byte lanes can pair up.  Measured in the decode step of
+    LFM2-1.2B, requests x keys, us: 4 x 4,096 (32 clusters of 8) 688 -> 654, 8 x 4,096 (64 of 8) 732 -> 724, 16 x 4,096
+    (128 of 4) 940 -> 932, 32 x 2,048 (256 of 2) 1,077 -> 1,062, 64 x 4,096 (no clusters) 1,560 -> 1,530."""
     k_pool = cache.k_pool
     if window:
         return False                 # (layers with a sliding window keep the two kernels: not measured, not tested)
-    if not (_fuse_rope and _use_mma and not _force_tiled and ctx.batch.max_segment == 1
+    return (_fuse_rope and _use_mma and not _force_tiled and ctx.batch.max_segment == 1
             and qkv.dtype == torch.bfloat16 and k_pool is not None and k_pool.dtype == torch.bfloat16
             and ctx.precision.act_dtype == torch.bfloat16 and rotary_dim % 16 == 0
-            and ops.attention_mma_shape_ok(n_heads, k_pool.shape[1], k_pool.shape[3], k_pool.shape[2])):
-        return False
-    n_kv, head_dim = k_pool.shape[1], k_pool.shape[3]
-    splits, _, in_cluster = decode_splits(ctx.batch.n_tokens, n_kv, block_table.shape[1], head_dim)
-    return not (in_cluster and ctx.batch.n_tokens * n_kv * splits >= FUSE_ROPE_CLUSTER_CTAS)
+            and ops.attention_mma_shape_ok(n_heads, k_pool.shape[1], k_pool.shape[3], k_pool.shape[2]))
 
 
 def fused_decode_attention(ctx, qkv, cache, block_table, n_heads, n_kv_in, window, scale, q_norm, k_norm, eps,
