@@ -85,7 +85,7 @@ gemm_simt_kernel(const TX* __restrict__ X, const TW* __restrict__ W, TY* __restr
 // 64 x 32 keeps eight warps busy, and a 201 x 1024 product fills 128 SMs.
 // Measured on B200 in a chain of launches over 300 MB of weights (us; gemm_simt_kernel, then this one):
 // 201 x 9216 x 1024 288 -> 121, 201 x 1024 x 4608 378 -> 76, 64 x 9216 x 1024 100 -> 39 (31 TFLOP/s),
-// 8 x 1024 x 4608 403 -> 35, 1 x 9216 x 1024 94 -> 21; relative error against 64 bits 5.7e-7 -> 2.1e-7 at K = 1024.
+// 8 x 1024 x 4608 403 -> 35, 1 x 9216 x 1024 94 -> 21 (matrices of that size have gone to the tensor cores since); relative error against 64 bits 5.7e-7 -> 2.1e-7 at K = 1024.
 constexpr int FK = 64, FSTRIDE = FK + 4, FSTAGES = 3;
 
 __device__ __forceinline__ void fma_four(float2& acc, const float4& a, const float4& b) {

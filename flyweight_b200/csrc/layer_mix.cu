@@ -6,7 +6,7 @@
 //                           with the mean of squares divided by count_r (zero padding inside a range does
 //                           not count)
 //   fwb_value_mix:          save: first[t][:] = rows[t][c0 .. c0+n);  mix: rows[t][c0+i] <- (1-lam) rows + lam first
-//   fwb_sigmoid_gate_mul:   y[t][h][c] *= sigmoid(gate[t][h*gw + (gw == 1 ? 0 : c)])
+//   fwb_sigmoid_gate_mul_strided:   y[t][h][c] *= sigmoid(gate[t][h*gw + (gw == 1 ? 0 : c)])
 //   fwb_scaled_add:         x[t][c] += s1[c] a[t][c] (+ s2[c] b[t][c])                        (fp32; a bf16 copy on request)
 //   fwb_unary_act:          out = act(in), act = relu squared | silu | sigmoid | gelu (tanh form)
 //   fwb_side_gate:          out[t][c] = gelu(g[t][c]) * table[token[t]][c0 + c]
@@ -366,18 +366,6 @@ FWB_API int fwb_value_mix(void* rows, int is_bf16, long long row_stride, int col
     return fwb_launch_status();
 }
 
-// y: [T][heads][head_dim], gate: [T][heads][gate_width] with gate_width 1 (a gate per head) or head_dim.
-FWB_API int fwb_sigmoid_gate_mul(void* y, const void* gate, int is_bf16, int T, int heads, int head_dim,
-                                 int gate_width, cudaStream_t stream) {
-    if (T <= 0) return FWB_OK;
-    if (!y || !gate || heads <= 0 || head_dim <= 0 || (gate_width != 1 && gate_width != head_dim)) return FWB_BAD_ARGUMENT;
-    const int blocks = blocks_for((size_t)T * heads * head_dim);
-    const long long stride = (long long)heads * gate_width;
-    if (is_bf16) fwb::pdl(sigmoid_gate_mul_kernel<bf, bf>, blocks, 256, 0, stream)((bf*)y, (const bf*)gate, stride, T, heads, head_dim, gate_width);
-    else fwb::pdl(sigmoid_gate_mul_kernel<float, float>, blocks, 256, 0, stream)((float*)y, (const float*)gate, stride, T, heads, head_dim, gate_width);
-    return fwb_launch_status();
-}
-
 // bfloat16 rows, eight entries (16 bytes) a thread and turn, a gate per head: one sigmoid for the eight.
 template <typename TG>
 __global__ void sigmoid_head_gate_mul_bf16x8_kernel(uint4* __restrict__ y, const TG* __restrict__ gate, long long gate_stride,
@@ -398,8 +386,9 @@ __global__ void sigmoid_head_gate_mul_bf16x8_kernel(uint4* __restrict__ y, const
     }
 }
 
-// The same with the gate inside the rows of another buffer (some columns of a fused projection): `gate` points at
-// the first gate entry of row 0, rows are `gate_stride` entries apart, and its type may differ from y's.
+// y: [T][heads][head_dim]; gate_width 1 (a gate per head) or head_dim entries a head lie in the rows of another buffer (some
+// columns of a fused projection): `gate` points at the first gate entry of row 0, rows are `gate_stride` entries apart,
+// and its type may differ from y's.
 FWB_API int fwb_sigmoid_gate_mul_strided(void* y, int y_bf16, const void* gate, int gate_bf16, long long gate_stride,
                                          int T, int heads, int head_dim, int gate_width, cudaStream_t stream) {
     if (T <= 0) return FWB_OK;

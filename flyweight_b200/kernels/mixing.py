@@ -100,25 +100,6 @@ def value_mix_(rows: torch.Tensor, col0: int, width: int, first: torch.Tensor,
              ptr(first), ptr(lam), rows.shape[0], 0 if lam is None else 1, stream())
 
 
-def sigmoid_gate_mul_(y: torch.Tensor, gate: torch.Tensor, heads: int, head_dim: int) -> torch.Tensor:
-    """``y[t][h][c] *= sigmoid(gate[t][h])`` (gate [T][heads]) or ``sigmoid(gate[t][h][c])`` (gate
-    [T][heads * head_dim]), in place; both of one dtype."""
-    check_tensor("attention output", y)
-    check_tensor("gate", gate, y.dtype)
-    T = y.shape[0]
-    if y.numel() != T * heads * head_dim:
-        raise KernelError(f"the gated rows hold {y.numel()} entries, expected {T * heads * head_dim}")
-    width = gate.numel() // max(T, 1)
-    if width == heads:
-        per_head = 1
-    elif width == heads * head_dim:
-        per_head = head_dim
-    else:
-        raise KernelError(f"a gate of {width} entries per token fits neither {heads} heads nor their channels")
-    lib.call("fwb_sigmoid_gate_mul", ptr(y), ptr(gate), is_bf16(y), T, heads, head_dim, per_head, stream())
-    return y
-
-
 def sigmoid_gate_cols_mul_(y: torch.Tensor, rows: torch.Tensor, col0: int, heads: int, head_dim: int,
                            per_channel: bool = False) -> torch.Tensor:
     """``y[t][h][c] *= sigmoid(rows[t][col0 + h])``, or ``sigmoid(rows[t][col0 + h * head_dim + c])``: a gate per head or

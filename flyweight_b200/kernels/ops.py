@@ -124,7 +124,8 @@ def cast(x: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
 def gemm_simt(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype,
               addend: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None
               ) -> torch.Tensor:
-    """``x @ w.T`` with fp32 FMA accumulation (no tensor cores).  x: [M][K], w: [N][K]."""
+    """``x @ w.T`` in true 32 bits: fp32 multiply-adds, or (fp32 operands, large matrices) exact thirds of the values on
+    the tensor cores.  x: [M][K], w: [N][K]."""
     check_tensor("gemm input", x)
     check_tensor("gemm weight", w)
     M, K = x.shape
@@ -146,7 +147,7 @@ def linear(x, w: torch.Tensor, out_dtype: torch.dtype,
            addend: Optional[torch.Tensor] = None) -> torch.Tensor:
     """The matrix product the model uses: picks the kernel for the dtypes and sizes.
 
-    float32 weights always take the SIMT kernel (true 32-bit).  bfloat16 weights take
+    float32 weights always take ``gemm_simt`` (true 32-bit).  bfloat16 weights take
     the tensor-core kernel when it accepts the shape, else the SIMT kernel.  ``x`` may be a
     norm not yet applied (``parts.base.DeferredNorm``): an RMS norm in front of a decode-sized
     bfloat16 product runs inside that product's kernel, otherwise its own kernel runs first.

@@ -407,7 +407,9 @@ class GQAttention(Mixer):
                                  f"{self.n_kv} value heads of {D}: the source layer runs first and has the same shape")
             mixing.value_mix_(qkv, v_at, self.n_kv * D, first, self.vmix)
         extra = self._encode_extra()
-        q = self.position.encode(ctx, qkv[:, :self._qkv_columns], n_heads=self.n_heads, n_kv_in=self._kv_in, head_dim=D,
+        if qkv.shape[1] != self._qkv_columns:                # the gate's columns behind them
+            qkv = qkv[:, :self._qkv_columns]
+        q = self.position.encode(ctx, qkv, n_heads=self.n_heads, n_kv_in=self._kv_in, head_dim=D,
                                  q_norm=None if whole else self.q_norm, k_norm=None if whole else self.k_norm,
                                  eps=None if whole else (self.eps if self.unit_rms_eps is None else self.unit_rms_eps),
                                  cache=cache, block_table=block_table, **extra)

@@ -166,6 +166,52 @@ def test_gemm_fp32_thirds_odd_values():
     assert torch.equal(out[same][:, clean], again[same][:, clean]) and torch.isfinite(plain).all()
 
 
+@pytest.mark.parametrize("group", [1, 2, 3, 5, 20])
+@pytest.mark.parametrize("hd", [64, 20, 132])
+@pytest.mark.parametrize("window,keep", [(0, 0), (17, 3), (-24, 0)])
+def test_fp32_attention_in_runs(group, hd, window, keep):
+    """Tokens of a segment share their key tiles: edges of the runs, of tiles and of pages, and every token's bits as
+    alone.  Sums of at most 80 products in 32 bits, in the order of the keys."""
+    from flyweight_b200.kernels import ops
+    g = torch.Generator().manual_seed(group * hd + window)
+    firsts, counts, nkv, page = [0, 60, 0, 31], [33, 9, 1, 7], 2, 64
+    T, nh, pages = sum(counts), 2 * group, 8
+    q = torch.randn(T, nh * hd, generator=g)
+    k, v = (torch.randn(pages, nkv, page, hd, generator=g) for _ in range(2))
+    table = torch.randperm(pages, generator=g).view(4, 2).to(torch.int32)
+    pos = torch.cat([torch.arange(f, f + c) for f, c in zip(firsts, counts)]).to(torch.int32)
+    seg = torch.repeat_interleave(torch.arange(4), torch.tensor(counts)).to(torch.int32)
+    sink = torch.randn(nh, generator=g)
+
+    def run(rows):
+        return ops.attention_simt(dev(q[rows]), dev(k), dev(v), dev(pos[rows]), dev(seg[rows]), dev(table), nh, window,
+                                  hd ** -0.5, torch.float32, sink=dev(sink), keep_first=keep).cpu()
+
+    out = run(slice(0, T))
+    for t in range(T):
+        p, keys = int(pos[t]), k[table[seg[t]].long()].double().permute(0, 2, 1, 3).reshape(-1, nkv, hd)
+        values = v[table[seg[t]].long()].double().permute(0, 2, 1, 3).reshape(-1, nkv, hd)
+        at = torch.arange(p + 1)
+        seen = (at > p - window) | (at < keep) if window > 0 else at // -window == p // -window if window < 0 else at >= 0
+        for h in range(nh):
+            s = torch.cat([keys[:p + 1, h // group] @ q[t].double().view(nh, hd)[h] * hd ** -0.5, sink[h:h + 1].double()])
+            s[:-1][~seen] = -math.inf
+            want = torch.softmax(s, 0)[:-1] @ values[:p + 1, h // group]
+            assert (out[t].view(nh, hd)[h].double() - want).abs().max() < 2e-6 * max(1.0, want.abs().max().item())
+        assert torch.equal(run(slice(t, t + 1)), out[t:t + 1])
+
+
+@pytest.mark.parametrize("y_dtype,rows_dtype", [(torch.bfloat16, torch.bfloat16), (torch.bfloat16, torch.float32),
+                                                (torch.float32, torch.float32)])
+def test_gate_per_channel_in_columns(y_dtype, rows_dtype):
+    from flyweight_b200.kernels import mixing
+    g = torch.Generator().manual_seed(4)
+    y, rows = torch.randn(5, 3 * 20, generator=g).to(y_dtype), torch.randn(5, 100, generator=g).to(rows_dtype)
+    want = y.double() * torch.sigmoid(rows[:, 24:84].double())
+    got = mixing.sigmoid_gate_cols_mul_(dev(y), dev(rows), 24, 3, 20, per_channel=True)
+    close(got, want, 2.0 ** -8 if y_dtype == torch.bfloat16 else 1e-6, "gate per channel")
+
+
 @pytest.mark.parametrize("M", [1, 8, 9, 16, 17, 32])
 @pytest.mark.parametrize("N,K", [(8, 8), (17, 40), (1000, 264), (2048, 1024), (2488, 1032), (9216, 1024)])
 def test_products_of_a_few_tokens(M, N, K):
