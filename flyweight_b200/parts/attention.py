@@ -137,9 +137,12 @@ class GQAttention(Mixer):
         # the head kernel reads them: one rounding, not two.  (Mixed values are rounded on both sides of the
         # mix in 16-bit runs: what the products' dtype means for a projection and for a cached value.)
         self._wide_qkv = self.qk_norm == "whole"
-        # an output gate's rows ride in the q|k|v product: what works on q, k and v in place leaves the columns behind
-        # them alone
-        self.w_qkv = self.w_o = self.q_norm = self.k_norm = self.sink = self.vmix = None
+        # a gate per head behind a convolution: its rows ride in the q|k|v product (the convolution writes a
+        # buffer of its own, so the gate's columns stay where the product left them).  Every other gate has a
+        # product of its own: its matrix keeps the type it is stored in and its rows leave in the activations',
+        # whatever q, k and v do
+        self._gate_in_projection = self.gate == "head" and self.conv_taps > 0
+        self.w_qkv = self.w_o = self.q_norm = self.k_norm = self.w_gate = self.sink = self.vmix = None
         self.taps = self.qkv_bias = self.temp = None
 
     @property
@@ -232,8 +235,8 @@ class GQAttention(Mixer):
         if not self.shares_cache:
             mats += [rows_padded(get(n["k"]), self.qk_dim), rows_padded(get(n["v"]), self.value_dim)]
         self._qkv_columns = sum(m.shape[0] for m in mats)
-        if self.gate:
-            gate_rows = rows_padded(get(n["g"]), self.value_dim) if self.gate == "element" else get(n["g"])
+        if self._gate_in_projection:
+            gate_rows = get(n["g"])
             pad = -gate_rows.shape[0] % 8                     # (a row count the products' tiles like)
             mats += [gate_rows] + ([gate_rows.new_zeros((pad, gate_rows.shape[1]))] if pad else [])
         dtypes = {m.dtype for m in mats}
@@ -262,6 +265,10 @@ class GQAttention(Mixer):
             if not self.shares_cache:
                 taps += [rows_padded(get(n["k_conv"]), self.qk_dim), rows_padded(get(n["v_conv"]), self.value_dim)]
             self.taps = precision.vector(torch.cat([t.to(torch.float32) for t in taps], dim=0), device)
+        if self.gate and not self._gate_in_projection:
+            w_gate = get(n["g"])
+            self.w_gate = precision.matrix(rows_padded(w_gate, self.value_dim) if self.gate == "element" else w_gate,
+                                           device)
         if self.value_mix == "mixed":
             self.vmix = precision.vector(get(n["vmix"]).reshape(1), device)
         if self.has_bias:
@@ -273,7 +280,7 @@ class GQAttention(Mixer):
         return rows
 
     def _matrices(self):
-        return tuple(m for m in (self.w_qkv, self.w_o) if m is not None)
+        return tuple(m for m in (self.w_qkv, self.w_o, self.w_gate) if m is not None)
 
     def weight_bytes(self):                       # (0 while the matrices belong to the mixer that joined this one)
         return sum(m.numel() * m.element_size() for m in self._matrices())
@@ -407,8 +414,6 @@ class GQAttention(Mixer):
                                  f"{self.n_kv} value heads of {D}: the source layer runs first and has the same shape")
             mixing.value_mix_(qkv, v_at, self.n_kv * D, first, self.vmix)
         extra = self._encode_extra()
-        if qkv.shape[1] != self._qkv_columns:                # the gate's columns behind them
-            qkv = qkv[:, :self._qkv_columns]
         q = self.position.encode(ctx, qkv, n_heads=self.n_heads, n_kv_in=self._kv_in, head_dim=D,
                                  q_norm=None if whole else self.q_norm, k_norm=None if whole else self.k_norm,
                                  eps=None if whole else (self.eps if self.unit_rms_eps is None else self.unit_rms_eps),
@@ -416,8 +421,11 @@ class GQAttention(Mixer):
         out = attention_kernels.paged_attention(ctx, q, cache, block_table, self.n_heads, self.span, self.scale,
                                                 act, sink=self.sink, softcap=self.softcap,
                                                 keep_first=self.keep_first)
-        if self.gate:
-            mixing.sigmoid_gate_cols_mul_(out, projected, self._qkv_columns, self.n_heads, D, per_channel=self.gate == "element")
+        if self._gate_in_projection:
+            mixing.sigmoid_gate_cols_mul_(out, projected, self._qkv_columns, self.n_heads, D)
+        elif self.gate:
+            mixing.sigmoid_gate_cols_mul_(out, ops.linear(h, self.w_gate, act), 0, self.n_heads, D,
+                                          per_channel=self.gate == "element")
         return ops.linear_into_residual(out, self.w_o, residual)
 
     def plan(self, builder, norm, cache):

@@ -257,3 +257,20 @@ def test_plain_layers_add_what_the_parts_give():
     x = x + P.token_side_input(x, ids, w, "l0.side.", 0, 4, eps)
     assert torch.allclose(streams[0], x, atol=1e-12)
     assert torch.allclose(logits, (P.unit(x, eps) * w["final.norm"]) @ w["head"].T, atol=1e-12)
+
+
+def test_an_output_gate_keeps_its_own_stored_type():
+    """A checkpoint may store its matrices in different types, and a 16-bit run keeps what is stored: a gate in 32 bits
+    leaves the 16-bit q, k and v alone, and the other way round."""
+    from flyweight_b200.parts import Precision, build_mixer
+    gated = [m for name in NAMES for layer in typed(TINY[name]).model_spec().layers
+             for m in (layer.parts["mixer"], layer.parts["mixer"].params.get("left"))
+             if m is not None and m.params.get("gate")]
+    assert {m.params["gate"] for m in gated} == {"element", "head"}
+    for part in gated:
+        for odd in (torch.float32, torch.bfloat16):
+            rest = torch.bfloat16 if odd == torch.float32 else torch.float32
+            mixer = build_mixer(part)
+            shapes = {name: (decl.shape, odd if name == part.tensors["g"] else rest) for name, decl in mixer.declare().items()}
+            mixer.bind(lambda name: torch.ones(shapes[name][0], dtype=shapes[name][1]), Precision("bfloat16"), "cpu")
+            assert mixer.w_qkv.dtype == rest and mixer.w_o.dtype == rest and mixer.w_gate.dtype == odd

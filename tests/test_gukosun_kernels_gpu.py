@@ -348,6 +348,28 @@ def test_decayed_linear_attention_part_and_the_pair(dtype, lin):
         close(got_pair[s], P.parallel_mixer(h, w, "l2.mix.", m, EPS, pos, rnd=rnd), TOL[dtype], f"pair, sequence {s}")
 
 
+@pytest.mark.parametrize("tokens", [1, 8, 40])
+@pytest.mark.parametrize("kind", ["element", "head"])
+def test_an_output_gate_is_rounded_like_every_projection(kind, tokens):
+    """The gated heads are the heads of the same mixer without a gate times the sigmoid of the gate's own product, a
+    bfloat16 row in a 16-bit run (also where a norm over the whole projection keeps q, k and v in 32 bits): bit for bit.
+    The output matrix is the identity, so the part gives the heads themselves."""
+    import dataclasses
+    from flyweight_b200.kernels import mixing, ops
+    raw = tiny_config(width=64, heads=4, kv=2, dim=16, vdim=16)
+    spec, w = random_weights(raw, 23, torch.bfloat16)
+    prefix = "l0.mix." if kind == "element" else "l2.mix.left."
+    part = spec.layers[0].parts["mixer"] if kind == "element" else spec.layers[2].parts["mixer"].params["left"]
+    assert part.params["gate"] == kind
+    w[prefix + "o"] = torch.eye(64, dtype=F64)
+    h = bf16_round(torch.randn(tokens, 64, generator=torch.Generator().manual_seed(tokens), dtype=F64))
+    ungated = dataclasses.replace(part, params={**part.params, "gate": None})
+    got, heads = (run_part(p, w, torch.bfloat16, [h], [[(0, tokens)]])[0] for p in (part, ungated))
+    gate = ops.linear(dev(h, torch.bfloat16), dev(w[prefix + "g"], torch.bfloat16), torch.bfloat16)
+    want = mixing.sigmoid_gate_cols_mul_(dev(heads, torch.bfloat16), gate, 0, 4, 16, per_channel=kind == "element")
+    assert torch.equal(got, want.float().cpu())
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_dense_feed_forward_and_token_side_input(dtype):
     from flyweight_b200.engine import Segment, StepBatch, StepContext
