@@ -186,10 +186,12 @@ __device__ __forceinline__ float gated_f32(int act, float limit, float g, float 
     return (act == GATED_GELU_TANH ? gelu_tanh_f32(g) : silu_f32(g)) * u;
 }
 
-// What a product without a gate may do to its output before it is stored.  0: nothing.  1: max(v, 0)^2.
-constexpr int OUTPUT_AS_IS = 0, OUTPUT_RELU_SQUARED = 1;
+// What a product without a gate may do to its output before it is stored.  0: nothing.  1: max(v, 0)^2.  2: the same of
+// v rounded to bfloat16, the bits of a product and a pass behind it.
+constexpr int OUTPUT_AS_IS = 0, OUTPUT_RELU_SQUARED = 1, OUTPUT_RELU_SQUARED_ROUNDED = 2;
 __device__ __forceinline__ float output_act_f32(int act, float v) {
-    if (act != OUTPUT_RELU_SQUARED) return v;
+    if (act == OUTPUT_AS_IS) return v;
+    if (act == OUTPUT_RELU_SQUARED_ROUNDED) v = __bfloat162float(__float2bfloat16_rn(v));
     const float r = fmaxf(v, 0.0f);
     return r * r;
 }

@@ -169,15 +169,18 @@ def linear(x, w: torch.Tensor, out_dtype: torch.dtype,
     return gemm_simt(x, w, out_dtype, addend)
 
 
-def linear_act(x: torch.Tensor, w: torch.Tensor, activation: str, out_dtype: torch.dtype) -> torch.Tensor:
-    """``act(x @ w.T)``, the activation (one of ``OUTPUT_ACTIVATIONS``) on the product's fp32 sums: in the tensor-core
-    product's epilogue when the output is bfloat16, else as a pass of its own."""
+def linear_act(x: torch.Tensor, w: torch.Tensor, activation: str, out_dtype: torch.dtype,
+               rounded: bool = False) -> torch.Tensor:
+    """``act(x @ w.T)``, the activation (one of ``FUSED_ACTIVATIONS``) on the product's fp32 sums, or, ``rounded``, on
+    them rounded to ``out_dtype`` (a matrix stored in 32 bits keeps its sums): in the tensor-core product's epilogue when
+    the output is bfloat16, else as a pass of its own."""
     from . import mixing, tensorcore
     if w.dtype == torch.bfloat16 and out_dtype == torch.bfloat16:
         x = cast(x, torch.bfloat16)
         if tensorcore.accepts(x, w, out_dtype):
-            return tensorcore.gemm(x, w, out_dtype, activation=activation)
-    return mixing.unary_act(linear(x, w, torch.float32), activation, out_dtype)
+            return tensorcore.gemm(x, w, out_dtype, activation=activation + "_rounded" if rounded else activation)
+    wide = not rounded or w.dtype == torch.float32
+    return mixing.unary_act(linear(x, w, torch.float32 if wide else out_dtype), activation, out_dtype)
 
 
 def linear_into_residual(x: torch.Tensor, w: torch.Tensor, residual: Optional[torch.Tensor]):
@@ -206,8 +209,10 @@ def silu_mul(gate_up: torch.Tensor, out_dtype: torch.dtype) -> torch.Tensor:
 # what a gated feed-forward makes of gate g and up u: silu(g) u, gelu(g) u (tanh form), or the clamped swish
 # min(g, L) sigmoid(1.702 min(g, L)) (clamp(u, -L, L) + 1) with a limit L, or max(g, 0) u
 GATE_ACTIVATIONS = {"silu": 0, "gelu_tanh": 1, "swish_clamped": 2, "relu": 3}
-# what a product without a gate may do to a bfloat16 output on its way out (in fp32, ahead of the rounding)
-OUTPUT_ACTIVATIONS = {None: 0, "relu_squared": 1}
+# what a product without a gate may do to a bfloat16 output on its way out: in fp32 ahead of the rounding, or, "_rounded",
+# on the rounded product
+OUTPUT_ACTIVATIONS = {None: 0, "relu_squared": 1, "relu_squared_rounded": 2}
+FUSED_ACTIVATIONS = ("relu_squared",)
 
 
 def gate_act_mul(gate_up: torch.Tensor, out_dtype: torch.dtype, activation: str = "silu",

@@ -1,5 +1,5 @@
 """Dense feed-forward without a gate: down( act(up h) ), no bias.  ``act`` is a parameter: the square of
-relu, silu, or the tanh form of gelu, computed in fp32."""
+relu, silu, or the tanh form of gelu, computed in fp32 on the product in its own dtype."""
 from __future__ import annotations
 
 import torch
@@ -42,8 +42,9 @@ class DenseMLP(FeedForward):
         act = ctx.precision.act_dtype
         if not isinstance(h, torch.Tensor):
             h = h.materialize(act)
-        if self.activation in ops.OUTPUT_ACTIVATIONS:        # in the product's epilogue, on its fp32 sums
-            a = ops.linear_act(h, self.w_up, self.activation, act)
+        # (the hidden row leaves its product in the products' dtype; the activation itself is computed in fp32)
+        if self.activation in ops.FUSED_ACTIVATIONS:         # in the product's epilogue
+            a = ops.linear_act(h, self.w_up, self.activation, act, rounded=True)
         else:
             a = mixing.unary_act(ops.linear(h, self.w_up, act), self.activation, act)
         return ops.linear(a, self.w_down, torch.float32)

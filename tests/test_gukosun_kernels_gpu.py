@@ -155,6 +155,11 @@ def tiny_config(window=37, heads=4, kv=2, dim=16, vdim=24, width=48, softcap=6.0
                        {"type": "parallel", "mixer": {"left": left, "right": right}, "mlp": mlp}]}
 
 
+def typed_spec(raw):
+    from flyweight_b200.config import GukosunConfig
+    return GukosunConfig.from_dict(raw).model_spec()
+
+
 def random_weights(raw, seed, dtype):
     """Every tensor the configuration declares, in float64 (rounded to bfloat16 first where that is the dtype)."""
     from flyweight_b200.config import GukosunConfig
@@ -368,6 +373,27 @@ def test_an_output_gate_is_rounded_like_every_projection(kind, tokens):
     gate = ops.linear(dev(h, torch.bfloat16), dev(w[prefix + "g"], torch.bfloat16), torch.bfloat16)
     want = mixing.sigmoid_gate_cols_mul_(dev(heads, torch.bfloat16), gate, 0, 4, 16, per_channel=kind == "element")
     assert torch.equal(got, want.float().cpu())
+
+
+@pytest.mark.parametrize("stored", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("tokens", [1, 9, 40, 70, 200, 600])
+def test_the_hidden_row_is_rounded_ahead_of_the_square(tokens, stored):
+    """The square of relu in the product's epilogue gives the bits of a bfloat16 product and a pass behind it, on each
+    of the product's kernels (few tokens, single CTAs, CTA pairs).  A matrix stored in 32 bits keeps its sums as they are."""
+    from types import SimpleNamespace
+    from flyweight_b200.kernels import mixing, ops
+    from flyweight_b200.parts import Precision
+    from flyweight_b200.parts.base import build_feed_forward
+    raw = tiny_config(width=256)
+    part = build_feed_forward(typed_spec(raw).layers[0].parts["feed_forward"])
+    g = torch.Generator().manual_seed(tokens)
+    w = {name: (torch.randn(decl.shape, generator=g) / 16).to(stored) for name, decl in part.declare().items()}
+    precision = Precision("bfloat16")
+    part.bind(lambda name: w[name], precision, DEV)
+    h = dev(torch.randn(tokens, 256, generator=g), torch.bfloat16)
+    hidden = mixing.unary_act(ops.linear(h, part.w_up, stored), "relu_squared", torch.bfloat16)
+    got = part.forward(SimpleNamespace(precision=precision), h)
+    assert torch.equal(got, ops.linear(hidden, part.w_down, torch.float32))
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
