@@ -424,8 +424,9 @@ class GQAttention(Mixer):
         if self._gate_in_projection:
             mixing.sigmoid_gate_cols_mul_(out, projected, self._qkv_columns, self.n_heads, D)
         elif self.gate:
-            mixing.sigmoid_gate_cols_mul_(out, ops.linear(h, self.w_gate, act), 0, self.n_heads, D,
-                                          per_channel=self.gate == "element")
+            # (a gate stored in 32 bits stays so: the 32-bit product has no 16-bit output)
+            gate = ops.linear(h, self.w_gate, torch.promote_types(act, self.w_gate.dtype))
+            mixing.sigmoid_gate_cols_mul_(out, gate, 0, self.n_heads, D, per_channel=self.gate == "element")
         return ops.linear_into_residual(out, self.w_o, residual)
 
     def plan(self, builder, norm, cache):

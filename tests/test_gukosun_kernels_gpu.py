@@ -185,10 +185,10 @@ def random_weights(raw, seed, dtype):
     return spec, w
 
 
-def run_part(part_spec, w, dtype, h_seqs, cuts, n_pages=24, seed=0, before=None):
+def run_part(part_spec, w, dtype, h_seqs, cuts, n_pages=24, seed=0, before=None, stored={}):
     """A mixer over several sequences fed in the portions ``cuts``; pages in shuffled order, slot = 3 - s.
     ``before``: a part that runs first in every step (the layer whose values this one mixes in).
-    Returns the outputs by sequence."""
+    ``stored``: types of single tensors.  Returns the outputs by sequence."""
     from flyweight_b200.engine import Segment, StepBatch, StepContext
     from flyweight_b200.parts import Precision, build_mixer
     from flyweight_b200.parts.base import FixedState, PagedKV
@@ -197,7 +197,7 @@ def run_part(part_spec, w, dtype, h_seqs, cuts, n_pages=24, seed=0, before=None)
 
     def made(spec):
         part = build_mixer(spec)
-        part.bind(lambda n: w[n].to(dtype), precision, DEV)
+        part.bind(lambda n: w[n].to(stored.get(n, dtype)), precision, DEV)
         part.prepare(1024, DEV)
         cache = type("Cache", (), {})()
         cache.k_pool = cache.v_pool = cache.state = None
@@ -353,12 +353,13 @@ def test_decayed_linear_attention_part_and_the_pair(dtype, lin):
         close(got_pair[s], P.parallel_mixer(h, w, "l2.mix.", m, EPS, pos, rnd=rnd), TOL[dtype], f"pair, sequence {s}")
 
 
+@pytest.mark.parametrize("stored", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("tokens", [1, 8, 40])
 @pytest.mark.parametrize("kind", ["element", "head"])
-def test_an_output_gate_is_rounded_like_every_projection(kind, tokens):
+def test_an_output_gate_is_rounded_like_every_projection(kind, tokens, stored):
     """The gated heads are the heads of the same mixer without a gate times the sigmoid of the gate's own product, a
     bfloat16 row in a 16-bit run (also where a norm over the whole projection keeps q, k and v in 32 bits): bit for bit.
-    The output matrix is the identity, so the part gives the heads themselves."""
+    A gate stored in 32 bits has a 32-bit product.  The output matrix is the identity, so the part gives the heads."""
     import dataclasses
     from flyweight_b200.kernels import mixing, ops
     raw = tiny_config(width=64, heads=4, kv=2, dim=16, vdim=16)
@@ -369,8 +370,8 @@ def test_an_output_gate_is_rounded_like_every_projection(kind, tokens):
     w[prefix + "o"] = torch.eye(64, dtype=F64)
     h = bf16_round(torch.randn(tokens, 64, generator=torch.Generator().manual_seed(tokens), dtype=F64))
     ungated = dataclasses.replace(part, params={**part.params, "gate": None})
-    got, heads = (run_part(p, w, torch.bfloat16, [h], [[(0, tokens)]])[0] for p in (part, ungated))
-    gate = ops.linear(dev(h, torch.bfloat16), dev(w[prefix + "g"], torch.bfloat16), torch.bfloat16)
+    got, heads = (run_part(p, w, torch.bfloat16, [h], [[(0, tokens)]], stored={prefix + "g": stored})[0] for p in (part, ungated))
+    gate = ops.linear(dev(h, torch.bfloat16), dev(w[prefix + "g"], stored), stored)
     want = mixing.sigmoid_gate_cols_mul_(dev(heads, torch.bfloat16), gate, 0, 4, 16, per_channel=kind == "element")
     assert torch.equal(got, want.float().cpu())
 
