@@ -44,6 +44,7 @@ struct SplitTile {
     static constexpr int SMEM = STAGES * STAGE + RAW_STAGES * RAW + 1024 + 256;
     static_assert(BUFFERS * NT + STAGES * A_COLS <= TMEM_COLS, "tensor memory");
     static_assert(NT * BM * 4 <= STAGES * STAGE + RAW_STAGES * RAW, "the parts of a cluster go where the rings were");
+    static_assert(RAW_STAGES >= STAGES && STAGES >= TEAMS, "a cutting warp's waits tell a slot's phases apart");
     static_assert(RAW % 1024 == 0 && STAGE * STAGES % 1024 == 0, "swizzled rows");
 };
 
@@ -215,8 +216,11 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
         const uint32_t swizzled = row0 * ROW_BYTES + ((((id & 7) >> 1) ^ ((row0 >> 1) & 3)) << 4) + (id & 1) * 8;
         for (int i = warp >> 2; i < n_blocks; i += T::TEAMS) {
             const int r = i % RAW_STAGES, s = i % STAGES;
-            bool ok = mbar_wait(&raw_full[r], (i / RAW_STAGES) & 1, abort_flag, 35, prm.status);
-            if (ok && i >= STAGES) ok = mbar_wait(&empty_bar[s], (i / STAGES - 1) & 1, abort_flag, 34, prm.status);
+            // The stage first: a wait goes by its phase's parity, and a team never waited for the blocks of the other
+            // teams.  Block i - STAGES multiplied means that every block up to it, the slot's last tenant too, has
+            // landed; the stage's own phases cannot run ahead, as this team's block before waited for i - TEAMS - STAGES.
+            bool ok = i < STAGES || mbar_wait(&empty_bar[s], (i / STAGES - 1) & 1, abort_flag, 34, prm.status);
+            if (ok) ok = mbar_wait(&raw_full[r], (i / RAW_STAGES) & 1, abort_flag, 35, prm.status);
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
             tc_fence_after();
