@@ -16,8 +16,8 @@
 //     distributed shared memory.
 //   * How K is cut depends on N and K alone and a value on its row of X and of W alone: the same bits in every batch.
 //   * Values without three bfloat16 parts (infinities, NaN, beyond the largest bfloat16, parts below the smallest
-//     normal one) show in the result: it is not finite, or below 2^-60.  Such an element is summed again as
-//     multiply-adds in the order of k.
+//     normal one) are found by what the element came to and the largest magnitudes of its two rows (see ``sure``); such
+//     an element is summed again as multiply-adds.  The warps that cut look at every value (sums of squares, packed).
 #include <float.h>
 
 #include "gemm_f32.cuh"
@@ -41,7 +41,7 @@ struct SplitTile {
     static constexpr int ADDERS = NT > 112 ? 16 : NT > 16 ? 8 : 4, THREADS = 32 * (CUTTERS + ADDERS + 2);
     static constexpr int COLUMNS = NT * 4 / ADDERS;     // of an accumulator, a warp's
     static constexpr int BUFFERS = NT > 112 ? 2 : NT > 64 ? 3 : 4, TMEM_COLS = 512;
-    static constexpr int SMEM = STAGES * STAGE + RAW_STAGES * RAW + 1024 + 256;
+    static constexpr int SMEM = STAGES * STAGE + RAW_STAGES * RAW + 1024 + 256 + (BM + NT + 1) * 4;
     static_assert(BUFFERS * NT + STAGES * A_COLS <= TMEM_COLS, "tensor memory");
     static_assert(NT * BM * 4 <= STAGES * STAGE + RAW_STAGES * RAW, "the parts of a cluster go where the rings were");
     static_assert(RAW_STAGES >= STAGES && STAGES >= TEAMS, "a cutting warp's waits tell a slot's phases apart");
@@ -54,6 +54,7 @@ struct SplitParams {
     int M, N, K, ldx, ldy;
     int splits, tile_tokens;
     bool vectors;                // rows of Y and the addend start on 16-byte borders
+    float lost;                  // see ``sure``
     int* status;
 };
 
@@ -110,38 +111,79 @@ __device__ __forceinline__ bool elect_one() {
         : "=r"(chosen));
     return chosen != 0;
 }
-// The leading bfloat16 parts of four values, which keep the rest.
-__device__ __forceinline__ uint2 take_bf16(float4& v) {
-    const __nv_bfloat162 a = __floats2bfloat162_rn(v.x, v.y), b = __floats2bfloat162_rn(v.z, v.w);
-    const float2 fa = __bfloat1622float2(a), fb = __bfloat1622float2(b);
-    v.x -= fa.x;
-    v.y -= fa.y;
-    v.z -= fb.x;
-    v.w -= fb.y;
-    return make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+// Two values in one register, as packed arithmetic takes them (half the instructions of the warps that cut).
+__device__ __forceinline__ float low(uint64_t v) { return __uint_as_float((uint32_t)v); }
+__device__ __forceinline__ float high(uint64_t v) { return __uint_as_float((uint32_t)(v >> 32)); }
+// The leading bfloat16 parts of two values, which keep the rest.
+__device__ __forceinline__ uint32_t take_bf16(uint64_t& v) {
+    uint32_t parts;
+    asm("{\n\t.reg .f32 a, b;\n\t.reg .b32 fa, fb;\n\t.reg .b64 both;\n\t"
+        "mov.b64 {a, b}, %1;\n\t"
+        "cvt.rn.bf16x2.f32 %0, b, a;\n\t"
+        "shl.b32 fa, %0, 16;\n\t"
+        "and.b32 fb, %0, 0xffff0000;\n\t"
+        "mov.b64 both, {fa, fb};\n\t"
+        "sub.rn.f32x2 %1, %1, both;\n\t}"
+        : "=&r"(parts), "+l"(v));
+    return parts;
+}
+__device__ __forceinline__ uint2 take_bf16(ulonglong2& v) {
+    uint64_t a = v.x, b = v.y;
+    const uint2 parts = make_uint2(take_bf16(a), take_bf16(b));
+    v.x = a;
+    v.y = b;
+    return parts;
 }
 
-// An element whose parts did not say what the values are.
+// What is asked of an element before its sum counts.  Of a value that has no three bfloat16 parts less than 2^-126 is
+// missing (or all of it: infinities, NaN and what rounds past the largest bfloat16 show in the sum, which is not finite),
+// and as much of a partial product that has no place among the normal floats.  With x and w the largest magnitudes in the
+// row of X and the row of W that is less than K 2^-126 (x + w + 6), so an element 2^24 times as large is right to a
+// rounding: K 2^-100 max(x, w), or 2^-40 while both are below TALL (K up to 2^24).  A sum over a row of zeros is zero.
+// What is asked is the two rows' own affair: bits do not depend on the batch.
+constexpr float TALL = 0x1p36f, TALL_SQUARE = 0x1p72f, SMALL = 0x1p-40f;
+__device__ __forceinline__ bool sure(float v) { return fabsf(v) <= FLT_MAX && fabsf(v) >= SMALL; }
+// x, w: 0 for a row of zeros, its largest magnitude from TALL on, else another positive number.
+__device__ __forceinline__ bool sure(float v, float x, float w, float lost) {
+    const float top = fmaxf(x, w), least = top >= TALL ? fmaxf(SMALL, lost * top) : SMALL;
+    return fabsf(v) <= FLT_MAX && (fabsf(v) >= least || x == 0.0f || w == 0.0f);
+}
+// An element whose parts did not say what the values are (rows of whole 16-byte pieces, on their borders).
 __device__ __noinline__ float plain_sum(const float* x, const float* w, int K) {
-    float sum = 0.0f;
-    for (int k = 0; k < K; ++k) sum = fmaf(x[k], w[k], sum);
-    return sum;
+    float sum[4] = {};
+    for (int k = 0; k < K; k += 4) {
+        const float4 a = *reinterpret_cast<const float4*>(x + k), b = *reinterpret_cast<const float4*>(w + k);
+        sum[0] = fmaf(a.x, b.x, sum[0]);
+        sum[1] = fmaf(a.y, b.y, sum[1]);
+        sum[2] = fmaf(a.z, b.z, sum[2]);
+        sum[3] = fmaf(a.w, b.w, sum[3]);
+    }
+    return (sum[0] + sum[1]) + (sum[2] + sum[3]);
+}
+// A token's sums that are not all sure, four features a lane: against the largest magnitudes that the cluster's CTAs found.
+__device__ __noinline__ float4 look_closer(const SplitParams& prm, float4 sum, uint32_t w_top, uint32_t x_top, int t, int f) {
+    const int splits = prm.splits, lane = threadIdx.x & 31;
+    float x = lane < splits ? ld_dsmem_f32(x_top, lane) : 0.0f;
+    x = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(x)));
+    float4 of[8], w = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+    for (int r = 0; r < 8; ++r) of[r] = r < splits ? ld_dsmem_f32x4(w_top, r) : w;
+#pragma unroll
+    for (int r = 0; r < 8; ++r) w = make_float4(fmaxf(w.x, of[r].x), fmaxf(w.y, of[r].y), fmaxf(w.z, of[r].z), fmaxf(w.w, of[r].w));
+    float v[4] = {sum.x, sum.y, sum.z, sum.w};
+    const float tops[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+        if (f + j < prm.N && !sure(v[j], x, tops[j], prm.lost))
+            v[j] = plain_sum(prm.x + (size_t)t * prm.ldx, prm.w + (size_t)(f + j) * prm.K, prm.K);
+    return make_float4(v[0], v[1], v[2], v[3]);
 }
 // Four neighbouring features of a token.
 __device__ __forceinline__ void finish(const SplitParams& prm, int t, int f, float4 sum) {
     const float v[4] = {sum.x, sum.y, sum.z, sum.w};
     float* y = prm.y + (size_t)t * prm.ldy + f;
     const float* addend = prm.addend ? prm.addend + (size_t)t * prm.ldy + f : nullptr;
-    auto in_range = [](float a) { return fabsf(a) >= 0x1p-60f && fabsf(a) <= FLT_MAX; };
-    if (!(in_range(v[0]) && in_range(v[1]) && in_range(v[2]) && in_range(v[3]))) {
-#pragma unroll 1
-        for (int j = 0; j < 4; ++j) {
-            if (f + j >= prm.N) break;
-            const float one = j == 0 ? v[0] : j == 1 ? v[1] : j == 2 ? v[2] : v[3];
-            const float sure = in_range(one) ? one : plain_sum(prm.x + (size_t)t * prm.ldx, prm.w + (size_t)(f + j) * prm.K, prm.K);
-            y[j] = addend ? sure + addend[j] : sure;
-        }
-    } else if (f + 3 < prm.N && prm.vectors) {
+    if (f + 3 < prm.N && prm.vectors) {
         if (addend) {
             const float4 a = *reinterpret_cast<const float4*>(addend);
             sum = make_float4(sum.x + a.x, sum.y + a.y, sum.z + a.z, sum.w + a.w);
@@ -153,6 +195,18 @@ __device__ __forceinline__ void finish(const SplitParams& prm, int t, int f, flo
             if (f + j < prm.N) y[j] = addend ? v[j] + addend[j] : v[j];
     }
 }
+// A maximum of floats that are not negative is one of their bits as integers.
+__device__ __forceinline__ void raise(float* at, float v) { atomicMax(reinterpret_cast<int*>(at), __float_as_int(v)); }
+__device__ __forceinline__ float top_of(float top, const float4& v) {
+    return fmaxf(fmaxf(fmaxf(top, fabsf(v.x)), fmaxf(fabsf(v.y), fabsf(v.z))), fabsf(v.w));
+}
+__device__ __forceinline__ bool not_zero(const float4& v) {
+    return ((__float_as_uint(v.x) | __float_as_uint(v.y) | __float_as_uint(v.z) | __float_as_uint(v.w)) << 1) != 0;
+}
+__device__ __forceinline__ void add_squares(uint64_t& s, const ulonglong2& v) {
+    asm("fma.rn.f32x2 %0, %1, %1, %0;\n\tfma.rn.f32x2 %0, %2, %2, %0;" : "+l"(s) : "l"(v.x), "l"(v.y));
+}
+__device__ __forceinline__ bool may_be_tall(uint64_t s) { return !(low(s) + high(s) < TALL_SQUARE); }      // (or not finite)
 
 template <int NT>
 __global__ void __launch_bounds__(SplitTile<NT>::THREADS, 1)
@@ -172,6 +226,10 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     uint64_t* acc_empty = acc_full + BUFFERS;
     uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(acc_empty + BUFFERS);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_holder + 1);
+    // of this CTA's k: what ``sure`` asks of its features and of its tokens, and whether any value is TALL
+    float* w_top = reinterpret_cast<float*>(raw + RAW_STAGES * T::RAW + 256);
+    float* x_top = w_top + BM;
+    float* any_tall = x_top + NT;
 
     pdl_launch_dependents();
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -197,6 +255,7 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    for (int i = tid; i < BM + NT + 1; i += T::THREADS) w_top[i] = 0.0f;
     if (warp == MMA_WARP) tmem_alloc(tmem_holder, T::TMEM_COLS);
     tc_fence_before();
     __syncthreads();
@@ -214,6 +273,10 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
         // of the tokens: piece p is 16 bytes at k = 4 (id & 7) of row row0 + 16 p
         const int id = tid & 127, row0 = id >> 3;
         const uint32_t swizzled = row0 * ROW_BYTES + ((((id & 7) >> 1) ^ ((row0 >> 1) & 3)) << 4) + (id & 1) * 8;
+        bool w_any = false;                              // this thread's feature has a value other than zero
+        uint32_t x_any = 0;                              // bit p: row row0 + 16 p of the tokens has one
+        const uint32_t x_all = tokens > row0 ? (1u << ((tokens - row0 + 15) >> 4)) - 1 : 0;
+        float w_most = 1.0f;
         for (int i = warp >> 2; i < n_blocks; i += T::TEAMS) {
             const int r = i % RAW_STAGES, s = i % STAGES;
             // The stage first: a wait goes by its phase's parity, and a team never waited for the blocks of the other
@@ -225,12 +288,15 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
             if (!ok) break;
             tc_fence_after();
             const uint8_t* from = raw + (size_t)r * T::RAW;
-            const float4* x = reinterpret_cast<const float4*>(from + T::RAW_W) + id;
+            const ulonglong2* x = reinterpret_cast<const ulonglong2*>(from + T::RAW_W) + id;
             uint8_t* x_to = ring + (size_t)s * T::STAGE + swizzled;
             const uint32_t w_to = a_base + lane_base + s * A_COLS;
-            float4 w[8];                                 // thread = feature: its 32 k
+            ulonglong2 w[8];                             // thread = feature: its 32 k
 #pragma unroll
-            for (int c = 0; c < 8; ++c) w[c] = *reinterpret_cast<const float4*>(from + id * 128 + ((c ^ (id & 7)) << 4));
+            for (int c = 0; c < 8; ++c) w[c] = *reinterpret_cast<const ulonglong2*>(from + id * 128 + ((c ^ (id & 7)) << 4));
+            uint64_t w_squares = 0, x_squares = 0;
+#pragma unroll
+            for (int c = 0; c < 8; ++c) add_squares(w_squares, w[c]);
 #pragma unroll
             for (int part = 0; part < 3; ++part)
 #pragma unroll
@@ -247,10 +313,13 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
 #pragma unroll
             for (int p0 = 0; p0 < PIECES; p0 += 4) {
                 if (p0 * 16 >= columns) break;
-                float4 v[4];                             // all asked for before the first one is cut
+                ulonglong2 v[4];                         // all asked for before the first one is cut
 #pragma unroll
                 for (int p = 0; p < 4; ++p)
                     if (p0 + p < PIECES && (p0 + p) * 16 < columns) v[p] = x[(p0 + p) * 128];
+#pragma unroll
+                for (int p = 0; p < 4; ++p)
+                    if (p0 + p < PIECES && (p0 + p) * 16 < columns) add_squares(x_squares, v[p]);
 #pragma unroll
                 for (int part = 0; part < 3; ++part)
 #pragma unroll
@@ -262,11 +331,44 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) {
-                mbar_arrive(&raw_empty[r]);
-                mbar_arrive(&full_bar[s]);
+            if (lane == 0) mbar_arrive(&full_bar[s]);
+            // what ``sure`` asks, where a block may add to it: read once more while the copies lie there
+            const float4* w_raw = reinterpret_cast<const float4*>(from + id * 128);          // (in another order)
+            const float4* x_raw = reinterpret_cast<const float4*>(x);
+            if (!w_any) {
+                w_any = low(w_squares) + high(w_squares) != 0.0f;
+                if (!w_any) {
+#pragma unroll
+                    for (int c = 0; c < 8; ++c) w_any |= not_zero(w_raw[c ^ (id & 7)]);
+                }
             }
+            if (x_any != x_all) {
+#pragma unroll
+                for (int p = 0; p < PIECES; ++p)
+                    if (p * 16 < columns && not_zero(x_raw[p * 128])) x_any |= 1u << p;
+            }
+            if (may_be_tall(w_squares)) {
+#pragma unroll 1
+                for (int c = 0; c < 8; ++c) w_most = top_of(w_most, w_raw[c]);
+            }
+            if (may_be_tall(x_squares)) {
+#pragma unroll 1
+                for (int p = 0; p * 16 < columns; ++p) {
+                    const float most = top_of(0.0f, x_raw[p * 128]);
+                    if (most >= TALL) {
+                        raise(x_top + row0 + p * 16, most);
+                        *any_tall = 1.0f;
+                    }
+                }
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&raw_empty[r]);
         }
+        if (w_any) raise(w_top + id, w_most >= TALL ? w_most : 1.0f);
+        if (w_most >= TALL) *any_tall = 1.0f;
+#pragma unroll 1
+        for (int p = 0; p < PIECES; ++p)
+            if (x_any >> p & 1) raise(x_top + row0 + p * 16, 1.0f);
     } else if (warp == LOAD_WARP) {
         if (lane == 0) {
             const uint32_t bytes = (BM + prm.tile_tokens) * KB * 4;
@@ -352,6 +454,8 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     if (splits == 1) __syncthreads();
     else cluster_sync_all();
     if (*abort_flag == 0) {
+        const float tall = splits == 1 ? *any_tall : lane < splits ? ld_dsmem_f32(smem_u32(any_tall), lane) : 0.0f;
+        const int f = f0 + lane * 4, features = prm.N - f;
 #pragma unroll 1
         for (int t = rank + warp * splits; t < tokens; t += (T::THREADS / 32) * splits) {
             const float* at = parts + t * BM + lane * 4;
@@ -368,7 +472,11 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
                     sum.w += part.w;
                 }
             }
-            finish(prm, t0 + t, f0 + lane * 4, sum);
+            const bool good = (sure(sum.x) || features < 1) && (sure(sum.y) || features < 2) &&
+                              (sure(sum.z) || features < 3) && (sure(sum.w) || features < 4);
+            if (!__all_sync(0xffffffffu, good && tall == 0.0f))
+                sum = look_closer(prm, sum, smem_u32(w_top + lane * 4), smem_u32(x_top + t), t0 + t, f);
+            finish(prm, t0 + t, f, sum);
         }
     }
     if (splits > 1) cluster_sync_all();                  // nobody leaves while a peer reads
@@ -420,10 +528,12 @@ int launch(const CUtensorMap& map_w, const CUtensorMap& map_x, const SplitParams
 }  // namespace
 
 // By the matrix alone, so that a row's bits do not depend on the batch.  Smaller matrices leave most SMs without a tile, and
-// what a CTA needs to start (tensor memory, rings) shows: us, multiply-adds then this, 1 | 64 | 201 tokens: 128 x 128 8.3 8.5 |
-// 8.9 8.3 | 8.5 12.5; 256 x 512 8.6 8.3 | 8.8 8.4 | 8.6 14.1; 1024 x 1024 10.5 11.0 | 15.2 8.4 | 19.0 16.4; 3072 x 1024
-// 11.9 11.1 | 22.5 11.6 | 47.7 22.0; 9216 x 1024 21.0 12.6 | 38.8 16.4 | 121 34.5; 1024 x 4608 40.5 12.5 | 60.3 17.0 |
-// 76.3 39.0; 65536 x 1024 130 68 | 260 92 | 832 230.  Relative error at K = 1,024 2.1e-7, then 0.9e-7 (one slice of 1,024:
+// what a CTA needs to start (tensor memory, rings) shows: single launches, us, multiply-adds then this, 1 | 64 | 201 tokens:
+// 128 x 128 8.3 8.5 | 8.9 8.3 | 8.5 12.5; 256 x 512 8.6 8.3 | 8.8 8.4 | 8.6 14.1.  In a chain of launches over 300 MB of
+// weights: 1024 x 1024 10.2 5.9 | 14.8 8.6 | 18.5 16.5; 3072 x 1024 11.0 8.1 | 21.9 11.1 | 47.1 21.5; 9216 x 1024 20.9 13.0 |
+// 38.7 17.3 | 121 34.8; 1024 x 4608 34.3 12.3 | 59.8 17.2 | 75.7 38.1; 65536 x 1024 132 72 | 262 98 | 834 229; 128 x 8192
+// 48.8 17.0 | 103 23.1 | 104 56.1; 8192 x 128 4.7 4.7 | 8.2 6.9 | 23.4 13.6; with half of W's or of X's rows zero at most
+// 1.2 times as long (3072 x 1024, 201 tokens).  Relative error at K = 1,024 2.1e-7, then 0.9e-7 (one slice of 1,024:
 // 1.2e-7), at 4,608 4.3e-7 and 1.1e-7, at 128 0.9e-7 and 0.7e-7.
 bool fwb::gemm_f32_split_takes(int N, int K) {
     return N >= 128 && K >= 128 && (long)N * K >= 1L << 20 && N <= 128 * 65535;
@@ -431,7 +541,7 @@ bool fwb::gemm_f32_split_takes(int N, int K) {
 
 int fwb::gemm_f32_split(const float* X, const float* W, float* Y, const float* addend, int M, int N, int K, int ldx, int ldy,
                         cudaStream_t stream) {
-    SplitParams prm{X, W, addend, Y, M, N, K, ldx, ldy, 1, 0, false, status_word()};
+    SplitParams prm{X, W, addend, Y, M, N, K, ldx, ldy, 1, 0, false, K * 0x1p-100f, status_word()};
     prm.vectors = !(ldy & 3) && !((uintptr_t)Y & 15) && !((uintptr_t)addend & 15);
     const int feature_tiles = (N + BM - 1) / BM, blocks = (K + KB - 1) / KB;
     // a CTA an SM; clusters of eight find room for sixteen, of four for some 34

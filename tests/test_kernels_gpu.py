@@ -166,6 +166,55 @@ def test_gemm_fp32_thirds_odd_values():
     assert torch.equal(out[same][:, clean], again[same][:, clean]) and torch.isfinite(plain).all()
 
 
+@pytest.mark.parametrize("M", [3, 40, 130])
+@pytest.mark.parametrize("x_scale,w_scale", [(-118, 64), (64, -118), (-125, 100), (-60, -66), (40, 40), (0, -30)])
+def test_gemm_fp32_thirds_far_from_one(M, x_scale, w_scale):
+    """Parts and partial products below the smallest normal float, whatever the other factor is: the bound of the usual
+    values, and K roundings of 2^-149 where the products themselves are that small.  Every third value is near 1, so the
+    rows' largest magnitudes alone do not tell; rows of zeros give zeros."""
+    from flyweight_b200.kernels import ops
+    g = torch.Generator().manual_seed(M + x_scale)
+    x, w = torch.randn(M, 1056, generator=g), torch.randn(1030, 1056, generator=g)
+    x[:, 1::3] *= 2.0 ** x_scale
+    w[:, 1::3] *= 2.0 ** w_scale
+    x[:, 2::3] *= 2.0 ** x_scale
+    w[:, 2::3] *= 2.0 ** w_scale
+    x[:, ::3] = 0.0                                      # (w's values near 1 meet zeros, and half of the features have none)
+    w[::2, ::3] = 0.0
+    x[1], w[7], w[1029] = 0.0, 0.0, 0.0
+    exact = x.double() @ w.double().T
+    out = ops.gemm_simt(dev(x), dev(w), torch.float32)
+    bound = 2.0 ** -22 * (x.double().abs() @ w.double().abs().T) + 1056 * 2.0 ** -149
+    assert ((out.cpu().double() - exact).abs() <= bound).all()
+    assert torch.equal(out[1:2].cpu(), torch.zeros(1, 1030)) and torch.equal(out[:, [7, 1029]].cpu(), torch.zeros(M, 2))
+    assert torch.equal(ops.gemm_simt(dev(x[-1:]), dev(w), torch.float32), out[-1:])
+
+
+def test_gemm_fp32_thirds_zeros_cost_nothing():
+    """Rows of zeros, of the matrix (heads padded to a common size) or of the tokens, take the time of other rows: half of
+    either made the product 140 and 350 times as long while zeros were summed again."""
+    from flyweight_b200.kernels import ops
+    g = torch.Generator().manual_seed(0)
+    x, w = dev(torch.randn(201, 1024, generator=g)), dev(torch.randn(9216, 1024, generator=g))
+    x_half, w_half = x.clone(), w.clone()
+    x_half[::2] = 0.0
+    w_half.view(-1, 16, 1024)[:, 8:] = 0.0
+
+    def shortest(a, b):
+        times = []
+        for _ in range(8):
+            first, last = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            first.record()
+            ops.gemm_simt(a, b, torch.float32)
+            last.record()
+            last.synchronize()
+            times.append(first.elapsed_time(last))
+        return min(times)
+
+    plain = shortest(x, w)
+    assert shortest(x_half, w) < 3 * plain and shortest(x, w_half) < 3 * plain
+
+
 @pytest.mark.parametrize("group", [1, 2, 3, 5, 20])
 @pytest.mark.parametrize("hd", [64, 20, 132])
 @pytest.mark.parametrize("window,keep", [(0, 0), (17, 3), (-24, 0)])
