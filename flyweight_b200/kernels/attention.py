@@ -148,7 +148,7 @@ def decode_fusable(ctx, qkv, cache, n_heads: int, rotary_dim: int, window: int =
     (128 of 4) 940 -> 932, 32 x 2,048 (256 of 2) 1,077 -> 1,062, 64 x 4,096 (no clusters) 1,560 -> 1,530."""
     k_pool = cache.k_pool
     if window:
-        return False                 # (layers with a sliding window keep the two kernels: not measured, not tested)
+        return False                 # (a sliding window or chunks keep the two kernels: not measured, not tested)
     return (_fuse_rope and _use_mma and not _force_tiled and ctx.batch.max_segment == 1
             and qkv.dtype == torch.bfloat16 and k_pool is not None and k_pool.dtype == torch.bfloat16
             and ctx.precision.act_dtype == torch.bfloat16 and rotary_dim % 16 == 0

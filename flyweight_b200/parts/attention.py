@@ -339,12 +339,12 @@ class GQAttention(Mixer):
         block_table = ctx.batch.block_tables[cache.group]
         from ..kernels import attention as attention_kernels
         rotation = self.position.rotation() if self.unit_rms_eps is None else None
-        if rotation is not None and attention_kernels.decode_fusable(ctx, qkv, cache, self.n_heads, rotation[1], self.window):
+        if rotation is not None and attention_kernels.decode_fusable(ctx, qkv, cache, self.n_heads, rotation[1], self.span):
             # a step of single tokens whose position part is a plain rotation: the decode attention
             # kernel norms, turns and stores its own token's heads (one kernel and one pass less)
             table, rotary_dim, pairing = rotation
             out = attention_kernels.fused_decode_attention(
-                ctx, qkv, cache, block_table, self.n_heads, self._kv_in, self.window, self.scale,
+                ctx, qkv, cache, block_table, self.n_heads, self._kv_in, self.span, self.scale,
                 self.q_norm, self.k_norm, self.eps, table, rotary_dim, pairing)
             return ops.linear_into_residual(out, self.w_o, residual)
         # positions are the position part's business: it norms, encodes and writes the pages

@@ -38,6 +38,33 @@ def test_the_measured_points_of_the_slicing_rule():
     assert chosen(1, 1985)[0] >= 32 and not chosen(1, 1985)[2]      # one long request: a merge kernel
 
 
+@pytest.mark.parametrize("mask,fused", [({}, True), ({"window": 64}, False), ({"chunk": 64}, False)])
+def test_the_decode_kernel_that_rotates_knows_no_mask(monkeypatch, mask, fused):
+    """It walks every earlier key, so a mixer with a window or with chunks goes by the kernels that take its span."""
+    from types import SimpleNamespace
+    import torch
+    from flyweight_b200.config import PartSpec
+    from flyweight_b200.kernels import ops
+    from flyweight_b200.parts import build_mixer
+    from flyweight_b200.parts.base import PositionEncoding
+    names = {role: role for role in ("q", "k", "v", "o")}
+    mixer = build_mixer(PartSpec("gqa_attention", {
+        "hidden_size": 64, "num_heads": 8, "num_kv_heads": 2, "head_dim": 64,
+        "position": PartSpec("rope_half_split", {"theta": 1e4, "rotary_dim": 64}), **mask}, names))
+    mixer.position.prepare(16, "cpu")
+    went = []
+    monkeypatch.setattr(ops, "linear", lambda h, w, dtype: torch.zeros(1, 12 * 64, dtype=dtype))
+    monkeypatch.setattr(ops, "linear_into_residual", lambda out, w, residual: out)
+    monkeypatch.setattr(attention, "fused_decode_attention", lambda *args: went.append("fused"))
+    monkeypatch.setattr(PositionEncoding, "encode", lambda self, *args, **kw: went.append("encode"))
+    monkeypatch.setattr(attention, "paged_attention", lambda ctx, q, cache, table, heads, span, *rest, **kw: went.append(span))
+    cache = SimpleNamespace(k_pool=torch.zeros(1, 2, 64, 64, dtype=torch.bfloat16), v_pool=None, group=0)
+    ctx = SimpleNamespace(batch=SimpleNamespace(block_tables=[torch.zeros(1, 1, dtype=torch.int32)], max_segment=1, n_tokens=1),
+                          precision=SimpleNamespace(act_dtype=torch.bfloat16))
+    mixer.forward(ctx, torch.zeros(1, 64, dtype=torch.bfloat16), cache)
+    assert went == (["fused"] if fused else ["encode", mixer.span])
+
+
 def test_a_convolution_step_refuses_what_the_convolution_refuses():
     """Fewer than two taps, more than sixteen, a slot shorter than its contents: the argument checks of the C entries
     answer before anything is launched, the folded step as the convolution's own kernel."""
