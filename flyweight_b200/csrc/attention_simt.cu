@@ -125,8 +125,9 @@ attention_simt_kernel(const TQ* __restrict__ q, const TC* __restrict__ k_pool,
 // multiply-adds) and that kernel spends its time on staging every tile once a token, a value at a time, and on two
 // reads of shared memory a multiply-add; here a tile serves a run of tokens, comes by 16-byte copies one tile ahead,
 // and a key is read once for all heads of a warp.
-// Tokens are cut into runs where their index is a multiple of the run's length and where the segment changes; a
-// block whose token begins no run ends at once, so single decoded tokens keep a block each.
+// Tokens are cut into runs where their index is a multiple of the run's length and where a token does not stand next to
+// the one before it in its sequence; a block whose token begins no run ends at once, so single decoded tokens keep a block
+// each.
 constexpr int F32_WARPS = 8;
 
 template <int HPW, int DPL>              // heads a warp, head channels a lane
@@ -141,9 +142,10 @@ attention_f32_kernel(const float* __restrict__ q, const float* __restrict__ k_po
     const int mine = group - g0 < WARPS * MAX_HPW ? group - g0 : WARPS * MAX_HPW;
     const int warps_a_token = (mine + HPW - 1) / HPW, run = F32_WARPS / warps_a_token;
     const int t0 = blockIdx.x, kvh = blockIdx.y, seg = tok_seg[t0];
-    if (t0 % run != 0 && tok_seg[t0 - 1] == seg) return;
+    auto goes_on = [&](int t) { return tok_seg[t] == tok_seg[t - 1] && positions[t] == positions[t - 1] + 1; };
+    if (t0 % run != 0 && goes_on(t0)) return;
     int n = 1;
-    while ((t0 + n) % run != 0 && t0 + n < T && tok_seg[t0 + n] == seg) ++n;
+    while ((t0 + n) % run != 0 && t0 + n < T && goes_on(t0 + n)) ++n;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int hd4 = hd >> 2, k_row = hd + 4, buffer = TILE * (k_row + hd);

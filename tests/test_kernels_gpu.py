@@ -250,6 +250,26 @@ def test_fp32_attention_in_runs(group, hd, window, keep):
         assert torch.equal(run(slice(t, t + 1)), out[t:t + 1])
 
 
+@pytest.mark.parametrize("window,keep", [(0, 0), (17, 3), (-24, 0)])
+def test_fp32_attention_of_tokens_in_any_order(window, keep):
+    """A segment's tokens backwards, twice the same and far apart: every token's bits as alone."""
+    from flyweight_b200.kernels import ops
+    g = torch.Generator().manual_seed(window)
+    pos = torch.tensor([90, 89, 88, 3, 4, 5, 5, 5, 100, 0, 1, 40, 39, 120, 121, 122, 122], dtype=torch.int32)
+    seg = torch.tensor([0] * 9 + [1] * 2 + [0] * 6, dtype=torch.int32)
+    q = torch.randn(17, 4 * 64, generator=g)
+    k, v = (torch.randn(4, 2, 64, 64, generator=g) for _ in range(2))
+    table = torch.tensor([[2, 0], [3, 1]], dtype=torch.int32)
+
+    def run(rows):
+        return ops.attention_simt(dev(q[rows]), dev(k), dev(v), dev(pos[rows]), dev(seg[rows]), dev(table), 4, window, 0.125,
+                                  torch.float32, keep_first=keep).cpu()
+
+    out = run(slice(0, 17))
+    for t in range(17):
+        assert torch.equal(run(slice(t, t + 1)), out[t:t + 1]), t
+
+
 @pytest.mark.parametrize("y_dtype,rows_dtype", [(torch.bfloat16, torch.bfloat16), (torch.bfloat16, torch.float32),
                                                 (torch.float32, torch.float32)])
 def test_gate_per_channel_in_columns(y_dtype, rows_dtype):
