@@ -191,6 +191,7 @@ __device__ __forceinline__ float gated_f32(int act, float limit, float g, float 
 constexpr int OUTPUT_AS_IS = 0, OUTPUT_RELU_SQUARED = 1, OUTPUT_RELU_SQUARED_ROUNDED = 2;
 __device__ __forceinline__ float output_act_f32(int act, float v) {
     if (act == OUTPUT_AS_IS) return v;
+    asm volatile("" : "+f"(v));      // a branch around the rest: as selects it made every plain product's epilogue longer
     if (act == OUTPUT_RELU_SQUARED_ROUNDED) v = __bfloat162float(__float2bfloat16_rn(v));
     const float r = fmaxf(v, 0.0f);
     return r * r;
