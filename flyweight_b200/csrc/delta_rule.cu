@@ -744,6 +744,26 @@ delta_runs_kernel(const float* __restrict__ r, const float* __restrict__ p, cons
     }
 }
 
+template <int DPL, int LPC, bool VEC>
+int launch_scan(const float* r, const float* p, float* state, long long slot_stride, const int* seg_start,
+                const int* seg_slot, float* o, int below, int segments, const DeltaShape& sh, cudaStream_t stream) {
+    // blocks that fit the SMs one by one must not meet on some of them, where they would land beside the last blocks of the
+    // kernel in front: they ask for more than half of an SM's shared memory (16 heads of 128, 128 blocks, all launches, us
+    // before and so: 256 tokens 149 117, 512 237 205, 1,024 449 385, 2,048 1,180 749, 4,096 2,580 1,476)
+    constexpr int ALONE = 116 * 1024, COLS = 128 / LPC;
+    auto kernel = delta_scan_kernel<DPL, LPC, VEC>;
+    static bool configured = false;
+    if (!configured) {
+        cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ALONE);
+        if (err != cudaSuccess) return (int)err;
+        configured = true;
+    }
+    const dim3 grid((sh.e + COLS - 1) / COLS, sh.H, segments);
+    const bool alone = (long)grid.x * grid.y * grid.z <= 148;
+    fwb::pdl(kernel, grid, 128, alone ? ALONE : 0, stream)(r, p, state, slot_stride, seg_start, seg_slot, o, below, sh);
+    return fwb_launch_status();
+}
+
 // Segments `first` .. of at least `from` tokens, the longest of `longest`.
 template <int D>
 int launch_runs(const float* r, const float* p, double* scratch, float* state, long long slot_stride, const int* seg_start,
@@ -830,15 +850,11 @@ FWB_API int fwb_delta_rule(const float* p, const float* taps, const float* a_log
                      ((uintptr_t)r & 15) == 0;
     const bool runs = scratch && vec && (d == 64 || d == 128) && ((uintptr_t)scratch & 15) == 0;
     const int below = runs ? from : 2147483647, scans = runs ? scanned : n_segments;
-#define FWB_SCAN(DPL, LPC)                                                                                 \
-    do {                                                                                                   \
-        const dim3 grid((e + 128 / LPC - 1) / (128 / LPC), H, scans);                                      \
-        if (vec)                                                                                           \
-            fwb::pdl(delta_scan_kernel<DPL, LPC, true>, grid, 128, 0, stream)(r, p, state, slot_stride,    \
-                                                                              seg_start, seg_slot, o, below, sh); \
-        else                                                                                               \
-            fwb::pdl(delta_scan_kernel<DPL, LPC, false>, grid, 128, 0, stream)(r, p, state, slot_stride,   \
-                                                                               seg_start, seg_slot, o, below, sh); \
+#define FWB_SCAN(DPL, LPC)                                                                                             \
+    do {                                                                                                               \
+        const int status = vec ? launch_scan<DPL, LPC, true>(r, p, state, slot_stride, seg_start, seg_slot, o, below, scans, sh, stream) \
+                               : launch_scan<DPL, LPC, false>(r, p, state, slot_stride, seg_start, seg_slot, o, below, scans, sh, stream); \
+        if (status != FWB_OK) return status;                                                                           \
     } while (0)
     if (scans > 0) {
         if (d <= 16) FWB_SCAN(4, 4);

@@ -456,6 +456,34 @@ def test_delta_chunks_against_the_scan_and_64_bits(H, G, d, e, strong):
     print("errors", errors)
 
 
+def test_the_scan_takes_four_times_as_long_for_four_times_the_tokens():
+    """128 blocks that walk a sequence token by token fit the SMs one by one.  Where some met on an SM, beside the last blocks
+    of the kernel in front of them, 2,048 tokens took 5.0 times as long as 512; apart they take 3.7 times."""
+    from flyweight_b200.kernels import recurrent
+    H, G, d, e, L = 16, 8, 128, 128, 4
+    C = 2 * G * d + H * e
+
+    def shortest(T):
+        p, zeros = torch.randn(T, C + H * e + 2 * H, device=DEV), torch.zeros(H, device=DEV)
+        taps, state = torch.randn(C, L, device=DEV), torch.zeros(1, recurrent.delta_state_size(H, G, d, e, L), device=DEV)
+        batch = type("Batch", (), {})()
+        batch.n_segments, batch.max_segment = 1, T
+        i32 = lambda values: torch.tensor(values, dtype=torch.int32, device=DEV)
+        batch.seg_start, batch.seg_slot, batch.tok_seg = i32([0, T]), i32([0]), torch.zeros(T, dtype=torch.int32, device=DEV)
+        times = []
+        for _ in range(8):
+            first, last = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            first.record()
+            for _ in range(4):
+                recurrent.delta_rule(p, taps, zeros, zeros, state, batch, H, G, d, e, chunks=False)
+            last.record()
+            last.synchronize()
+            times.append(first.elapsed_time(last))
+        return min(times)
+
+    assert shortest(2048) < 4.4 * shortest(512)
+
+
 @pytest.mark.parametrize("d", [64, 128])
 @pytest.mark.parametrize("part,bad", [("k", "nan"), ("v", "nan"), ("v", "inf"), ("q", "nan")])
 def test_a_value_that_is_not_finite_reaches_no_earlier_token(d, part, bad):
