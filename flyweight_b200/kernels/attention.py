@@ -141,18 +141,32 @@ def set_rope_fusion(flag: bool) -> None:
     _fuse_rope = bool(flag)
 
 
-def decode_fusable(ctx, qkv, cache, n_heads: int, rotary_dim: int, window: int = 0) -> bool:
+FUSE_ROPE_CLUSTER_CTAS, FUSE_ROPE_FRONT_BYTES = 256, 8 << 20
+
+
+def decode_fusable(ctx, qkv, cache, block_table, n_heads: int, rotary_dim: int, span: int, front_bytes: int) -> bool:
     """Whether ``fused_decode_attention`` takes this step: single tokens only, everything bfloat16, a shape the
-    tensor-core decode kernel has, a rotary width the 16-byte lanes can pair up.  Measured in the decode step of
-    LFM2-1.2B, requests x keys, us: 4 x 4,096 (32 clusters of 8) 688 -> 654, 8 x 4,096 (64 of 8) 732 -> 724, 16 x 4,096
-    (128 of 4) 940 -> 932, 32 x 2,048 (256 of 2) 1,077 -> 1,062, 64 x 4,096 (no clusters) 1,560 -> 1,530."""
+    tensor-core decode kernel has, a rotary width the 16-byte lanes can pair up, no sliding window and no chunks -- and a
+    launch that gains by it.  ``front_bytes``: the weights of the q|k|v product in front.
+
+    Decode steps, us, apart and fused, eight blocks of each in turn (their spread 3 to 6 us).  Behind the 12.6 MB of LFM2-1.2B
+    every launch gains: 4 requests x 4,096 keys (32 clusters of 8) 688.8 652.5, 8 x 4,096 (64 of 8) 729.4 722.1, 16 x 4,096
+    (128 of 4) 939.1 931.8, 32 x 2,048 (256 of 2) 1,080.6 1,065.8, 6 x 30,000 1,208 1,143.  Behind the 4.2 MB of LFM2-350M
+    many clusters of five to eight lose: 4 x 4,096 446.7 453.9, 6 x 4,096 469.9 477.7, 8 x 4,096 484.0 489.8, 8 x 8,000 561.0 565.3 --
+    the small kernel is the window in which they find their SMs, which a product that short is not; fewer or smaller
+    clusters do not need it: 2 x 8,000 (16 of 8) 391.7 389.9, 8 x 2,048 (64 of 4) 426.5 422.8, 16 x 4,096 617.6 616.5."""
     k_pool = cache.k_pool
-    if window:
+    if span:
         return False                 # (a sliding window or chunks keep the two kernels: not measured, not tested)
-    return (_fuse_rope and _use_mma and not _force_tiled and ctx.batch.max_segment == 1
+    if not (_fuse_rope and _use_mma and not _force_tiled and ctx.batch.max_segment == 1
             and qkv.dtype == torch.bfloat16 and k_pool is not None and k_pool.dtype == torch.bfloat16
             and ctx.precision.act_dtype == torch.bfloat16 and rotary_dim % 16 == 0
-            and ops.attention_mma_shape_ok(n_heads, k_pool.shape[1], k_pool.shape[3], k_pool.shape[2]))
+            and ops.attention_mma_shape_ok(n_heads, k_pool.shape[1], k_pool.shape[3], k_pool.shape[2])):
+        return False
+    n_kv, head_dim = k_pool.shape[1], k_pool.shape[3]
+    splits, _, in_cluster = decode_splits(ctx.batch.n_tokens, n_kv, block_table.shape[1], head_dim)
+    return not (in_cluster and splits > 4 and ctx.batch.n_tokens * n_kv * splits >= FUSE_ROPE_CLUSTER_CTAS
+                and front_bytes < FUSE_ROPE_FRONT_BYTES)
 
 
 def fused_decode_attention(ctx, qkv, cache, block_table, n_heads, n_kv_in, window, scale, q_norm, k_norm, eps,

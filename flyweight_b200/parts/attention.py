@@ -339,7 +339,9 @@ class GQAttention(Mixer):
         block_table = ctx.batch.block_tables[cache.group]
         from ..kernels import attention as attention_kernels
         rotation = self.position.rotation() if self.unit_rms_eps is None else None
-        if rotation is not None and attention_kernels.decode_fusable(ctx, qkv, cache, self.n_heads, rotation[1], self.span):
+        if rotation is not None and attention_kernels.decode_fusable(
+                ctx, qkv, cache, block_table, self.n_heads, rotation[1], self.span,
+                self.w_qkv.numel() * self.w_qkv.element_size()):
             # a step of single tokens whose position part is a plain rotation: the decode attention
             # kernel norms, turns and stores its own token's heads (one kernel and one pass less)
             table, rotary_dim, pairing = rotation

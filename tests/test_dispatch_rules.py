@@ -52,6 +52,7 @@ def test_the_decode_kernel_that_rotates_knows_no_mask(monkeypatch, mask, fused):
         "hidden_size": 64, "num_heads": 8, "num_kv_heads": 2, "head_dim": 64,
         "position": PartSpec("rope_half_split", {"theta": 1e4, "rotary_dim": 64}), **mask}, names))
     mixer.position.prepare(16, "cpu")
+    mixer.w_qkv = torch.zeros(12 * 64, 64, dtype=torch.bfloat16)
     went = []
     monkeypatch.setattr(ops, "linear", lambda h, w, dtype: torch.zeros(1, 12 * 64, dtype=dtype))
     monkeypatch.setattr(ops, "linear_into_residual", lambda out, w, residual: out)
@@ -63,6 +64,20 @@ def test_the_decode_kernel_that_rotates_knows_no_mask(monkeypatch, mask, fused):
                           precision=SimpleNamespace(act_dtype=torch.bfloat16))
     mixer.forward(ctx, torch.zeros(1, 64, dtype=torch.bfloat16), cache)
     assert went == (["fused"] if fused else ["encode", mixer.span])
+
+
+@pytest.mark.parametrize("requests,tiles,front_bytes,fused", [
+    (4, 65, 4 << 20, False), (8, 65, 4 << 20, False), (8, 126, 4 << 20, False), (4, 65, 12 << 20, True),
+    (2, 126, 4 << 20, True), (8, 33, 4 << 20, True), (16, 65, 4 << 20, True), (64, 17, 4 << 20, True)])
+def test_many_clusters_of_eight_keep_the_small_kernel_behind_a_short_product(requests, tiles, front_bytes, fused):
+    """The measured points of the rule (8 KV heads of 64, pages of 64 keys)."""
+    from types import SimpleNamespace
+    import torch
+    cache = SimpleNamespace(k_pool=torch.zeros(1, 8, 64, 64, dtype=torch.bfloat16))
+    ctx = SimpleNamespace(batch=SimpleNamespace(max_segment=1, n_tokens=requests),
+                          precision=SimpleNamespace(act_dtype=torch.bfloat16))
+    qkv, table = torch.zeros(1, 1, dtype=torch.bfloat16), torch.zeros(requests, tiles, dtype=torch.int32)
+    assert attention.decode_fusable(ctx, qkv, cache, table, 16, 64, 0, front_bytes) == fused
 
 
 def test_a_convolution_step_refuses_what_the_convolution_refuses():
