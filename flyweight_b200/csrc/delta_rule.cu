@@ -372,8 +372,8 @@ delta_scan_kernel(const float* __restrict__ r, const float* __restrict__ p, floa
 // results are 32 bits wide.  Error against 64 bits over the scan's, 600 tokens on B200, keys behind silu, keys that come
 // again, keys that nearly coincide and keys of both signs, decays from none to e^-60 a token: 0.76 to 0.90 in the
 // read-out, 0.72 to 1.00 in the state (what is left is the inputs' own rounding).  64-bit multiply-adds run at half the
-// rate of 32-bit ones here and do not bind; 16 heads of 128, 2,048 tokens, all launches: 302 us in 32 bits, 388 so by
-// multiply-adds, 290 with the 64-bit tensor cores, 900 by the scan.
+// rate of 32-bit ones here and do not bind; 16 heads of 128, 2,048 tokens, all launches: 302 us in 32 bits, 378 so by
+// multiply-adds, 268 with the 64-bit tensor cores, 749 by the scan.
 //
 // A token reads nothing of a later one: T and P are summed up to the token's own column, so a value that is not finite
 // stays where the scan leaves it.

@@ -1,15 +1,16 @@
 // Y[M][N] = X[M][K] * W[N][K]^T (+ addend) in 32 bits on the tensor cores, sm_100a.
 //
-// A float is the exact sum of three bfloat16 values (8 bits of the significand each), so a product of floats is nine
-// products of bfloat16 values, each of them exact in 32 bits.  The three that lie below 2^-27 of the largest are left
-// out (together less than a quarter of one rounding of the product); the other six are summed by tcgen05.mma.  The
-// tensor cores cut off what they add instead of rounding it, so an accumulator lives for one block of 32 k only: it is
-// read back, added to a sum in registers (rounded to nearest) and begun again.
+// A float is the exact sum of three bfloat16 values (8 bits of the significand each; the second at most 2^-8, the third
+// 2^-17 of the float's power of two), so a product of floats is nine products of bfloat16 values, each of them exact in 32
+// bits.  The three smallest are left out: together less than 2^-24 of the product, a rounding of it, and 2^-28 on average.
+// The other six are summed by tcgen05.mma.  The tensor cores cut off what they add instead of rounding it, so an accumulator
+// lives for one block of 32 k only: it is read back, added to a sum in registers (rounded to nearest) and begun again.
 //
 //   * TMA brings blocks of both operands into a ring in shared memory and eight or twelve warps, four to a block, cut
 //     them in three: the weights, operand A, into tensor memory (a lane a feature), the tokens, operand B, back into
-//     shared memory (K-major, 64-byte swizzle).  Shared memory's bandwidth is what binds: with the weights' parts in it
-//     too a block of 128 x 128 took 1,650 clocks of it (768 of the tensor cores).
+//     shared memory (K-major, 64-byte swizzle).  With the weights' parts in shared memory too its bandwidth bound (a block of
+//     128 x 128 took 1,650 clocks of it, 768 of the tensor cores); as it is the cutting warps' latency does (9216 x 1024,
+//     201 tokens: issue slots 51 % busy, shared memory 31 %, tensor memory 35 %, DRAM 12 %).
 //   * One lane issues the MMAs, 128 features by up to 208 tokens; four to sixteen warps add finished accumulators up.
 //     Each role runs as far ahead as the rings and the accumulators let it.
 //   * K is cut over a cluster where a matrix has too few feature tiles; the parts are added in rank order through
@@ -544,7 +545,9 @@ int fwb::gemm_f32_split(const float* X, const float* W, float* Y, const float* a
     SplitParams prm{X, W, addend, Y, M, N, K, ldx, ldy, 1, 0, false, K * 0x1p-100f, status_word()};
     prm.vectors = !(ldy & 3) && !((uintptr_t)Y & 15) && !((uintptr_t)addend & 15);
     const int feature_tiles = (N + BM - 1) / BM, blocks = (K + KB - 1) / KB;
-    // a CTA an SM; clusters of eight find room for sixteen, of four for some 34
+    // a CTA an SM; 15 clusters of eight find room at once, 33 of four.  So 1024 x 1024, eight feature tiles, takes two rounds
+    // from 209 to some 300 tokens: 209 | 225 | 300 tokens 18.6 | 21.1 | 24.1 us by multiply-adds, 23.4 | 23.3 | 26.5 so (the
+    // slices may not follow the tokens)
     for (int s = 8; s > 1 && prm.splits == 1; s >>= 1)
         if (feature_tiles * s <= (s == 8 ? 128 : s == 4 ? 136 : 148) && blocks >= 4 * s) prm.splits = s;
     // (how the tokens are cut changes no value)

@@ -1,12 +1,11 @@
-// Y[M][N] = X[M][K] * W[N][K]^T (+ addend), plain SIMT with fp32 FMA accumulation.
+// Y[M][N] = X[M][K] * W[N][K]^T (+ addend): the entry point of the true 32-bit matrix product, and the fallback of the
+// bfloat16 path for shapes the tensor-core kernel refuses.  Any M, N, K >= 1.  The order in which an output element's
+// products are added depends on the kernel alone, and which kernel runs on the types, N, K, ldx and the operands' alignment
+// alone: the value at [m][n] does not depend on M or on which other rows share the launch.
 //
-// This is the true 32-bit matrix product of the engine, and the fallback of the bfloat16
-// path for shapes the tensor-core kernel refuses.  Any M, N, K >= 1.  The order in which an output element's products are added depends
-// on the kernel alone, and which kernel runs on the types, K, ldx and the operands' alignment alone:
-// the value at [m][n] does not depend on M or on which other rows share the launch.
-//
-//   gemm_f32_tcgen05.cu   fp32 throughout, 16-byte copies, N and K from 128 on: exact thirds of
-//                     the values on the tensor cores, closer to the exact sum than the others.
+//   gemm_f32_tcgen05.cu   fp32 throughout, 16-byte copies, N and K from 128 and N K from 2^20 on:
+//                     exact thirds of the values on the tensor cores, closer to the exact sum than the
+//                     others, which are plain multiply-adds.
 //   gemm_f32_kernel   fp32 throughout, rows that 16-byte copies can read (K, ldx multiples of 4):
 //                     eight partial sums an element (four quarters of every 64 k, even and odd k
 //                     apart), added in a fixed order.
@@ -85,7 +84,8 @@ gemm_simt_kernel(const TX* __restrict__ X, const TW* __restrict__ W, TY* __restr
 // 64 x 32 keeps eight warps busy, and a 201 x 1024 product fills 128 SMs.
 // Measured on B200 in a chain of launches over 300 MB of weights (us; gemm_simt_kernel, then this one):
 // 201 x 9216 x 1024 288 -> 121, 201 x 1024 x 4608 378 -> 76, 64 x 9216 x 1024 100 -> 39 (31 TFLOP/s),
-// 8 x 1024 x 4608 403 -> 35, 1 x 9216 x 1024 94 -> 21 (matrices of that size have gone to the tensor cores since); relative error against 64 bits 5.7e-7 -> 2.1e-7 at K = 1024.
+// 8 x 1024 x 4608 403 -> 35, 1 x 9216 x 1024 94 -> 21 (matrices of that
+// size have gone to the tensor cores since); relative error against 64 bits 5.7e-7 -> 2.1e-7 at K = 1024.
 constexpr int FK = 64, FSTRIDE = FK + 4, FSTAGES = 3;
 
 __device__ __forceinline__ void fma_four(float2& acc, const float4& a, const float4& b) {

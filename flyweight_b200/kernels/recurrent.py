@@ -19,11 +19,12 @@ def delta_state_size(heads: int, kv_heads: int, dim: int, vdim: int, taps: int) 
 # A segment of this many tokens and more runs in chunks of 32 tokens (head sizes 64 and 128); shorter ones, decoding
 # requests above all, walk token by token, whatever else the step holds.  Measured on B200 (16 heads of 128, all
 # launches, us a layer with that segment in chunks, and with every segment by the scan):
-#   one segment of 64 tokens 54 and 68, of 128 63 and 93, of 512 118 and 368, of 2,048 388 and 900;
-#   behind 8 decoding requests 64 tokens 84 and 69, 96 88 and 85, 128 96 and 112; behind 64, 96 tokens 117 and 112,
-#   128 121 and 122, 512 174 and 302;  4 segments of 128 101 and 138, 8 of 128 175 and 171, 8 of 256 321 and 323.
-# Steps that fill the SMs several times over are dearer in chunks (16 of 128 320 and 286, 16 of 512 1,144 and 1,043): the
-# line cannot follow the number of segments without a request's bits following its company.
+#   one segment of 64 tokens 33 and 51, of 128 40 and 73, of 512 86 and 205, of 2,048 268 and 749;
+#   behind 8 decoding requests 64 tokens 58 and 56, 96 62 and 70, 128 68 and 84; behind 64, 96 tokens 90 and 95,
+#   128 93 and 107, 512 144 and 288;  4 segments of 128 74 and 110, 8 of 128 116 and 157, 8 of 256 217 and 295,
+#   16 of 128 219 and 260, 16 of 512 765 and 986.
+# (Below, chunks win alone and lose a little behind decoding requests; the line was drawn when they won from 128 on only, and
+# moving it moves bits.)
 CHUNKS_FROM = 128
 _CHUNK_TOKENS, _CHUNK_DOUBLES = 32, 2 * 32 * 34
 

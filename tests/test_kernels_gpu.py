@@ -129,7 +129,7 @@ def test_gemm_fp32_tiles(M, N, K):
 @pytest.mark.parametrize("N,K", [(8192, 128), (8193, 132), (1025, 1028), (259, 8200), (19000, 160)])
 def test_gemm_fp32_thirds(M, N, K):
     """The tensor-core form: edges of its tiles of tokens, features and k, one slice of K and several.  Six of nine
-    partial products (the rest below 2^-26 of a product), sums of 32 cut off at 2^-23, then rounded sums: within
+    partial products (the rest below 2^-24 of a product), sums of 32 cut off at 2^-23, then rounded sums: within
     2^-22 of the products' magnitudes; rows do not depend on the batch."""
     from flyweight_b200.kernels import ops
     g = torch.Generator().manual_seed(M * N + K)
