@@ -746,10 +746,11 @@ delta_runs_kernel(const float* __restrict__ r, const float* __restrict__ p, cons
 
 template <int DPL, int LPC, bool VEC>
 int launch_scan(const float* r, const float* p, float* state, long long slot_stride, const int* seg_start,
-                const int* seg_slot, float* o, int below, int segments, const DeltaShape& sh, cudaStream_t stream) {
+                const int* seg_slot, float* o, int below, int T, int segments, const DeltaShape& sh, cudaStream_t stream) {
     // blocks that fit the SMs one by one must not meet on some of them, where they would land beside the last blocks of the
     // kernel in front: they ask for more than half of an SM's shared memory (16 heads of 128, 128 blocks, all launches, us
-    // before and so: 256 tokens 149 117, 512 237 205, 1,024 449 385, 2,048 1,180 749, 4,096 2,580 1,476)
+    // before and so: 256 tokens 149 117, 512 237 205, 1,024 449 385, 2,048 1,180 749, 4,096 2,580 1,476).  A walk of a few
+    // tokens does not pay for waiting until an SM has that much free (a decode step of Diforax, ten such layers: 960 us, 972)
     constexpr int ALONE = 116 * 1024, COLS = 128 / LPC;
     auto kernel = delta_scan_kernel<DPL, LPC, VEC>;
     static bool configured = false;
@@ -759,7 +760,7 @@ int launch_scan(const float* r, const float* p, float* state, long long slot_str
         configured = true;
     }
     const dim3 grid((sh.e + COLS - 1) / COLS, sh.H, segments);
-    const bool alone = (long)grid.x * grid.y * grid.z <= 148;
+    const bool alone = T >= 64 && (long)grid.x * grid.y * grid.z <= 148;
     fwb::pdl(kernel, grid, 128, alone ? ALONE : 0, stream)(r, p, state, slot_stride, seg_start, seg_slot, o, below, sh);
     return fwb_launch_status();
 }
@@ -852,8 +853,8 @@ FWB_API int fwb_delta_rule(const float* p, const float* taps, const float* a_log
     const int below = runs ? from : 2147483647, scans = runs ? scanned : n_segments;
 #define FWB_SCAN(DPL, LPC)                                                                                             \
     do {                                                                                                               \
-        const int status = vec ? launch_scan<DPL, LPC, true>(r, p, state, slot_stride, seg_start, seg_slot, o, below, scans, sh, stream) \
-                               : launch_scan<DPL, LPC, false>(r, p, state, slot_stride, seg_start, seg_slot, o, below, scans, sh, stream); \
+        const int status = vec ? launch_scan<DPL, LPC, true>(r, p, state, slot_stride, seg_start, seg_slot, o, below, T, scans, sh, stream) \
+                               : launch_scan<DPL, LPC, false>(r, p, state, slot_stride, seg_start, seg_slot, o, below, T, scans, sh, stream); \
         if (status != FWB_OK) return status;                                                                           \
     } while (0)
     if (scans > 0) {
