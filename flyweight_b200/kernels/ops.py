@@ -169,6 +169,15 @@ def linear(x, w: torch.Tensor, out_dtype: torch.dtype,
     return gemm_simt(x, w, out_dtype, addend)
 
 
+def one_launch_changes_no_bit(x: torch.Tensor, w: torch.Tensor, parts, out_dtype: torch.dtype) -> bool:
+    """Whether ``linear(x, w, out_dtype)`` has the bits of the products with ``parts``, ``w``'s rows in pieces: where the
+    reader of a few tokens' weights runs them all, which sums a feature the same way whatever the others are."""
+    from . import tensorcore
+    M, K = x.shape
+    return (M <= 16 and out_dtype == torch.bfloat16 and x.dtype == torch.bfloat16
+            and all(tensorcore.accepts(x, m, out_dtype) and tensorcore._rows_takes(M, m.shape[0], K) for m in (w, *parts)))
+
+
 def linear_act(x: torch.Tensor, w: torch.Tensor, activation: str, out_dtype: torch.dtype,
                rounded: bool = False) -> torch.Tensor:
     """``act(x @ w.T)``, the activation (one of ``FUSED_ACTIVATIONS``) on the product's fp32 sums, or, ``rounded``, on

@@ -140,9 +140,9 @@ class GQAttention(Mixer):
         # a gate per head behind a convolution: its rows ride in the q|k|v product (the convolution writes a
         # buffer of its own, so the gate's columns stay where the product left them).  Every other gate has a
         # product of its own: its matrix keeps the type it is stored in and its rows leave in the activations',
-        # whatever q, k and v do
+        # whatever q, k and v do; a few tokens read both matrices in one launch where that changes no bit
         self._gate_in_projection = self.gate == "head" and self.conv_taps > 0
-        self.w_qkv = self.w_o = self.q_norm = self.k_norm = self.w_gate = self.sink = self.vmix = None
+        self.w_qkv = self.w_o = self.q_norm = self.k_norm = self.w_gate = self.w_both = self.sink = self.vmix = None
         self.taps = self.qkv_bias = self.temp = None
 
     @property
@@ -205,6 +205,10 @@ class GQAttention(Mixer):
 
     def bind(self, get, precision: Precision, device):
         self.w_qkv = precision.matrix(self._bind_inner(get, precision, device), device)
+        if (self.w_gate is not None and not self._wide_qkv and self.w_gate.dtype == self.w_qkv.dtype == torch.bfloat16
+                and self.w_gate.shape[0] % 8 == 0):
+            self.w_both = torch.cat([self.w_qkv, self.w_gate])
+            self.w_qkv, self.w_gate = self.w_both[:self._qkv_columns], self.w_both[self._qkv_columns:]
         w_o = self._output_columns(get) if self._placed else get(self.names["o"])
         D = self.head_dim
         if not self._placed and self.value_dim != D:      # zero columns where the padded channels of a head arrive
@@ -386,7 +390,8 @@ class GQAttention(Mixer):
         if not isinstance(h, torch.Tensor):
             h = h.materialize(act)
         D = self.head_dim
-        qkv = ops.linear(h, self.w_qkv, torch.float32 if self._wide_qkv else act)
+        both = self.w_both is not None and ops.one_launch_changes_no_bit(h, self.w_both, (self.w_qkv, self.w_gate), act)
+        qkv = ops.linear(h, self.w_both if both else self.w_qkv, torch.float32 if self._wide_qkv else act)
         block_table = ctx.batch.block_tables[cache.group]
         k_at, v_at = self.n_heads * D, (self.n_heads + self._kv_in) * D
         whole = self.qk_norm == "whole"
@@ -416,6 +421,8 @@ class GQAttention(Mixer):
                                  f"{self.n_kv} value heads of {D}: the source layer runs first and has the same shape")
             mixing.value_mix_(qkv, v_at, self.n_kv * D, first, self.vmix)
         extra = self._encode_extra()
+        if both:                                             # (the gate's columns behind them)
+            qkv = qkv[:, :self._qkv_columns]
         q = self.position.encode(ctx, qkv, n_heads=self.n_heads, n_kv_in=self._kv_in, head_dim=D,
                                  q_norm=None if whole else self.q_norm, k_norm=None if whole else self.k_norm,
                                  eps=None if whole else (self.eps if self.unit_rms_eps is None else self.unit_rms_eps),
@@ -423,8 +430,9 @@ class GQAttention(Mixer):
         out = attention_kernels.paged_attention(ctx, q, cache, block_table, self.n_heads, self.span, self.scale,
                                                 act, sink=self.sink, softcap=self.softcap,
                                                 keep_first=self.keep_first)
-        if self._gate_in_projection:
-            mixing.sigmoid_gate_cols_mul_(out, projected, self._qkv_columns, self.n_heads, D)
+        if self._gate_in_projection or both:
+            mixing.sigmoid_gate_cols_mul_(out, projected, self._qkv_columns, self.n_heads, D,
+                                          per_channel=self.gate == "element")
         elif self.gate:
             # (a gate stored in 32 bits stays so: the 32-bit product has no 16-bit output)
             gate = ops.linear(h, self.w_gate, torch.promote_types(act, self.w_gate.dtype))

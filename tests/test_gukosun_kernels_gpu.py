@@ -353,6 +353,32 @@ def test_decayed_linear_attention_part_and_the_pair(dtype, lin):
         close(got_pair[s], P.parallel_mixer(h, w, "l2.mix.", m, EPS, pos, rnd=rnd), TOL[dtype], f"pair, sequence {s}")
 
 
+@pytest.mark.parametrize("tokens", [1, 2, 8, 9, 16, 17])
+@pytest.mark.parametrize("width,kv,mix", [(512, 4, None), (512, 4, "source"), (1032, 1, None), (1024, 8, None)])
+def test_a_gate_beside_the_projection_changes_no_bit(tokens, width, kv, mix):
+    """A few tokens' q, k, v and gate come from one launch over both matrices; the same mixer with the matrices apart."""
+    import dataclasses
+    from flyweight_b200.kernels import ops
+    raw = tiny_config(width=width, heads=8, kv=kv, dim=32, vdim=32)
+    spec, w = random_weights(raw, 29, torch.bfloat16)
+    part = spec.layers[0].parts["mixer"]
+    part = dataclasses.replace(part, params={**part.params, "value_mix": mix})
+    h = bf16_round(torch.randn(tokens, width, generator=torch.Generator().manual_seed(tokens), dtype=F64))
+    before, asked = ops.one_launch_changes_no_bit, []
+
+    def answer(*args):
+        asked.append(before(*args))
+        return asked[-1] and len(asked) == 1
+
+    ops.one_launch_changes_no_bit = answer
+    try:
+        one, apart = (run_part(part, w, torch.bfloat16, [h], [[(0, tokens)]])[0] for _ in range(2))
+    finally:
+        ops.one_launch_changes_no_bit = before
+    assert torch.equal(one, apart)
+    assert asked == [tokens <= 16] * 2
+
+
 @pytest.mark.parametrize("stored", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("tokens", [1, 8, 40])
 @pytest.mark.parametrize("kind", ["element", "head"])
